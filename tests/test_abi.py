@@ -34,6 +34,15 @@ def test_version_and_status_strings_without_a_gpu():
     assert lib.xlstm_mlstm_chunkwise_workspace_bytes(1, 1, 64, 64, 64, 64, 0) == 0
 
 
+def test_workspace_query_below_one_tile():
+    """A bf16 sequence shorter than the 128-token tile needs no scratch; the query used to divide by zero."""
+    from xlstm_cuda import _lib
+    lib = _lib.load()
+    for S in (1, 15, 63, 64, 127):
+        assert lib.xlstm_mlstm_chunkwise_workspace_bytes(1, 8, S, 256, 512, 64, 1) == 0
+    assert lib.xlstm_mlstm_chunkwise_workspace_bytes(1, 8, 128, 256, 512, 64, 1) > 0
+
+
 def test_no_product_module_imports_the_oracle():
     pkg = ROOT / "xlstm-metal_b200"
     for path in pkg.rglob("*.py"):
