@@ -468,6 +468,48 @@ def test_slstm_scan_oracle(ops, B, S, NH, H, dtype):
         assert relerr(host(got), want) < FP32_TOL
 
 
+@pytest.mark.parametrize("B,S,NH,H,dtype,with_state", [
+    (1, 95, 1, 64, torch.float32, False),     # two gate tiles: one pass
+    (1, 97, 2, 128, torch.float32, True),     # three segments, the last one a single step
+    (1, 1000, 2, 1024, torch.float32, True),  # many segments, several unit slices, ragged end
+    (2, 333, 1, 37, torch.float32, False),    # width without 16-byte vectors
+    (1, 1024, 4, 40, torch.bfloat16, True),   # a slice with idle lanes
+])
+def test_slstm_scan_segments(ops, B, S, NH, H, dtype, with_state):
+    """Segments of the sequence in parallel against the oracle, raw gates capped inside, and an in-place state (which
+    takes the single pass) through the C ABI."""
+    rng = np.random.default_rng(S)
+    rnd = (lambda a: xo.bf16_round(a)) if dtype == torch.bfloat16 else (lambda a: a)
+    z = rnd(rng.standard_normal((B, S, NH, H)).astype(np.float32))
+    i, f, o = (rnd((rng.standard_normal((B, S, NH)) * 3 + s).astype(np.float32)) for s in (0, 2, 0))
+    st0 = None
+    if with_state:
+        st0 = (rng.standard_normal((B, NH, H)).astype(np.float32), rng.uniform(0.5, 2, (B, NH, H)).astype(np.float32),
+               rng.standard_normal((B, NH)).astype(np.float32))
+    cap = 5.0
+    h_ref, st_ref = xo.slstm_scan(z, *(xo.softcap(g, cap) for g in (i, f, o)), st0)
+    st = None if st0 is None else tuple(dev(s) for s in st0)
+    args = [dev(a, dtype) for a in (z, i, f, o)]
+    h, st1 = ops.slstm_scan(*args, state=st, gate_cap=cap)
+    tol = FP32_TOL if dtype == torch.float32 else BF16_TOL
+    assert relerr(host(h), h_ref) < tol
+    for a, r in zip(st1, st_ref):
+        assert relerr(host(a), r) < tol
+    if st is not None:
+        from xlstm_cuda import _lib
+        c, n, m1 = st[0].clone(), st[1].clone(), torch.empty_like(st[2])
+        h2 = torch.empty_like(h)
+        code = _lib.F32 if dtype == torch.float32 else _lib.BF16
+        need = _lib.load().xlstm_slstm_scan_workspace_bytes(B, S, NH, H, code)
+        assert need > 0
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+        rc = _lib.load().xlstm_slstm_scan_ex(*(a.data_ptr() for a in args), c.data_ptr(), n.data_ptr(), st[2].data_ptr(),
+                                             h2.data_ptr(), c.data_ptr(), n.data_ptr(), m1.data_ptr(), B, S, NH, H, 1e-6, cap,
+                                             code, ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        assert relerr(host(h2), h_ref) < tol and relerr(host(c), st_ref[0]) < tol and relerr(host(n), st_ref[1]) < tol
+
+
 def test_slstm_recurrent_fixture(ops, golden):
     g = golden("slstm_b")
     nh = int(g["num_heads"])

@@ -6,52 +6,9 @@
 // kernels - one CTA of 16 warps per SM, inputs arriving through per-lane rings of 16-byte cp.async slots in
 // shared memory a fixed distance ahead, so the bytes in flight do not depend on the register allocation.
 #include "common.cuh"
+#include "vec16.cuh"
 
 namespace xl {
-
-template <typename T> struct Vec16 { static constexpr int N = 16 / sizeof(T); };
-
-template <typename T> __device__ __forceinline__ void ld16(const T *p, float *f);
-template <> __device__ __forceinline__ void ld16<float>(const float *p, float *f) {
-    const float4 a = *reinterpret_cast<const float4 *>(p);
-    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-}
-template <> __device__ __forceinline__ void ld16<__nv_bfloat16>(const __nv_bfloat16 *p, float *f) {
-    const uint4 u = *reinterpret_cast<const uint4 *>(p);
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-}
-template <typename T> __device__ __forceinline__ void st16(T *p, const float *f);
-template <> __device__ __forceinline__ void st16<float>(float *p, const float *f) {
-    *reinterpret_cast<float4 *>(p) = make_float4(f[0], f[1], f[2], f[3]);
-}
-template <> __device__ __forceinline__ void st16<__nv_bfloat16>(__nv_bfloat16 *p, const float *f) {
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-        w[i] = *reinterpret_cast<uint32_t *>(&v);
-    }
-    *reinterpret_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// 16 raw bytes already in registers -> VN floats
-template <typename T> __device__ __forceinline__ void unpack16(const uint4 &u, float *f);
-template <> __device__ __forceinline__ void unpack16<float>(const uint4 &u, float *f) {
-    f[0] = __uint_as_float(u.x); f[1] = __uint_as_float(u.y); f[2] = __uint_as_float(u.z); f[3] = __uint_as_float(u.w);
-}
-template <> __device__ __forceinline__ void unpack16<__nv_bfloat16>(const uint4 &u, float *f) {
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-}
 
 // sigmoid / SiLU: exact division and expf for fp32 outputs; for bf16 outputs (8 elements per 16 bytes,
 // where these kernels would otherwise be bound by instruction issue, not by HBM) the approximate

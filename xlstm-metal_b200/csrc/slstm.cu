@@ -1,16 +1,6 @@
-// sLSTM kernels.
-//
-// (1) slstm_scan: the packaged cell (scalar gates per head, no recurrent
-//     weights) has no dependence on h_{t-1}, so the whole sequence is one
-//     first-order scan per (batch, head): a single launch walks S timesteps,
-//     the per-step gate scalars are computed once per head (not once per
-//     unit) and the unit state lives in registers.  HBM-bound on z and h.
-//
-// (2) slstm_recurrent: the block-diagonal variant is truly sequential through
-//     h_{t-1}.  A thread-block cluster owns one (head, batch group); every CTA
-//     keeps its slice of the four recurrent matrices resident in shared memory
-//     for all timesteps and the CTAs exchange their slice of h_t through
-//     distributed shared memory once per step.  Latency-bound.
+// sLSTM with block-diagonal recurrent weights: truly sequential through h_{t-1}.  A thread-block cluster owns one (head,
+// batch group); every CTA keeps its slice of the four recurrent matrices resident in shared memory for all timesteps
+// and the CTAs exchange their slice of h_t through distributed shared memory once per step.  Latency-bound.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -20,92 +10,7 @@ namespace cg = cooperative_groups;
 namespace xl {
 
 // ---------------------------------------------------------------------------
-// (1) scan over S timesteps, packaged cell
-// ---------------------------------------------------------------------------
-constexpr int SCAN_TT = 32;  // timesteps per gate tile (one warp lane each)
-constexpr int SCAN_HPT = 4;  // units per thread at most
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-slstm_scan_kernel(const T *__restrict__ z, const T *__restrict__ ig, const T *__restrict__ fg,
-                  const T *__restrict__ og, const float *c0, const float *n0, const float *__restrict__ m0,
-                  T *__restrict__ h, float *c1, float *n1, float *__restrict__ m1, int S, int NH, int H, float eps) {
-    __shared__ float s_f[SCAN_TT], s_i[SCAN_TT], s_o[SCAN_TT];
-    __shared__ float s_m;
-    const int bh = blockIdx.x, b = bh / NH, hd = bh % NH;
-    const int tid = threadIdx.x;
-    float c[SCAN_HPT], n[SCAN_HPT];
-#pragma unroll
-    for (int u = 0; u < SCAN_HPT; ++u) {
-        const int j = tid + u * blockDim.x;
-        c[u] = (c0 && j < H) ? c0[(size_t)bh * H + j] : 0.f;
-        n[u] = (c0 && j < H) ? n0[(size_t)bh * H + j] : 0.f;
-    }
-    if (tid == 0) s_m = c0 ? m0[bh] : 0.f;
-    __syncthreads();
-
-    for (int t0 = 0; t0 < S; t0 += SCAN_TT) {
-        const int nt = min(SCAN_TT, S - t0);
-        if (tid < 32) {
-            // lane = timestep: transcendental work in parallel, then the exact
-            // sequential stabiliser recurrence m_t = max(m_{t-1} + logsig f_t, i_t)
-            const size_t g = ((size_t)b * S + t0 + tid) * NH + hd;
-            const bool valid = tid < nt;
-            const float lf = valid ? logsigmoid(Elem<T>::ld(fg + g)) : 0.f;
-            const float it = valid ? Elem<T>::ld(ig + g) : 0.f;
-            const float ot = valid ? sigmoidf(Elem<T>::ld(og + g)) : 0.f;
-            float m = s_m, m_prev_mine = 0.f, m_mine = 0.f;
-            for (int s = 0; s < nt; ++s) {
-                const float lfs = __shfl_sync(0xffffffffu, lf, s);
-                const float is = __shfl_sync(0xffffffffu, it, s);
-                const float mn = fmaxf(m + lfs, is);
-                if (s == tid) { m_prev_mine = m; m_mine = mn; }
-                m = mn;
-            }
-            if (valid) {
-                s_f[tid] = expf(m_prev_mine + lf - m_mine);
-                s_i[tid] = expf(it - m_mine);
-                s_o[tid] = ot;
-            }
-            if (tid == 0) s_m = m;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < SCAN_HPT; ++u) {
-            const int j = tid + u * blockDim.x;
-            if (j < H) {
-                const T *zp = z + (((size_t)b * S + t0) * NH + hd) * H + j;
-                T *hp = h + (((size_t)b * S + t0) * NH + hd) * H + j;
-                const size_t tstride = (size_t)NH * H;
-                float cc = c[u], nn = n[u];
-                for (int s0 = 0; s0 < nt; s0 += 8) {
-                    float zz[8];
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) zz[s] = (s0 + s < nt) ? Elem<T>::ld(zp + (s0 + s) * tstride) : 0.f;
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) {
-                        if (s0 + s < nt) {
-                            cc = fmaf(s_f[s0 + s], cc, s_i[s0 + s] * tanhf(zz[s]));
-                            nn = fmaf(s_f[s0 + s], nn, s_i[s0 + s]);
-                            Elem<T>::st(hp + (s0 + s) * tstride, s_o[s0 + s] * cc / (fabsf(nn) + eps));
-                        }
-                    }
-                }
-                c[u] = cc; n[u] = nn;
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < SCAN_HPT; ++u) {
-        const int j = tid + u * blockDim.x;
-        if (j < H) { c1[(size_t)bh * H + j] = c[u]; n1[(size_t)bh * H + j] = n[u]; }
-    }
-    if (tid == 0) m1[bh] = s_m;
-}
-
-// ---------------------------------------------------------------------------
-// (2) block-diagonal recurrent sLSTM, recurrent weights resident in shared memory
+// block-diagonal recurrent sLSTM, recurrent weights resident in shared memory
 // ---------------------------------------------------------------------------
 constexpr int REC_THREADS = 256;
 #ifndef XL_REC_BG
@@ -290,28 +195,6 @@ int slstm_recurrent_tc(const void *gx, const void *R, const float *rb, const flo
                        const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH,
                        float cap, cudaStream_t st);
 }  // namespace xl
-
-extern "C" int xlstm_slstm_scan(const void *z, const void *ig, const void *fg, const void *og, const float *c0,
-                                const float *n0, const float *m0, void *h, float *c1, float *n1, float *m1, int B,
-                                int S, int NH, int H, float eps, int dtype, void *stream) {
-    if (!z || !ig || !fg || !og || !h || !c1 || !n1 || !m1) return XLSTM_ERR_INVALID;
-    if (B <= 0 || S <= 0 || NH <= 0 || H <= 0) return XLSTM_ERR_INVALID;
-    if (c0 && (!n0 || !m0)) return XLSTM_ERR_INVALID;
-    if (dtype != XLSTM_F32 && dtype != XLSTM_BF16) return XLSTM_ERR_UNSUPPORTED;
-    int threads = H >= 256 ? 256 : ((H + 31) / 32) * 32;
-    if (H > threads * xl::SCAN_HPT) return XLSTM_ERR_UNSUPPORTED;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == XLSTM_F32)
-        xl::slstm_scan_kernel<float><<<B * NH, threads, 0, st>>>(
-            static_cast<const float *>(z), static_cast<const float *>(ig), static_cast<const float *>(fg),
-            static_cast<const float *>(og), c0, n0, m0, static_cast<float *>(h), c1, n1, m1, S, NH, H, eps);
-    else
-        xl::slstm_scan_kernel<__nv_bfloat16><<<B * NH, threads, 0, st>>>(
-            static_cast<const __nv_bfloat16 *>(z), static_cast<const __nv_bfloat16 *>(ig),
-            static_cast<const __nv_bfloat16 *>(fg), static_cast<const __nv_bfloat16 *>(og), c0, n0, m0,
-            static_cast<__nv_bfloat16 *>(h), c1, n1, m1, S, NH, H, eps);
-    return xl::launch_status();
-}
 
 extern "C" int xlstm_slstm_recurrent(const void *gx, const void *R, const float *rb, const float *c0, const float *n0,
                                      const float *h0, const float *m0, void *hs, float *c1, float *n1, float *h1,

@@ -35,6 +35,9 @@ _SIGNATURES = {
     "xlstm_mlstm_chunkwise_fwd_static": (c_int, [c_void_p] * 5 + [c_void_p] * 3 + [c_void_p] * 4 + [c_int] * 6
                                          + [c_float, c_int, ctypes.POINTER(c_int64), c_void_p]),
     "xlstm_slstm_scan": (c_int, [c_void_p] * 4 + [c_void_p] * 3 + [c_void_p] * 4 + [c_int] * 4 + [c_float, c_int, c_void_p]),
+    "xlstm_slstm_scan_workspace_bytes": (c_size_t, [c_int] * 5),
+    "xlstm_slstm_scan_ex": (c_int, [c_void_p] * 4 + [c_void_p] * 3 + [c_void_p] * 4 + [c_int] * 4
+                            + [c_float, c_float, c_int, c_void_p, c_size_t, c_void_p]),
     "xlstm_slstm_recurrent": (c_int, [c_void_p] * 3 + [c_void_p] * 4 + [c_void_p] * 5 + [c_int] * 4 + [c_float, c_int, c_void_p]),
     "xlstm_mlstm_step_gatecap": (c_int, [c_void_p] * 5 + [c_void_p] * 3 + [c_void_p] * 4 + [c_int] * 4
                                  + [c_float, c_float, c_int, c_void_p]),

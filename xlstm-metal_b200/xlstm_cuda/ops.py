@@ -253,8 +253,9 @@ def mlstm_chunkwise_scatter(q, k, v, i, f, state, h_rank_ptrs, tokens_per_rank: 
     return C1, n1, m1
 
 
-def slstm_scan(z, i, f, o, state=None, eps: float = 1e-6):
-    """Packaged sLSTM cell over S steps.  z: [B,S,NH,H]; i,f,o: [B,S,NH]; state (c,n,m) or None."""
+def slstm_scan(z, i, f, o, state=None, eps: float = 1e-6, gate_cap: Optional[float] = None):
+    """Packaged sLSTM cell over S steps.  z: [B,S,NH,H]; i,f,o: [B,S,NH]; state (c,n,m) or None.
+    ``gate_cap`` > 0: the gates are raw projections, soft-capped inside the kernel."""
     _need_cuda(z, i, f, o)
     B, S, NH, H = z.shape
     dt = _dtype_code(z)
@@ -269,10 +270,12 @@ def slstm_scan(z, i, f, o, state=None, eps: float = 1e-6):
     c1 = torch.empty(B, NH, H, dtype=torch.float32, device=dev)
     n1 = torch.empty(B, NH, H, dtype=torch.float32, device=dev)
     m1 = torch.empty(B, NH, dtype=torch.float32, device=dev)
-    _lib.check(_lib.load().xlstm_slstm_scan(
+    need = int(_lib.load().xlstm_slstm_scan_workspace_bytes(B, S, NH, H, dt))
+    ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+    _lib.check(_lib.load().xlstm_slstm_scan_ex(
         z.data_ptr(), i.data_ptr(), f.data_ptr(), o.data_ptr(), _ptr(c0), _ptr(n0), _ptr(m0),
-        h.data_ptr(), c1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, S, NH, H, float(eps), dt, _stream()),
-        "xlstm_slstm_scan")
+        h.data_ptr(), c1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, S, NH, H, float(eps),
+        float(gate_cap) if gate_cap is not None else 0.0, dt, _ptr(ws), need, _stream()), "xlstm_slstm_scan_ex")
     return h, (c1, n1, m1)
 
 
