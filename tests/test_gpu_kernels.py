@@ -441,6 +441,34 @@ def test_chunkwise_full_length_properties(ops):
     assert torch.equal(h, h_again)
 
 
+@pytest.mark.parametrize("B,NH,S,dqk,dv,dtype,with_state", [
+    (1, 2, 65, 20, 36, torch.float32, True),       # partial pieces of dqk and dv, one token in the second chunk
+    (1, 4, 64, 64, 64, torch.float32, False),      # one chunk: no scratch
+    (2, 3, 31, 128, 256, torch.float32, True),     # less than one state tile
+    (1, 2, 200, 256, 192, torch.float32, False),   # 64-column CTAs, ragged last chunk
+    (2, 8, 1606, 256, 512, torch.float32, True),   # 128-column CTAs, a second group of chunks continuing in place
+    (1, 2, 130, 64, 128, torch.bfloat16, True),    # bf16 head shape outside the tensor-core kernels
+])
+def test_chunkwise_fp32_two_kernels(ops, B, NH, S, dqk, dv, dtype, with_state):
+    """The fp32 forward at the edges of its tiles, chunks and groups, against the step-by-step oracle."""
+    rng = np.random.default_rng(S + dqk)
+    rnd = xo.bf16_round if dtype == torch.bfloat16 else (lambda a: a)
+    q, k = (rnd(rng.standard_normal((B, NH, S, dqk)).astype(np.float32)) for _ in range(2))
+    v = rnd(rng.standard_normal((B, NH, S, dv)).astype(np.float32))
+    i, f = (rnd(a) for a in gates(rng, (B, NH, S)))
+    st0 = None
+    if with_state:
+        st0 = ((rng.standard_normal((B, NH, dqk, dv)) * 0.1).astype(np.float32),
+               (rng.standard_normal((B, NH, dqk)) * 0.1).astype(np.float32), rng.standard_normal((B, NH)).astype(np.float32))
+    h_ref, st_ref = xo.mlstm_recurrent(q, k, v, i, f, st0)
+    st = None if st0 is None else tuple(dev(a) for a in st0)
+    h, st1 = ops.mlstm_chunkwise(*(dev(a, dtype) for a in (q, k, v, i, f)), state=st)
+    tol = FP32_TOL if dtype == torch.float32 else BF16_TOL
+    assert relerr(host(h), h_ref) < tol
+    for a, r in zip(st1, st_ref):
+        assert relerr(host(a), r) < FP32_TOL
+
+
 # ---- sLSTM ------------------------------------------------------------------------
 @pytest.mark.parametrize("tag", ["a", "b", "x", "z"])
 def test_slstm_scan_fixture(ops, golden, tag):

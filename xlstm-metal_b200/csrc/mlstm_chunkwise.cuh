@@ -22,7 +22,12 @@ struct ChunkwiseParams {
     int tok_per_rank;
 };
 
-// exact-fp32 CUDA-core path: any dqk <= 512, dv, S, L <= 64
+// fp32 arithmetic, any dqk, dv, S: two launches per group of chunks, chunk states in scratch
+size_t mlstm_chunkwise_f32_workspace(int B, int NH, int S, int dqk, int dv);
+bool mlstm_chunkwise_f32_supported(const ChunkwiseParams &p, int dtype);
+int mlstm_chunkwise_f32(const ChunkwiseParams &p, int dtype, void *workspace, cudaStream_t st);
+
+// the same in one launch without scratch: dqk <= 512, L <= 64
 int mlstm_chunkwise_simt(const ChunkwiseParams &p, int dtype, cudaStream_t st);
 
 // tcgen05 / TMEM / TMA path: bf16, L == 64, dqk == 256 (or 128/64), dv % 128 == 0, whole chunks

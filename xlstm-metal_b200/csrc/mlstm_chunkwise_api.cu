@@ -43,8 +43,9 @@ extern "C" int xlstm_mlstm_chunkwise_status(const void *workspace, void *stream)
 }
 
 extern "C" size_t xlstm_mlstm_chunkwise_workspace_bytes(int B, int NH, int S, int dqk, int dv, int L, int dtype) {
-    if (dtype != XLSTM_BF16) return 0;
-    return xl::mlstm_chunkwise_tc_workspace(B, NH, S, dqk, dv, L);
+    if (B <= 0 || NH <= 0 || S <= 0 || dqk <= 0 || dv <= 0) return 0;
+    const size_t tc = dtype == XLSTM_BF16 ? xl::mlstm_chunkwise_tc_workspace(B, NH, S, dqk, dv, L) : 0;
+    return tc ? tc : xl::mlstm_chunkwise_f32_workspace(B, NH, S, dqk, dv);
 }
 
 static int chunkwise_dispatch(const void *q, const void *k, const void *v, const void *ig, const void *fg,
@@ -87,7 +88,11 @@ static int chunkwise_dispatch(const void *q, const void *k, const void *v, const
     }
     if (!xl::mlstm_chunkwise_tc_supported(p, dtype)) {
         if (n_peers) return XLSTM_ERR_UNSUPPORTED;   // peer stores exist in the tensor-core kernel only
-        return xl::mlstm_chunkwise_simt(p, dtype, st);
+        const size_t f32_need = xl::mlstm_chunkwise_f32_workspace(B, NH, S, dqk, dv);
+        if (xl::mlstm_chunkwise_f32_supported(p, dtype) &&
+            (f32_need == 0 || (workspace && workspace_bytes >= f32_need && !(reinterpret_cast<uintptr_t>(workspace) & 255u))))
+            return xl::mlstm_chunkwise_f32(p, dtype, workspace, st);
+        return xl::mlstm_chunkwise_simt(p, dtype, st);   // no scratch, or strides the other one does not take
     }
 
     // Whole 128-token tiles on the tensor cores, then the remaining tokens (with the carried

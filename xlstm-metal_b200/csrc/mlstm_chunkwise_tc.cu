@@ -773,7 +773,7 @@ std::atomic<int> g_segments{-1};       // -1: planned from the grid size; >= 1: 
 size_t mlstm_chunkwise_tc_workspace(int B, int NH, int S, int dqk, int dv, int L) {
     (void)L;
     const int nch = S / LT;
-    if (nch < 1) return 0;     // shorter than a tile: the exact kernel, which needs no scratch
+    if (nch < 1 || (dqk != 256 && dqk != 128) || dv % DVS) return 0;     // not a shape of this path
     const int forced = g_segments.load();
     const int P = forced >= 1 ? (forced > nch ? (nch > 0 ? nch : 1) : forced) : plan_segments(B * NH, dv, nch);
     return ws_layout(B, NH, S, dqk, dv, P).total;
