@@ -572,8 +572,8 @@ def test_slstm_recurrent_oracle(ops, B, S, NH, dh, dtype):
 
 @pytest.mark.parametrize("B,S,NH", [(1, 5, 1), (33, 70, 2), (32, 600, 4)])
 def test_slstm_recurrent_tensor_core_path(ops, B, S, NH):
-    """bf16 with head dimension 256 runs the tcgen05 kernel (R resident in tensor memory, h fed back as
-    bf16): ragged batch groups, a carried state, and a long sequence for drift."""
+    """bf16 with head dimension 256 runs on the tensor cores (h fed back as bf16): ragged batch groups, a carried
+    state, and a long sequence for drift."""
     dh, D = 256, NH * 256
     rng = np.random.default_rng(B * 1000 + S)
     gx = rng.standard_normal((B, S, 4, D)).astype(np.float32)
@@ -591,6 +591,34 @@ def test_slstm_recurrent_tensor_core_path(ops, B, S, NH):
     assert relerr(host(hs), hs_ref) < BF16_TOL
     for got, want in zip(st2, st_ref):
         assert relerr(host(got), want) < BF16_TOL
+
+
+BF, FP = torch.bfloat16, torch.float32
+
+
+@pytest.mark.parametrize("B,S,NH,dh,dtype", [(1, 1, 1, 64, BF), (16, 2, 2, 64, BF), (17, 3, 4, 128, BF), (5, 64, 2, 128, BF),
+                                             (16, 1, 1, 256, BF), (15, 2, 2, 256, BF), (34, 7, 3, 256, BF)])
+def test_slstm_recurrent_edges(ops, B, S, NH, dh, dtype):
+    """One, two and three steps (each h buffer unused, used once, reused), rows around the groups of a cluster (16), a
+    carried state.  bf16 heads of 64 and 128 feed h back unrounded and use the exact exponentials: their states stay within
+    the fp32 tolerance and their outputs within half a bf16 ulp (8 significant bits: 2^-8 of the value) of it."""
+    rng = np.random.default_rng(dh + B)
+    rd = xo.bf16_round if dtype == BF else (lambda a: a)
+    D = NH * dh
+    gx = rng.standard_normal((B, S, 4, D)).astype(np.float32)
+    gx[:, :, 1] += np.linspace(3, 6, D, dtype=np.float32)
+    gx = rd(gx)
+    R = rd((rng.standard_normal((4, NH, dh, dh)) * 0.05).astype(np.float32))
+    rb = (rng.standard_normal((4, D)) * 0.05).astype(np.float32)
+    st0 = [rng.standard_normal((B, D)).astype(np.float32) for _ in range(4)]
+    st0[1] = np.abs(st0[1]) + 1
+    hs_ref, st_ref = xo.slstm_recurrent(gx, R, rb, tuple(st0), NH, 15.0)
+    hs, st = ops.slstm_recurrent(dev(gx, dtype), dev(R, dtype), dev(rb), tuple(dev(s) for s in st0), NH, 15.0)
+    ops.slstm_recurrent_status()
+    rounded = dtype == BF and dh == 256
+    for got, want in zip(st, st_ref):
+        assert relerr(host(got), want) < (BF16_TOL if rounded else FP32_TOL)
+    assert relerr(host(hs), hs_ref) < (BF16_TOL if rounded else FP32_TOL if dtype == FP else 2.0 ** -8 + FP32_TOL)
 
 
 # ---- error behaviour of the C ABI --------------------------------------------------

@@ -188,12 +188,16 @@ static int slstm_recurrent_launch(const void *gx, const void *R, const float *rb
 }  // namespace xl
 
 namespace xl {
-// tensor-core version (slstm_tc.cu): bf16, head dimension 256
-bool slstm_recurrent_tc_supported(int dtype, int dh, const void *R, const void *gx, const void *hs);
-int slstm_recurrent_tc_status(cudaStream_t st);
-int slstm_recurrent_tc(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
-                       const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH,
-                       float cap, cudaStream_t st);
+// bf16 with head dimension 64, 128 or 256 on the tensor cores (slstm_mma.cu); a wait that gives up sets *timeout
+bool slstm_recurrent_mma_supported(int dtype, int dh, const void *R, const void *gx, const void *hs);
+int slstm_recurrent_mma(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
+                        const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH, int dh,
+                        float cap, int *timeout, cudaStream_t st);
+
+namespace {
+// set by any CTA whose bounded wait gave up; read and cleared by xlstm_slstm_recurrent_status()
+__device__ int g_rec_timeout = 0;
+}  // namespace
 }  // namespace xl
 
 extern "C" int xlstm_slstm_recurrent(const void *gx, const void *R, const float *rb, const float *c0, const float *n0,
@@ -206,13 +210,27 @@ extern "C" int xlstm_slstm_recurrent(const void *gx, const void *R, const float 
     if (dtype != XLSTM_F32 && dtype != XLSTM_BF16) return XLSTM_ERR_UNSUPPORTED;
     if (NH > 65535 || (B + xl::REC_BG - 1) / xl::REC_BG > 65535) return XLSTM_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (xl::slstm_recurrent_tc_supported(dtype, dh, R, gx, hs))
-        return xl::slstm_recurrent_tc(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, st);
+    if (xl::slstm_recurrent_mma_supported(dtype, dh, R, gx, hs)) {
+        void *timeout = nullptr;
+        if (cudaGetSymbolAddress(&timeout, xl::g_rec_timeout) != cudaSuccess) return XLSTM_ERR_CUDA;
+        return xl::slstm_recurrent_mma(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap,
+                                       static_cast<int *>(timeout), st);
+    }
     if (dtype == XLSTM_F32)
         return xl::slstm_recurrent_launch<float>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap, st);
     return xl::slstm_recurrent_launch<__nv_bfloat16>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap, st);
 }
 
 extern "C" int xlstm_slstm_recurrent_status(void *stream) {
-    return xl::slstm_recurrent_tc_status(static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    int v = 0;
+    if (cudaMemcpyFromSymbolAsync(&v, xl::g_rec_timeout, sizeof(int), 0, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return XLSTM_ERR_CUDA;
+    if (!v) return XLSTM_OK;
+    const int zero = 0;
+    if (cudaMemcpyToSymbolAsync(xl::g_rec_timeout, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return XLSTM_ERR_CUDA;
+    return XLSTM_ERR_TIMEOUT;
 }
