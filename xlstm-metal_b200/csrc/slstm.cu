@@ -188,11 +188,16 @@ static int slstm_recurrent_launch(const void *gx, const void *R, const float *rb
 }  // namespace xl
 
 namespace xl {
-// bf16 with head dimension 64, 128 or 256 on the tensor cores (slstm_mma.cu); a wait that gives up sets *timeout
+// bf16 with head dimension 64, 128 or 256 on the tensor cores (slstm_mma.cu), fp32 with the same head dimensions from
+// registers (slstm_regs.cu); a wait that gives up sets *timeout
 bool slstm_recurrent_mma_supported(int dtype, int dh, const void *R, const void *gx, const void *hs);
 int slstm_recurrent_mma(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
                         const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH, int dh,
                         float cap, int *timeout, cudaStream_t st);
+bool slstm_recurrent_regs_supported(int dtype, int dh, const void *R);
+int slstm_recurrent_regs(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
+                         const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH, int dh,
+                         float cap, int *timeout, cudaStream_t st);
 
 namespace {
 // set by any CTA whose bounded wait gave up; read and cleared by xlstm_slstm_recurrent_status()
@@ -210,11 +215,12 @@ extern "C" int xlstm_slstm_recurrent(const void *gx, const void *R, const float 
     if (dtype != XLSTM_F32 && dtype != XLSTM_BF16) return XLSTM_ERR_UNSUPPORTED;
     if (NH > 65535 || (B + xl::REC_BG - 1) / xl::REC_BG > 65535) return XLSTM_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (xl::slstm_recurrent_mma_supported(dtype, dh, R, gx, hs)) {
+    const bool mma = xl::slstm_recurrent_mma_supported(dtype, dh, R, gx, hs);
+    if (mma || xl::slstm_recurrent_regs_supported(dtype, dh, R)) {
         void *timeout = nullptr;
         if (cudaGetSymbolAddress(&timeout, xl::g_rec_timeout) != cudaSuccess) return XLSTM_ERR_CUDA;
-        return xl::slstm_recurrent_mma(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap,
-                                       static_cast<int *>(timeout), st);
+        auto run = mma ? xl::slstm_recurrent_mma : xl::slstm_recurrent_regs;
+        return run(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap, static_cast<int *>(timeout), st);
     }
     if (dtype == XLSTM_F32)
         return xl::slstm_recurrent_launch<float>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, dh, cap, st);
