@@ -32,7 +32,8 @@
 // scratch buffer, releases all roles and frees TMEM before the CTA returns.
 #include <atomic>
 
-#include "mlstm_chunkwise_tc.cuh"
+#include "mlstm_chunkwise_tc_fast.cuh"
+#include "mlstm_chunkwise_tc_scan.cuh"
 
 namespace xl {
 
@@ -43,13 +44,16 @@ using namespace tcw;
 
 // ---------------------------------------------------------------------------
 // gate pre-pass.  Only the stabiliser m couples the tiles, and only through two numbers per tile
-// (G = sum of log-sigmoid f, U = max of u = i - b), so it runs as three small launches:
-//   mlstm_gate_stats_kernel   one warp per (head, tile): G_c, U_c                      -> scratch
-//   mlstm_gate_chain_kernel   one warp per head: m_{c+1} = G_c + max(m_c, U_c), the frame rho of the
-//                             lazily rescaled accumulator, the head's path flag        -> scratch
-//   mlstm_gate_write_kernel   one warp per (head, tile): the per-token scalars          -> scratch
+// (G = sum of log-sigmoid f, U = max of u = i - b):  m' = G + max(m, U).  Three phases:
+//   stats   one warp per (head, tile): G_c, U_c
+//   chain   one warp per (head, segment): m at every tile of the segment, the frame rho of the lazily rescaled
+//           accumulator, the segment's path flag and total decay
+//   write   one warp per (head, tile): the per-token scalars
+// One launch with a CTA per head up to FUSED_TILES tiles (a warp per tile, the phases between barriers); three launches
+// beyond that, where one CTA per head would do on one SM what the tiles' warps do on all of them.
 // Sums and maxima are kept in double so that differences of large cumulative sums stay exact.
 // ---------------------------------------------------------------------------
+constexpr int FUSED_TILES = 32;
 constexpr int GP_THREADS = 256;        // 8 warps = 8 tiles per CTA
 constexpr int GC = 6;                  // doubles of chain scratch per (head, tile): G, U, m_in, rho_in, rho_out, mul
 constexpr double RESCALE_AT = 30.0;    // general kernel: rescale C~ when the frame exponent would exceed e^30
@@ -59,6 +63,19 @@ constexpr double RESCALE_AT = 30.0;    // general kernel: rescale C~ when the fr
 // margin of e^10 below overflow.
 constexpr double SPREAD_LIMIT = 45.0;
 constexpr double RESCALE_AT_B = 20.0;
+
+struct GateParams {
+    const void *ig, *fg;
+    const float *m0;            // [BH] or NULL (zero)
+    double *chain;              // [BH][NCH][GC] (three-launch form)
+    float *gates;               // [BH][NCH][GW]
+    float *m_final;             // [BH] stabiliser after the last tile
+    float *decay;               // [BH * P] total decay of a segment, or NULL
+    int *path, *status;         // [BH * P] 1: bounded-spread path; status word, cleared here
+    int64_t sg[3];
+    int NH, NCH, P, seg_tiles, general_only;
+    float qscale, cap;
+};
 
 template <typename T>
 __device__ __forceinline__ void gate_tile_scan(const T *ip, const T *fp, int64_t sg_s, float cap, int c, int lane,
@@ -100,65 +117,64 @@ __device__ __forceinline__ void gate_tile_scan(const T *ip, const T *fp, int64_t
     G = __shfl_sync(0xffffffffu, bcum[3], 31);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(GP_THREADS)
-mlstm_gate_stats_kernel(const T *__restrict__ ig, const T *__restrict__ fg, int64_t sg_b, int64_t sg_h, int64_t sg_s,
-                        double *__restrict__ chain, int NH, int NCH, float cap) {
-    const int bh = blockIdx.y, b = bh / NH, hd = bh % NH;
-    const int lane = threadIdx.x & 31, c = blockIdx.x * (GP_THREADS / 32) + (threadIdx.x >> 5);
-    if (c >= NCH) return;
-    double bcum[4], u[4], pmax[4], excl, G, U;
-    gate_tile_scan<T>(ig + b * sg_b + hd * sg_h, fg + b * sg_b + hd * sg_h, sg_s, cap, c, lane, bcum, u, pmax, excl, G, U);
-    if (lane == 0) {
-        double *o = chain + ((size_t)bh * NCH + c) * GC;
-        o[0] = G; o[1] = U;
-    }
-}
-
-// One warp per (head, segment).  The chain is sequential but tiny; the warp loads 32 tiles' (G, U) at once and
-// every lane walks them through shuffles, keeping the results of "its" tile for a coalesced write.
-// m0_auto: the segment starts from an EMPTY state (C = n = 0): any stabiliser below the first maximum gives the
-// same end state, so the chain starts at the first tile's U (spread 0) instead of -inf.
-__global__ void __launch_bounds__(32)
-mlstm_gate_chain_kernel(const float *__restrict__ m0, double *__restrict__ chain, float *__restrict__ m_out,
-                        int *__restrict__ path, int NCH, int P, int seg_tiles, int general_only, int m0_auto) {
-    const int bhv = blockIdx.x, lane = threadIdx.x;
-    const int tile0 = (bhv % P) * seg_tiles, n = min(seg_tiles, NCH - tile0);
-    double *ch = chain + ((size_t)(bhv / P) * NCH + tile0) * GC;
-    // pass 1: the stabiliser chain, and whether every tile's spread x_last - m is bounded
-    double m = m0_auto ? ch[1] : (m0 ? (double)m0[bhv] : 0.0);
-    bool bounded = !general_only;
-    for (int c0 = 0; c0 < n; c0 += 32) {
-        const int c = c0 + lane;
-        const double Gl = c < n ? ch[(size_t)c * GC + 0] : 0.0, Ul = c < n ? ch[(size_t)c * GC + 1] : 0.0;
-        double m_mine = 0.0;
-        const int nb = min(32, n - c0);
-        for (int j = 0; j < nb; ++j) {
-            const double Gj = __shfl_sync(0xffffffffu, Gl, j), Uj = __shfl_sync(0xffffffffu, Ul, j);
-            const double x_last = fmax(m, Uj);
-            if (x_last - m > SPREAD_LIMIT) bounded = false;
-            if (j == lane) m_mine = m;
-            m = Gj + x_last;
+// the chain of one segment, by one warp: ch = the head's [NCH][GC] scratch (global or shared memory)
+__device__ __forceinline__ void gate_chain(double *ch, double m, int tile0, int n, bool general_only, int lane, float *m_out,
+                                           int *path, float *decay) {
+    // (G, U) as a map m -> max(G + m, M) with M = G + U; maps compose associatively, first tile on the left
+    auto tile_map = [&](int c, int end, double &G, double &M) {
+        const bool ok = c < end;
+        G = ok ? ch[(size_t)c * GC + 0] : 0.0;
+        M = ok ? G + ch[(size_t)c * GC + 1] : -INFINITY;
+    };
+    for (int c0 = 0; c0 < tile0; c0 += 32) {       // the tiles before the segment, 32 at a time
+        double G, M;
+        tile_map(c0 + lane, tile0, G, M);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double G2 = __shfl_down_sync(0xffffffffu, G, o), M2 = __shfl_down_sync(0xffffffffu, M, o);
+            M = fmax(G2 + M, M2);
+            G += G2;
         }
-        if (c < n) ch[(size_t)c * GC + 2] = m_mine;    // stabiliser carried INTO tile c
+        m = fmax(__shfl_sync(0xffffffffu, G, 0) + m, __shfl_sync(0xffffffffu, M, 0));
     }
-    if (lane == 0) { m_out[bhv] = (float)m; path[bhv] = bounded ? 1 : 0; }
-    // pass 2: C is kept in TMEM as C~ = C e^{-rho}: rho absorbs the per-tile decay so that the accumulator is
+    // the stabiliser carried into every tile, and whether every tile's spread x_last - m is bounded
+    bool bounded = !general_only;
+    const int end = tile0 + n;
+    for (int c0 = tile0; c0 < end; c0 += 32) {
+        const int c = c0 + lane;
+        double G, M;
+        tile_map(c, end, G, M);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double G1 = __shfl_up_sync(0xffffffffu, G, o), M1 = __shfl_up_sync(0xffffffffu, M, o);
+            if (lane >= o) { M = fmax(G + M1, M); G += G1; }
+        }
+        const double m_after = fmax(G + m, M);
+        double m_in = __shfl_up_sync(0xffffffffu, m_after, 1);
+        if (lane == 0) m_in = m;
+        if (c < end) ch[(size_t)c * GC + 2] = m_in;
+        const bool wide = c < end && fmax(m_in, ch[(size_t)c * GC + 1]) - m_in > SPREAD_LIMIT;
+        if (__any_sync(0xffffffffu, wide)) bounded = false;
+        m = __shfl_sync(0xffffffffu, m_after, 31);
+    }
+    if (lane == 0) { if (m_out) *m_out = (float)m; *path = bounded ? 1 : 0; }
+    // C is kept in TMEM as C~ = C e^{-rho}: rho absorbs the per-tile decay so that the accumulator is
     // NOT rescaled every tile; only when -rho would exceed the threshold is C~ multiplied once (mul).
-    // General kernel: the multiplication happens BEFORE tile c's update (mul also carries the decay of that
-    // tile); bounded-spread kernel: AFTER tile c's update, so that update and read-out of a tile share one
+    // General path: the multiplication happens BEFORE tile c's update (mul also carries the decay of that
+    // tile); bounded-spread path: AFTER tile c's update, so that update and read-out of a tile share one
     // frame.  rho_in = frame the read-out of tile c sees, rho_out = frame after tile c's update.
-    double rho = 0.0;
-    for (int c0 = 0; c0 < n; c0 += 32) {
+    double rho = 0.0, total = 0.0;
+    for (int c0 = tile0; c0 < end; c0 += 32) {
         const int c = c0 + lane;
         double ld = 0.0;
-        if (c < n) ld = ch[(size_t)c * GC + 2] - fmax(ch[(size_t)c * GC + 2], ch[(size_t)c * GC + 1]);   // m - x_last <= 0
+        if (c < end) ld = ch[(size_t)c * GC + 2] - fmax(ch[(size_t)c * GC + 2], ch[(size_t)c * GC + 1]);   // m - x_last <= 0
         double rin = 0.0, rout = 0.0, mul = 1.0;
-        const int nb = min(32, n - c0);
+        const int nb = min(32, end - c0);
         for (int j = 0; j < nb; ++j) {
             const double logdec = __shfl_sync(0xffffffffu, ld, j);
             const double r_in = rho;
             double r_out, mu = 1.0;
+            total += logdec;
             if (bounded) {
                 rho += logdec;
                 r_out = rho;
@@ -170,52 +186,26 @@ mlstm_gate_chain_kernel(const float *__restrict__ m0, double *__restrict__ chain
             }
             if (j == lane) { rin = r_in; rout = r_out; mul = mu; }
         }
-        if (c < n) {
+        if (c < end) {
             ch[(size_t)c * GC + 3] = rin; ch[(size_t)c * GC + 4] = rout; ch[(size_t)c * GC + 5] = mul;
         }
     }
+    if (lane == 0 && decay) *decay = (float)exp(total);
 }
 
-// Segment-parallel prefill: the end state of segment j from an EMPTY state (Cl, nl, ml) and the total log-decay
-// G_j of the segment combine associatively with the state before it,
-//   m' = max(G_j + m, ml);  C' = e^{G_j + m - m'} C + e^{ml - m'} Cl;  n' likewise,
-// so one cheap pass over the P local states yields the true state at the start of every segment (Cs, ns, ms)
-// and the final state.  One CTA per (head, slab of elements); the scalar chain is recomputed per CTA.
+// Segment-parallel prefill: the end state of segment j from an EMPTY state (Cl, nl, in the frame of the true stabiliser)
+// and the segment's total decay combine associatively with the state before it,
+//   C' = e^{sum of m - x_last} C + Cl;  n' likewise,
+// so one cheap pass over the P local states yields the true state at the start of every segment (Cs, ns)
+// and the final state.  One CTA per (head, slab of elements).
 constexpr int COMB_THREADS = 256;
 constexpr int COMB_VEC = 4;        // elements per thread (one 16-byte vector)
 __global__ void __launch_bounds__(COMB_THREADS)
-mlstm_segment_combine_kernel(const float *__restrict__ C0, const float *__restrict__ n0, const float *__restrict__ m0,
-                             const float *__restrict__ Cl, const float *__restrict__ nl, const float *__restrict__ ml,
-                             const double *__restrict__ chain, float *__restrict__ Cs, float *__restrict__ ns,
-                             float *__restrict__ ms, float *__restrict__ C1, float *__restrict__ n1, float *__restrict__ m1,
-                             int NCH, int P, int seg_tiles, int dqk, int dv) {
-    __shared__ float s_wc[64], s_wl[64];   // weights of the carried and of the local state per segment (P <= 64)
-    __shared__ double s_G[64];             // summed log forget gates per segment
+mlstm_segment_combine_kernel(const float *__restrict__ C0, const float *__restrict__ n0, const float *__restrict__ Cl,
+                             const float *__restrict__ nl, const float *__restrict__ decay, float *__restrict__ Cs,
+                             float *__restrict__ ns, float *__restrict__ C1, float *__restrict__ n1, int P, int dqk, int dv) {
+    grid_dependency_wait();
     const int bh = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // per-segment sums by the warps (lanes stride over the segment's tiles), then one thread chains the P segments
-    for (int j = warp; j < P; j += COMB_THREADS / 32) {
-        const int tile0 = j * seg_tiles, n = min(seg_tiles, NCH - tile0);
-        double G = 0.0;
-        for (int c = lane; c < n; c += 32) G += chain[((size_t)bh * NCH + tile0 + c) * GC + 0];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) G += __shfl_xor_sync(0xffffffffu, G, o);
-        if (lane == 0) s_G[j] = G;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = C0 ? (double)m0[bh] : 0.0;
-        for (int j = 0; j < P; ++j) {
-            const double mloc = (double)ml[(size_t)bh * P + j];
-            const double mn = fmax(s_G[j] + m, mloc);
-            if (blockIdx.y == 0) ms[(size_t)bh * P + j] = (float)m;
-            s_wc[j] = (float)exp(s_G[j] + m - mn);
-            s_wl[j] = (float)exp(mloc - mn);
-            m = mn;
-        }
-        if (blockIdx.y == 0) m1[bh] = (float)m;
-    }
-    __syncthreads();
     // elements of C, then of n, as 16-byte vectors (dqk * dv and dqk are multiples of 4); a thread owns one vector
     // of every segment: its P loads are independent of the chain and are issued ahead of it, 8 at a time
     const size_t CE = (size_t)dqk * dv, total_vec = (CE + dqk) / COMB_VEC;
@@ -236,45 +226,47 @@ mlstm_segment_combine_kernel(const float *__restrict__ C0, const float *__restri
                 if (j0 + u < P) {
                     const int j = j0 + u;
                     stg_stream(st + ((size_t)bh * P + j) * per + off, v);
-                    const float wc = s_wc[j], wl = s_wl[j];
-                    v.x = wc * v.x + wl * l[u].x;
-                    v.y = wc * v.y + wl * l[u].y;
-                    v.z = wc * v.z + wl * l[u].z;
-                    v.w = wc * v.w + wl * l[u].w;
+                    const float wc = decay[(size_t)bh * P + j];
+                    v.x = fmaf(wc, v.x, l[u].x);
+                    v.y = fmaf(wc, v.y, l[u].y);
+                    v.z = fmaf(wc, v.z, l[u].z);
+                    v.w = fmaf(wc, v.w, l[u].w);
                 }
         }
         *reinterpret_cast<float4 *>(fin + (size_t)bh * per + off) = v;
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(GP_THREADS)
-mlstm_gate_write_kernel(const T *__restrict__ ig, const T *__restrict__ fg, int64_t sg_b, int64_t sg_h, int64_t sg_s,
-                        const double *__restrict__ chain, const int *__restrict__ path, float *__restrict__ gates,
-                        int NH, int NCH, int P, int seg_tiles, float qscale, float cap) {
-    const int bh = blockIdx.y, b = bh / NH, hd = bh % NH;
-    const int lane = threadIdx.x & 31, c = blockIdx.x * (GP_THREADS / 32) + (threadIdx.x >> 5);
-    if (c >= NCH) return;
-    const bool bounded = path[(size_t)bh * P + c / seg_tiles] != 0;
+// gates of one tile, in the registers of its warp (lane = four tokens)
+struct GateScan {
     double bcum[4], u[4], pmax[4], excl, G, U;
-    gate_tile_scan<T>(ig + b * sg_b + hd * sg_h, fg + b * sg_b + hd * sg_h, sg_s, cap, c, lane, bcum, u, pmax, excl, G, U);
-    const double *ch = chain + ((size_t)bh * NCH + c) * GC;
+};
+template <typename T>
+__device__ __forceinline__ GateScan gate_tile(const GateParams &p, int bh, int c, int lane) {
+    const int b = bh / p.NH, hd = bh % p.NH;
+    const int64_t off = b * p.sg[0] + hd * p.sg[1];
+    GateScan s;
+    gate_tile_scan<T>(static_cast<const T *>(p.ig) + off, static_cast<const T *>(p.fg) + off, p.sg[2], p.cap, c, lane, s.bcum,
+                      s.u, s.pmax, s.excl, s.G, s.U);
+    return s;
+}
+
+__device__ __forceinline__ void gate_write(const GateScan &s, const double *ch, bool bounded, float *g, int lane, float qscale) {
     const double m = ch[2], rho_in = ch[3], rho_out = ch[4];
-    const double x_last = fmax(U, m);
-    const double carry = fmax(excl, m);
-    float *g = gates + ((size_t)bh * NCH + c) * GW;
+    const double x_last = fmax(s.U, m);
+    const double carry = fmax(s.excl, m);
     float4 o_u2, o_x2, o_wq, o_w, o_em;
     float *pu = &o_u2.x, *px = &o_x2.x, *pq = &o_wq.x, *pw = &o_w.x, *pe = &o_em.x;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const double xt = fmax(pmax[e], carry);
-        pu[e] = (float)(u[e] * (double)LOG2E);
+        const double xt = fmax(s.pmax[e], carry);
+        pu[e] = (float)(s.u[e] * (double)LOG2E);
         px[e] = (float)(xt * (double)LOG2E);
         pq[e] = expf((float)(m - xt + rho_in)) * qscale;   // read-out sees C~ = C e^{-rho_in}
-        // weight of token s in the update: general kernel e^{u_s - x_last - rho_out} (<= e^{RESCALE_AT});
-        // bounded-spread kernel a_s = e^{u_s - m - rho_in} (the same number except on rescale tiles)
-        pw[e] = bounded ? expf((float)(u[e] - m - rho_in)) : expf((float)(u[e] - x_last - rho_out));
-        pe[e] = expf(-(float)(bcum[e] + xt));
+        // weight of token s in the update: general path e^{u_s - x_last - rho_out} (<= e^{RESCALE_AT});
+        // bounded-spread path a_s = e^{u_s - m - rho_in} (the same number except on rescale tiles)
+        pw[e] = bounded ? expf((float)(s.u[e] - m - rho_in)) : expf((float)(s.u[e] - x_last - rho_out));
+        pe[e] = expf(-(float)(s.bcum[e] + xt));
     }
     *reinterpret_cast<float4 *>(g + G_U2 + lane * 4) = o_u2;
     *reinterpret_cast<float4 *>(g + G_X2 + lane * 4) = o_x2;
@@ -283,9 +275,72 @@ mlstm_gate_write_kernel(const T *__restrict__ ig, const T *__restrict__ fg, int6
     *reinterpret_cast<float4 *>(g + G_EMT + lane * 4) = o_em;
     if (lane == 0) {
         g[G_SCAL + 0] = (float)ch[5];               // multiplier for C~ and n~: before this tile (general) / after its update (bounded)
-        g[G_SCAL + 1] = (float)(G + x_last);        // stabiliser after this tile
+        g[G_SCAL + 1] = (float)(s.G + x_last);      // stabiliser after this tile
         g[G_SCAL + 2] = expf((float)rho_out);       // C = C~ * this after the tile's update (used for the final state)
     }
+}
+
+__device__ __forceinline__ void gate_segment(const GateParams &p, double *ch, int bh, int j, int lane) {
+    const int tile0 = j * p.seg_tiles, n = min(p.seg_tiles, p.NCH - tile0);
+    gate_chain(ch, p.m0 ? (double)p.m0[bh] : 0.0, tile0, n, p.general_only != 0, lane, j == p.P - 1 ? p.m_final + bh : nullptr,
+               p.path + (size_t)bh * p.P + j, p.decay ? p.decay + (size_t)bh * p.P + j : nullptr);
+}
+
+template <typename T> __global__ void __launch_bounds__(FUSED_TILES * 32) mlstm_gate_kernel(const GateParams p) {
+    __shared__ double s_chain[FUSED_TILES * GC];
+    __shared__ int s_path[FUSED_TILES];
+    grid_dependency_wait();
+    allow_dependents();
+    const int bh = blockIdx.x, lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+    const GateScan s = gate_tile<T>(p, bh, c, lane);
+    if (lane == 0) { s_chain[c * GC] = s.G; s_chain[c * GC + 1] = s.U; }
+    if (bh == 0 && threadIdx.x == 0) *p.status = 0;
+    __syncthreads();
+    if (c < p.P) {
+        gate_segment(p, s_chain, bh, c, lane);
+        if (lane == 0) s_path[c] = p.path[(size_t)bh * p.P + c];
+    }
+    __syncthreads();
+    gate_write(s, s_chain + c * GC, s_path[c / p.seg_tiles] != 0, p.gates + ((size_t)bh * p.NCH + c) * GW, lane, p.qscale);
+}
+
+template <typename T> __global__ void __launch_bounds__(GP_THREADS) mlstm_gate_stats_kernel(const GateParams p) {
+    grid_dependency_wait();
+    allow_dependents();
+    const int bh = blockIdx.y, lane = threadIdx.x & 31, c = blockIdx.x * (GP_THREADS / 32) + (threadIdx.x >> 5);
+    if (bh == 0 && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
+    if (c >= p.NCH) return;
+    const GateScan s = gate_tile<T>(p, bh, c, lane);
+    if (lane == 0) {
+        double *o = p.chain + ((size_t)bh * p.NCH + c) * GC;
+        o[0] = s.G; o[1] = s.U;
+    }
+}
+
+__global__ void __launch_bounds__(32) mlstm_gate_chain_kernel(const GateParams p) {
+    grid_dependency_wait();
+    allow_dependents();
+    const int bh = blockIdx.x / p.P;
+    gate_segment(p, p.chain + (size_t)bh * p.NCH * GC, bh, blockIdx.x % p.P, threadIdx.x);
+}
+
+template <typename T> __global__ void __launch_bounds__(GP_THREADS) mlstm_gate_write_kernel(const GateParams p) {
+    grid_dependency_wait();
+    allow_dependents();
+    const int bh = blockIdx.y, lane = threadIdx.x & 31, c = blockIdx.x * (GP_THREADS / 32) + (threadIdx.x >> 5);
+    if (c >= p.NCH) return;
+    const GateScan s = gate_tile<T>(p, bh, c, lane);
+    gate_write(s, p.chain + ((size_t)bh * p.NCH + c) * GC, p.path[(size_t)bh * p.P + c / p.seg_tiles] != 0,
+               p.gates + ((size_t)bh * p.NCH + c) * GW, lane, p.qscale);
+}
+
+template <typename T> int gate_prepass(const GateParams &p, int BH, cudaStream_t st) {
+    if (p.NCH <= FUSED_TILES) return launch_overlapped(mlstm_gate_kernel<T>, dim3(BH), dim3(p.NCH * 32), 0, st, p);
+    const dim3 tg((p.NCH + GP_THREADS / 32 - 1) / (GP_THREADS / 32), BH);
+    int rc = launch_overlapped(mlstm_gate_stats_kernel<T>, tg, dim3(GP_THREADS), 0, st, p);
+    if (rc == XLSTM_OK) rc = launch_overlapped(mlstm_gate_chain_kernel, dim3(BH * p.P), dim3(32), 0, st, p);
+    if (rc == XLSTM_OK) rc = launch_overlapped(mlstm_gate_write_kernel<T>, tg, dim3(GP_THREADS), 0, st, p);
+    return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -347,7 +402,7 @@ __device__ __forceinline__ void c_pass_half(unsigned char *smem, uint32_t t_half
 }
 
 template <int DQK>
-__global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
+__device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     using SM = Smem<DQK>;
     constexpr int NBOX = SM::NBOX;
     constexpr int NHALF = DQK / 128;
@@ -361,7 +416,6 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bh = blockIdx.x;     // (batch, head, segment): index of the states and of the path flag
-    if (p.path[bh] != 0) return;   // this segment runs in the bounded-spread kernel (CTA-uniform, before any set-up)
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;   // (batch, head) and first tile of this segment
     const int b = bhr / p.NH, hd = bhr % p.NH;
     const int col0 = blockIdx.y * DVS;
@@ -693,6 +747,26 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __
     if (tid == 0 && *abort_flag) atomicExch(p.status, 1);
 }
 
+// One launch for all (head, segment)s: a CTA takes the path that the gate pre-pass has found for its gates.  Heads of
+// both kinds run side by side (two launches, each with half of the CTAs returning at once, ran them one after the
+// other).  STATE_ONLY: the first pass of the segment-parallel mode, where the bounded path needs no h.
+template <int DQK, bool STATE_ONLY>
+__global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
+    grid_dependency_wait();
+    if (p.path[blockIdx.x] == 0) chunkwise_general<DQK>(p);
+    else if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
+    else chunkwise_bounded<DQK>(p);
+}
+
+template <int DQK, bool STATE_ONLY>
+int launch_tc(const TcParams &tp, dim3 grid, cudaStream_t st) {
+    constexpr uint32_t bytes = STATE_ONLY && ScanSmem<DQK>::TOTAL > Smem<DQK>::TOTAL ? ScanSmem<DQK>::TOTAL : Smem<DQK>::TOTAL;
+    auto kern = mlstm_chunkwise_tc_kernel<DQK, STATE_ONLY>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+        return XLSTM_ERR_CUDA;
+    return launch_overlapped(kern, grid, dim3(THREADS), bytes, st, tp);
+}
+
 }  // namespace
 
 bool mlstm_chunkwise_tc_shape_ok(const ChunkwiseParams &p, int dtype) {
@@ -719,7 +793,7 @@ namespace {
 
 // Layout of the caller-provided scratch.  P > 1 adds the per-segment states of the segment-parallel mode.
 struct WsLayout {
-    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], seg_m[2], total;
+    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], decay, total;
     int P, seg_tiles;
 };
 
@@ -758,8 +832,8 @@ WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P) {
         for (int set = 0; set < 2; ++set) {
             w.seg_C[set] = o; o = up(o + VH * dqk * dv * sizeof(float));
             w.seg_n[set] = o; o = up(o + VH * dqk * sizeof(float));
-            w.seg_m[set] = o; o = up(o + VH * sizeof(float));
         }
+        w.decay = o; o = up(o + VH * sizeof(float));
     }
     w.total = o + 256;
     return w;
@@ -811,20 +885,11 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     const size_t CE = (size_t)p.dqk * p.dv;                         // elements of one C
     // set A: pass 1 local end states (pass 2: end states, unused); set B: the true start state of every segment
     float *segA_C = reinterpret_cast<float *>(ws + w.seg_C[0]), *segA_n = reinterpret_cast<float *>(ws + w.seg_n[0]);
-    float *segA_m = reinterpret_cast<float *>(ws + w.seg_m[0]);
     float *segB_C = reinterpret_cast<float *>(ws + w.seg_C[1]), *segB_n = reinterpret_cast<float *>(ws + w.seg_n[1]);
-    float *segB_m = reinterpret_cast<float *>(ws + w.seg_m[1]);
+    float *decay = reinterpret_cast<float *>(ws + w.decay);
     const bool tail = s_full < p.S;
     if (tail && p.n_peer) return XLSTM_ERR_UNSUPPORTED;   // the exact tail path writes the local h only
     if (p.tok_per_rank > 0 && (p.tok_per_rank % LT || (long long)p.tok_per_rank * p.n_peer != s_full)) return XLSTM_ERR_INVALID;
-    if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return XLSTM_ERR_CUDA;
-
-    const __nv_bfloat16 *ig = static_cast<const __nv_bfloat16 *>(p.ig), *fg = static_cast<const __nv_bfloat16 *>(p.fg);
-    const dim3 tg((nch + GP_THREADS / 32 - 1) / (GP_THREADS / 32), BH);
-    mlstm_gate_stats_kernel<__nv_bfloat16><<<tg, GP_THREADS, 0, st>>>(ig, fg, p.sg[0], p.sg[1], p.sg[2], chain, p.NH, nch,
-                                                                      p.gate_cap);
-    if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
-
     TcParams tp{};
     if (!make_tmap_bf16_4d(&tp.tq, p.q, p.dqk, s_full, p.NH, p.B, p.sq[2], p.sq[1], p.sq[0], LT) ||
         !make_tmap_bf16_4d(&tp.tk, p.k, p.dqk, s_full, p.NH, p.B, p.sk[2], p.sk[1], p.sk[0], LT) ||
@@ -844,51 +909,43 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     for (int d = 0; d < 3; ++d) tp.sh[d] = p.sh[d];
     const dim3 grid(BH * P, p.dv / DVS);
 
-    // one forward over all (head, segment) pairs: chain + per-token scalars of the gate pre-pass, then the two
-    // tensor-core kernels.  Two launches over the same grid: every CTA looks at its path flag (written by the
-    // pre-pass) and returns at once if it belongs to the other kernel, so the choice needs no host round trip.
-    auto forward = [&](const float *m0v, int m0_auto, float *m_out, bool state_only) -> int {
-        mlstm_gate_chain_kernel<<<BH * P, 32, 0, st>>>(m0v, chain, m_out, path, nch, P, seg_tiles, g_general_only.load(),
-                                                       m0_auto);
-        mlstm_gate_write_kernel<__nv_bfloat16><<<tg, GP_THREADS, 0, st>>>(ig, fg, p.sg[0], p.sg[1], p.sg[2], chain, path, gates,
-                                                                          p.NH, nch, P, seg_tiles, p.qscale, p.gate_cap);
-        if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
-        const int rc = state_only ? mlstm_chunkwise_tc_scan_launch(tp, grid, p.dqk, st) : mlstm_chunkwise_tc_fast_launch(tp, grid, p.dqk, st);
-        if (rc != XLSTM_OK) return rc;
-        if (p.dqk == 256) {
-            auto kern = mlstm_chunkwise_tc_kernel<256>;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<256>::TOTAL) != cudaSuccess)
-                return XLSTM_ERR_CUDA;
-            kern<<<grid, THREADS, Smem<256>::TOTAL, st>>>(tp);
-        } else {
-            auto kern = mlstm_chunkwise_tc_kernel<128>;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<128>::TOTAL) != cudaSuccess)
-                return XLSTM_ERR_CUDA;
-            kern<<<grid, THREADS, Smem<128>::TOTAL, st>>>(tp);
-        }
-        return cudaGetLastError() == cudaSuccess ? XLSTM_OK : XLSTM_ERR_CUDA;
+    auto forward = [&](bool state_only) -> int {
+        if (p.dqk == 256) return state_only ? launch_tc<256, true>(tp, grid, st) : launch_tc<256, false>(tp, grid, st);
+        return state_only ? launch_tc<128, true>(tp, grid, st) : launch_tc<128, false>(tp, grid, st);
     };
-
     float *n_final = tail ? tail_n : p.n1, *m_final = tail ? tail_m : p.m1;
+    float *C_final = p.C1;
+
+    // the gate pre-pass (chain, path flags and per-token scalars for both passes of the segment-parallel mode), then the
+    // tensor-core kernel, whose CTAs read their path flag: the choice needs no host round trip
+    GateParams gp{};
+    gp.ig = p.ig; gp.fg = p.fg; gp.m0 = p.C0 ? p.m0 : nullptr;
+    gp.chain = chain; gp.gates = gates; gp.m_final = m_final; gp.decay = P > 1 ? decay : nullptr;
+    gp.path = path; gp.status = status;
+    for (int d = 0; d < 3; ++d) gp.sg[d] = p.sg[d];
+    gp.NH = p.NH; gp.NCH = nch; gp.P = P; gp.seg_tiles = seg_tiles; gp.general_only = g_general_only.load();
+    gp.qscale = p.qscale; gp.cap = p.gate_cap;
+    int rc = gate_prepass<__nv_bfloat16>(gp, BH, st);
+    if (rc != XLSTM_OK) return rc;
     if (P == 1) {
-        tp.C0 = p.C0; tp.n0 = p.n0; tp.C1 = p.C1; tp.n1 = n_final; tp.n_h = n_dest;
-        const int rc = forward(p.C0 ? p.m0 : nullptr, 0, m_final, false);
+        tp.C0 = p.C0; tp.n0 = p.n0; tp.C1 = C_final; tp.n1 = n_final; tp.n_h = n_dest;
+        rc = forward(false);
         if (rc != XLSTM_OK) return rc;
     } else {
-        // pass 1: every segment from an empty state -> its local end state: the state-only scan kernel (segments whose
-        // gates need the general kernel run that one in full, with nothing stored)
+        // pass 1: every segment from an empty state -> its local end state: the state-only scan (segments whose
+        // gates need the general path run that one in full, with nothing stored)
         tp.C0 = nullptr; tp.n0 = nullptr; tp.C1 = segA_C; tp.n1 = segA_n; tp.n_h = 0;
-        int rc = forward(nullptr, 1, segA_m, true);
+        rc = forward(true);
         if (rc != XLSTM_OK) return rc;
         // the true state at the start of every segment, and the final state
         const int slabs = (int)(((CE + p.dqk) / COMB_VEC + COMB_THREADS - 1) / COMB_THREADS);   // one vector per thread
-        mlstm_segment_combine_kernel<<<dim3(BH, slabs), COMB_THREADS, 0, st>>>(
-            p.C0, p.n0, p.C0 ? p.m0 : nullptr, segA_C, segA_n, segA_m, chain, segB_C, segB_n, segB_m, p.C1, n_final,
-            m_final, nch, P, seg_tiles, p.dqk, p.dv);
-        if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
+        rc = launch_overlapped(mlstm_segment_combine_kernel, dim3(BH, slabs), dim3(COMB_THREADS), 0, st, p.C0, p.n0,
+                               static_cast<const float *>(segA_C), static_cast<const float *>(segA_n),
+                               static_cast<const float *>(decay), segB_C, segB_n, C_final, n_final, P, p.dqk, p.dv);
+        if (rc != XLSTM_OK) return rc;
         // pass 2: every segment from its true start state
         tp.C0 = segB_C; tp.n0 = segB_n; tp.C1 = segA_C; tp.n1 = segA_n; tp.n_h = n_dest;
-        rc = forward(segB_m, 0, segA_m, false);
+        rc = forward(false);
         if (rc != XLSTM_OK) return rc;
     }
     if (!tail) return XLSTM_OK;

@@ -32,6 +32,7 @@
 // once P V~ has read it).
 // Every mbarrier wait is bounded; a time-out sets the status word in the scratch buffer, releases all roles
 // and frees TMEM before the CTA returns.
+#pragma once
 #include "mlstm_chunkwise_tc.cuh"
 
 namespace xl {
@@ -146,14 +147,13 @@ __device__ __forceinline__ float p_pass_part(uint32_t t_rows, int q, int lane, c
 }
 
 template <int DQK>
-__global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(const __grid_constant__ TcParams p) {
+__device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
     using SM = Smem<DQK>;
     constexpr int NBOX = SM::NBOX;
     constexpr int NHALF = DQK / 128;
     constexpr int F_UPDLAST = (NHALF == 2) ? F_UPDB : F_UPDA;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int bh = blockIdx.x;     // (batch, head, segment): index of the states and of the path flag
-    if (p.path[bh] != 1) return;   // these gates need the general kernel (CTA-uniform, before any set-up)
 
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + SM::BARS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + SM::MISC);
@@ -473,20 +473,5 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(con
 }
 
 }  // namespace
-
-int mlstm_chunkwise_tc_fast_launch(const tcw::TcParams &tp, dim3 grid, int dqk, cudaStream_t st) {
-    if (dqk == 256) {
-        auto kern = mlstm_chunkwise_tc_fast_kernel<256>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<256>::TOTAL) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
-        kern<<<grid, THREADS, Smem<256>::TOTAL, st>>>(tp);
-    } else {
-        auto kern = mlstm_chunkwise_tc_fast_kernel<128>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<128>::TOTAL) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
-        kern<<<grid, THREADS, Smem<128>::TOTAL, st>>>(tp);
-    }
-    return cudaGetLastError() == cudaSuccess ? XLSTM_OK : XLSTM_ERR_CUDA;
-}
 
 }  // namespace xl

@@ -13,6 +13,7 @@
 // V~ = diag(a) V in place, warps 8-11 n~ += K^T a, warps 12-15 / 16-19 the rows [0,128) / [128,256) of C~:
 // the occasional rescale in TMEM and, after the last tile, the fp32 state to global memory.
 // Every mbarrier wait is bounded; a time-out sets the status word, releases all roles and frees TMEM.
+#pragma once
 #include "mlstm_chunkwise_tc.cuh"
 
 namespace xl {
@@ -38,13 +39,12 @@ template <int DQK> struct ScanSmem {
 };
 
 template <int DQK>
-__global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_scan_kernel(const __grid_constant__ TcParams p) {
+__device__ __forceinline__ void chunkwise_state_scan(const TcParams &p) {
     using SM = ScanSmem<DQK>;
     constexpr int NBOX = SM::NBOX;
     constexpr int NHALF = DQK / 128;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int bh = blockIdx.x;     // (batch, head, segment)
-    if (p.path[bh] != 1) return;   // this segment's gates need the general kernel
 
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + SM::BARS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + SM::MISC);
@@ -203,20 +203,5 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_scan_kernel(con
 }
 
 }  // namespace
-
-int mlstm_chunkwise_tc_scan_launch(const tcw::TcParams &tp, dim3 grid, int dqk, cudaStream_t st) {
-    if (dqk == 256) {
-        auto kern = mlstm_chunkwise_tc_scan_kernel<256>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanSmem<256>::TOTAL) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
-        kern<<<grid, THREADS, ScanSmem<256>::TOTAL, st>>>(tp);
-    } else {
-        auto kern = mlstm_chunkwise_tc_scan_kernel<128>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanSmem<128>::TOTAL) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
-        kern<<<grid, THREADS, ScanSmem<128>::TOTAL, st>>>(tp);
-    }
-    return cudaGetLastError() == cudaSuccess ? XLSTM_OK : XLSTM_ERR_CUDA;
-}
 
 }  // namespace xl
