@@ -253,9 +253,53 @@ def test_linear_token_norm_and_swiglu(ops, M, F, K):
     assert relerr(host(act), host(sep)) <= BF16_TOL
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 4096, 4096), (5, 33, 64), (9, 264, 10944), (16, 31, 32), (1, 1, 288), (12, 50, 2080)])
+def test_linear_rows(ops, M, N, K):
+    """Rows around the 8-row halves of the x operand, weight rows and k blocks around a CTA's and a warp's share."""
+    rng = np.random.default_rng(M * 7 + N + K)
+    x = bf(rng.standard_normal((M, K)).astype(np.float32))
+    W = bf((rng.standard_normal((N, K)) * 0.05).astype(np.float32))
+    b = bf((rng.standard_normal(N) * 0.1).astype(np.float32))
+    r = bf(rng.standard_normal((M, N)).astype(np.float32))
+    t = torch.bfloat16
+    ref = xo.linear(x, W, b)
+    y = ops.linear_rows(dev(W, t), dev(x, t), bias=dev(b, t))
+    assert y.shape == (M, N) and relerr(host(y), ref) <= BF16_TOL
+    assert relerr(host(ops.linear_rows(dev(W, t), dev(x, t))), xo.linear(x, W)) <= BF16_TOL
+    yr = ops.linear_rows(dev(W, t), dev(x, t), bias=dev(b, t), residual=dev(r, t))
+    assert relerr(host(yr), bf(ref) + r) <= BF16_TOL
+    W2 = bf((rng.standard_normal((2 * N, K)) * 0.05).astype(np.float32))
+    act = ops.linear_rows(dev(W2, t), dev(x, t), swiglu_pair=True)
+    assert act.shape == (M, N)
+    assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
+
+
+@pytest.mark.parametrize("B", [2, 4, 5, 16, 17])
+def test_block_token_step_matches_separate_launches(ops, B):
+    """The single-token launch sequences of a block against the same block cell by cell, on a carried state."""
+    from xlstm_cuda.blocks import mLSTMBlock
+    t = torch.bfloat16
+    torch.manual_seed(B)
+    with torch.device("cuda"):
+        blk = mLSTMBlock(0, embedding_dim=512, num_heads=2, compute_dtype=t).to(t)
+    blk.fuse_projections()
+    x = torch.randn(B, 1, 512, device="cuda", dtype=t)
+    st = (torch.randn(B, 2, 128, 256, device="cuda") * 0.1, torch.randn(B, 2, 128, device="cuda") * 0.1, torch.zeros(B, 2, device="cuda"))
+    with torch.inference_mode():
+        y, s1 = blk(x, st)
+        out, s2 = blk.mlstm_cell(blk.norm_mlstm(x), st)
+        x1, xn = ops.add_rms_norm(x, out, blk.norm_ffn.weight, blk.norm_ffn.eps)
+        ref = x1 + blk.ffn_proj_down(ops.swiglu(blk.ffn_proj_up_gate(xn), blk.ffn_proj_up(xn)))
+    assert relerr(host(y), host(ref)) <= BF16_TOL
+    for a, b in zip(s1, s2):
+        assert relerr(host(a), host(b)) <= BF16_TOL
+
+
 def test_linear_token_rejects_what_it_does_not_do(ops):
     t = torch.bfloat16
     with pytest.raises(ValueError):
         ops.linear_token(torch.zeros(8, 16, device="cuda", dtype=t), torch.zeros(5, 16, device="cuda", dtype=t))
     with pytest.raises(TypeError):
         ops.linear_token(torch.zeros(8, 16, device="cuda"), torch.zeros(1, 16, device="cuda"))
+    with pytest.raises(ValueError):
+        ops.linear_rows(torch.zeros(8, 32, device="cuda", dtype=t), torch.zeros(17, 32, device="cuda", dtype=t))

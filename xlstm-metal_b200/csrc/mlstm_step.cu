@@ -30,6 +30,12 @@ struct StepGate {
     const void *norm_w;     // [NH*dv] or nullptr
     long long ogate_ld;
     float norm_eps;
+};
+
+// element distance between the sequences' rows of q, k, v and the gates: dense tensors, or column blocks of the merged
+// projection output as it stands (five copies of them took longer than the launch gap of the step)
+struct StepRows {
+    long long q, k, v, g;
     int NH;
 };
 
@@ -39,7 +45,7 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
                   const T *__restrict__ ig, const T *__restrict__ fg,
                   const float *C0, const float *__restrict__ n0, const float *__restrict__ m0,
                   T *__restrict__ h, float *C1, float *__restrict__ n1, float *__restrict__ m1,
-                  int dqk, int dv, float eps, float qscale, float gate_cap, int state_settled, StepGate gate) {
+                  int dqk, int dv, float eps, float qscale, float gate_cap, int state_settled, StepRows rows, StepGate gate) {
     constexpr int CV = DVT / 4;       // 128-bit column vectors per row of the tile
     constexpr int RG = THREADS / CV;  // row groups walking the rows in parallel
     extern __shared__ float smem[];
@@ -53,6 +59,7 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     const int tile = blockIdx.y;
     const int tid = threadIdx.x;
     const bool has_state = (C0 != nullptr);
+    const int seq = bh / rows.NH, head = bh - seq * rows.NH;
     const int cv = tid % CV, rg = tid / CV;
     const int col = tile * DVT + cv * 4;
     const bool active = col < dv;
@@ -81,18 +88,19 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     }
 
     // stabilised gates (every thread: two exps and a log1p are cheaper than a broadcast)
-    const float it = gate_softcap(Elem<T>::ld(ig + bh), gate_cap);
-    const float flog = logsigmoid(gate_softcap(Elem<T>::ld(fg + bh), gate_cap));
+    const float it = gate_softcap(Elem<T>::ld(ig + seq * rows.g + head), gate_cap);
+    const float flog = logsigmoid(gate_softcap(Elem<T>::ld(fg + seq * rows.g + head), gate_cap));
     const float mold = has_state ? m0[bh] : 0.0f;
     const float mnew = fmaxf(flog + mold, it);
     const float fgate = expf(flog + mold - mnew);
     const float igate = expf(it - mnew);
 
     // q~, gated k, normaliser update and q~ . n'
+    const T *qrow = q + seq * rows.q + (size_t)head * dqk, *krow = k + seq * rows.k + (size_t)head * dqk;
     float qn = 0.0f;
     for (int j = tid; j < dqk; j += THREADS) {
-        const float qj = Elem<T>::ld(q + (size_t)bh * dqk + j) * qscale;
-        const float kj = Elem<T>::ld(k + (size_t)bh * dqk + j);
+        const float qj = Elem<T>::ld(qrow + j) * qscale;
+        const float kj = Elem<T>::ld(krow + j);
         const float nj = fgate * (has_state ? n0[(size_t)bh * dqk + j] : 0.0f) + igate * kj;
         s_q[j] = qj;
         s_kw[j] = igate * kj;
@@ -112,7 +120,7 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
 
     float4 acc = zero4;
     if (active) {
-        const float4 v4 = ld4(v + (size_t)bh * dv + col);
+        const float4 v4 = ld4(v + seq * rows.v + (size_t)head * dv + col);
         for (int j0 = rg; j0 < dqk; j0 += RG * UNROLL) {
             // next batch goes out before this one is consumed
             float4 nx[UNROLL];
@@ -177,10 +185,9 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
             const unsigned nc = cluster.num_blocks();
             for (unsigned p = 0; p < nc; ++p) tot += cluster.map_shared_rank(s_ss, p)[0];
             const float inv = 1.0f / sqrtf(tot / (float)dv + gate.norm_eps);
-            const int b = bh / gate.NH, head = bh % gate.NH;
             const int c = tile * DVT + tid;
             const float w = gate.norm_w ? Elem<T>::ld(static_cast<const T *>(gate.norm_w) + (size_t)head * dv + c) : 1.0f;
-            const float og = Elem<T>::ld(static_cast<const T *>(gate.ogate) + (size_t)b * gate.ogate_ld + (size_t)head * dv + c);
+            const float og = Elem<T>::ld(static_cast<const T *>(gate.ogate) + (size_t)seq * gate.ogate_ld + (size_t)head * dv + c);
             Elem<T>::st(h + (size_t)bh * dv + c, hv * inv * w * gate_sigmoid<T>(og));
         }
         cluster.sync();                    // nobody leaves while a peer still reads its shared memory
@@ -191,7 +198,7 @@ template <typename T>
 static int mlstm_step_launch(const void *q, const void *k, const void *v, const void *ig, const void *fg,
                              const float *C0, const float *n0, const float *m0, void *h, float *C1, float *n1,
                              float *m1, int BH, int dqk, int dv, float eps, float gate_cap, int state_settled,
-                             const StepGate *gate, cudaStream_t st) {
+                             const StepRows &rows, const StepGate *gate, cudaStream_t st) {
     constexpr int DVT = STEP_DVT, THREADS = STEP_THREADS, UNROLL = STEP_UNROLL;
     dim3 grid(BH, (dv + DVT - 1) / DVT);
     size_t smem = sizeof(float) * (2 * (size_t)dqk + (THREADS / (DVT / 4)) * DVT);
@@ -205,7 +212,7 @@ static int mlstm_step_launch(const void *q, const void *k, const void *v, const 
         return launch_overlapped(kern, grid, dim3(THREADS), smem, st, static_cast<const T *>(q), static_cast<const T *>(k),
                                  static_cast<const T *>(v), static_cast<const T *>(ig), static_cast<const T *>(fg), C0, n0,
                                  m0, static_cast<T *>(h), C1, n1, m1, dqk, dv, eps, qscale, gate_cap, state_settled,
-                                 StepGate{});
+                                 rows, StepGate{});
     }
     // fused output epilogue: the column tiles of a head form one cluster (portable size: at most 8)
     if (grid.y > 8) return XLSTM_ERR_UNSUPPORTED;
@@ -229,7 +236,7 @@ static int mlstm_step_launch(const void *q, const void *k, const void *v, const 
     cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, kern, static_cast<const T *>(q), static_cast<const T *>(k), static_cast<const T *>(v),
                            static_cast<const T *>(ig), static_cast<const T *>(fg), C0, n0, m0, static_cast<T *>(h), C1, n1, m1,
-                           dqk, dv, eps, qscale, gate_cap, state_settled, *gate) != cudaSuccess)
+                           dqk, dv, eps, qscale, gate_cap, state_settled, rows, *gate) != cudaSuccess)
         return XLSTM_ERR_CUDA;
     return launch_status();
 }
@@ -239,7 +246,7 @@ static int mlstm_step_launch(const void *q, const void *k, const void *v, const 
 static int mlstm_step_checked(const void *q, const void *k, const void *v, const void *ig, const void *fg,
                               const float *C0, const float *n0, const float *m0, void *h, float *C1, float *n1,
                               float *m1, int B, int NH, int dqk, int dv, float eps, float gate_cap, int flags,
-                              const xl::StepGate *gate, int dtype, void *stream) {
+                              const xl::StepGate *gate, int dtype, void *stream, const int64_t *row_pitch = nullptr) {
     if (!q || !k || !v || !ig || !fg || !h || !C1 || !n1 || !m1) return XLSTM_ERR_INVALID;
     if (B <= 0 || NH <= 0 || dqk <= 0 || dv <= 0) return XLSTM_ERR_INVALID;
     if (C0 && (!n0 || !m0)) return XLSTM_ERR_INVALID;
@@ -249,12 +256,17 @@ static int mlstm_step_checked(const void *q, const void *k, const void *v, const
     if ((int64_t)B * NH > 2147483647LL || (dv + xl::STEP_DVT - 1) / xl::STEP_DVT > 65535) return XLSTM_ERR_UNSUPPORTED;
     if (flags & ~XLSTM_STEP_STATE_SETTLED) return XLSTM_ERR_INVALID;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    xl::StepRows rows{(long long)NH * dqk, (long long)NH * dqk, (long long)NH * dv, NH, NH};
+    if (row_pitch) {
+        rows.q = row_pitch[0]; rows.k = row_pitch[1]; rows.v = row_pitch[2]; rows.g = row_pitch[3];
+        if (rows.v % 4 || (reinterpret_cast<uintptr_t>(v) & (dtype == XLSTM_F32 ? 15u : 7u))) return XLSTM_ERR_UNSUPPORTED;
+    }
     const int settled = (flags & XLSTM_STEP_STATE_SETTLED) ? 1 : 0;
     if (dtype == XLSTM_F32)
         return xl::mlstm_step_launch<float>(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap,
-                                            settled, gate, st);
+                                            settled, rows, gate, st);
     return xl::mlstm_step_launch<__nv_bfloat16>(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap,
-                                                settled, gate, st);
+                                                settled, rows, gate, st);
 }
 
 extern "C" int xlstm_mlstm_step(const void *q, const void *k, const void *v, const void *ig, const void *fg,
@@ -277,18 +289,26 @@ extern "C" int xlstm_mlstm_step_ex(const void *q, const void *k, const void *v, 
     return mlstm_step_checked(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B, NH, dqk, dv, eps, gate_cap, flags, nullptr, dtype, stream);
 }
 
-extern "C" int xlstm_mlstm_step_gated(const void *q, const void *k, const void *v, const void *ig, const void *fg,
-                                      const float *C0, const float *n0, const float *m0, const void *ogate,
-                                      int64_t ogate_ld, const void *norm_w, float norm_eps, void *y, float *C1, float *n1,
-                                      float *m1, int B, int NH, int dqk, int dv, float eps, float gate_cap, int flags,
-                                      int dtype, void *stream) {
+extern "C" int xlstm_mlstm_step_gated_rows(const void *q, const void *k, const void *v, const void *ig, const void *fg,
+                                           const int64_t *row_pitch, const float *C0, const float *n0, const float *m0,
+                                           const void *ogate, int64_t ogate_ld, const void *norm_w, float norm_eps, void *y,
+                                           float *C1, float *n1, float *m1, int B, int NH, int dqk, int dv, float eps,
+                                           float gate_cap, int flags, int dtype, void *stream) {
     if (!ogate || ogate_ld < (int64_t)NH * dv) return XLSTM_ERR_INVALID;
     xl::StepGate g;
     g.ogate = ogate;
     g.norm_w = norm_w;
     g.ogate_ld = ogate_ld;
     g.norm_eps = norm_eps;
-    g.NH = NH;
     return mlstm_step_checked(q, k, v, ig, fg, C0, n0, m0, y, C1, n1, m1, B, NH, dqk, dv, eps, gate_cap, flags, &g, dtype,
-                              stream);
+                              stream, row_pitch);
+}
+
+extern "C" int xlstm_mlstm_step_gated(const void *q, const void *k, const void *v, const void *ig, const void *fg,
+                                      const float *C0, const float *n0, const float *m0, const void *ogate,
+                                      int64_t ogate_ld, const void *norm_w, float norm_eps, void *y, float *C1, float *n1,
+                                      float *m1, int B, int NH, int dqk, int dv, float eps, float gate_cap, int flags,
+                                      int dtype, void *stream) {
+    return xlstm_mlstm_step_gated_rows(q, k, v, ig, fg, nullptr, C0, n0, m0, ogate, ogate_ld, norm_w, norm_eps, y, C1, n1, m1, B,
+                                       NH, dqk, dv, eps, gate_cap, flags, dtype, stream);
 }

@@ -45,6 +45,9 @@ _SIGNATURES = {
                             + [c_float, c_float, c_int, c_int, c_void_p]),
     "xlstm_mlstm_step_gated": (c_int, [c_void_p] * 5 + [c_void_p] * 3 + [c_void_p, c_int64, c_void_p, c_float]
                                + [c_void_p] * 4 + [c_int] * 4 + [c_float, c_float, c_int, c_int, c_void_p]),
+    "xlstm_mlstm_step_gated_rows": (c_int, [c_void_p] * 5 + [ctypes.POINTER(c_int64)] + [c_void_p] * 3
+                                    + [c_void_p, c_int64, c_void_p, c_float] + [c_void_p] * 4 + [c_int] * 4
+                                    + [c_float, c_float, c_int, c_int, c_void_p]),
     "xlstm_mlstm_chunkwise_fwd_gatecap": (c_int, [c_void_p] * 5 + [c_void_p] * 3 + [c_void_p] * 4 + [c_int] * 6
                                           + [c_float, c_float, c_int, ctypes.POINTER(c_int64), c_void_p, c_size_t, c_void_p]),
     "xlstm_rms_norm": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_float, c_int, c_void_p]),
@@ -52,6 +55,7 @@ _SIGNATURES = {
     "xlstm_mlstm_output_gate": (c_int, [c_void_p] * 4 + [c_int] * 4 + [ctypes.POINTER(c_int64), c_int64, c_float, c_int, c_void_p]),
     "xlstm_swiglu": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_int64, c_int, c_void_p]),
     "xlstm_linear_token": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
+    "xlstm_linear_rows": (c_int, [c_void_p] * 5 + [c_int] * 5 + [c_void_p]),
     "xlstm_causal_conv1d": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_void_p]),
 }
 

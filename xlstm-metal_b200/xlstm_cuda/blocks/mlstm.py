@@ -351,17 +351,26 @@ class mLSTMBlock(nn.Module):
         self.state_dtype = state_dtype
 
     def _token_step(self, x: torch.Tensor, state: Optional[State]):
-        """Single-token path (at most 4 sequences, bf16, fused weights): every Linear is one
-        weight-streaming kernel with its norm / bias / residual / SwiGLU folded in, so a block is five
-        launches: projections, cell step with the output epilogue, out-projection, FFN up, FFN down."""
+        """Single-token path (bf16, fused weights).  Up to 4 sequences every Linear is one weight-streaming kernel with
+        its norm / bias / residual / SwiGLU folded in, so a block is five launches: projections, cell step with the
+        output epilogue, out-projection, FFN up, FFN down.  Up to 16 the streaming kernel multiplies on the tensor cores
+        and the two norms are launches of their own; beyond that the Linears are GEMMs.  The cell step reads q, k, v and
+        the gates where the merged projection has written them."""
         cell = self.mlstm_cell
         W, b = cell._fused_weights()
         B = x.shape[0]
         NH, dqk, dv = cell.num_heads, cell.qk_dim_per_head, cell.v_dim_per_head
         x2 = x.reshape(B, -1)
-        y = ops.linear_token(W, x2, bias=b, norm_weight=self.norm_mlstm.weight, norm_eps=self.norm_mlstm.eps)
+        few = B <= ops.LINEAR_TOKEN_MAX_ROWS
+        rows = not few and B <= ops.LINEAR_ROWS_MAX and self._rows_ok()
+        if few:
+            y = ops.linear_token(W, x2, bias=b, norm_weight=self.norm_mlstm.weight, norm_eps=self.norm_mlstm.eps)
+        else:
+            xn = self.norm_mlstm(x2)
+            y = ops.linear_rows(W, xn, bias=b) if rows else F.linear(xn, W, b)
         o_k, o_v, o_g, o_o = NH * dqk, 2 * NH * dqk, 2 * NH * dqk + NH * dv, 2 * NH * dqk + NH * dv + 2 * NH
-        q, k, v = y[:, :o_k].view(B, NH, dqk), y[:, o_k:o_v].view(B, NH, dqk), y[:, o_v:o_g].view(B, NH, dv)
+        heads = lambda lo, hi, d: y[:, lo:hi].unflatten(1, (NH, d))
+        q, k, v = heads(0, o_k, dqk), heads(o_k, o_v, dqk), heads(o_v, o_g, dv)
         rk = cell.recurrent_kernel
         oc = cell.output_cell
         if dv <= 512 and dv % 4 == 0:
@@ -375,11 +384,24 @@ class mLSTMBlock(nn.Module):
                                           inplace=rk.inplace_state, gate_cap=cell.projection_cell.gate_soft_cap,
                                           state_settled=True)
             gated = ops.mlstm_output_gate(h.unsqueeze(2), y[:, o_o:].unsqueeze(1), oc.norm.weight, oc.norm.eps)
-        x1 = ops.linear_token(oc.out_proj.weight, gated.reshape(B, -1), bias=oc.out_proj.bias, residual=x2)
-        act = ops.linear_token(self._fused_ffn(), x1, norm_weight=self.norm_ffn.weight, norm_eps=self.norm_ffn.eps,
-                               swiglu_pair=True)
-        x3 = ops.linear_token(self.ffn_proj_down.weight, act, bias=self.ffn_proj_down.bias, residual=x1)
+        gated = gated.reshape(B, -1)
+        ffn, down = self._fused_ffn(), self.ffn_proj_down
+        if few:
+            x1 = ops.linear_token(oc.out_proj.weight, gated, bias=oc.out_proj.bias, residual=x2)
+            act = ops.linear_token(ffn, x1, norm_weight=self.norm_ffn.weight, norm_eps=self.norm_ffn.eps, swiglu_pair=True)
+            x3 = ops.linear_token(down.weight, act, bias=down.bias, residual=x1)
+        elif rows:
+            x1 = ops.linear_rows(oc.out_proj.weight, gated, bias=oc.out_proj.bias, residual=x2)
+            act = ops.linear_rows(ffn, self.norm_ffn(x1), swiglu_pair=True)
+            x3 = ops.linear_rows(down.weight, act, bias=down.bias, residual=x1)
+        else:
+            x1, xn = ops.add_rms_norm(x2, oc.out_proj(gated), self.norm_ffn.weight, self.norm_ffn.eps)
+            up = F.linear(xn, ffn)
+            x3 = x1 + down(ops.swiglu(up[:, :self.ffn_hidden_dim], up[:, self.ffn_hidden_dim:]))
         return x3.view_as(x), rk._cast_state(new_state)
+
+    def _rows_ok(self) -> bool:
+        return all(K % 32 == 0 for K in (self.embedding_dim, self.hidden_size, self.ffn_hidden_dim))
 
     def shard_heads(self, rank: int, world: int, group=None) -> None:
         """Head-sharded mLSTM layer (see ``mLSTMNeuron.shard_heads``); norms and the FFN stay replicated."""
@@ -392,7 +414,7 @@ class mLSTMBlock(nn.Module):
     def _token_step_ok(self, x: torch.Tensor) -> bool:
         if getattr(self.mlstm_cell, "_shard", None) is not None:
             return False   # the single-token launch sequence has no gather step
-        return (x.shape[1] == 1 and x.shape[0] <= ops.LINEAR_TOKEN_MAX_ROWS and x.dtype == torch.bfloat16 and
+        return (x.shape[1] == 1 and x.dtype == torch.bfloat16 and
                 self.mlstm_cell._fused_weights() is not None and self._fused_ffn() is not None and
                 self.mlstm_cell.compute_dtype == torch.bfloat16)
 

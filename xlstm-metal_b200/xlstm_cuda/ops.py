@@ -87,6 +87,10 @@ def mlstm_step(q, k, v, i, f, state=None, eps: float = 1e-6, inplace: bool = Fal
     return h, (C1, n1, m1)
 
 
+def _dense_heads(t: torch.Tensor) -> bool:
+    return t.stride(2) == 1 and (t.shape[1] == 1 or t.stride(1) == t.shape[2])
+
+
 def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float = 1e-6, norm_eps: float = 1e-6,
                      inplace: bool = False, gate_cap: Optional[float] = None, state_settled: bool = False):
     """Decode step with the output epilogue fused in: returns ``y [B, NH*dv] = MultiHeadRMSNorm(h) * weight *
@@ -96,8 +100,12 @@ def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float =
     B, NH, dqk = q.shape
     dv = v.shape[-1]
     dt = _dtype_code(q)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    i, f = i.to(q.dtype).contiguous(), f.to(q.dtype).contiguous()
+    i, f = i.to(q.dtype), f.to(q.dtype)
+    if not (_dense_heads(q) and _dense_heads(k) and _dense_heads(v) and i.stride(1) == f.stride(1) == 1 and
+            (B == 1 or i.stride(0) == f.stride(0)) and (B == 1 or v.stride(0) % 4 == 0) and
+            v.data_ptr() % (4 * v.element_size()) == 0):
+        q, k, v, i, f = q.contiguous(), k.contiguous(), v.contiguous(), i.contiguous(), f.contiguous()
+    pitch = (ctypes.c_int64 * 4)(*((0, 0, 0, 0) if B == 1 else (q.stride(0), k.stride(0), v.stride(0), i.stride(0))))
     og = ogate.to(q.dtype)
     if og.dim() != 2 or og.stride(1) != 1 or og.shape[1] != NH * dv:
         og = og.reshape(B, NH * dv).contiguous()
@@ -116,11 +124,11 @@ def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float =
     n1 = torch.empty(B, NH, dqk, dtype=torch.float32, device=dev)
     m1 = torch.empty(B, NH, dtype=torch.float32, device=dev)
     flags = _lib.STEP_STATE_SETTLED if (state_settled and state is not None) else 0
-    _lib.check(_lib.load().xlstm_mlstm_step_gated(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), _ptr(C0), _ptr(n0), _ptr(m0),
+    _lib.check(_lib.load().xlstm_mlstm_step_gated_rows(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, _ptr(C0), _ptr(n0), _ptr(m0),
         og.data_ptr(), int(ld), _ptr(w), float(norm_eps), y.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(),
         B, NH, dqk, dv, float(eps), float(gate_cap) if gate_cap is not None else 0.0, flags, dt, _stream()),
-        "xlstm_mlstm_step_gated")
+        "xlstm_mlstm_step_gated_rows")
     return y, (C1, n1, m1)
 
 
@@ -432,4 +440,29 @@ def linear_token(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Ten
     epi = 2 if swiglu_pair else (1 if r is not None else 0)
     _lib.check(_lib.load().xlstm_linear_token(w.data_ptr(), x2.data_ptr(), _ptr(b), _ptr(nw), float(norm_eps), _ptr(r),
                                               y.data_ptr(), M, N, K, epi, _lib.BF16, _stream()), "xlstm_linear_token")
+    return y
+
+
+LINEAR_ROWS_MAX = 16
+
+
+def linear_rows(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                residual: Optional[torch.Tensor] = None, swiglu_pair: bool = False) -> torch.Tensor:
+    """The same for up to 16 token rows (bf16, ``K`` a multiple of 32), without the norm."""
+    _need_cuda(weight, x, bias, residual)
+    if weight.dtype != torch.bfloat16:
+        raise TypeError("linear_rows is a bf16 kernel")
+    K = x.shape[-1]
+    x2 = x.reshape(-1, K).to(torch.bfloat16).contiguous()
+    M = x2.shape[0]
+    if M > LINEAR_ROWS_MAX:
+        raise ValueError(f"linear_rows takes at most {LINEAR_ROWS_MAX} rows, got {M}")
+    w = weight if weight.is_contiguous() else weight.contiguous()
+    N = w.shape[0] // 2 if swiglu_pair else w.shape[0]
+    b = None if bias is None else bias.to(torch.bfloat16).contiguous()
+    r = None if residual is None else residual.reshape(-1, N).to(torch.bfloat16).contiguous()
+    y = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=x.device)
+    epi = 2 if swiglu_pair else (1 if r is not None else 0)
+    _lib.check(_lib.load().xlstm_linear_rows(w.data_ptr(), x2.data_ptr(), _ptr(b), _ptr(r), y.data_ptr(), M, N, K, epi,
+                                             _lib.BF16, _stream()), "xlstm_linear_rows")
     return y
