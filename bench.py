@@ -408,7 +408,7 @@ def run_ours(args):
             "gather_check": prefill["gather_check"], "gather_gbs_per_rank": prefill["gather_gbs_per_rank"],
             "token_sharded_outproj_ms": prefill["token_sharded_outproj_ms"], "token_sharded_check": prefill["token_sharded_check"],
             "workload": f"B=4 S={args.prefill_seq} NH=8 256/512 bf16 (BASELINE configs[3]), heads x{world}",
-            "kernel": "mlstm_chunkwise_tc_fast_kernel", "bound": "tensor"}
+            "kernel": "mlstm_chunkwise_tc_kernel", "bound": "tensor"}
         details["prefill"] = prefill
     launches = K
     if not args.no_extras:

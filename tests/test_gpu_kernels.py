@@ -601,8 +601,8 @@ BF, FP = torch.bfloat16, torch.float32
                                              (1, 1, 1, 256, FP), (4, 2, 2, 128, FP), (5, 3, 2, 64, FP), (33, 40, 4, 256, FP),
                                              (70, 5, 4, 128, FP), (140, 4, 4, 64, FP)])
 def test_slstm_recurrent_edges(ops, B, S, NH, dh, dtype):
-    """One, two and three steps (each h buffer unused, used once, reused), rows around the groups of a cluster (16 in bf16;
-    4, or 8 when many, in fp32), a carried state.  bf16 heads of 64 and 128 feed h back unrounded and use the exact exponentials: their states stay within
+    """One, two and three steps (each h buffer unused, used once, reused), rows around the groups of a cluster (16 in bf16,
+    4 in fp32), a carried state.  bf16 heads of 64 and 128 feed h back unrounded and use the exact exponentials: their states stay within
     the fp32 tolerance and their outputs within half a bf16 ulp (8 significant bits: 2^-8 of the value) of it."""
     rng = np.random.default_rng(dh + B)
     rd = xo.bf16_round if dtype == BF else (lambda a: a)

@@ -53,16 +53,20 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
 #pragma unroll
     for (int r = 0; r < 2; ++r) xp[r] = x + (size_t)min(r * 8 + g, M - 1) * K + c * 8;
 
-    uint4 wr[LR_U][4];
-    auto load_w = [&](int b0) {
+    // a ring of LR_U k blocks: slot u is refilled as soon as its block has been multiplied
+    uint4 wr[LR_U][4], xr[LR_U][2];
+    auto load_w = [&](int u, int b) {
+        b = min(b, blocks - 1);
 #pragma unroll
-        for (int u = 0; u < LR_U; ++u) {
-            const int b = min(b0 + u * LR_WARPS, blocks - 1);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) wr[u][r] = ldg_weights(wp[r] + (size_t)b * 32);
-        }
+        for (int r = 0; r < 4; ++r) wr[u][r] = ldg_weights(wp[r] + (size_t)b * 32);
     };
-    load_w(warp);
+    auto load_x = [&](int u, int b) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            xr[u][r] = b < blocks ? *reinterpret_cast<const uint4 *>(xp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
+    };
+#pragma unroll
+    for (int u = 0; u < LR_U; ++u) load_w(u, warp + u * LR_WARPS);
     grid_dependency_wait();
     allow_dependents();
 
@@ -73,17 +77,11 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[t][n][e] = 0.f;
+#pragma unroll
+    for (int u = 0; u < LR_U; ++u) load_x(u, warp + u * LR_WARPS);
     for (int b0 = warp; b0 < blocks; b0 += LR_U * LR_WARPS) {
-        uint4 xr[LR_U][2];
 #pragma unroll
         for (int u = 0; u < LR_U; ++u) {
-            const int b = b0 + u * LR_WARPS;
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-                xr[u][r] = b < blocks ? *reinterpret_cast<const uint4 *>(xp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int u = 0; u < LR_U; ++u)
 #pragma unroll
             for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -91,7 +89,9 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
                     mma_bf16(acc[t][n], wr[u][2 * t].x, wr[u][2 * t + 1].x, wr[u][2 * t].y, wr[u][2 * t + 1].y, xr[u][n].x, xr[u][n].y);
                     mma_bf16(acc[t][n], wr[u][2 * t].z, wr[u][2 * t + 1].z, wr[u][2 * t].w, wr[u][2 * t + 1].w, xr[u][n].z, xr[u][n].w);
                 }
-        if (b0 + LR_U * LR_WARPS < blocks) load_w(b0 + LR_U * LR_WARPS);
+            const int b = b0 + (u + LR_U) * LR_WARPS;
+            if (b0 + LR_U * LR_WARPS < blocks) { load_w(u, b); load_x(u, b); }
+        }
     }
     // element e of a tile: weight row g + 8 (e / 2), x row 2c + (e & 1)
 #pragma unroll

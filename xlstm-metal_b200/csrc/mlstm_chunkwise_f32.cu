@@ -88,13 +88,22 @@ __device__ __forceinline__ GateTile gate_tile(const ChunkwiseParams &p, int bb, 
     return g;
 }
 
+// 16 bytes global -> shared memory, zeros if not ok; arrives by cp_async_wait_all() in the issuing thread
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(ok ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <typename T> __device__ __forceinline__ float4 ld4_or_zero(const T *ptr, bool ok) {
     return ok ? ld4(ptr) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// Two CTAs per SM: a scheduler's 16 K registers hold three of the ten warps only up to 168 registers a thread (with 182 it
+// was one CTA, 1.25 warps per scheduler, 30 % of the FMA issue slots).
 template <typename T, int CT>
-__global__ void __launch_bounds__(MAIN + 32) mlstm_f32_state_kernel(const F32Params P) {
+__global__ void __launch_bounds__(MAIN + 32, 2) mlstm_f32_state_kernel(const F32Params P) {
     constexpr int NG = CT / 64;                       // groups of 4 columns per thread
     constexpr int KV = TT * JT / 4 / MAIN, VV = TT * CT / 4 / MAIN;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -107,6 +116,8 @@ __global__ void __launch_bounds__(MAIN + 32) mlstm_f32_state_kernel(const F32Par
     const int j0 = blockIdx.y * JT, col0 = blockIdx.z * CT;
     const int t_begin = P.c_begin * CH, t_end = min(p.S, P.c_end * CH);
     const int tiles = (t_end - t_begin + TT - 1) / TT;
+    grid_dependency_wait();
+    allow_dependents();
 
     if (tid >= MAIN) {
         // ---- gate warp: weights two tiles ahead, stabiliser chain, normaliser (first column tile only)
@@ -223,6 +234,7 @@ __global__ void __launch_bounds__(MAIN + 32) mlstm_f32_state_kernel(const F32Par
     load(0);
     __syncthreads();
     store(0);
+    cp_async_wait_all();
     __syncthreads();
     for (int k = 0; k < tiles; ++k) {
         if (k + 1 < tiles) load(k + 1);
@@ -266,14 +278,18 @@ template <int DVT> struct OutSmem {
     static constexpr uint32_t K = Q + 2 * KP * CH * 8;                 // float  [2][KP][CH]  transposed
     static constexpr uint32_t C = K + 2 * KP * CH * 4;                 // float  [2][KP][DVT]
     static constexpr uint32_t V = C + 2 * KP * DVT * 4;                // float  [CH][DVT]
-    static constexpr uint32_t PM = V + CH * DVT * 4;                   // float2 [CH s][CH t] (P, P), 16-byte units swizzled
-    static constexpr uint32_t U = PM + CH * CH * 8;                    // double [CH] u, [CH] x
+    static constexpr uint32_t PM = Q;                                  // float2 [CH s][CH t] (P, P), 16-byte units swizzled:
+                                                                       // over Q, K and C, which the last piece leaves free
+    static constexpr uint32_t U = V + CH * DVT * 4;                    // double [CH] u, [CH] x
     static constexpr uint32_t WIN = U + 2 * CH * 8;                    // float [CH] e^{m - x_t}, [CH] e^{-m_t}, [2][CH] q.n, [CH] row sums
     static constexpr uint32_t TOTAL = WIN + 5 * CH * 4;
+    static_assert(CH * CH * 8 <= V, "P fits the buffers it replaces");
 };
 
+// 128 columns: three CTAs per SM (77 KB each); with two, 1.84 warps per scheduler left 60 % of the FMA issue slots to
+// latency.  64 columns are taken for grids that do not fill the GPU, where a CTA has the registers to itself.
 template <typename T, int DVT>
-__global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Params P) {
+__global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_kernel(const F32Params P) {
     using SM = OutSmem<DVT>;
     constexpr int NG = DVT / 64;
     constexpr int QV = KP * CH / 4 / MAIN, CV = KP * DVT / 4 / MAIN;
@@ -296,8 +312,8 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
     const T *kb = static_cast<const T *>(p.k) + b * p.sk[0] + hd * p.sk[1] + (int64_t)t0 * p.sk[2];
     const T *vb = static_cast<const T *>(p.v) + b * p.sv[0] + hd * p.sv[1] + (int64_t)t0 * p.sv[2] + col0;
 
-    float4 qr[QV], kr[QV], cr[CV];
-    auto load = [&](int j0) {
+    float4 qr[QV], kr[QV];
+    auto load_qk = [&](int j0) {
 #pragma unroll
         for (int i = 0; i < QV; ++i) {                       // lane = token: the transposed stores are conflict-free
             const int e = tid + i * MAIN, t = e % CH, j = j0 + (e / CH) * 4;
@@ -305,11 +321,14 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
             qr[i] = ld4_or_zero(qb + (int64_t)t * p.sq[2] + j, ok);
             kr[i] = ld4_or_zero(kb + (int64_t)t * p.sk[2] + j, ok);
         }
+    };
+    auto load_c = [&](int j0, int buf) {                     // straight into shared memory
         if (has_C) {
 #pragma unroll
             for (int i = 0; i < CV; ++i) {
                 const int e = tid + i * MAIN, j = j0 + e / (DVT / 4), cc = (e % (DVT / 4)) * 4;
-                cr[i] = ld4_or_zero(Cs + (size_t)j * p.dv + col0 + cc, j < p.dqk && col0 + cc < p.dv);
+                const bool ok = j < p.dqk && col0 + cc < p.dv;
+                cp_async16(reinterpret_cast<float4 *>(sC + buf * KP * DVT) + e, Cs + (ok ? (size_t)j * p.dv + col0 + cc : 0), ok);
             }
         }
     };
@@ -323,12 +342,24 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
             dq[2 * CH] = make_float2(qr[i].z, qr[i].z); dq[3 * CH] = make_float2(qr[i].w, qr[i].w);
             dk[0] = kr[i].x; dk[CH] = kr[i].y; dk[2 * CH] = kr[i].z; dk[3 * CH] = kr[i].w;
         }
-        if (has_C) {
-#pragma unroll
-            for (int i = 0; i < CV; ++i) reinterpret_cast<float4 *>(sC + buf * KP * DVT)[tid + i * MAIN] = cr[i];
-        }
     };
-    load(0);
+    // The kernel before this one (state) has waited for its own predecessor before it let this one start, so the inputs are
+    // there; what it writes itself (C, n, m) is read after the wait.  A single chunk starts from the caller's state and
+    // needs nothing of it: the two kernels then run side by side, and one CTA waits at the end, so that this launch is
+    // complete only when that one is.
+    const bool single = P.m_all == nullptr;
+    load_qk(0);
+    // V of the chunk: needed after the last piece
+#pragma unroll 4
+    for (int e = tid; e < CH * DVT / 4; e += MAIN) {
+        const int t = e / (DVT / 4), cc = (e % (DVT / 4)) * 4;
+        reinterpret_cast<float4 *>(sV)[e] = ld4_or_zero(vb + (int64_t)t * p.sv[2] + cc, t0 + t < p.S && col0 + cc < p.dv);
+    }
+    if (!single) {
+        grid_dependency_wait();
+        allow_dependents();
+    }
+    load_c(0, 0);
     if (tid < 32) {
         const float m = P.m_all ? P.m_all[(size_t)bh * (P.NC + 1) + c] : (P.m0 ? P.m0[bh] : 0.f);
         double bsum = 0.0, mx = (double)m;
@@ -345,12 +376,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
         }
     }
     store(0);
-    // V of the chunk: needed after the last piece
-#pragma unroll 4
-    for (int e = tid; e < CH * DVT / 4; e += MAIN) {
-        const int t = e / (DVT / 4), cc = (e % (DVT / 4)) * 4;
-        reinterpret_cast<float4 *>(sV)[e] = ld4_or_zero(vb + (int64_t)t * p.sv[2] + cc, t0 + t < p.S && col0 + cc < p.dv);
-    }
+    cp_async_wait_all();
     __syncthreads();
 
     u64 accS[8][2], accH[8][2 * NG];
@@ -365,7 +391,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
     const int pieces = (p.dqk + KP - 1) / KP;
     for (int pc = 0; pc < pieces; ++pc) {
         const int buf = pc & 1;
-        if (pc + 1 < pieces) load((pc + 1) * KP);
+        if (pc + 1 < pieces) { load_qk((pc + 1) * KP); load_c((pc + 1) * KP, buf ^ 1); }
         const float2 *qa = sQ + buf * KP * CH + ty * 8;
         const float *ka = sK + buf * KP * CH + tx * 4;
         const float *ca = sC + buf * KP * DVT + tx * 4;
@@ -414,6 +440,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
             }
         }
         if (pc + 1 < pieces) store(buf ^ 1);
+        cp_async_wait_all();
         __syncthreads();
     }
     sQn[nh * CH + nt] = qn;
@@ -479,7 +506,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int t = ty * 8 + r;
-        if (t0 + t >= p.S) break;
+        if (t0 + t >= p.S) break;   // the later rows are beyond the end too
         const float den = sWin[t] * qs * (sQn[t] + sQn[CH + t]) + sRow[t];
         const float inv = 1.0f / (fmaxf(fabsf(den), sEmt[t]) + p.eps);
 #pragma unroll
@@ -491,6 +518,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
             }
         }
     }
+    if (single && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) grid_dependency_wait();
 }
 
 template <typename T> int run_group(const F32Params &P, cudaStream_t st) {
@@ -506,10 +534,9 @@ template <typename T> int run_group(const F32Params &P, cudaStream_t st) {
     if (cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s) != cudaSuccess ||
         cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_o) != cudaSuccess)
         return XLSTM_ERR_CUDA;
-    ks<<<dim3(BH, jt, (p.dv + cs - 1) / cs), MAIN + 32, sm_s, st>>>(P);
-    if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
-    ko<<<dim3(chunks, (p.dv + co - 1) / co, BH), MAIN, sm_o, st>>>(P);
-    return launch_status();
+    const int rc = launch_overlapped(ks, dim3(BH, jt, (p.dv + cs - 1) / cs), dim3(MAIN + 32), sm_s, st, P);
+    if (rc != XLSTM_OK) return rc;
+    return launch_overlapped(ko, dim3(chunks, (p.dv + co - 1) / co, BH), dim3(MAIN), sm_o, st, P);
 }
 
 int group_chunks(int BH, int S, int dqk, int dv) {

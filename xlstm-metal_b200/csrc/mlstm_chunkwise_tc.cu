@@ -747,24 +747,39 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     if (tid == 0 && *abort_flag) atomicExch(p.status, 1);
 }
 
-// One launch for all (head, segment)s: a CTA takes the path that the gate pre-pass has found for its gates.  Heads of
-// both kinds run side by side (two launches, each with half of the CTAs returning at once, ran them one after the
-// other).  STATE_ONLY: the first pass of the segment-parallel mode, where the bounded path needs no h.
-template <int DQK, bool STATE_ONLY>
+// Two launches over the same (head, segment)s, for the gates of either kind; the choice is the pre-pass's path flag, so it
+// needs no host round trip, and a CTA of the other kind returns at once.  They run side by side: the general launch lets
+// the second one start as soon as its own CTAs have, and that one reads nothing the first has written, so the CTAs of both
+// kinds share the GPU (one after the other, heads with widely spread gates took twice as long).  One kernel with both bodies
+// made the bounded path spill (prefill of 4 x 32768: 1.61 -> 1.71 ms).
+template <int DQK>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
     grid_dependency_wait();
+    allow_dependents();
     if (p.path[blockIdx.x] == 0) chunkwise_general<DQK>(p);
-    else if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
-    else chunkwise_bounded<DQK>(p);
+}
+// STATE_ONLY: the first pass of the segment-parallel mode, where the bounded path needs no h.
+// The wait for the general launch comes last, in one CTA: this launch is complete only when that one is.
+template <int DQK, bool STATE_ONLY>
+__global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(const __grid_constant__ TcParams p) {
+    if (p.path[blockIdx.x] != 0) {
+        if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
+        else chunkwise_bounded<DQK>(p);
+    }
+    if (blockIdx.x == 0 && blockIdx.y == 0) grid_dependency_wait();
 }
 
 template <int DQK, bool STATE_ONLY>
 int launch_tc(const TcParams &tp, dim3 grid, cudaStream_t st) {
-    constexpr uint32_t bytes = STATE_ONLY && ScanSmem<DQK>::TOTAL > Smem<DQK>::TOTAL ? ScanSmem<DQK>::TOTAL : Smem<DQK>::TOTAL;
-    auto kern = mlstm_chunkwise_tc_kernel<DQK, STATE_ONLY>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    constexpr uint32_t bytes = STATE_ONLY ? ScanSmem<DQK>::TOTAL : Smem<DQK>::TOTAL;
+    auto general = mlstm_chunkwise_tc_kernel<DQK>;
+    auto fast = mlstm_chunkwise_tc_fast_kernel<DQK, STATE_ONLY>;
+    if (cudaFuncSetAttribute(general, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<DQK>::TOTAL) != cudaSuccess ||
+        cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return XLSTM_ERR_CUDA;
-    return launch_overlapped(kern, grid, dim3(THREADS), bytes, st, tp);
+    const int rc = launch_overlapped(general, grid, dim3(THREADS), Smem<DQK>::TOTAL, st, tp);
+    if (rc != XLSTM_OK) return rc;
+    return launch_overlapped(fast, grid, dim3(THREADS), bytes, st, tp);
 }
 
 }  // namespace
@@ -798,20 +813,27 @@ struct WsLayout {
 };
 
 constexpr int SM_COUNT = 148;          // B200
-constexpr int MIN_SEG_TILES = 16;      // a shorter segment is dominated by its prologue (state in) and epilogue (state out)
+constexpr int MIN_SEG_TILES = 2;
 
-// Number of segments every sequence is cut into: while the grid of persistent CTAs (one per head and 128 dv
-// columns) fills at most half of the SMs, cutting the sequence buys parallelism at the price of the state-only
-// first pass (about a quarter of a full pass) and of the states going through HBM once.
+// Number of segments every sequence is cut into.  Cutting buys parallelism while the grid of persistent CTAs (one per head
+// and 128 dv columns) leaves SMs idle, at the price of the state-only first pass, of the states going through HBM and of
+// three more launches.  Microseconds fitted to forced segment counts at 256/512, 8 to 128 CTAs, 2 to 32 tiles a segment:
+//   one pass    13 + tiles x (4.55 up to 32 CTAs, 5.3 at 64, 6.75 at 128)
+//   two passes  35 + tiles of a segment x (7.1 at 64 CTAs, 9 at 128)
+// e.g. 8 heads, S = 2048: 85 us in one pass, 72 in 4 segments; S = 4096: 167 and 109; 2 heads, S = 8192: 283, 127 in 4
+// segments and 72 in 16; 8 heads, S = 1024: 51 and 54.  128/256 follows the same order (S = 8192, 4 heads: 250 and 51).
 int plan_segments(int BH, int dv, int nch) {
     const int ctas = BH * (dv / DVS);
-    int P = SM_COUNT / ctas;
-    if (P > nch / MIN_SEG_TILES) P = nch / MIN_SEG_TILES;
-    if (P > 64) P = 64;
-    if (P < 2) return 1;
-    for (int d = P; 4 * d >= 3 * P; --d)      // segments of equal length, if a count close to P divides the tiles
-        if (nch % d == 0) return d;
-    return P;
+    int pmax = SM_COUNT / ctas;
+    if (pmax > nch / MIN_SEG_TILES) pmax = nch / MIN_SEG_TILES;
+    if (pmax > 64) pmax = 64;
+    int best = 1;
+    float best_us = 13.0f + nch * (ctas <= 32 ? 4.55f : 3.9f + 0.022f * ctas);
+    for (int P = 2; P <= pmax; ++P) {
+        const float us = 35.0f + ((nch + P - 1) / P) * (5.2f + 0.03f * ctas * P);
+        if (us < best_us) { best_us = us; best = P; }
+    }
+    return best;
 }
 
 // tail: tokens after the last whole tile that get the state and scratch of the fp32 kernels (0: none, or in place)

@@ -20,6 +20,7 @@ typedef unsigned long long u64;
 constexpr int GU = 32;                 // units per CTA
 constexpr int GCOL = 4 * GU;           // gate columns per CTA
 constexpr int GK = 64;                 // k's per thread
+constexpr int BG = 4;                  // batch rows per cluster (8 doubled the step and saved no wave of clusters)
 
 __device__ __forceinline__ u64 ffma2(u64 a, u64 b, u64 c) {
     u64 d;
@@ -32,7 +33,7 @@ __device__ __forceinline__ float sum2(u64 v) {
     return x + y;
 }
 
-template <int DH, int BG>
+template <int DH>
 __global__ void __launch_bounds__(DH, 1)
 slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restrict__ R, const float *__restrict__ rb,
                             const float *__restrict__ c0, const float *__restrict__ n0, const float *__restrict__ h0,
@@ -101,6 +102,7 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
     cluster.sync();                 // barriers armed and buffer 0 complete in every CTA before any of h_0 can land
     load_gx(0);
 
+    const bool capped = cap > 0.f;
     const uint32_t h_s = smem_u32(s_h), bar_s = smem_u32(hbar);
     for (int t = 0; t < S; ++t) {
         const int p = t & 1;
@@ -142,8 +144,8 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
                     pre[q] = gn[i][q] + (s + bias[q]);
                 }
                 float it = pre[0], ft = pre[1];
-                if (cap > 0.f) { it = cap * tanhf(it / cap); ft = cap * tanhf(ft / cap); }
-                const float zt = tanhf(pre[2]), ot = sigmoidf(pre[3]);
+                if (capped) { it = cap * tanh_quotient(it / cap); ft = cap * tanh_quotient(ft / cap); }
+                const float zt = tanh_quotient(pre[2]), ot = sigmoidf(pre[3]);
                 const float mt = fmaxf(ft + sm[i], it);
                 const float ie = expf(it - mt), fe = expf(ft - mt + sm[i]);
                 sc[i] = fmaf(fe, sc[i], ie * zt);
@@ -183,7 +185,7 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
     cluster.sync();   // no CTA leaves while a peer may still write into its shared memory
 }
 
-template <int DH, int BG>
+template <int DH>
 int launch_regs(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
                 const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH, float cap,
                 int *timeout, cudaStream_t st) {
@@ -198,7 +200,7 @@ int launch_regs(const void *gx, const void *R, const float *rb, const float *c0,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, slstm_recurrent_regs_kernel<DH, BG>, static_cast<const float *>(gx),
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, slstm_recurrent_regs_kernel<DH>, static_cast<const float *>(gx),
                                              static_cast<const float *>(R), rb, c0, n0, h0, m0, static_cast<float *>(hs), c1,
                                              n1, h1, m1, B, S, NH, cap, timeout);
     return e == cudaSuccess ? launch_status() : XLSTM_ERR_CUDA;
@@ -213,17 +215,9 @@ bool slstm_recurrent_regs_supported(int dtype, int dh, const void *R) {
 int slstm_recurrent_regs(const void *gx, const void *R, const float *rb, const float *c0, const float *n0, const float *h0,
                          const float *m0, void *hs, float *c1, float *n1, float *h1, float *m1, int B, int S, int NH, int dh,
                          float cap, int *timeout, cudaStream_t st) {
-    // eight rows per cluster once groups of four no longer all fit on the GPU at once
-    const bool small = (long long)(dh / GU) * NH * ((B + 3) / 4) * dh <= 128LL * 256;
-#define XL_REGS(DHV) \
-    if (dh == DHV) \
-        return small ? launch_regs<DHV, 4>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, timeout, st) \
-                     : launch_regs<DHV, 8>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, timeout, st);
-    XL_REGS(256)
-    XL_REGS(128)
-    XL_REGS(64)
-#undef XL_REGS
-    return XLSTM_ERR_UNSUPPORTED;
+    if (dh == 256) return launch_regs<256>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, timeout, st);
+    if (dh == 128) return launch_regs<128>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, timeout, st);
+    return launch_regs<64>(gx, R, rb, c0, n0, h0, m0, hs, c1, n1, h1, m1, B, S, NH, cap, timeout, st);
 }
 
 }  // namespace xl
