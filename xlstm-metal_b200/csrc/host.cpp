@@ -1,0 +1,200 @@
+// Tensor-level front end of the C ABI for the calls that decode loops and short prompts make: argument checks, output
+// allocation, the current stream and the call, in native code.  Through Python and ctypes the same work took 30 to 40 us a
+// call (a decode step of one sequence runs 3 us on the GPU, one of sixteen 25), so these calls were bound by it.
+//
+// Every function returns the status of the C ABI first; the Python wrappers (ops.py) raise on it.  Inputs are normalised as
+// there: activations of one dtype, states in fp32, contiguous where the ABI has no strides.  Nothing is kept between calls.
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include "xlstm_cuda.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = c10::optional<Tensor>;
+
+void need_cuda(const Tensor &t) {
+    if (!t.is_cuda()) throw std::runtime_error("xlstm_cuda kernels need CUDA tensors (no CPU fallback exists)");
+}
+void need_cuda(const OptTensor &t) {
+    if (t) need_cuda(*t);
+}
+int dtype_code(const Tensor &t) {
+    if (t.scalar_type() == at::kBFloat16) return XLSTM_BF16;
+    if (t.scalar_type() == at::kFloat) return XLSTM_F32;
+    throw py::type_error(std::string("xlstm_cuda kernels take float32 or bfloat16 activations, got ") + at::toString(t.scalar_type()));
+}
+void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+const void *ptr(const OptTensor &t) { return t ? t->data_ptr() : nullptr; }
+const float *fptr(const OptTensor &t) { return t ? static_cast<const float *>(t->data_ptr()) : nullptr; }
+float *fptr(const Tensor &t) { return static_cast<float *>(t.data_ptr()); }
+OptTensor cast_contiguous(const OptTensor &t, at::ScalarType dt) {
+    return t ? OptTensor(t->to(dt).contiguous()) : OptTensor();
+}
+
+struct State {
+    OptTensor C, n, m;
+    State(const OptTensor &c, const OptTensor &nn, const OptTensor &mm, int64_t B, int64_t NH)
+        : C(cast_contiguous(c, at::kFloat)), n(cast_contiguous(nn, at::kFloat)), m(cast_contiguous(mm, at::kFloat)) {
+        if (m) m = m->reshape({B, NH});
+    }
+};
+struct NewState {
+    Tensor C, n, m;
+    NewState(const Tensor &q, const State &st, int64_t B, int64_t NH, int64_t dqk, int64_t dv, bool inplace) {
+        const auto f32 = q.options().dtype(at::kFloat);
+        C = inplace && st.C ? *st.C : at::empty({B, NH, dqk, dv}, f32);
+        n = at::empty({B, NH, dqk}, f32);
+        m = at::empty({B, NH}, f32);
+    }
+};
+
+// q, k: [B, NH, dqk], v: [B, NH, dv], i, f: [B, NH], or the same with a token dimension of one ([B, NH, 1, d], [B, NH, 1])
+py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const OptTensor &C0, const OptTensor &n0,
+                     const OptTensor &m0, double eps, bool inplace, double gate_cap, bool state_settled) {
+    for (const Tensor *t : {&q, &k, &v, &i, &f}) need_cuda(*t);
+    const bool token_dim = q.dim() == 4;
+    if (q.dim() != 3 && !(token_dim && q.size(2) == 1))
+        throw py::value_error("mlstm_step takes q as [B, NH, dqk] or [B, NH, 1, dqk]");
+    const int64_t B = q.size(0), NH = q.size(1), dqk = q.size(-1), dv = v.size(-1);
+    const int dt = dtype_code(q);
+    q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+    i = i.to(q.scalar_type()).contiguous(); f = f.to(q.scalar_type()).contiguous();
+    const State st(C0, n0, m0, B, NH);
+    const Tensor h = token_dim ? at::empty({B, NH, 1, dv}, q.options()) : at::empty({B, NH, dv}, q.options());
+    const NewState out(q, st, B, NH, dqk, dv, inplace);
+    const int flags = state_settled && st.C ? XLSTM_STEP_STATE_SETTLED : 0;
+    const int rc = xlstm_mlstm_step_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C),
+                                       fptr(st.n), fptr(st.m), h.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B,
+                                       (int)NH, (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    return py::make_tuple(rc, h, out.C, out.n, out.m);
+}
+
+bool dense_heads(const Tensor &t) { return t.stride(2) == 1 && (t.size(1) == 1 || t.stride(1) == t.size(2)); }
+
+py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Tensor ogate, const OptTensor &norm_weight,
+                           const OptTensor &C0, const OptTensor &n0, const OptTensor &m0, double eps, double norm_eps,
+                           bool inplace, double gate_cap, bool state_settled) {
+    for (const Tensor *t : {&q, &k, &v, &i, &f, &ogate}) need_cuda(*t);
+    need_cuda(norm_weight);
+    if (q.dim() != 3) throw py::value_error("mlstm_step_gated takes q as [B, NH, dqk]");
+    const int64_t B = q.size(0), NH = q.size(1), dqk = q.size(2), dv = v.size(-1);
+    const int dt = dtype_code(q);
+    const auto type = q.scalar_type();
+    i = i.to(type); f = f.to(type);
+    const bool in_place = dense_heads(q) && dense_heads(k) && dense_heads(v) && i.stride(1) == 1 && f.stride(1) == 1 &&
+                          (B == 1 || (i.stride(0) == f.stride(0) && v.stride(0) % 4 == 0)) &&
+                          reinterpret_cast<uintptr_t>(v.data_ptr()) % (4 * v.element_size()) == 0;
+    if (!in_place) {
+        q = q.contiguous(); k = k.contiguous(); v = v.contiguous(); i = i.contiguous(); f = f.contiguous();
+    }
+    const int64_t pitch[4] = {B == 1 ? 0 : q.stride(0), B == 1 ? 0 : k.stride(0), B == 1 ? 0 : v.stride(0), B == 1 ? 0 : i.stride(0)};
+    Tensor og = ogate.to(type);
+    if (og.dim() != 2 || og.stride(1) != 1 || og.size(1) != NH * dv) og = og.reshape({B, NH * dv}).contiguous();
+    int64_t ld = B > 1 ? og.stride(0) : NH * dv;
+    if (ld < NH * dv) { og = og.contiguous(); ld = NH * dv; }
+    const OptTensor w = cast_contiguous(norm_weight, type);
+    const State st(C0, n0, m0, B, NH);
+    const Tensor y = at::empty({B, NH * dv}, q.options());
+    const NewState out(q, st, B, NH, dqk, dv, inplace);
+    const int flags = state_settled && st.C ? XLSTM_STEP_STATE_SETTLED : 0;
+    const int rc = xlstm_mlstm_step_gated_rows(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, fptr(st.C), fptr(st.n), fptr(st.m),
+        og.data_ptr(), ld, ptr(w), (float)norm_eps, y.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH,
+        (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    return py::make_tuple(rc, y, out.C, out.n, out.m);
+}
+
+py::tuple mlstm_chunkwise(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const OptTensor &C0, const OptTensor &n0,
+                          const OptTensor &m0, int64_t chunk_size, double eps, OptTensor workspace, const OptTensor &h_out,
+                          double gate_cap) {
+    for (const Tensor *t : {&q, &k, &v, &i, &f}) need_cuda(*t);
+    if (q.dim() != 4) throw py::value_error("mlstm_chunkwise takes q as [B, NH, S, dqk]");
+    const int64_t B = q.size(0), NH = q.size(1), S = q.size(2), dqk = q.size(3), dv = v.size(-1);
+    const int dt = dtype_code(q);
+    const auto type = q.scalar_type();
+    auto fix = [](const Tensor &t) { return t.stride(-1) == 1 ? t : t.contiguous(); };
+    q = fix(q); k = fix(k.to(type)); v = fix(v.to(type));
+    i = i.to(type); f = f.to(type);
+    if (i.strides() != f.strides()) { i = i.contiguous(); f = f.contiguous(); }
+    const State st(C0, n0, m0, B, NH);
+    const Tensor h = h_out ? *h_out : at::empty({B, NH, S, dv}, q.options());
+    const NewState out(q, st, B, NH, dqk, dv, false);
+    int64_t strides[15];
+    const Tensor *ts[5] = {&q, &k, &v, &h, &i};
+    for (int t = 0; t < 5; ++t)
+        for (int d = 0; d < 3; ++d) strides[3 * t + d] = ts[t]->stride(d);
+    const size_t need = xlstm_mlstm_chunkwise_workspace_bytes((int)B, (int)NH, (int)S, (int)dqk, (int)dv, (int)chunk_size, dt);
+    if (need && (!workspace || workspace->nbytes() < need)) workspace = at::empty({(int64_t)need}, q.options().dtype(at::kByte));
+    const size_t bytes = workspace ? workspace->nbytes() : 0;
+    void *ws = workspace ? workspace->data_ptr() : nullptr;
+    const int rc = xlstm_mlstm_chunkwise_fwd_gatecap(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C), fptr(st.n), fptr(st.m), h.data_ptr(),
+        fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH, (int)S, (int)dqk, (int)dv, (int)chunk_size, (float)eps,
+        (float)gate_cap, dt, strides, ws, bytes, stream());
+    return py::make_tuple(rc, h, out.C, out.n, out.m);
+}
+
+// rows of x as [M, K] bf16 and the output [.., N]
+std::vector<int64_t> with_last(const Tensor &x, int64_t n) {
+    auto s = x.sizes().vec();
+    s.back() = n;
+    return s;
+}
+
+py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight,
+                       double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows) {
+    need_cuda(weight); need_cuda(x); need_cuda(bias); need_cuda(norm_weight); need_cuda(residual);
+    if (weight.scalar_type() != at::kBFloat16) throw py::type_error("linear_token and linear_rows are bf16 kernels");
+    const int64_t K = x.size(-1);
+    const Tensor x2 = x.reshape({-1, K}).to(at::kBFloat16).contiguous();
+    const int64_t M = x2.size(0);
+    if (M > max_rows)
+        throw py::value_error("this Linear takes at most " + std::to_string(max_rows) + " rows, got " + std::to_string(M));
+    const Tensor w = weight.contiguous();
+    const int64_t N = swiglu_pair ? w.size(0) / 2 : w.size(0);
+    const OptTensor b = cast_contiguous(bias, at::kBFloat16), nw = cast_contiguous(norm_weight, at::kBFloat16);
+    const OptTensor r = residual ? cast_contiguous(residual->reshape({-1, N}), at::kBFloat16) : OptTensor();
+    const Tensor y = at::empty(with_last(x, N), x.options().dtype(at::kBFloat16));
+    const int epi = swiglu_pair ? 2 : (r ? 1 : 0);
+    const int rc = max_rows <= 4
+        ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M, (int)N,
+                             (int)K, epi, XLSTM_BF16, stream())
+        : xlstm_linear_rows(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, XLSTM_BF16,
+                            stream());
+    return py::make_tuple(rc, y);
+}
+
+py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
+    need_cuda(x); need_cuda(weight);
+    const int64_t cols = x.size(-1);
+    const Tensor xc = x.contiguous();
+    const OptTensor w = cast_contiguous(weight, xc.scalar_type());
+    const Tensor y = at::empty_like(xc);
+    const int rc = xlstm_rms_norm(xc.data_ptr(), ptr(w), y.data_ptr(), cols ? xc.numel() / cols : 0, (int)cols, (float)eps,
+                                  dtype_code(xc), stream());
+    return py::make_tuple(rc, y);
+}
+
+py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor &weight, double eps) {
+    need_cuda(x); need_cuda(residual); need_cuda(weight);
+    const int64_t cols = x.size(-1);
+    const Tensor xc = x.contiguous(), rc_ = residual.to(x.scalar_type()).contiguous();
+    const OptTensor w = cast_contiguous(weight, xc.scalar_type());
+    const Tensor s = at::empty_like(xc), y = at::empty_like(xc);
+    const int rc = xlstm_add_rms_norm(xc.data_ptr(), rc_.data_ptr(), ptr(w), s.data_ptr(), y.data_ptr(),
+                                      cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dtype_code(xc), stream());
+    return py::make_tuple(rc, s, y);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("mlstm_step", &mlstm_step);
+    m.def("mlstm_step_gated", &mlstm_step_gated);
+    m.def("mlstm_chunkwise", &mlstm_chunkwise);
+    m.def("linear_token", &linear_token);
+    m.def("rms_norm", &rms_norm);
+    m.def("add_rms_norm", &add_rms_norm);
+}

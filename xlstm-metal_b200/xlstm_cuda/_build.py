@@ -11,6 +11,8 @@ CSRC = PKG.parent / "csrc"
 INCLUDE = PKG.parent.parent / "include"
 OBJ = CSRC / "build"
 LIB = PKG / "libxlstm_cuda.so"
+HOST_SRC = CSRC / "host.cpp"     # tensor-level front end: a Python extension over the C ABI
+HOST = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -35,9 +37,31 @@ def needs_build() -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def build_host(force: bool = False) -> Path:
+    """Compile the tensor-level front end against the installed torch."""
+    deps = [HOST_SRC, *INCLUDE.glob("*.h")]
+    if not force and HOST.exists() and all(d.stat().st_mtime <= HOST.stat().st_mtime for d in deps):
+        return HOST
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{d}" for d in (*include_paths("cuda"), sysconfig.get_paths()["include"], INCLUDE)),
+           str(HOST_SRC), "-o", str(HOST), *(f"-L{d}" for d in library_paths("cuda")),
+           "-lc10", "-ltorch_cpu", "-lc10_cuda", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+           f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{HOST_SRC.name} failed to build:\n{r.stderr}")
+    return HOST
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile every ``.cu`` to an object (in parallel) and link the shared library."""
     if not force and not needs_build():
+        build_host()
         return LIB
     OBJ.mkdir(parents=True, exist_ok=True)
     nvcc = _nvcc()
@@ -63,6 +87,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stderr}")
+    build_host(force)
     return LIB
 
 

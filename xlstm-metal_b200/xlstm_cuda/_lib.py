@@ -87,6 +87,23 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native tensor-level front end (``csrc/host.cpp``), linked against the library that ``load()`` opens."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise ImportError(f"the native front end of xlstm_cuda is missing or stale ({e}): build it with "
+                              "`python -m xlstm_cuda._build`") from e
+        _host = mod
+    return _host
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         msg = load().xlstm_strerror(status).decode()

@@ -97,9 +97,8 @@ class mLSTMRecurrentKernelCell(_KernelCellBase):
         applies the soft-cap itself."""
         q, k, v, i_preact, f_preact = self._cast_in(q, k, v, i_preact, f_preact)
         if q.shape[2] == 1:
-            h, st = ops.mlstm_step(q[:, :, 0], k[:, :, 0], v[:, :, 0], i_preact[:, :, 0], f_preact[:, :, 0],
-                                   state, self.eps, inplace=self.inplace_state, gate_cap=gate_cap)
-            return h.unsqueeze(2), self._cast_state(st)
+            h, st = ops.mlstm_step(q, k, v, i_preact, f_preact, state, self.eps, inplace=self.inplace_state, gate_cap=gate_cap)
+            return h, self._cast_state(st)
         h, st = ops.mlstm_chunkwise(q, k, v, i_preact, f_preact, state, 64, self.eps, gate_cap=gate_cap)
         return h, self._cast_state(st)
 

@@ -40,6 +40,9 @@ def _state32(t: torch.Tensor) -> torch.Tensor:
     return t.to(torch.float32).contiguous()
 
 
+_NO_STATE = (None, None, None)
+
+
 def softcap(x: torch.Tensor, cap: Optional[float], out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``cap * tanh(x / cap)``; ``cap`` None or <= 0 returns ``x`` unchanged."""
     if cap is None or cap <= 0:
@@ -56,6 +59,8 @@ def mlstm_step(q, k, v, i, f, state=None, eps: float = 1e-6, inplace: bool = Fal
                gate_cap: Optional[float] = None, state_settled: bool = False):
     """One decode step.  q,k: [B,NH,dqk]; v: [B,NH,dv]; i,f: [B,NH]; state (C,n,m) fp32 or None.
 
+    Inputs may carry a token dimension of one ([B,NH,1,d], [B,NH,1]); ``h`` then does too.
+
     Returns ``h [B,NH,dv]`` and the new state.  ``inplace=True`` overwrites the
     caller's ``C`` (the 2 x dqk x dv x 4 byte stream then hits one buffer).
     ``gate_cap`` > 0: ``i`` and ``f`` are the raw gate projections and are soft-capped inside the kernel.
@@ -63,32 +68,10 @@ def mlstm_step(q, k, v, i, f, state=None, eps: float = 1e-6, inplace: bool = Fal
     (a layer stack: the launch before a layer's step is its projection); the kernel then starts streaming the
     state while that kernel drains.
     """
-    _need_cuda(q, k, v, i, f)
-    B, NH, dqk = q.shape
-    dv = v.shape[-1]
-    dt = _dtype_code(q)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    i, f = i.to(q.dtype).contiguous(), f.to(q.dtype).contiguous()
-    if state is not None:
-        C0, n0, m0 = (_state32(s) for s in state)
-        m0 = m0.reshape(B, NH)
-    else:
-        C0 = n0 = m0 = None
-    dev = q.device
-    h = torch.empty(B, NH, dv, dtype=q.dtype, device=dev)
-    C1 = C0 if (inplace and C0 is not None) else torch.empty(B, NH, dqk, dv, dtype=torch.float32, device=dev)
-    n1 = torch.empty(B, NH, dqk, dtype=torch.float32, device=dev)
-    m1 = torch.empty(B, NH, dtype=torch.float32, device=dev)
-    flags = _lib.STEP_STATE_SETTLED if (state_settled and state is not None) else 0
-    _lib.check(_lib.load().xlstm_mlstm_step_ex(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), _ptr(C0), _ptr(n0), _ptr(m0),
-        h.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, NH, dqk, dv, float(eps),
-        float(gate_cap) if gate_cap is not None else 0.0, flags, dt, _stream()), "xlstm_mlstm_step_ex")
-    return h, (C1, n1, m1)
-
-
-def _dense_heads(t: torch.Tensor) -> bool:
-    return t.stride(2) == 1 and (t.shape[1] == 1 or t.stride(1) == t.shape[2])
+    rc, h, C, n, m = _lib.host().mlstm_step(q, k, v, i, f, *(state or _NO_STATE), eps, inplace, gate_cap or 0.0, state_settled)
+    if rc:
+        _lib.check(rc, "xlstm_mlstm_step_ex")
+    return h, (C, n, m)
 
 
 def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float = 1e-6, norm_eps: float = 1e-6,
@@ -96,40 +79,11 @@ def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float =
     """Decode step with the output epilogue fused in: returns ``y [B, NH*dv] = MultiHeadRMSNorm(h) * weight *
     sigmoid(ogate)`` and the new state; ``h`` itself is never written.  ``ogate: [B, NH*dv]``, possibly a column
     block of a wider one-row-per-sequence tensor (row stride >= NH*dv).  ``dv`` must be at most 512."""
-    _need_cuda(q, k, v, i, f, ogate, norm_weight)
-    B, NH, dqk = q.shape
-    dv = v.shape[-1]
-    dt = _dtype_code(q)
-    i, f = i.to(q.dtype), f.to(q.dtype)
-    if not (_dense_heads(q) and _dense_heads(k) and _dense_heads(v) and i.stride(1) == f.stride(1) == 1 and
-            (B == 1 or i.stride(0) == f.stride(0)) and (B == 1 or v.stride(0) % 4 == 0) and
-            v.data_ptr() % (4 * v.element_size()) == 0):
-        q, k, v, i, f = q.contiguous(), k.contiguous(), v.contiguous(), i.contiguous(), f.contiguous()
-    pitch = (ctypes.c_int64 * 4)(*((0, 0, 0, 0) if B == 1 else (q.stride(0), k.stride(0), v.stride(0), i.stride(0))))
-    og = ogate.to(q.dtype)
-    if og.dim() != 2 or og.stride(1) != 1 or og.shape[1] != NH * dv:
-        og = og.reshape(B, NH * dv).contiguous()
-    ld = og.stride(0) if B > 1 else NH * dv
-    if ld < NH * dv:
-        og, ld = og.contiguous(), NH * dv
-    w = None if norm_weight is None else norm_weight.to(q.dtype).contiguous()
-    if state is not None:
-        C0, n0, m0 = (_state32(s) for s in state)
-        m0 = m0.reshape(B, NH)
-    else:
-        C0 = n0 = m0 = None
-    dev = q.device
-    y = torch.empty(B, NH * dv, dtype=q.dtype, device=dev)
-    C1 = C0 if (inplace and C0 is not None) else torch.empty(B, NH, dqk, dv, dtype=torch.float32, device=dev)
-    n1 = torch.empty(B, NH, dqk, dtype=torch.float32, device=dev)
-    m1 = torch.empty(B, NH, dtype=torch.float32, device=dev)
-    flags = _lib.STEP_STATE_SETTLED if (state_settled and state is not None) else 0
-    _lib.check(_lib.load().xlstm_mlstm_step_gated_rows(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, _ptr(C0), _ptr(n0), _ptr(m0),
-        og.data_ptr(), int(ld), _ptr(w), float(norm_eps), y.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(),
-        B, NH, dqk, dv, float(eps), float(gate_cap) if gate_cap is not None else 0.0, flags, dt, _stream()),
-        "xlstm_mlstm_step_gated_rows")
-    return y, (C1, n1, m1)
+    rc, y, C, n, m = _lib.host().mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, *(state or _NO_STATE), eps, norm_eps,
+                                                  inplace, gate_cap or 0.0, state_settled)
+    if rc:
+        _lib.check(rc, "xlstm_mlstm_step_gated_rows")
+    return y, (C, n, m)
 
 
 def _strides3(t: torch.Tensor):
@@ -173,8 +127,17 @@ def mlstm_chunkwise(q, k, v, i, f, state=None, chunk_size: int = 64, eps: float 
     ``[B,S,NH_total,dv]`` buffer); ``h_peer_ptrs`` (optional) are raw device pointers to the same
     slot in peer GPUs' buffers: the kernel stores every h tile there too (fused all-gather).
     ``gate_cap`` > 0: ``i`` and ``f`` are the raw gate projections, soft-capped inside the kernels."""
+    if not h_peer_ptrs:
+        if h_out is not None and (tuple(h_out.shape) != (*q.shape[:3], v.shape[-1]) or h_out.dtype != q.dtype or
+                                  h_out.stride(-1) != 1):
+            raise ValueError("h_out must be a [B,NH,S,dv] view of the activation dtype with a contiguous last dimension")
+        rc, h, C, n, m = _lib.host().mlstm_chunkwise(q, k, v, i, f, *(state or _NO_STATE), int(chunk_size), eps, workspace, h_out,
+                                                     gate_cap or 0.0)
+        if rc:
+            _lib.check(rc, "xlstm_mlstm_chunkwise_fwd")
+        return h, (C, n, m)
     _need_cuda(q, k, v, i, f)
-    if gate_cap is not None and gate_cap > 0 and h_peer_ptrs:
+    if gate_cap is not None and gate_cap > 0:
         i, f, gate_cap = softcap(i, gate_cap), softcap(f, gate_cap), None   # the gather entry takes capped gates
     B, NH, S, dqk = q.shape
     dv = v.shape[-1]
@@ -205,23 +168,11 @@ def mlstm_chunkwise(q, k, v, i, f, state=None, chunk_size: int = 64, eps: float 
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
     wbytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
-    if h_peer_ptrs:
-        peers = (ctypes.c_void_p * len(h_peer_ptrs))(*[int(x) for x in h_peer_ptrs])
-        _lib.check(_lib.load().xlstm_mlstm_chunkwise_fwd_gather(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), _ptr(C0), _ptr(n0), _ptr(m0),
-            h.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, NH, S, dqk, dv, int(chunk_size), float(eps),
-            dt, sarr, _ptr(workspace), wbytes, peers, len(h_peer_ptrs), _stream()), "xlstm_mlstm_chunkwise_fwd_gather")
-        return h, (C1, n1, m1)
-    if gate_cap is not None and gate_cap > 0:
-        _lib.check(_lib.load().xlstm_mlstm_chunkwise_fwd_gatecap(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), _ptr(C0), _ptr(n0), _ptr(m0),
-            h.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, NH, S, dqk, dv, int(chunk_size), float(eps),
-            float(gate_cap), dt, sarr, _ptr(workspace), wbytes, _stream()), "xlstm_mlstm_chunkwise_fwd_gatecap")
-        return h, (C1, n1, m1)
-    _lib.check(_lib.load().xlstm_mlstm_chunkwise_fwd(
+    peers = (ctypes.c_void_p * len(h_peer_ptrs))(*[int(x) for x in h_peer_ptrs])
+    _lib.check(_lib.load().xlstm_mlstm_chunkwise_fwd_gather(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), _ptr(C0), _ptr(n0), _ptr(m0),
-        h.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, NH, S, dqk, dv, int(chunk_size), float(eps), dt,
-        sarr, _ptr(workspace), wbytes, _stream()), "xlstm_mlstm_chunkwise_fwd")
+        h.data_ptr(), C1.data_ptr(), n1.data_ptr(), m1.data_ptr(), B, NH, S, dqk, dv, int(chunk_size), float(eps),
+        dt, sarr, _ptr(workspace), wbytes, peers, len(h_peer_ptrs), _stream()), "xlstm_mlstm_chunkwise_fwd_gather")
     return h, (C1, n1, m1)
 
 
@@ -315,27 +266,17 @@ def slstm_recurrent(gx, R, rb, state=None, num_heads: int = 4, cap: Optional[flo
 
 def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6) -> torch.Tensor:
     """RMSNorm over the last dimension; ``weight`` (or None) is cast to ``x.dtype``."""
-    _need_cuda(x, weight)
-    cols = x.shape[-1]
-    xc = x.contiguous()
-    w = None if weight is None else weight.to(xc.dtype).contiguous()
-    y = torch.empty_like(xc)
-    rows = xc.numel() // cols if cols else 0
-    _lib.check(_lib.load().xlstm_rms_norm(xc.data_ptr(), _ptr(w), y.data_ptr(), rows, cols, float(eps), _dtype_code(xc),
-                                          _stream()), "xlstm_rms_norm")
+    rc, y = _lib.host().rms_norm(x, weight, eps)
+    if rc:
+        _lib.check(rc, "xlstm_rms_norm")
     return y
 
 
 def add_rms_norm(x: torch.Tensor, residual: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6):
     """``s = x + residual`` and ``RMSNorm(s) * weight`` in one pass; returns ``(s, normed)``."""
-    _need_cuda(x, residual, weight)
-    cols = x.shape[-1]
-    xc, rc = x.contiguous(), residual.to(x.dtype).contiguous()
-    w = None if weight is None else weight.to(xc.dtype).contiguous()
-    s, y = torch.empty_like(xc), torch.empty_like(xc)
-    rows = xc.numel() // cols if cols else 0
-    _lib.check(_lib.load().xlstm_add_rms_norm(xc.data_ptr(), rc.data_ptr(), _ptr(w), s.data_ptr(), y.data_ptr(), rows, cols,
-                                              float(eps), _dtype_code(xc), _stream()), "xlstm_add_rms_norm")
+    rc, s, y = _lib.host().add_rms_norm(x, residual, weight, eps)
+    if rc:
+        _lib.check(rc, "xlstm_add_rms_norm")
     return s, y
 
 
@@ -422,24 +363,9 @@ def linear_token(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Ten
     most 4 rows, ``weight: [N, K]``.  Optional RMSNorm of ``x`` first (``norm_weight``), optional
     ``residual + (...)``, or ``swiglu_pair``: ``weight`` holds gate rows then up rows (``[2F, K]``) and
     the result is ``silu(gate) * up`` of width ``F``."""
-    _need_cuda(weight, x, bias, norm_weight, residual)
-    if weight.dtype != torch.bfloat16:
-        raise TypeError("linear_token is a bf16 kernel")
-    K = x.shape[-1]
-    x2 = x.reshape(-1, K).to(torch.bfloat16).contiguous()
-    M = x2.shape[0]
-    if M > LINEAR_TOKEN_MAX_ROWS:
-        raise ValueError(f"linear_token takes at most {LINEAR_TOKEN_MAX_ROWS} rows, got {M}")
-    w = weight if weight.is_contiguous() else weight.contiguous()
-    rows = w.shape[0]
-    N = rows // 2 if swiglu_pair else rows
-    b = None if bias is None else bias.to(torch.bfloat16).contiguous()
-    nw = None if norm_weight is None else norm_weight.to(torch.bfloat16).contiguous()
-    r = None if residual is None else residual.reshape(-1, N).to(torch.bfloat16).contiguous()
-    y = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=x.device)
-    epi = 2 if swiglu_pair else (1 if r is not None else 0)
-    _lib.check(_lib.load().xlstm_linear_token(w.data_ptr(), x2.data_ptr(), _ptr(b), _ptr(nw), float(norm_eps), _ptr(r),
-                                              y.data_ptr(), M, N, K, epi, _lib.BF16, _stream()), "xlstm_linear_token")
+    rc, y = _lib.host().linear_token(weight, x, bias, norm_weight, norm_eps, residual, swiglu_pair, LINEAR_TOKEN_MAX_ROWS)
+    if rc:
+        _lib.check(rc, "xlstm_linear_token")
     return y
 
 
@@ -449,20 +375,7 @@ LINEAR_ROWS_MAX = 16
 def linear_rows(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 residual: Optional[torch.Tensor] = None, swiglu_pair: bool = False) -> torch.Tensor:
     """The same for up to 16 token rows (bf16, ``K`` a multiple of 32), without the norm."""
-    _need_cuda(weight, x, bias, residual)
-    if weight.dtype != torch.bfloat16:
-        raise TypeError("linear_rows is a bf16 kernel")
-    K = x.shape[-1]
-    x2 = x.reshape(-1, K).to(torch.bfloat16).contiguous()
-    M = x2.shape[0]
-    if M > LINEAR_ROWS_MAX:
-        raise ValueError(f"linear_rows takes at most {LINEAR_ROWS_MAX} rows, got {M}")
-    w = weight if weight.is_contiguous() else weight.contiguous()
-    N = w.shape[0] // 2 if swiglu_pair else w.shape[0]
-    b = None if bias is None else bias.to(torch.bfloat16).contiguous()
-    r = None if residual is None else residual.reshape(-1, N).to(torch.bfloat16).contiguous()
-    y = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=x.device)
-    epi = 2 if swiglu_pair else (1 if r is not None else 0)
-    _lib.check(_lib.load().xlstm_linear_rows(w.data_ptr(), x2.data_ptr(), _ptr(b), _ptr(r), y.data_ptr(), M, N, K, epi,
-                                             _lib.BF16, _stream()), "xlstm_linear_rows")
+    rc, y = _lib.host().linear_token(weight, x, bias, None, 0.0, residual, swiglu_pair, LINEAR_ROWS_MAX)
+    if rc:
+        _lib.check(rc, "xlstm_linear_rows")
     return y
