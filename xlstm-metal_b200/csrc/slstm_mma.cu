@@ -117,7 +117,8 @@ slstm_recurrent_mma_kernel(const __nv_bfloat16 *__restrict__ gx, const __nv_bflo
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const bool ok = c0 != nullptr && b0 + g + 8 * (e >> 1) < B;
-        sc[e] = ok ? c0[cell(e)] : 0.f;
+        // (rows beyond the batch: nonzero, off the slow path of the division)
+        sc[e] = ok ? c0[cell(e)] : b0 + g + 8 * (e >> 1) < B ? 0.f : 1.f;
         sn[e] = ok ? n0[cell(e)] : 1.f;
         sm[e] = ok ? m0[cell(e)] : 0.f;
         hv[e] = 0.f;
@@ -232,8 +233,8 @@ slstm_recurrent_mma_kernel(const __nv_bfloat16 *__restrict__ gx, const __nv_bflo
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 float it = pre[0][e], ft = pre[1][e];
-                if (capped) { it = cap * tanh_quotient(it / cap); ft = cap * tanh_quotient(ft / cap); }
-                const float zt = tanh_quotient(pre[2][e]), ot = sigmoidf(pre[3][e]);
+                if (capped) { it = cap * tanh_quotient<true>(it / cap); ft = cap * tanh_quotient<true>(ft / cap); }
+                const float zt = tanh_quotient<true>(pre[2][e]), ot = quotient<true>(1.0f, 1.0f + expf(-pre[3][e]));
                 const float mt = fmaxf(ft + sm[e], it);
                 const float ie = expf(it - mt), fe = expf(ft - mt + sm[e]);
                 sc[e] = fmaf(fe, sc[e], ie * zt);

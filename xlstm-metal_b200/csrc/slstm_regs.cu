@@ -84,7 +84,7 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
 #pragma unroll
     for (int i = 0; i < CPT; ++i) {
         const bool ok = c0 != nullptr && row_ok(i);
-        sc[i] = ok ? c0[cell(i)] : 0.f;
+        sc[i] = ok ? c0[cell(i)] : row_ok(i) ? 0.f : 1.f;   // rows beyond the batch: nonzero, off the slow path of the division
         sn[i] = ok ? n0[cell(i)] : 1.f;
         sm[i] = ok ? m0[cell(i)] : 0.f;
         hv[i] = 0.f;
@@ -144,8 +144,8 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
                     pre[q] = gn[i][q] + (s + bias[q]);
                 }
                 float it = pre[0], ft = pre[1];
-                if (capped) { it = cap * tanh_quotient(it / cap); ft = cap * tanh_quotient(ft / cap); }
-                const float zt = tanh_quotient(pre[2]), ot = sigmoidf(pre[3]);
+                if (capped) { it = cap * tanh_quotient<false>(it / cap); ft = cap * tanh_quotient<false>(ft / cap); }
+                const float zt = tanh_quotient<false>(pre[2]), ot = sigmoidf(pre[3]);
                 const float mt = fmaxf(ft + sm[i], it);
                 const float ie = expf(it - mt), fe = expf(ft - mt + sm[i]);
                 sc[i] = fmaf(fe, sc[i], ie * zt);
