@@ -142,20 +142,17 @@ __device__ __forceinline__ void gate_chain(double *ch, double m, int tile0, int 
     const int end = tile0 + n;
     for (int c0 = tile0; c0 < end; c0 += 32) {
         const int c = c0 + lane;
-        double G, M;
-        tile_map(c, end, G, M);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double G1 = __shfl_up_sync(0xffffffffu, G, o), M1 = __shfl_up_sync(0xffffffffu, M, o);
-            if (lane >= o) { M = fmax(G + M1, M); G += G1; }
+        const double Gl = c < end ? ch[(size_t)c * GC + 0] : 0.0, Ul = c < end ? ch[(size_t)c * GC + 1] : 0.0;
+        double m_mine = 0.0;
+        const int nb = min(32, end - c0);
+        for (int j = 0; j < nb; ++j) {
+            const double Gj = __shfl_sync(0xffffffffu, Gl, j), Uj = __shfl_sync(0xffffffffu, Ul, j);
+            const double x_last = fmax(m, Uj);
+            if (x_last - m > SPREAD_LIMIT) bounded = false;
+            if (j == lane) m_mine = m;
+            m = Gj + x_last;
         }
-        const double m_after = fmax(G + m, M);
-        double m_in = __shfl_up_sync(0xffffffffu, m_after, 1);
-        if (lane == 0) m_in = m;
-        if (c < end) ch[(size_t)c * GC + 2] = m_in;
-        const bool wide = c < end && fmax(m_in, ch[(size_t)c * GC + 1]) - m_in > SPREAD_LIMIT;
-        if (__any_sync(0xffffffffu, wide)) bounded = false;
-        m = __shfl_sync(0xffffffffu, m_after, 31);
+        if (c < end) ch[(size_t)c * GC + 2] = m_mine;
     }
     if (lane == 0) { if (m_out) *m_out = (float)m; *path = bounded ? 1 : 0; }
     // C is kept in TMEM as C~ = C e^{-rho}: rho absorbs the per-tile decay so that the accumulator is
@@ -821,25 +818,29 @@ struct WsLayout {
 };
 
 constexpr int SM_COUNT = 148;          // B200
-constexpr int MIN_SEG_TILES = 2;
+constexpr int MIN_SEG_TILES = 2, LONG_SEG_TILES = 16;
 
 // Number of segments every sequence is cut into.  Cutting buys parallelism while the grid of persistent CTAs (one per head
 // and 128 dv columns) leaves SMs idle, at the price of the state-only first pass, of the states going through HBM and of
 // three more launches.  Microseconds fitted to forced segment counts at 256/512, 8 to 128 CTAs, 2 to 32 tiles a segment:
 //   one pass    13 + tiles x (4.55 up to 32 CTAs, 5.3 at 64, 6.75 at 128)
 //   two passes  35 + tiles of a segment x (7.1 at 64 CTAs, 9 at 128)
-// e.g. 8 heads, S = 2048: 85 us in one pass, 72 in 4 segments; S = 4096: 167 and 109; 2 heads, S = 8192: 283, 127 in 4
-// segments and 72 in 16; 8 heads, S = 1024: 51 and 54.  128/256 follows the same order (S = 8192, 4 heads: 250 and 51).
+// and with segments of less than LONG_SEG_TILES a quarter has to be gained (less is not worth states of 0.5 MB per head and
+// segment): 8 heads, S = 4096: 167 us in one
+// pass, 109 in 4 segments; 4 heads, S = 2048: 84 and 54 (8); 2 heads, S = 8192: 283, 127 in 4 segments and 72 in 16; but 8
+// heads, S = 2048: 85 and 74 (4), S = 1024: 51 and 54.  128/256 follows the same order (S = 8192, 4 heads: 250 and 51).
 int plan_segments(int BH, int dv, int nch) {
     const int ctas = BH * (dv / DVS);
     int pmax = SM_COUNT / ctas;
     if (pmax > nch / MIN_SEG_TILES) pmax = nch / MIN_SEG_TILES;
     if (pmax > 64) pmax = 64;
+    const float one = 13.0f + nch * (ctas <= 32 ? 4.55f : 3.9f + 0.022f * ctas);
     int best = 1;
-    float best_us = 13.0f + nch * (ctas <= 32 ? 4.55f : 3.9f + 0.022f * ctas);
+    float best_us = one;
     for (int P = 2; P <= pmax; ++P) {
-        const float us = 35.0f + ((nch + P - 1) / P) * (5.2f + 0.03f * ctas * P);
-        if (us < best_us) { best_us = us; best = P; }
+        const int tiles = (nch + P - 1) / P;
+        const float us = 35.0f + tiles * (5.2f + 0.03f * ctas * P);
+        if (us < best_us && (tiles >= LONG_SEG_TILES || us < 0.75f * one)) { best_us = us; best = P; }
     }
     return best;
 }
