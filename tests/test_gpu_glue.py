@@ -253,6 +253,15 @@ def test_linear_token_norm_and_swiglu(ops, M, F, K):
     assert relerr(host(act), host(sep)) <= BF16_TOL
 
 
+@pytest.mark.parametrize("rows,cols,dtype", [(1, 8, torch.bfloat16), (33, 1368, torch.bfloat16), (5, 4, torch.float32), (700, 344, torch.float32)])
+def test_geglu_matches_separate_ops(ops, rows, cols, dtype):
+    """One 16-byte vector, odd row counts; bf16 equal up to one ulp of the product (erff here and in torch agree to an ulp)."""
+    torch.manual_seed(rows)
+    x = (torch.randn(rows, 2 * cols, device="cuda") * 3).to(dtype)
+    ref = x[:, :cols] * torch.nn.functional.gelu(x[:, cols:])
+    assert relerr(host(ops.geglu(x)), host(ref)) <= (2.0 ** -7 if dtype == torch.bfloat16 else 1e-6)
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 4096, 4096), (5, 33, 64), (9, 264, 10944), (16, 31, 32), (1, 1, 288), (12, 50, 2080)])
 def test_linear_rows(ops, M, N, K):
     """Rows around the 8-row halves of the x operand, weight rows and k blocks around a CTA's and a warp's share."""
@@ -274,7 +283,7 @@ def test_linear_rows(ops, M, N, K):
     assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
 
 
-@pytest.mark.parametrize("B", [2, 3, 5, 16, 17])
+@pytest.mark.parametrize("B", [2, 3, 8, 9, 17])
 def test_block_token_step_matches_separate_launches(ops, B):
     """The single-token launch sequences of a block against the same block cell by cell, on a carried state."""
     from xlstm_cuda.blocks import mLSTMBlock

@@ -1,4 +1,4 @@
-// Linear layers for 5 to 16 rows of x (one token of a small serving batch): y[m] = epilogue(W . x[m] + bias), bf16.
+// Linear layers for 3 to 16 rows of x (one token of a small serving batch): y[m] = epilogue(W . x[m] + bias), bf16.
 // Still a weight-streaming pass (every weight is used 16 times at most, HBM-bound up to ~100 rows), but 16 fp32
 // multiply-adds per weight on the CUDA cores would bind before HBM does, so the products are mma.sync.m16n8k16 with the
 // WEIGHTS as the 16-row operand and the 16 rows of x as two 8-column operands.
@@ -11,6 +11,8 @@
 // turn; the partial sums meet in shared memory, where the epilogue (bias, residual, SwiGLU with the separate layers'
 // roundings) runs.  x comes through L2, half a byte per byte of W.  The first U blocks of weights are loaded BEFORE the
 // wait on the preceding kernel, which cannot have written them.
+// Measured (weights cold, 5 rows): 12304 x 4096 24 us (floor 15.2 at 6.65 TB/s; 385 CTAs in 1.3 waves), 4096 x 10944 23.6
+// (13.5), 21888 x 4096 36 (27).
 #include "common.cuh"
 
 namespace xl {

@@ -64,12 +64,23 @@ struct F32Params {
 struct GateTile {
     double b, u, mx;
 };
-template <typename T>
-__device__ __forceinline__ GateTile gate_tile(const ChunkwiseParams &p, int bb, int hd, int t, int lane, double b_in) {
-    const bool valid = t < p.S;
-    const int64_t off = bb * p.sg[0] + hd * p.sg[1] + (int64_t)t * p.sg[2];
-    const float lf = valid ? logsigmoid(gate_softcap(Elem<T>::ld(static_cast<const T *>(p.fg) + off), p.gate_cap)) : 0.f;
-    const float it = valid ? gate_softcap(Elem<T>::ld(static_cast<const T *>(p.ig) + off), p.gate_cap) : -INFINITY;
+// the raw gates of one token: loaded ahead of their use, the scan below is latency enough
+struct GateRaw {
+    float i, f;
+    bool valid;
+};
+template <typename T> __device__ __forceinline__ GateRaw gate_load(const ChunkwiseParams &p, int bb, int hd, int t) {
+    GateRaw r{0.f, 0.f, t < p.S};
+    if (r.valid) {
+        const int64_t off = bb * p.sg[0] + hd * p.sg[1] + (int64_t)t * p.sg[2];
+        r.i = Elem<T>::ld(static_cast<const T *>(p.ig) + off);
+        r.f = Elem<T>::ld(static_cast<const T *>(p.fg) + off);
+    }
+    return r;
+}
+__device__ __forceinline__ GateTile gate_tile(const GateRaw &r, float cap, int lane, double b_in) {
+    const float lf = r.valid ? logsigmoid(gate_softcap(r.f, cap)) : 0.f;
+    const float it = r.valid ? gate_softcap(r.i, cap) : -INFINITY;
     GateTile g;
     g.b = (double)lf;
 #pragma unroll
@@ -129,11 +140,12 @@ __global__ void __launch_bounds__(MAIN + 32, 2) mlstm_f32_state_kernel(const F32
             if (j < p.dqk) n0 = P.n0[(size_t)bh * p.dqk + j];
             if (j + 1 < p.dqk) n1 = P.n0[(size_t)bh * p.dqk + j + 1];
         }
+        GateRaw raw = gate_load<T>(p, b, hd, t_begin + lane);
         auto gates = [&](int k) {
             if (k >= tiles) return;
-            const int t = t_begin + k * TT + lane;
             if (own_m && lane == 0 && (k & 1) == 0 && P.m_all) P.m_all[(size_t)bh * (P.NC + 1) + P.c_begin + (k >> 1)] = m;
-            const GateTile g = gate_tile<T>(p, b, hd, t, lane, 0.0);
+            const GateTile g = gate_tile(raw, p.gate_cap, lane, 0.0);
+            raw = gate_load<T>(p, b, hd, t_begin + (k + 1) * TT + lane);
             const double xl = fmax((double)m, __shfl_sync(0xffffffffu, g.mx, 31));
             s_w[k & 3][lane] = expf((float)(g.u - xl));
             if (lane == 0) s_decay[k & 3] = expf((float)((double)m - xl));
@@ -282,14 +294,16 @@ template <int DVT> struct OutSmem {
                                                                        // over Q, K and C, which the last piece leaves free
     static constexpr uint32_t U = V + CH * DVT * 4;                    // double [CH] u, [CH] x
     static constexpr uint32_t WIN = U + 2 * CH * 8;                    // float [CH] e^{m - x_t}, [CH] e^{-m_t}, [2][CH] q.n, [CH] row sums
-    static constexpr uint32_t TOTAL = WIN + 5 * CH * 4;
+    static constexpr uint32_t NV = WIN + 5 * CH * 4;                   // float [2][KP] n of the piece
+    static constexpr uint32_t TOTAL = NV + 2 * KP * 4;
     static_assert(CH * CH * 8 <= V, "P fits the buffers it replaces");
 };
 
-// 128 columns: three CTAs per SM (77 KB each); with two, 1.84 warps per scheduler left 60 % of the FMA issue slots to
-// latency.  64 columns are taken for grids that do not fill the GPU, where a CTA has the registers to itself.
+// Two CTAs per SM by registers; a third (168 registers, a few spilled) measured the same, so it is latency inside the
+// warps and the shared-memory return path (an LDS.128 takes 2.4 to 4 clocks of it, 7 for 48 packed multiply-adds of 2.3)
+// that bind, not their number.
 template <typename T, int DVT>
-__global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_kernel(const F32Params P) {
+__global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Params P) {
     using SM = OutSmem<DVT>;
     constexpr int NG = DVT / 64;
     constexpr int QV = KP * CH / 4 / MAIN, CV = KP * DVT / 4 / MAIN;
@@ -300,6 +314,7 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
     float2 *sP = reinterpret_cast<float2 *>(smem + SM::PM);
     double *sU = reinterpret_cast<double *>(smem + SM::U), *sX = sU + CH;
     float *sWin = reinterpret_cast<float *>(smem + SM::WIN), *sEmt = sWin + CH, *sQn = sEmt + CH, *sRow = sQn + 2 * CH;
+    float *sN = reinterpret_cast<float *>(smem + SM::NV);
     const ChunkwiseParams &p = P.p;
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 4, tx = tid & 15;
     const int ci = blockIdx.x, c = P.c_begin + ci, t0 = c * CH, col0 = blockIdx.y * DVT;
@@ -313,6 +328,7 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
     const T *vb = static_cast<const T *>(p.v) + b * p.sv[0] + hd * p.sv[1] + (int64_t)t0 * p.sv[2] + col0;
 
     float4 qr[QV], kr[QV];
+    float nr = 0.f;
     auto load_qk = [&](int j0) {
 #pragma unroll
         for (int i = 0; i < QV; ++i) {                       // lane = token: the transposed stores are conflict-free
@@ -324,6 +340,7 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
     };
     auto load_c = [&](int j0, int buf) {                     // straight into shared memory
         if (has_C) {
+            if (tid < KP) nr = j0 + tid < p.dqk ? ns[j0 + tid] : 0.f;
 #pragma unroll
             for (int i = 0; i < CV; ++i) {
                 const int e = tid + i * MAIN, j = j0 + e / (DVT / 4), cc = (e % (DVT / 4)) * 4;
@@ -342,12 +359,14 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
             dq[2 * CH] = make_float2(qr[i].z, qr[i].z); dq[3 * CH] = make_float2(qr[i].w, qr[i].w);
             dk[0] = kr[i].x; dk[CH] = kr[i].y; dk[2 * CH] = kr[i].z; dk[3 * CH] = kr[i].w;
         }
+        if (tid < KP) sN[buf * KP + tid] = nr;
     };
     // The kernel before this one (state) has waited for its own predecessor before it let this one start, so the inputs are
     // there; what it writes itself (C, n, m) is read after the wait.  A single chunk starts from the caller's state and
     // needs nothing of it: the two kernels then run side by side, and one CTA waits at the end, so that this launch is
     // complete only when that one is.
     const bool single = P.m_all == nullptr;
+    const GateRaw raw[2] = {gate_load<T>(p, b, hd, t0 + lane), gate_load<T>(p, b, hd, t0 + 32 + lane)};
     load_qk(0);
     // V of the chunk: needed after the last piece
 #pragma unroll 4
@@ -365,7 +384,7 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
         double bsum = 0.0, mx = (double)m;
 #pragma unroll 1
         for (int h = 0; h < CH; h += 32) {
-            const GateTile g = gate_tile<T>(p, b, hd, t0 + h + lane, lane, bsum);
+            const GateTile g = gate_tile(h == 0 ? raw[0] : raw[1], p.gate_cap, lane, bsum);
             const double x = fmax(mx, g.mx);
             sU[h + lane] = g.u;
             sX[h + lane] = x;
@@ -422,8 +441,8 @@ __global__ void __launch_bounds__(MAIN, DVT == 128 ? 3 : 2) mlstm_f32_output_ker
             }
 #pragma unroll
             for (int j = 0; j < KP / 2; ++j) {
-                const int jj = nh * (KP / 2) + j, jg = pc * KP + jj;
-                if (jg < p.dqk) qn = fmaf(sQ[(buf * KP + jj) * CH + nt].x, ns[jg], qn);
+                const int jj = nh * (KP / 2) + j;
+                qn = fmaf(sQ[(buf * KP + jj) * CH + nt].x, sN[buf * KP + jj], qn);
             }
         } else {
 #pragma unroll 4

@@ -171,8 +171,7 @@ class sLSTMBlock(nn.Module):
 
     def forward(self, x: torch.Tensor, state=None):
         out, new_state = self.slstm_cell(self.norm_slstm(x), state)
-        x = x + out
-        xn = self.norm_ffn(x)
+        x, xn = ops.add_rms_norm(x, out, self.norm_ffn.weight, self.norm_ffn.eps)   # residual + pre-norm
         x = x + self.ffn_proj_down(ops.swiglu(self.ffn_proj_up_gate(xn), self.ffn_proj_up(xn)))
         return x, new_state
 
@@ -301,7 +300,7 @@ class sLSTMBlockDiag(nn.Module):
         out = self.hid_norm(hs)
         Wu, bu, Wd, Pp = self._ffn_weights()
         y = F.linear(out, Wu, bu)
-        out = F.linear(y[..., :Pp] * F.gelu(y[..., Pp:]), Wd, self.down_proj.bias) + xs
+        out = F.linear(ops.geglu(y), Wd, self.down_proj.bias) + xs
         return (out[:, 0] if single else out), state
 
     def _ffn_weights(self):

@@ -332,6 +332,16 @@ def swiglu(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return y
 
 
+def geglu(x: torch.Tensor) -> torch.Tensor:
+    """``x[..., :P] * gelu(x[..., P:])`` over the last dimension of size ``2 P`` (``P`` a multiple of 16 bytes)."""
+    _need_cuda(x)
+    P = x.shape[-1] // 2
+    xc = x.contiguous()
+    y = torch.empty(*x.shape[:-1], P, dtype=x.dtype, device=x.device)
+    _lib.check(_lib.load().xlstm_geglu(xc.data_ptr(), y.data_ptr(), y.numel() // P, P, _dtype_code(xc), _stream()), "xlstm_geglu")
+    return y
+
+
 def causal_conv1d(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, silu: bool = False,
                   state: Optional[torch.Tensor] = None, return_state: bool = False):
     """Causal depthwise convolution over tokens of ``x [B,S,C]`` (channels last) with ``weight [C,K]``
