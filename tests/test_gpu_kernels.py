@@ -682,6 +682,29 @@ def test_gate_cap_inside_the_kernels(ops, dtype, shape):
     assert torch.equal(h0, h1)
 
 
+@pytest.mark.parametrize("S", [128, 4096, 4224])
+def test_chunkwise_gate_prepass_forms_and_mixed_heads(ops, S):
+    """1, 32 and 33 tiles: the one-launch gate pre-pass, its last size, and the three-launch form; one head of bounded gate
+    spread beside one that forgets within a token, so both tensor-core paths share the launches; one pass and segments."""
+    rng = np.random.default_rng(S)
+    NH, d = 2, 128
+    q, k, v = (xo.bf16_round(rng.standard_normal((1, NH, S, d)).astype(np.float32)) for _ in range(3))
+    i, f = (a.astype(np.float32) for a in gates(rng, (1, NH, S)))
+    f[:, 1] -= 8
+    i, f = xo.bf16_round(i), xo.bf16_round(f)
+    h_ref, st_ref = xo.mlstm_recurrent(q, k, v, i, f)
+    args = [dev(a, torch.bfloat16) for a in (q, k, v, i, f)]
+    try:
+        for P in (1, 3):
+            ops.chunkwise_segments(P)
+            h, st = ops.mlstm_chunkwise(*args)
+            assert relerr(host(h), h_ref) < BF16_TOL
+            for a, r in zip(st, st_ref):
+                assert relerr(host(a), r) < BF16_TOL
+    finally:
+        ops.chunkwise_segments(None)
+
+
 @pytest.mark.parametrize("general", [False, True])
 def test_chunkwise_segment_parallel_equals_single_pass(ops, general):
     """The segment-parallel two-pass mode (every segment from an empty state, states combined, every segment again
