@@ -682,6 +682,35 @@ def test_gate_cap_inside_the_kernels(ops, dtype, shape):
     assert torch.equal(h0, h1)
 
 
+@pytest.mark.parametrize("S", [128 + 1, 128 + 64, 128 + 65, 128 + 127, 128 + 128])
+def test_chunkwise_tail_forms(ops, S):
+    """Tails of one chunk (one-kernel form, in place), of two (two launches, from a copy of the state), and with scratch for
+    the minimum only (one-kernel form again): outputs of the tail agree to one bf16 ulp (2^-7 of the value)."""
+    rng = np.random.default_rng(S)
+    NH, dqk, dv = 2, 128, 256
+    q, k = (xo.bf16_round(rng.standard_normal((1, NH, S, dqk)).astype(np.float32)) for _ in range(2))
+    v = xo.bf16_round(rng.standard_normal((1, NH, S, dv)).astype(np.float32))
+    i, f = (xo.bf16_round(a) for a in gates(rng, (1, NH, S)))
+    h_ref, st_ref = xo.mlstm_recurrent(q, k, v, i, f)
+    args = [dev(a, torch.bfloat16) for a in (q, k, v, i, f)]
+    h, st = ops.mlstm_chunkwise(*args)
+    assert relerr(host(h), h_ref) < BF16_TOL
+    for a, r in zip(st, st_ref):
+        assert relerr(host(a), r) < BF16_TOL
+    from xlstm_cuda import _lib
+    least = _lib.load().xlstm_mlstm_chunkwise_workspace_bytes(1, NH, 128, dqk, dv, 64, _lib.BF16)   # one tile, no tail
+    ws = torch.empty(least, dtype=torch.uint8, device="cuda")
+    C, n, m = torch.empty_like(st[0]), torch.empty_like(st[1]), torch.empty_like(st[2])
+    h2 = torch.empty_like(h)
+    rc = _lib.load().xlstm_mlstm_chunkwise_fwd(*(a.data_ptr() for a in args), None, None, None, h2.data_ptr(), C.data_ptr(), n.data_ptr(),
+                                               m.data_ptr(), 1, NH, S, dqk, dv, 64, 1e-6, _lib.BF16, None, ws.data_ptr(), least,
+                                               torch.cuda.current_stream().cuda_stream)
+    assert (rc == 0) == (S < 256)        # 256 tokens are two tiles
+    if rc == 0:
+        assert relerr(host(h2)[:, :, 128:], host(h)[:, :, 128:]) < 2.0 ** -7 + FP32_TOL
+        assert relerr(host(C), host(st[0])) < FP32_TOL
+
+
 @pytest.mark.parametrize("S", [128, 4096, 4224])
 def test_chunkwise_gate_prepass_forms_and_mixed_heads(ops, S):
     """1, 32 and 33 tiles: the one-launch gate pre-pass, its last size, and the three-launch form; one head of bounded gate

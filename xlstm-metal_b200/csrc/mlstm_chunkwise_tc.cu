@@ -813,7 +813,7 @@ namespace {
 
 // Layout of the caller-provided scratch.  P > 1 adds the per-segment states of the segment-parallel mode.
 struct WsLayout {
-    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], decay, total;
+    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], decay, tail_C, tail_ws, total;
     int P, seg_tiles;
 };
 
@@ -845,7 +845,13 @@ int plan_segments(int BH, int dv, int nch) {
     return best;
 }
 
-WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P) {
+// Tokens after the last whole tile that run on the two-launch fp32 kernels (their state and scratch is in the workspace); 0:
+// none, or the one-kernel form in place.  That one walks 64-token chunks, 54 us each at 256/512; the two launches take both
+// chunks of a longer tail at once, but for a single chunk they gain nothing (54 and 51 us).
+int tail_for_f32(int S) { return S % LT > 64 ? S % LT : 0; }
+
+// tail: see tail_for_f32()
+WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P, int tail) {
     WsLayout w{};
     const size_t BH = (size_t)B * NH, nch = (size_t)(S / LT);
     w.P = P;
@@ -866,6 +872,10 @@ WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P) {
         }
         w.decay = o; o = up(o + VH * sizeof(float));
     }
+    if (tail) {
+        w.tail_C = o;  o = up(o + BH * dqk * dv * sizeof(float));
+        w.tail_ws = o; o = up(o + mlstm_chunkwise_f32_workspace(B, NH, tail, dqk, dv));
+    }
     w.total = o + 256;
     return w;
 }
@@ -881,11 +891,11 @@ size_t mlstm_chunkwise_tc_workspace(int B, int NH, int S, int dqk, int dv, int L
     if (nch < 1 || (dqk != 256 && dqk != 128) || dv % DVS) return 0;     // not a shape of this path
     const int forced = g_segments.load();
     const int P = forced >= 1 ? (forced > nch ? (nch > 0 ? nch : 1) : forced) : plan_segments(B * NH, dv, nch);
-    return ws_layout(B, NH, S, dqk, dv, P).total;
+    return ws_layout(B, NH, S, dqk, dv, P, tail_for_f32(S)).total;
 }
 
 size_t mlstm_chunkwise_tc_workspace_min(int B, int NH, int S, int dqk, int dv) {
-    return S < LT ? 0 : ws_layout(B, NH, S, dqk, dv, 1).total;
+    return S < LT ? 0 : ws_layout(B, NH, S, dqk, dv, 1, 0).total;
 }
 
 void mlstm_chunkwise_tc_set_general_only(int on) { g_general_only.store(on ? 1 : 0); }
@@ -896,14 +906,15 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     const int nch = s_full / LT;
     const int BH = p.B * p.NH;
     if (!workspace) return XLSTM_ERR_WORKSPACE;
-    // the segment-parallel mode if the scratch holds its states, else the plain single pass
+    // the segment-parallel mode, and the fp32 kernels for a tail, if the scratch holds their states; else the plain
+    // single pass, and the tail in place
     const int forced = g_segments.load();
     int P = forced >= 1 ? (forced > nch ? nch : forced) : plan_segments(BH, p.dv, nch);
-    WsLayout w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, P);
-    if (workspace_bytes < w.total) {
-        w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1);
-        if (workspace_bytes < w.total) return XLSTM_ERR_WORKSPACE;
-    }
+    int tail_f32 = tail_for_f32(p.S);
+    WsLayout w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, P, tail_f32);
+    if (workspace_bytes < w.total) w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1, tail_f32);
+    if (workspace_bytes < w.total) w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1, tail_f32 = 0);
+    if (workspace_bytes < w.total) return XLSTM_ERR_WORKSPACE;
     P = w.P;
     const int seg_tiles = w.seg_tiles;
     unsigned char *ws = static_cast<unsigned char *>(workspace);
@@ -945,7 +956,23 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         return state_only ? launch_tc<128, true>(tp, grid, st) : launch_tc<128, false>(tp, grid, st);
     };
     float *n_final = tail ? tail_n : p.n1, *m_final = tail ? tail_m : p.m1;
-    float *C_final = p.C1;
+    // the fp32 kernels write C1 before the last read of C0, so they start from a copy; the one-kernel form runs in place
+    ChunkwiseParams t = p;
+    if (tail) {
+        const size_t esz = 2;
+        t.q = static_cast<const unsigned char *>(p.q) + (size_t)s_full * p.sq[2] * esz;
+        t.k = static_cast<const unsigned char *>(p.k) + (size_t)s_full * p.sk[2] * esz;
+        t.v = static_cast<const unsigned char *>(p.v) + (size_t)s_full * p.sv[2] * esz;
+        t.h = static_cast<unsigned char *>(p.h) + (size_t)s_full * p.sh[2] * esz;
+        t.ig = static_cast<const unsigned char *>(p.ig) + (size_t)s_full * p.sg[2] * esz;
+        t.fg = static_cast<const unsigned char *>(p.fg) + (size_t)s_full * p.sg[2] * esz;
+        t.S = p.S - s_full;
+        t.L = 64;
+        t.C0 = tail_f32 ? reinterpret_cast<float *>(ws + w.tail_C) : p.C1;
+        t.n0 = tail_n; t.m0 = tail_m;
+        if (tail_f32 && !mlstm_chunkwise_f32_supported(t, XLSTM_BF16)) { tail_f32 = 0; t.C0 = p.C1; }
+    }
+    float *C_final = tail ? const_cast<float *>(t.C0) : p.C1;
 
     // the gate pre-pass (chain, path flags and per-token scalars for both passes of the segment-parallel mode), then the
     // tensor-core kernel, whose CTAs read their path flag: the choice needs no host round trip
@@ -981,20 +1008,8 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     }
     if (!tail) return XLSTM_OK;
 
-    // S mod 128 tail on the exact path, continuing from (C1, tail_n, tail_m).  C is handed over in
-    // place: every CTA of that kernel reads only the columns it later writes.
-    ChunkwiseParams t = p;
-    const size_t esz = 2;
-    t.q = static_cast<const unsigned char *>(p.q) + (size_t)s_full * p.sq[2] * esz;
-    t.k = static_cast<const unsigned char *>(p.k) + (size_t)s_full * p.sk[2] * esz;
-    t.v = static_cast<const unsigned char *>(p.v) + (size_t)s_full * p.sv[2] * esz;
-    t.h = static_cast<unsigned char *>(p.h) + (size_t)s_full * p.sh[2] * esz;
-    t.ig = static_cast<const unsigned char *>(p.ig) + (size_t)s_full * p.sg[2] * esz;
-    t.fg = static_cast<const unsigned char *>(p.fg) + (size_t)s_full * p.sg[2] * esz;
-    t.S = p.S - s_full;
-    t.L = 64;
-    t.C0 = p.C1; t.n0 = tail_n; t.m0 = tail_m;
-    return mlstm_chunkwise_simt(t, XLSTM_BF16, st);
+    // S mod 128 tail on the exact path, continuing from (t.C0, tail_n, tail_m)
+    return tail_f32 ? mlstm_chunkwise_f32(t, XLSTM_BF16, ws + w.tail_ws, st) : mlstm_chunkwise_simt(t, XLSTM_BF16, st);
 }
 
 }  // namespace xl
