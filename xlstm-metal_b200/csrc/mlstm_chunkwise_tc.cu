@@ -846,8 +846,9 @@ int plan_segments(int BH, int dv, int nch) {
 }
 
 // Tokens after the last whole tile that run on the two-launch fp32 kernels (their state and scratch is in the workspace); 0:
-// none, or the one-kernel form in place.  That one walks 64-token chunks, 54 us each at 256/512; the two launches take both
-// chunks of a longer tail at once, but for a single chunk they gain nothing (54 and 51 us).
+// none, or the one-kernel form in place.  That one walks 64-token chunks, 51 us each at 8 heads of 256/512; the two launches
+// take both chunks of a longer tail at once (101 -> 66 us; 64 heads: 486 -> 309 for 612 tokens in all), but for a single
+// chunk they gain nothing (52 and 51 us).
 int tail_for_f32(int S) { return S % LT > 64 ? S % LT : 0; }
 
 // tail: see tail_for_f32()

@@ -352,16 +352,18 @@ class mLSTMBlock(nn.Module):
     def _token_step(self, x: torch.Tensor, state: Optional[State]):
         """Single-token path (bf16, fused weights).  Up to 2 sequences every Linear is one weight-streaming kernel with
         its norm / bias / residual / SwiGLU folded in, so a block is five launches: projections, cell step with the
-        output epilogue, out-projection, FFN up, FFN down.  Up to 8 the streaming kernel multiplies on the tensor cores
+        output epilogue, out-projection, FFN up, FFN down.  Up to 16 the streaming kernel multiplies on the tensor cores
         (the CUDA-core one is bound by its multiply-adds from 3 rows on: 143 us for the four Linears of a 4096-wide block at 4
-        rows, 99 us on the tensor cores) and the two norms are launches of their own; beyond that the Linears are GEMMs (8
-        rows: 97 us with the separate gate and add, 96 us streamed; 16 rows: 92 and 98).  The cell step reads q, k, v and the gates where the merged projection has written them."""
+        rows, 99 us on the tensor cores) and the two norms are launches of their own; beyond that the Linears are GEMMs (with
+        the separate gate and add 97 us at 8 rows and 92 at 16, against 96 and 98 streamed, but two more launches: 16
+        sequences through 8 blocks without a graph 1.54 ms against 1.31).  The cell step reads q, k, v and the gates where
+        the merged projection has written them."""
         cell = self.mlstm_cell
         W, b = cell._fused_weights()
         B = x.shape[0]
         NH, dqk, dv = cell.num_heads, cell.qk_dim_per_head, cell.v_dim_per_head
         x2 = x.reshape(B, -1)
-        rows = 2 < B <= 8 and self._rows_ok()
+        rows = 2 < B <= ops.LINEAR_ROWS_MAX and self._rows_ok()
         few = not rows and B <= ops.LINEAR_TOKEN_MAX_ROWS
         if few:
             y = ops.linear_token(W, x2, bias=b, norm_weight=self.norm_mlstm.weight, norm_eps=self.norm_mlstm.eps)
