@@ -538,6 +538,33 @@ def test_slstm_scan_segments(ops, B, S, NH, H, dtype, with_state):
         assert relerr(host(h2), h_ref) < tol and relerr(host(c), st_ref[0]) < tol and relerr(host(n), st_ref[1]) < tol
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("closed", [-1e4, -1e6, -1e9, float(np.finfo(np.float32).min), -np.inf])
+def test_slstm_scan_closed_gates(ops, closed, dtype):
+    """Tokens that reset the state (a forget gate closed for good) or that are masked out (input gate closed), in the middle and
+    at the edges of segments: what lies after them keeps the accuracy of the step-by-step oracle."""
+    rng = np.random.default_rng(11)
+    rnd = xo.bf16_round if dtype == torch.bfloat16 else (lambda a: a)
+    B, S, NH, H = 1, 1024, 2, 128
+    z = rnd(rng.standard_normal((B, S, NH, H)).astype(np.float32))
+    i, f, o = (rnd((rng.standard_normal((B, S, NH)) + s).astype(np.float32)) for s in (0, 3, 0))
+    f[:, [200, 511, 768], 0] = closed
+    f[:, 40, 1] = closed
+    i[:, 100:180, 1] = closed
+    f, i = rnd(f), rnd(i)
+    st0 = (rng.standard_normal((B, NH, H)).astype(np.float32), rng.uniform(0.5, 2, (B, NH, H)).astype(np.float32),
+           rng.standard_normal((B, NH)).astype(np.float32))
+    args = [dev(a, dtype) for a in (z, i, f, o)]
+    tol = FP32_TOL if dtype == torch.float32 else BF16_TOL
+    for st in (None, st0):
+        h_ref, st_ref = xo.slstm_scan(*(host(a) for a in args), st)
+        assert np.isfinite(h_ref).all()
+        h, st1 = ops.slstm_scan(*args, state=None if st is None else tuple(dev(s) for s in st))
+        assert relerr(host(h), h_ref) < tol
+        for a, r in zip(st1, st_ref):
+            assert relerr(host(a), r) < tol
+
+
 def test_slstm_recurrent_fixture(ops, golden):
     g = golden("slstm_b")
     nh = int(g["num_heads"])

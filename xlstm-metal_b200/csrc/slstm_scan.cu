@@ -97,7 +97,11 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
                 const float up = __shfl_down_sync(FULL, incl, o);
                 if (lane + o < 32) incl += up;
             }
-            const float total = __shfl_sync(FULL, incl, 0), suf = incl - s4.x;
+            const float total = __shfl_sync(FULL, incl, 0);
+            // the EXCLUSIVE suffix as the neighbour's sum: taken as incl - s4.x, one large term (a gate closed for good)
+            // would swallow the later ones, and an infinite one make it NaN
+            float suf = __shfl_down_sync(FULL, incl, 1);
+            if (lane == 31) suf = 0.f;
             const float ms = fmaxf(m + total, warp_max(s4.y + suf));
             const float w = lane < seg ? expf(s4.y + suf - ms) : 0.f;
             P = expf(m + total - ms);
