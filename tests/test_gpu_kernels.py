@@ -565,6 +565,18 @@ def test_slstm_scan_closed_gates(ops, closed, dtype):
             assert relerr(host(a), r) < tol
 
 
+@pytest.mark.parametrize("S", [4, 1024])
+def test_slstm_scan_keeps_small_inputs(ops, S):
+    """c is fp32 whatever the activations are: small z (where 1 - 2 / (1 + e^2z) would leave two digits) keep fp32 accuracy."""
+    rng = np.random.default_rng(S)
+    z = xo.bf16_round((rng.standard_normal((1, S, 2, 64)) * 1e-5).astype(np.float32))
+    i, f, o = (xo.bf16_round((rng.standard_normal((1, S, 2)) + s).astype(np.float32)) for s in (0, 3, 0))
+    _, st_ref = xo.slstm_scan(z, i, f, o)
+    _, st = ops.slstm_scan(*(dev(a, torch.bfloat16) for a in (z, i, f, o)))
+    for a, r in zip(st, st_ref):
+        assert relerr(host(a), r) < FP32_TOL
+
+
 def test_slstm_recurrent_fixture(ops, golden):
     g = golden("slstm_b")
     nh = int(g["num_heads"])

@@ -6,12 +6,14 @@
 // Nothing depends on h_{t-1}, so both recurrences are associative: (A, B) -> m' = max(m + A, B) for the stabiliser
 // and (f, i) -> x' = f x + i for c and n.  The floor is one read of z and one write of h (134 MB at B=4, S=2048, 4 x
 // 1024 units in bf16: 21 us); a CTA per (batch, head) walking all S steps, which this replaces, left 132 SMs idle and
-// paid the sequential stabiliser and two barriers per 32 steps (1916 us; the two launches below 29 + 35 us).
+// paid the sequential stabiliser and two barriers per 32 steps (1912 us; the two launches below 82, with a state 113).
 //
 // One WARP is one work item: (batch, head) x 32*VEC adjacent units x a segment of the sequence.  Lane = timestep while
 // the gates of 32 steps are worked out (transcendentals and both scans by warp shuffles, no shared memory, no
-// barrier), lane = VEC adjacent units (one 16-byte vector) while the state walks those steps.  n needs no per-unit
-// arithmetic: it is P_t n_0 + N_t with scalars per step, and without an initial n the whole factor of c is one scalar.
+// barrier), lane = VEC adjacent units (one 16-byte vector) while the state walks those steps.  Without an initial n the
+// normaliser is one scalar per step, and so is the whole factor of c.  The state is fp32 whatever the activations are, so
+// tanh and the quotients are the exact ones in both types (in bf16 the special-function forms took 69 and 79 us, but left two
+// digits of a z of 1e-5 in c).
 // Few (batch, head) pairs: the sequence is cut into segments of whole 32-step tiles.  A first launch leaves each
 // segment's end state from an empty start (reads z once), the second one chains those of the earlier segments (at
 // most 31 independent loads per unit) into its own start state and does the full walk.  z is read twice; that costs
@@ -37,20 +39,19 @@ struct ScanParams {
     float eps, cap;
 };
 
-// tanh of a bf16 pre-activation: exp and reciprocal on the special-function unit, absolute error ~1e-7
-template <typename T> __device__ __forceinline__ float cell_tanh(float x) {
-    if (sizeof(T) == 2) return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * x));
-    return tanhf(x);
-}
-
 template <typename T, int VEC> struct Units {   // VEC adjacent units of one timestep
     uint4 raw;
+    __device__ __forceinline__ void one() {
+        const uint32_t w = sizeof(T) == 2 ? 0x3f803f80u : 0x3f800000u;
+        raw = make_uint4(w, w, w, w);
+    }
     __device__ __forceinline__ void load(const T *p) { raw = *reinterpret_cast<const uint4 *>(p); }
     __device__ __forceinline__ void get(float *f) const { unpack16<T>(raw, f); }
     static __device__ __forceinline__ void put(T *p, const float *f) { st16<T>(p, f); }
 };
 template <typename T> struct Units<T, 1> {      // widths or addresses that do not allow 16-byte accesses
     float v;
+    __device__ __forceinline__ void one() { v = 1.f; }
     __device__ __forceinline__ void load(const T *p) { v = Elem<T>::ld(p); }
     __device__ __forceinline__ void get(float *f) const { f[0] = v; }
     static __device__ __forceinline__ void put(T *p, const float *f) { Elem<T>::st(p, f[0]); }
@@ -69,22 +70,21 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
     T *hp = static_cast<T *>(p.h) + ((size_t)b * p.S * p.NH + hd) * p.H + j0;
     const T *ig = static_cast<const T *>(p.ig), *fg = static_cast<const T *>(p.fg), *og = static_cast<const T *>(p.og);
 
-    // ---- state at the start of the segment: c per unit, n = P n_0 + N, m
-    float c[VEC], m = -INFINITY, P = 0.f, N = 0.f, Asum = 0.f;
+    // ---- state at the start of the segment: c and n per unit (N: n without an initial one), m
+    float c[VEC], m = -INFINITY, N = 0.f, Asum = 0.f;
 #pragma unroll
     for (int e = 0; e < VEC; ++e) c[e] = 0.f;
     const bool has_state = FINAL && p.c0 != nullptr;
-    float n0[VEC];
+    float n[VEC];
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) n0[e] = 0.f;
+    for (int e = 0; e < VEC; ++e) n[e] = 0.f;
     if (FINAL) {
         m = has_state ? p.m0[bh] : 0.f;
-        P = 1.f;
         if (has_state && active) {
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
                 c[e] = p.c0[(size_t)bh * p.H + j0 + e];
-                n0[e] = p.n0[(size_t)bh * p.H + j0 + e];
+                n[e] = p.n0[(size_t)bh * p.H + j0 + e];
             }
         }
         if (seg > 0) {
@@ -104,11 +104,14 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
             if (lane == 31) suf = 0.f;
             const float ms = fmaxf(m + total, warp_max(s4.y + suf));
             const float w = lane < seg ? expf(s4.y + suf - ms) : 0.f;
-            P = expf(m + total - ms);
+            const float P = expf(m + total - ms);
             N = warp_sum(w * s4.z);
             m = ms;
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) c[e] *= P;
+            for (int e = 0; e < VEC; ++e) {
+                c[e] *= P;
+                n[e] = fmaf(P, n[e], N);
+            }
             const float *lc = p.loc_c + (size_t)bh * p.nseg * p.H + j0;
 #pragma unroll 8
             for (int l = 0; l < seg; ++l) {
@@ -134,7 +137,8 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
     Units<T, VEC> zb[SC_BATCH];
 #pragma unroll
     for (int s = 0; s < SC_BATCH; ++s)
-        if (active && t0 + s < t1) zb[s].load(zp + (size_t)(t0 + s) * tstride);
+        if (!active) zb[s].one();           // lanes without a unit: a nonzero c keeps them off the slow path of the division
+        else if (t0 + s < t1) zb[s].load(zp + (size_t)(t0 + s) * tstride);
 
     for (int tt = t0; tt < t1; tt += SC_TILE) {
         const int nt = min(SC_TILE, t1 - tt);
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
             const float pp = __shfl_up_sync(FULL, pt, o), np = __shfl_up_sync(FULL, nn, o);
             if (lane >= o) { nn = fmaf(pt, np, nn); pt *= pp; }
         }
-        const float Nt = fmaf(pt, N, nn), Pt = pt * P;
+        const float Nt = fmaf(pt, N, nn);
         const float rt = has_state ? ot : ot / (fabsf(Nt) + p.eps);
         // ---- lane = units: walk the tile, the next batch of z in flight
         for (int s0 = 0; s0 < nt; s0 += SC_BATCH) {
@@ -179,16 +183,15 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
                     float zf[VEC];
                     zc[s].get(zf);
 #pragma unroll
-                    for (int e = 0; e < VEC; ++e) c[e] = fmaf(f, c[e], i * cell_tanh<T>(zf[e]));
+                    for (int e = 0; e < VEC; ++e) c[e] = fmaf(f, c[e], i * tanhf(zf[e]));
                     if (FINAL) {
                         const float r = __shfl_sync(FULL, rt, s0 + s);
                         float hv[VEC];
                         if (has_state) {
-                            const float Ps = __shfl_sync(FULL, Pt, s0 + s), Ns = __shfl_sync(FULL, Nt, s0 + s);
 #pragma unroll
                             for (int e = 0; e < VEC; ++e) {
-                                const float den = fabsf(fmaf(Ps, n0[e], Ns)) + p.eps;
-                                hv[e] = sizeof(T) == 2 ? __fdividef(r * c[e], den) : r * c[e] / den;
+                                n[e] = fmaf(f, n[e], i);
+                                hv[e] = r * c[e] / (fabsf(n[e]) + p.eps);
                             }
                         } else {
 #pragma unroll
@@ -201,7 +204,6 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
         }
         m = __shfl_sync(FULL, mt, 31);              // lanes past the end carry the last valid step on unchanged
         N = __shfl_sync(FULL, Nt, 31);
-        P = __shfl_sync(FULL, Pt, 31);
         Asum += __shfl_sync(FULL, A, 31);
     }
 
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(32) slstm_scan_kernel(const ScanParams p) {
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
                 p.c1[(size_t)bh * p.H + j0 + e] = c[e];
-                p.n1[(size_t)bh * p.H + j0 + e] = fmaf(P, n0[e], N);
+                p.n1[(size_t)bh * p.H + j0 + e] = has_state ? n[e] : N;
             }
         }
         if (blockIdx.y == 0 && lane == 0) p.m1[bh] = m;
