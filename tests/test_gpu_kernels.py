@@ -539,6 +539,24 @@ def test_slstm_scan_segments(ops, B, S, NH, H, dtype, with_state):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,with_state", [(36, False), (37, False), (197, True), (198, True)])
+def test_slstm_scan_single_pass_forms(ops, B, with_state, dtype):
+    """Around the numbers of warps at which the single pass changes from one unit a lane to a 16-byte vector."""
+    rng = np.random.default_rng(B)
+    rnd = xo.bf16_round if dtype == torch.bfloat16 else (lambda a: a)
+    S, NH, H = 43, 4, 72
+    z = rnd(rng.standard_normal((B, S, NH, H)).astype(np.float32))
+    i, f, o = (rnd((rng.standard_normal((B, S, NH)) + s).astype(np.float32)) for s in (0, 3, 0))
+    st0 = (rng.standard_normal((B, NH, H)).astype(np.float32), rng.uniform(0.5, 2, (B, NH, H)).astype(np.float32),
+           rng.standard_normal((B, NH)).astype(np.float32)) if with_state else None
+    h_ref, st_ref = xo.slstm_scan(z, i, f, o, st0)
+    h, st1 = ops.slstm_scan(*(dev(a, dtype) for a in (z, i, f, o)), state=None if st0 is None else tuple(dev(s) for s in st0))
+    assert relerr(host(h), h_ref) < (FP32_TOL if dtype == torch.float32 else BF16_TOL)
+    for a, r in zip(st1, st_ref):
+        assert relerr(host(a), r) < FP32_TOL
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("closed", [-1e4, -1e6, -1e9, float(np.finfo(np.float32).min), -np.inf])
 def test_slstm_scan_closed_gates(ops, closed, dtype):
     """Tokens that reset the state (a forget gate closed for good) or that are masked out (input gate closed), in the middle and

@@ -270,7 +270,12 @@ int scan(const void *z, const void *ig, const void *fg, const void *og, const fl
     p.loc_s = static_cast<float *>(ws);
     p.loc_c = p.loc_s ? p.loc_s + (size_t)bh * p.nseg * 4 : nullptr;
     if (bh * p.nseg > 2147483647LL || (H + 31) / 32 > 65535) return XLSTM_ERR_UNSUPPORTED;
-    const bool al = ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(h)) & 15u) == 0;
+    // One pass of few warps is bound by the instructions of a step in a warp: one unit a lane then, in place of 4 or 8.  Without a
+    // state (no quotient per unit) that pays up to about one warp per SM (bf16, 128 warps of 256 units: 310 -> 259 us, 512: 310
+    // -> 352), with one as long as the narrow warps do not fill the GPU several times over (128: 629 -> 302, 512: 630 -> 423).
+    const int64_t warps = bh * (((int64_t)H * (dtype == XLSTM_BF16 ? 2 : 4) + 511) / 512);
+    const bool narrow = p.nseg == 1 && warps < (c0 ? SC_FULL / 3 : SC_FULL / 16);
+    const bool al = !narrow && ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(h)) & 15u) == 0;
     if (dtype == XLSTM_F32) return al && H % 4 == 0 ? launch<float, 4>(p, bh, st) : launch<float, 1>(p, bh, st);
     return al && H % 8 == 0 ? launch<__nv_bfloat16, 8>(p, bh, st) : launch<__nv_bfloat16, 1>(p, bh, st);
 }
