@@ -849,6 +849,31 @@ def test_bounded_wait_gives_up_and_status_queries_report_ok(ops):
     ops.slstm_recurrent_status()
 
 
+@pytest.mark.parametrize("dtype,S,full", [(torch.float32, 200, True), (torch.float32, 40, True), (torch.float32, 200, False),
+                                          (torch.bfloat16, 200, True)])
+def test_status_after_forwards_without_waits(ops, dtype, S, full):
+    """The fp32 kernels (fp32 inputs, and bf16 head shapes outside the tensor-core kernels) cannot time out: whatever the
+    scratch held before, and with a stabiliser that is not zero, the status of a forward that was handed it is fine; with scratch
+    too small for the chunk states too."""
+    rng = np.random.default_rng(S)
+    B, NH, d = 1, 2, 64
+    q, k, v = (dev(rng.standard_normal((B, NH, S, d)).astype(np.float32), dtype) for _ in range(3))
+    i, f = (dev(a, dtype) for a in gates(rng, (B, NH, S)))
+    st = tuple(dev(a) for a in (rng.standard_normal((B, NH, d, d)).astype(np.float32),
+                                rng.standard_normal((B, NH, d)).astype(np.float32), np.full((B, NH), 2.5, np.float32)))
+    need = max(ops.chunkwise_workspace_bytes(B, NH, S, d, d, 64, dtype), 256)
+    ws = torch.full((need if full else 256,), 255, dtype=torch.uint8, device="cuda")
+    h, st1 = ops.mlstm_chunkwise(q, k, v, i, f, state=st, workspace=torch.full_like(ws, 255))
+    from xlstm_cuda import _lib
+    code = _lib.F32 if dtype == torch.float32 else _lib.BF16
+    h2, C, n, m = torch.empty_like(h), *(torch.empty_like(a) for a in st1)
+    rc = _lib.load().xlstm_mlstm_chunkwise_fwd(*(a.data_ptr() for a in (q, k, v, i, f, *st, h2, C, n, m)), B, NH, S, d, d, 64, 1e-6,
+                                               code, None, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    ops.chunkwise_status(ws)
+    assert relerr(host(h2), host(h)) < FP32_TOL and relerr(host(C), host(st1[0])) < FP32_TOL
+
+
 def test_chunkwise_scatter_entry_point_single_rank(ops):
     """The token-sharded store mode with one rank: h lands in the [B, S, NH, dv] buffer exactly as the regular
     entry point writes it into a strided view of the same layout (the multi-rank routing is covered by the

@@ -20,7 +20,11 @@ struct ChunkwiseParams {
     // > 0: token-sharded destinations instead of replicas - h_peer[r] (r = 0 .. n_peer-1, this rank included, `h` unused)
     // is rank r's [B, tok_per_rank, NH_total, dv] buffer and a tile of tokens goes ONLY to the rank that owns them
     int tok_per_rank;
+    int *status;      // status word of the caller's scratch, cleared by the fp32 kernels (no wait of theirs can give up), or NULL
 };
+
+// the first bytes of every scratch buffer: the status word that xlstm_mlstm_chunkwise_status() reads
+constexpr size_t WS_HEADER = 256;
 
 // fp32 arithmetic, any dqk, dv, S: two launches per group of chunks, chunk states in scratch
 size_t mlstm_chunkwise_f32_workspace(int B, int NH, int S, int dqk, int dv);

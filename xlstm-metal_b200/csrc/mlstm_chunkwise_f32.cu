@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(MAIN + 32, 2) mlstm_f32_state_kernel(const F32
     const int tiles = (t_end - t_begin + TT - 1) / TT;
     grid_dependency_wait();
     allow_dependents();
+    if (p.status && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) *p.status = 0;
 
     if (tid >= MAIN) {
         // ---- gate warp: weights two tiles ahead, stabiliser chain, normaliser (first column tile only)
@@ -572,7 +573,7 @@ size_t mlstm_chunkwise_f32_workspace(int B, int NH, int S, int dqk, int dv) {
     const int NC = (S + CH - 1) / CH, BH = B * NH;
     if (NC < 2) return 0;
     const int g = group_chunks(BH, S, dqk, dv);
-    return (((size_t)BH * (NC + 1) * sizeof(float) + 255) & ~(size_t)255) +
+    return WS_HEADER + (((size_t)BH * (NC + 1) * sizeof(float) + 255) & ~(size_t)255) +
            (size_t)BH * g * ((size_t)dqk * dv + dqk) * sizeof(float);
 }
 
@@ -596,9 +597,9 @@ int mlstm_chunkwise_f32(const ChunkwiseParams &p, int dtype, void *workspace, cu
     P.NC = NC;
     P.slots = g;
     if (NC > 1) {
-        P.m_all = static_cast<float *>(workspace);
-        P.slot_C = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) +
-                                             (((size_t)BH * (NC + 1) * sizeof(float) + 255) & ~(size_t)255));
+        unsigned char *ws = static_cast<unsigned char *>(workspace) + WS_HEADER;
+        P.m_all = reinterpret_cast<float *>(ws);
+        P.slot_C = reinterpret_cast<float *>(ws + (((size_t)BH * (NC + 1) * sizeof(float) + 255) & ~(size_t)255));
         P.slot_n = P.slot_C + (size_t)BH * g * p.dqk * p.dv;
     }
     P.C1 = p.C1; P.n1 = p.n1;

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_simt_kernel(Chunkw
     float *sW = sWin + LT;               // [LT] e^{a_t-m'}
     float *sQn = sW + LT;                // [LT] q~ . n
     float *sRow = sQn + LT;              // [LT] row sums of P
+    if (p.status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *p.status = 0;
     __shared__ float s_m;                // carried stabiliser
     __shared__ double sBd[LT], sUd[LT], sXd[LT];  // cumsum b, u = i - b, running max x
 

@@ -16,7 +16,6 @@ constexpr int THREADS = 640;
 constexpr int GW = 6 * LT;     // floats of gate scratch per (head, tile)
 constexpr int G_U2 = 0, G_X2 = LT, G_WINQ = 2 * LT, G_W = 3 * LT, G_EMT = 4 * LT, G_SCAL = 5 * LT;
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr size_t WS_HEADER = 256;  // status word lives in the first bytes of the scratch
 
 struct TcParams {
     CUtensorMap tq, tk, tv;
