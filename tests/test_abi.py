@@ -32,6 +32,7 @@ def test_version_and_status_strings_without_a_gpu():
     # argument checks run before any CUDA call
     assert lib.xlstm_softcap(None, None, 5, 15.0, 0, None) == -1
     assert lib.xlstm_mlstm_chunkwise_workspace_bytes(1, 1, 64, 64, 64, 64, 0) == 0
+    assert lib.xlstm_linear_rows_ex(64, 64, None, None, 64, 1, 32, 32, 0, 2, 1, None) == -1      # an unknown flag
 
 
 def test_workspace_query_below_one_tile():

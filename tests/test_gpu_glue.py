@@ -283,6 +283,26 @@ def test_linear_rows(ops, M, N, K):
     assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
 
 
+def test_linear_rows_reads_weights_written_just_before(ops):
+    """A weight that the launch right before the call writes (an update in place; the dense copy that the call itself makes of a
+    transposed one, also where the caller vouches for the weight it passes) is not read early."""
+    t = torch.bfloat16
+    torch.manual_seed(0)
+    M, N, K = 8, 512, 4096
+    x = torch.randn(M, K, device="cuda").to(t)
+    Ws = [(torch.randn(N, K, device="cuda") * 0.05).to(t) for _ in range(4)]
+    refs = [x.float() @ W.float().T for W in Ws]
+    W = torch.zeros(N, K, device="cuda", dtype=t)
+    Wt = torch.zeros(K, N, device="cuda", dtype=t)
+    for n in range(40):
+        W.copy_(Ws[n % 4])
+        y = ops.linear_rows(W, x)
+        Wt.copy_(Ws[n % 4].T)
+        yt = ops.linear_rows(Wt.T, x, weights_settled=True)
+        assert relerr(host(y), host(refs[n % 4])) <= BF16_TOL
+        assert torch.equal(y, yt)
+
+
 @pytest.mark.parametrize("B", [2, 3, 9, 16, 17])
 def test_block_token_step_matches_separate_launches(ops, B):
     """The single-token launch sequences of a block against the same block cell by cell, on a carried state."""

@@ -144,7 +144,7 @@ std::vector<int64_t> with_last(const Tensor &x, int64_t n) {
 }
 
 py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight,
-                       double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows) {
+                       double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows, bool weights_settled) {
     need_cuda(weight); need_cuda(x); need_cuda(bias); need_cuda(norm_weight); need_cuda(residual);
     if (weight.scalar_type() != at::kBFloat16) throw py::type_error("linear_token and linear_rows are bf16 kernels");
     const int64_t K = x.size(-1);
@@ -158,11 +158,13 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
     const OptTensor r = residual ? cast_contiguous(residual->reshape({-1, N}), at::kBFloat16) : OptTensor();
     const Tensor y = at::empty(with_last(x, N), x.options().dtype(at::kBFloat16));
     const int epi = swiglu_pair ? 2 : (r ? 1 : 0);
+    // a dense copy made here is written by the launch right before the call
+    const int flags = weights_settled && w.is_same(weight) ? XLSTM_LINEAR_WEIGHTS_SETTLED : 0;
     const int rc = max_rows <= 4
         ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M, (int)N,
                              (int)K, epi, XLSTM_BF16, stream())
-        : xlstm_linear_rows(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, XLSTM_BF16,
-                            stream());
+        : xlstm_linear_rows_ex(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, flags,
+                               XLSTM_BF16, stream());
     return py::make_tuple(rc, y);
 }
 

@@ -9,8 +9,8 @@
 //
 // A CTA owns 2 x 16 weight rows (16 gate and 16 up rows for the SwiGLU pair) and its 8 warps take the 32-wide k blocks in
 // turn; the partial sums meet in shared memory, where the epilogue (bias, residual, SwiGLU with the separate layers'
-// roundings) runs.  x comes through L2, half a byte per byte of W.  The first U blocks of weights are loaded BEFORE the
-// wait on the preceding kernel, which cannot have written them.
+// roundings) runs.  x comes through L2, half a byte per byte of W.  With XLSTM_LINEAR_WEIGHTS_SETTLED the first U blocks
+// of weights are loaded BEFORE the wait on the preceding kernel, which the caller promises not to have written them.
 // Measured (weights cold, 5 rows): 12304 x 4096 24 us (floor 15.2 at 6.65 TB/s; 385 CTAs in 1.3 waves), 4096 x 10944 23.6
 // (13.5), 21888 x 4096 36 (27).
 #include "common.cuh"
@@ -39,7 +39,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 template <int EPI>
 __global__ void __launch_bounds__(LR_THREADS, 2)
 linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, const __nv_bfloat16 *__restrict__ bias,
-                   const __nv_bfloat16 *residual, __nv_bfloat16 *__restrict__ y, int M, int N, int K) {
+                   const __nv_bfloat16 *residual, __nv_bfloat16 *__restrict__ y, int M, int N, int K, int weights_settled) {
     constexpr int STRIDE = EPI == 2 ? 16 : 32;                 // outputs per CTA
     __shared__ float s_part[LR_WARPS][LR_M][LR_ROWS + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
@@ -67,10 +67,14 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
         for (int r = 0; r < 2; ++r)
             xr[u][r] = b < blocks ? *reinterpret_cast<const uint4 *>(xp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
     };
+    auto load_first = [&]() {
 #pragma unroll
-    for (int u = 0; u < LR_U; ++u) load_w(u, warp + u * LR_WARPS);
+        for (int u = 0; u < LR_U; ++u) load_w(u, warp + u * LR_WARPS);
+    };
+    if (weights_settled) load_first();
     grid_dependency_wait();
     allow_dependents();
+    if (!weights_settled) load_first();
 
     float acc[2][2][4];
 #pragma unroll
@@ -132,25 +136,32 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
 
 template <int EPI>
 int linear_rows_launch(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N, int K,
-                       cudaStream_t st) {
+                       int settled, cudaStream_t st) {
     const int per = EPI == 2 ? 16 : 32;
     return launch_overlapped(linear_rows_kernel<EPI>, dim3((N + per - 1) / per), dim3(LR_THREADS), 0, st,
                              static_cast<const __nv_bfloat16 *>(W), static_cast<const __nv_bfloat16 *>(x),
                              static_cast<const __nv_bfloat16 *>(bias), static_cast<const __nv_bfloat16 *>(residual),
-                             static_cast<__nv_bfloat16 *>(y), M, N, K);
+                             static_cast<__nv_bfloat16 *>(y), M, N, K, settled);
 }
 
 }  // namespace
 }  // namespace xl
 
-extern "C" int xlstm_linear_rows(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
-                                 int K, int epilogue, int dtype, void *stream) {
+extern "C" int xlstm_linear_rows_ex(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
+                                    int K, int epilogue, int flags, int dtype, void *stream) {
     if (M <= 0 || N <= 0 || K <= 0 || !W || !x || !y) return XLSTM_ERR_INVALID;
     if (epilogue < 0 || epilogue > 2 || (epilogue == 1 && !residual)) return XLSTM_ERR_INVALID;
+    if (flags & ~XLSTM_LINEAR_WEIGHTS_SETTLED) return XLSTM_ERR_INVALID;
     if (dtype != XLSTM_BF16 || M > xl::LR_M || K % 32) return XLSTM_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15u) return XLSTM_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (epilogue == 2) return xl::linear_rows_launch<2>(W, x, bias, residual, y, M, N, K, st);
-    if (epilogue == 1) return xl::linear_rows_launch<1>(W, x, bias, residual, y, M, N, K, st);
-    return xl::linear_rows_launch<0>(W, x, bias, residual, y, M, N, K, st);
+    const int settled = flags & XLSTM_LINEAR_WEIGHTS_SETTLED ? 1 : 0;
+    if (epilogue == 2) return xl::linear_rows_launch<2>(W, x, bias, residual, y, M, N, K, settled, st);
+    if (epilogue == 1) return xl::linear_rows_launch<1>(W, x, bias, residual, y, M, N, K, settled, st);
+    return xl::linear_rows_launch<0>(W, x, bias, residual, y, M, N, K, settled, st);
+}
+
+extern "C" int xlstm_linear_rows(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
+                                 int K, int epilogue, int dtype, void *stream) {
+    return xlstm_linear_rows_ex(W, x, bias, residual, y, M, N, K, epilogue, 0, dtype, stream);
 }

@@ -56,6 +56,7 @@ _SIGNATURES = {
     "xlstm_swiglu": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_int64, c_int, c_void_p]),
     "xlstm_linear_token": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "xlstm_linear_rows": (c_int, [c_void_p] * 5 + [c_int] * 5 + [c_void_p]),
+    "xlstm_linear_rows_ex": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_void_p]),
     "xlstm_geglu": (c_int, [c_void_p] * 2 + [c_int64, c_int, c_int, c_void_p]),
     "xlstm_causal_conv1d": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_void_p]),
 }

@@ -369,7 +369,7 @@ class mLSTMBlock(nn.Module):
             y = ops.linear_token(W, x2, bias=b, norm_weight=self.norm_mlstm.weight, norm_eps=self.norm_mlstm.eps)
         else:
             xn = self.norm_mlstm(x2)
-            y = ops.linear_rows(W, xn, bias=b) if rows else F.linear(xn, W, b)
+            y = ops.linear_rows(W, xn, bias=b, weights_settled=True) if rows else F.linear(xn, W, b)
         o_k, o_v, o_g, o_o = NH * dqk, 2 * NH * dqk, 2 * NH * dqk + NH * dv, 2 * NH * dqk + NH * dv + 2 * NH
         heads = lambda lo, hi, d: y[:, lo:hi].unflatten(1, (NH, d))
         q, k, v = heads(0, o_k, dqk), heads(o_k, o_v, dqk), heads(o_v, o_g, dv)
@@ -393,9 +393,10 @@ class mLSTMBlock(nn.Module):
             act = ops.linear_token(ffn, x1, norm_weight=self.norm_ffn.weight, norm_eps=self.norm_ffn.eps, swiglu_pair=True)
             x3 = ops.linear_token(down.weight, act, bias=down.bias, residual=x1)
         elif rows:
-            x1 = ops.linear_rows(oc.out_proj.weight, gated, bias=oc.out_proj.bias, residual=x2)
-            act = ops.linear_rows(ffn, self.norm_ffn(x1), swiglu_pair=True)
-            x3 = ops.linear_rows(down.weight, act, bias=down.bias, residual=x1)
+            # weights_settled: the launches before these four are a norm, the cell step, a norm and the Linear above
+            x1 = ops.linear_rows(oc.out_proj.weight, gated, bias=oc.out_proj.bias, residual=x2, weights_settled=True)
+            act = ops.linear_rows(ffn, self.norm_ffn(x1), swiglu_pair=True, weights_settled=True)
+            x3 = ops.linear_rows(down.weight, act, bias=down.bias, residual=x1, weights_settled=True)
         else:
             x1, xn = ops.add_rms_norm(x2, oc.out_proj(gated), self.norm_ffn.weight, self.norm_ffn.eps)
             up = F.linear(xn, ffn)

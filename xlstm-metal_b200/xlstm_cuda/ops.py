@@ -373,7 +373,8 @@ def linear_token(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Ten
     most 4 rows, ``weight: [N, K]``.  Optional RMSNorm of ``x`` first (``norm_weight``), optional
     ``residual + (...)``, or ``swiglu_pair``: ``weight`` holds gate rows then up rows (``[2F, K]``) and
     the result is ``silu(gate) * up`` of width ``F``."""
-    rc, y = _lib.host().linear_token(weight, x, bias, norm_weight, norm_eps, residual, swiglu_pair, LINEAR_TOKEN_MAX_ROWS)
+    rc, y = _lib.host().linear_token(weight, x, bias, norm_weight, norm_eps, residual, swiglu_pair, LINEAR_TOKEN_MAX_ROWS,
+                                      False)
     if rc:
         _lib.check(rc, "xlstm_linear_token")
     return y
@@ -383,9 +384,11 @@ LINEAR_ROWS_MAX = 16
 
 
 def linear_rows(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                residual: Optional[torch.Tensor] = None, swiglu_pair: bool = False) -> torch.Tensor:
-    """The same for up to 16 token rows (bf16, ``K`` a multiple of 32), without the norm."""
-    rc, y = _lib.host().linear_token(weight, x, bias, None, 0.0, residual, swiglu_pair, LINEAR_ROWS_MAX)
+                residual: Optional[torch.Tensor] = None, swiglu_pair: bool = False, weights_settled: bool = False) -> torch.Tensor:
+    """The same for up to 16 token rows (bf16, ``K`` a multiple of 32), without the norm.  ``weights_settled`` promises that
+    the launch right before this one on the stream does not write ``weight``: its first blocks are then loaded while that
+    launch drains."""
+    rc, y = _lib.host().linear_token(weight, x, bias, None, 0.0, residual, swiglu_pair, LINEAR_ROWS_MAX, weights_settled)
     if rc:
-        _lib.check(rc, "xlstm_linear_rows")
+        _lib.check(rc, "xlstm_linear_rows_ex")
     return y
