@@ -680,6 +680,29 @@ def test_slstm_recurrent_edges(ops, B, S, NH, dh, dtype):
     assert relerr(host(hs), hs_ref) < (BF16_TOL if rounded else FP32_TOL if dtype == FP else 2.0 ** -8 + FP32_TOL)
 
 
+@pytest.mark.parametrize("dh,dtype", [(64, BF), (128, BF), (256, BF), (64, FP), (128, FP), (256, FP), (32, FP)])
+@pytest.mark.parametrize("cap", [15.0, 0.0])
+def test_slstm_recurrent_keeps_nan_and_inf(ops, dh, dtype, cap):
+    """A NaN in any gate's pre-activation reaches the same outputs and states as in the oracle; an infinite cell input or
+    output gate saturates."""
+    B, S, NH = 5, 2, 1
+    rng = np.random.default_rng(dh)
+    rd = xo.bf16_round if dtype == BF else (lambda a: a)
+    gx = rd(rng.standard_normal((B, S, 4, dh)).astype(np.float32))
+    for g in range(4):
+        gx[g, 0, g, 3 + g] = np.nan
+    gx[4, 0, 2, 5], gx[4, 1, 2, 6], gx[4, 0, 3, 7], gx[4, 1, 3, 8] = np.inf, -np.inf, np.inf, -np.inf
+    R = rd((rng.standard_normal((4, NH, dh, dh)) * 0.05).astype(np.float32))
+    rb = np.zeros((4, dh), np.float32)
+    hs_ref, st_ref = xo.slstm_recurrent(gx, R, rb, None, NH, cap)
+    hs, st = ops.slstm_recurrent(dev(gx, dtype), dev(R, dtype), dev(rb), None, NH, cap)
+    ops.slstm_recurrent_status()
+    for got, want in zip((hs, *st), (hs_ref, *st_ref)):
+        got = host(got)
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        assert relerr(np.nan_to_num(got), np.nan_to_num(want)) < BF16_TOL
+
+
 # ---- error behaviour of the C ABI --------------------------------------------------
 def test_errors_are_statuses_not_crashes(ops):
     from xlstm_cuda import _lib

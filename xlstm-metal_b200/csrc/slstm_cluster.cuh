@@ -48,21 +48,6 @@ __device__ __forceinline__ void mbar_wait_cluster(uint64_t *bar, uint32_t parity
     }
 }
 
-// tanh for the recurrences that feed h back unrounded, without a branch so that several cells' chains interleave: Lambert's
-// continued fraction x / (1 + y / (3 + y / (5 + y / (7 + y / 9)))), y = x^2, as one quotient up to |x| = 0.8 (its
-// truncation error there is below 1e-8), and (e^{2x} - 1) / (e^{2x} + 1) beyond, where the subtraction loses less than a
-// bit.  Within 1.4e-7 of tanh, rms 2.7e-8, over the whole range.
-// FAST: the approximate division (2 ulp), for results that are not kept in fp32.
-template <bool FAST> __device__ __forceinline__ float quotient(float a, float b) { return FAST ? __fdividef(a, b) : a / b; }
-template <bool FAST> __device__ __forceinline__ float tanh_quotient(float x) {
-    x = fminf(fmaxf(x, -10.0f), 10.0f);   // 1 - tanh(10) is below half an ulp
-    const float y = x * x, e = expf(2.0f * x);
-    const bool near0 = fabsf(x) < 0.8f;
-    const float num = near0 ? x * fmaf(y, 105.0f + y, 945.0f) : e - 1.0f;
-    const float den = near0 ? fmaf(y, fmaf(y, 15.0f, 420.0f), 945.0f) : e + 1.0f;
-    return quotient<FAST>(num, den);
-}
-
 // after a wait that gave up: time for stores still under way to land before the CTA may leave (normally every one has
 // been waited for)
 __device__ __forceinline__ void drain_after_abort() {

@@ -144,8 +144,8 @@ slstm_recurrent_regs_kernel(const float *__restrict__ gx, const float *__restric
                     pre[q] = gn[i][q] + (s + bias[q]);
                 }
                 float it = pre[0], ft = pre[1];
-                if (capped) { it = cap * tanh_quotient<false>(it / cap); ft = cap * tanh_quotient<false>(ft / cap); }
-                const float zt = tanh_quotient<false>(pre[2]), ot = sigmoidf(pre[3]);
+                if (capped) { it = cap * tanhf(it / cap); ft = cap * tanhf(ft / cap); }
+                const float zt = tanhf(pre[2]), ot = sigmoidf(pre[3]);
                 const float mt = fmaxf(ft + sm[i], it);
                 const float ie = expf(it - mt), fe = expf(ft - mt + sm[i]);
                 sc[i] = fmaf(fe, sc[i], ie * zt);
