@@ -703,6 +703,29 @@ def test_slstm_recurrent_keeps_nan_and_inf(ops, dh, dtype, cap):
         assert relerr(np.nan_to_num(got), np.nan_to_num(want)) < BF16_TOL
 
 
+@pytest.mark.parametrize("state_dtype,strided", [(torch.bfloat16, False), (torch.float32, True)])
+def test_step_with_a_state_that_is_converted(ops, state_dtype, strided):
+    """A state in bf16 or with strides is copied by the launch right before the step: it is not read early, also where the
+    caller vouches for the state that it passes."""
+    torch.manual_seed(1)
+    B, NH, dqk, dv = 16, 8, 256, 512
+    bf = torch.bfloat16
+    q, k = (torch.randn(B, NH, dqk, device="cuda").to(bf) for _ in range(2))
+    v = torch.randn(B, NH, dv, device="cuda").to(bf)
+    i, f, og = (torch.randn(*s, device="cuda").to(bf) for s in ((B, NH), (B, NH), (B, NH * dv)))
+    w = torch.ones(NH * dv, device="cuda", dtype=bf)
+    n, m = torch.randn(B, NH, dqk, device="cuda"), torch.zeros(B, NH, device="cuda")
+    for _ in range(20):
+        C = torch.randn(B, NH, dqk, dv, device="cuda").to(state_dtype)
+        given = C.transpose(2, 3).contiguous().transpose(2, 3) if strided else C
+        h, (C1, _, _) = ops.mlstm_step(q, k, v, i, f, (C.float(), n, m))
+        h2, (C2, _, _) = ops.mlstm_step(q, k, v, i, f, (given, n, m), state_settled=True)
+        assert torch.equal(h, h2) and torch.equal(C1, C2)
+        y, _ = ops.mlstm_step_gated(q, k, v, i, f, og, w, (C.float(), n, m))
+        y2, _ = ops.mlstm_step_gated(q, k, v, i, f, og, w, (given, n, m), state_settled=True)
+        assert torch.equal(y, y2)
+
+
 # ---- error behaviour of the C ABI --------------------------------------------------
 def test_errors_are_statuses_not_crashes(ops):
     from xlstm_cuda import _lib

@@ -35,10 +35,13 @@ OptTensor cast_contiguous(const OptTensor &t, at::ScalarType dt) {
 
 struct State {
     OptTensor C, n, m;
+    bool converted;   // C is a copy made here, by the launch right before the step's: not settled, whatever the caller says
     State(const OptTensor &c, const OptTensor &nn, const OptTensor &mm, int64_t B, int64_t NH)
         : C(cast_contiguous(c, at::kFloat)), n(cast_contiguous(nn, at::kFloat)), m(cast_contiguous(mm, at::kFloat)) {
         if (m) m = m->reshape({B, NH});
+        converted = c && !C->is_same(*c);
     }
+    int step_flags(bool settled) const { return settled && C && !converted ? XLSTM_STEP_STATE_SETTLED : 0; }
 };
 struct NewState {
     Tensor C, n, m;
@@ -64,7 +67,7 @@ py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const Opt
     const State st(C0, n0, m0, B, NH);
     const Tensor h = token_dim ? at::empty({B, NH, 1, dv}, q.options()) : at::empty({B, NH, dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
-    const int flags = state_settled && st.C ? XLSTM_STEP_STATE_SETTLED : 0;
+    const int flags = st.step_flags(state_settled);
     const int rc = xlstm_mlstm_step_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C),
                                        fptr(st.n), fptr(st.m), h.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B,
                                        (int)NH, (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
@@ -98,7 +101,7 @@ py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Ten
     const State st(C0, n0, m0, B, NH);
     const Tensor y = at::empty({B, NH * dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
-    const int flags = state_settled && st.C ? XLSTM_STEP_STATE_SETTLED : 0;
+    const int flags = st.step_flags(state_settled);
     const int rc = xlstm_mlstm_step_gated_rows(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, fptr(st.C), fptr(st.n), fptr(st.m),
         og.data_ptr(), ld, ptr(w), (float)norm_eps, y.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH,
