@@ -703,6 +703,61 @@ def test_slstm_recurrent_keeps_nan_and_inf(ops, dh, dtype, cap):
         assert relerr(np.nan_to_num(got), np.nan_to_num(want)) < BF16_TOL
 
 
+def test_front_end_refuses_sizes_that_do_not_fit(ops):
+    """The ABI takes bare pointers, so operands that are too small, of another dtype or incomplete are refused before a launch."""
+    z = lambda *s, dt=torch.bfloat16: torch.zeros(*s, device="cuda", dtype=dt)
+    B, NH, dqk, dv, S = 2, 2, 16, 32, 8
+    f32 = torch.float32
+    st = (z(B, NH, dqk, dv, dt=f32), z(B, NH, dqk, dt=f32), z(B, NH, dt=f32))
+    step = dict(q=z(B, NH, dqk), k=z(B, NH, dqk), v=z(B, NH, dv), i=z(B, NH), f=z(B, NH), state=st)
+    gated = dict(step, ogate=z(B, NH * dv), norm_weight=z(NH * dv))
+    chunk = dict(q=z(B, NH, S, dqk), k=z(B, NH, S, dqk), v=z(B, NH, S, dv), i=z(B, NH, S), f=z(B, NH, S), state=st)
+    lin = dict(weight=z(64, 32), x=z(3, 32), bias=z(64), residual=z(3, 64))
+    small = [(ops.mlstm_step, step, dict(k=z(B, NH, 8))), (ops.mlstm_step, step, dict(v=z(1, NH, dv))),
+             (ops.mlstm_step, step, dict(f=z(B, 1))), (ops.mlstm_step, step, dict(state=(st[0][:1], st[1], st[2]))),
+             (ops.mlstm_step, step, dict(state=(st[0], st[1][:1], st[2]))), (ops.mlstm_step, step, dict(state=(st[0], None, None))),
+             (ops.mlstm_step, step, dict(state=(None, st[1], st[2]))),
+             (ops.mlstm_step_gated, gated, dict(k=z(B, NH, 8))), (ops.mlstm_step_gated, gated, dict(ogate=z(1, NH * dv))),
+             (ops.mlstm_step_gated, gated, dict(norm_weight=z(dv))), (ops.mlstm_step_gated, gated, dict(i=z(1, NH))),
+             (ops.mlstm_chunkwise, chunk, dict(k=z(B, NH, S, 8))), (ops.mlstm_chunkwise, chunk, dict(v=z(B, NH, 4, dv))),
+             (ops.mlstm_chunkwise, chunk, dict(i=z(B, NH, 4), f=z(B, NH, 4))),
+             (ops.mlstm_chunkwise, chunk, dict(state=(st[0], st[1][:1], st[2])))]
+    for fn in (ops.linear_token, ops.linear_rows):
+        small += [(fn, lin, dict(weight=z(64, 16))), (fn, lin, dict(bias=z(32))), (fn, lin, dict(residual=z(2, 64))),
+                  (fn, lin, dict(weight=z(63, 32), bias=None, residual=None, swiglu_pair=True))]
+    small += [(ops.rms_norm, dict(x=z(4, 64), weight=z(32), eps=1e-6), {}),
+              (ops.add_rms_norm, dict(x=z(4, 64), residual=z(3, 64), weight=z(64)), {})]
+    for fn, good, bad in small:
+        with pytest.raises(ValueError):
+            fn(**dict(good, **bad))
+    for bad in (dict(k=z(B, NH, dqk, dt=f32)), dict(v=z(B, NH, dv, dt=f32))):
+        with pytest.raises(TypeError):
+            ops.mlstm_step(**dict(step, **bad))
+        with pytest.raises(TypeError):
+            ops.mlstm_step_gated(**dict(gated, **bad))
+    with pytest.raises((ValueError, TypeError)):
+        ops.mlstm_step(**dict(step, state=()))
+    for fn, good in ((ops.mlstm_step, step), (ops.mlstm_step_gated, gated), (ops.mlstm_chunkwise, chunk), (ops.linear_rows, lin)):
+        fn(**good)
+
+
+def test_step_with_an_unaligned_v(ops):
+    """v is read four elements at a time: a view at an odd offset is copied, in the plain and in the gated step."""
+    torch.manual_seed(0)
+    B, NH, dqk, dv = 2, 2, 16, 32
+    for dt in (torch.float32, torch.bfloat16):
+        q, k = (torch.randn(B, NH, dqk, device="cuda").to(dt) for _ in range(2))
+        v = torch.randn(B * NH * dv + 1, device="cuda").to(dt)[1:].view(B, NH, dv)
+        i, f, og = (torch.randn(*s, device="cuda").to(dt) for s in ((B, NH), (B, NH), (B, NH * dv)))
+        assert torch.equal(ops.mlstm_step(q, k, v, i, f)[0], ops.mlstm_step(q, k, v.clone(), i, f)[0])
+        assert torch.equal(ops.mlstm_step_gated(q, k, v, i, f, og, None)[0],
+                           ops.mlstm_step_gated(q, k, v.clone(), i.reshape(-1), f.unsqueeze(-1), og, None)[0])
+    from xlstm_cuda import _lib
+    C = torch.zeros(B * NH * dqk * dv + 1, device="cuda")[1:].view(B, NH, dqk, dv)
+    with pytest.raises(_lib.XlstmCudaError):
+        ops.mlstm_step(q, k, v.clone(), i, f, (C, torch.zeros(B, NH, dqk, device="cuda"), torch.zeros(B, NH, device="cuda")))
+
+
 @pytest.mark.parametrize("state_dtype,strided", [(torch.bfloat16, False), (torch.float32, True)])
 def test_step_with_a_state_that_is_converted(ops, state_dtype, strided):
     """A state in bf16 or with strides is copied by the launch right before the step: it is not read early, also where the

@@ -20,6 +20,13 @@ void need_cuda(const Tensor &t) {
 void need_cuda(const OptTensor &t) {
     if (t) need_cuda(*t);
 }
+// The ABI takes bare pointers: whatever could make a kernel read beyond a tensor is refused here.
+void need(bool ok, const char *what) {
+    if (!ok) throw py::value_error(what);
+}
+void need_type(const Tensor &t, at::ScalarType type, const char *what) {
+    if (t.scalar_type() != type) throw py::type_error(what);
+}
 int dtype_code(const Tensor &t) {
     if (t.scalar_type() == at::kBFloat16) return XLSTM_BF16;
     if (t.scalar_type() == at::kFloat) return XLSTM_F32;
@@ -36,9 +43,15 @@ OptTensor cast_contiguous(const OptTensor &t, at::ScalarType dt) {
 struct State {
     OptTensor C, n, m;
     bool converted;   // C is a copy made here, by the launch right before the step's: not settled, whatever the caller says
-    State(const OptTensor &c, const OptTensor &nn, const OptTensor &mm, int64_t B, int64_t NH)
+    State(const OptTensor &c, const OptTensor &nn, const OptTensor &mm, int64_t B, int64_t NH, int64_t dqk, int64_t dv)
         : C(cast_contiguous(c, at::kFloat)), n(cast_contiguous(nn, at::kFloat)), m(cast_contiguous(mm, at::kFloat)) {
-        if (m) m = m->reshape({B, NH});
+        need(C.has_value() == n.has_value() && C.has_value() == m.has_value(), "a state is (C, n, m), all three or None");
+        if (C) {
+            need_cuda(C); need_cuda(n); need_cuda(m);
+            need(C->numel() == B * NH * dqk * dv && n->numel() == B * NH * dqk && m->numel() == B * NH,
+                 "state of another size than [B,NH,dqk,dv], [B,NH,dqk], [B,NH]");
+            m = m->reshape({B, NH});
+        }
         converted = c && !C->is_same(*c);
     }
     int step_flags(bool settled) const { return settled && C && !converted ? XLSTM_STEP_STATE_SETTLED : 0; }
@@ -53,6 +66,18 @@ struct NewState {
     }
 };
 
+void step_inputs(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &i, const Tensor &f, int64_t B, int64_t NH,
+                 int64_t dqk, int64_t dv) {
+    need_type(k, q.scalar_type(), "q, k and v of one dtype");
+    need_type(v, q.scalar_type(), "q, k and v of one dtype");
+    need(k.numel() == B * NH * dqk && v.numel() == B * NH * dv && i.numel() == B * NH && f.numel() == B * NH,
+         "k, v or gates of another size than q: [B,NH,dqk], [B,NH,dv], [B,NH]");
+}
+// v is read four elements at a time
+Tensor aligned4(const Tensor &t) {
+    return reinterpret_cast<uintptr_t>(t.data_ptr()) % (4 * t.element_size()) ? t.clone() : t;
+}
+
 // q, k: [B, NH, dqk], v: [B, NH, dv], i, f: [B, NH], or the same with a token dimension of one ([B, NH, 1, d], [B, NH, 1])
 py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const OptTensor &C0, const OptTensor &n0,
                      const OptTensor &m0, double eps, bool inplace, double gate_cap, bool state_settled) {
@@ -62,9 +87,10 @@ py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const Opt
         throw py::value_error("mlstm_step takes q as [B, NH, dqk] or [B, NH, 1, dqk]");
     const int64_t B = q.size(0), NH = q.size(1), dqk = q.size(-1), dv = v.size(-1);
     const int dt = dtype_code(q);
-    q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+    step_inputs(q, k, v, i, f, B, NH, dqk, dv);
+    q = q.contiguous(); k = k.contiguous(); v = aligned4(v.contiguous());
     i = i.to(q.scalar_type()).contiguous(); f = f.to(q.scalar_type()).contiguous();
-    const State st(C0, n0, m0, B, NH);
+    const State st(C0, n0, m0, B, NH, dqk, dv);
     const Tensor h = token_dim ? at::empty({B, NH, 1, dv}, q.options()) : at::empty({B, NH, dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
     const int flags = st.step_flags(state_settled);
@@ -85,20 +111,25 @@ py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Ten
     const int64_t B = q.size(0), NH = q.size(1), dqk = q.size(2), dv = v.size(-1);
     const int dt = dtype_code(q);
     const auto type = q.scalar_type();
+    step_inputs(q, k, v, i, f, B, NH, dqk, dv);
     i = i.to(type); f = f.to(type);
+    if (i.dim() != 2) i = i.reshape({B, NH});
+    if (f.dim() != 2) f = f.reshape({B, NH});
     const bool in_place = dense_heads(q) && dense_heads(k) && dense_heads(v) && i.stride(1) == 1 && f.stride(1) == 1 &&
                           (B == 1 || (i.stride(0) == f.stride(0) && v.stride(0) % 4 == 0)) &&
                           reinterpret_cast<uintptr_t>(v.data_ptr()) % (4 * v.element_size()) == 0;
     if (!in_place) {
-        q = q.contiguous(); k = k.contiguous(); v = v.contiguous(); i = i.contiguous(); f = f.contiguous();
+        q = q.contiguous(); k = k.contiguous(); v = aligned4(v.contiguous()); i = i.contiguous(); f = f.contiguous();
     }
     const int64_t pitch[4] = {B == 1 ? 0 : q.stride(0), B == 1 ? 0 : k.stride(0), B == 1 ? 0 : v.stride(0), B == 1 ? 0 : i.stride(0)};
     Tensor og = ogate.to(type);
+    need(og.numel() == B * NH * dv && (!norm_weight || norm_weight->numel() == NH * dv),
+         "output gate or norm weight of another size than [B,NH*dv], [NH*dv]");
     if (og.dim() != 2 || og.stride(1) != 1 || og.size(1) != NH * dv) og = og.reshape({B, NH * dv}).contiguous();
     int64_t ld = B > 1 ? og.stride(0) : NH * dv;
     if (ld < NH * dv) { og = og.contiguous(); ld = NH * dv; }
     const OptTensor w = cast_contiguous(norm_weight, type);
-    const State st(C0, n0, m0, B, NH);
+    const State st(C0, n0, m0, B, NH, dqk, dv);
     const Tensor y = at::empty({B, NH * dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
     const int flags = st.step_flags(state_settled);
@@ -118,10 +149,18 @@ py::tuple mlstm_chunkwise(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, cons
     const int dt = dtype_code(q);
     const auto type = q.scalar_type();
     auto fix = [](const Tensor &t) { return t.stride(-1) == 1 ? t : t.contiguous(); };
+    auto covers = [](const Tensor &t, at::IntArrayRef s) {
+        bool ok = t.dim() >= (int64_t)s.size();
+        for (size_t d = 0; ok && d < s.size(); ++d) ok = t.size(d) >= s[d];
+        return ok;
+    };
+    need(covers(k, {B, NH, S, dqk}) && covers(v, {B, NH, S, dv}) && covers(i, {B, NH, S}) && covers(f, {B, NH, S}),
+         "k, v or gates smaller than q: [B,NH,S,dqk], [B,NH,S,dv], [B,NH,S]");
+    need_cuda(h_out); need_cuda(workspace);
     q = fix(q); k = fix(k.to(type)); v = fix(v.to(type));
     i = i.to(type); f = f.to(type);
     if (i.strides() != f.strides()) { i = i.contiguous(); f = f.contiguous(); }
-    const State st(C0, n0, m0, B, NH);
+    const State st(C0, n0, m0, B, NH, dqk, dv);
     const Tensor h = h_out ? *h_out : at::empty({B, NH, S, dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, false);
     int64_t strides[15];
@@ -151,6 +190,10 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
     need_cuda(weight); need_cuda(x); need_cuda(bias); need_cuda(norm_weight); need_cuda(residual);
     if (weight.scalar_type() != at::kBFloat16) throw py::type_error("linear_token and linear_rows are bf16 kernels");
     const int64_t K = x.size(-1);
+    need(weight.dim() == 2 && weight.size(1) == K, "weight must be [N, K] for rows of K elements");
+    need(!swiglu_pair || weight.size(0) % 2 == 0, "a SwiGLU pair has as many gate rows as up rows");
+    need(!bias || bias->numel() == weight.size(0), "bias must have one element per weight row");
+    need(!norm_weight || norm_weight->numel() == K, "norm weight must have K elements");
     const Tensor x2 = x.reshape({-1, K}).to(at::kBFloat16).contiguous();
     const int64_t M = x2.size(0);
     if (M > max_rows)
@@ -158,6 +201,7 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
     const Tensor w = weight.contiguous();
     const int64_t N = swiglu_pair ? w.size(0) / 2 : w.size(0);
     const OptTensor b = cast_contiguous(bias, at::kBFloat16), nw = cast_contiguous(norm_weight, at::kBFloat16);
+    need(!residual || residual->numel() == M * N, "residual must have the size of the result");
     const OptTensor r = residual ? cast_contiguous(residual->reshape({-1, N}), at::kBFloat16) : OptTensor();
     const Tensor y = at::empty(with_last(x, N), x.options().dtype(at::kBFloat16));
     const int epi = swiglu_pair ? 2 : (r ? 1 : 0);
@@ -174,6 +218,7 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
 py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
     need_cuda(x); need_cuda(weight);
     const int64_t cols = x.size(-1);
+    need(!weight || weight->numel() == cols, "norm weight must have one element per column");
     const Tensor xc = x.contiguous();
     const OptTensor w = cast_contiguous(weight, xc.scalar_type());
     const Tensor y = at::empty_like(xc);
@@ -185,6 +230,8 @@ py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
 py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor &weight, double eps) {
     need_cuda(x); need_cuda(residual); need_cuda(weight);
     const int64_t cols = x.size(-1);
+    need(residual.numel() == x.numel() && (!weight || weight->numel() == cols),
+         "residual of another size than x, or norm weight of another size than a row");
     const Tensor xc = x.contiguous(), rc_ = residual.to(x.scalar_type()).contiguous();
     const OptTensor w = cast_contiguous(weight, xc.scalar_type());
     const Tensor s = at::empty_like(xc), y = at::empty_like(xc);

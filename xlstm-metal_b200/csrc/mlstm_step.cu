@@ -262,8 +262,12 @@ static int mlstm_step_checked(const void *q, const void *k, const void *v, const
     xl::StepRows rows{(long long)NH * dqk, (long long)NH * dqk, (long long)NH * dv, NH, NH};
     if (row_pitch) {
         rows.q = row_pitch[0]; rows.k = row_pitch[1]; rows.v = row_pitch[2]; rows.g = row_pitch[3];
-        if (rows.v % 4 || (reinterpret_cast<uintptr_t>(v) & (dtype == XLSTM_F32 ? 15u : 7u))) return XLSTM_ERR_UNSUPPORTED;
+        if (rows.v % 4) return XLSTM_ERR_UNSUPPORTED;
     }
+    // v and C move four elements at a time
+    if ((reinterpret_cast<uintptr_t>(v) & (dtype == XLSTM_F32 ? 15u : 7u)) ||
+        ((reinterpret_cast<uintptr_t>(C0) | reinterpret_cast<uintptr_t>(C1)) & 15u))
+        return XLSTM_ERR_UNSUPPORTED;
     const int settled = (flags & XLSTM_STEP_STATE_SETTLED) ? 1 : 0;
     if (dtype == XLSTM_F32)
         return xl::mlstm_step_launch<float>(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap,

@@ -68,7 +68,7 @@ def mlstm_step(q, k, v, i, f, state=None, eps: float = 1e-6, inplace: bool = Fal
     (a layer stack: the launch before a layer's step is its projection); the kernel then starts streaming the
     state while that kernel drains.
     """
-    rc, h, C, n, m = _lib.host().mlstm_step(q, k, v, i, f, *(state or _NO_STATE), eps, inplace, gate_cap or 0.0, state_settled)
+    rc, h, C, n, m = _lib.host().mlstm_step(q, k, v, i, f, *(_NO_STATE if state is None else state), eps, inplace, gate_cap or 0.0, state_settled)
     if rc:
         _lib.check(rc, "xlstm_mlstm_step_ex")
     return h, (C, n, m)
@@ -79,7 +79,7 @@ def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float =
     """Decode step with the output epilogue fused in: returns ``y [B, NH*dv] = MultiHeadRMSNorm(h) * weight *
     sigmoid(ogate)`` and the new state; ``h`` itself is never written.  ``ogate: [B, NH*dv]``, possibly a column
     block of a wider one-row-per-sequence tensor (row stride >= NH*dv).  ``dv`` must be at most 512."""
-    rc, y, C, n, m = _lib.host().mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, *(state or _NO_STATE), eps, norm_eps,
+    rc, y, C, n, m = _lib.host().mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, *(_NO_STATE if state is None else state), eps, norm_eps,
                                                   inplace, gate_cap or 0.0, state_settled)
     if rc:
         _lib.check(rc, "xlstm_mlstm_step_gated_rows")
@@ -131,7 +131,7 @@ def mlstm_chunkwise(q, k, v, i, f, state=None, chunk_size: int = 64, eps: float 
         if h_out is not None and (tuple(h_out.shape) != (*q.shape[:3], v.shape[-1]) or h_out.dtype != q.dtype or
                                   h_out.stride(-1) != 1):
             raise ValueError("h_out must be a [B,NH,S,dv] view of the activation dtype with a contiguous last dimension")
-        rc, h, C, n, m = _lib.host().mlstm_chunkwise(q, k, v, i, f, *(state or _NO_STATE), int(chunk_size), eps, workspace, h_out,
+        rc, h, C, n, m = _lib.host().mlstm_chunkwise(q, k, v, i, f, *(_NO_STATE if state is None else state), int(chunk_size), eps, workspace, h_out,
                                                      gate_cap or 0.0)
         if rc:
             _lib.check(rc, "xlstm_mlstm_chunkwise_fwd")
