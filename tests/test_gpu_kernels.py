@@ -741,6 +741,28 @@ def test_front_end_refuses_sizes_that_do_not_fit(ops):
         fn(**good)
 
 
+def test_front_end_releases_the_interpreter_lock(ops):
+    """Other Python threads run while a launch is on its way (as through ctypes): with thread switching on request put off for
+    good, a waiting thread can only get the lock where a call gives it up."""
+    import threading
+    x = torch.zeros(4, 64, device="cuda")
+    ops.rms_norm(x, None)
+    go, ran, interval = threading.Lock(), [], sys.getswitchinterval()
+    go.acquire()
+    other = threading.Thread(target=lambda: (go.acquire(), ran.append(True)))
+    other.start()
+    kept = []                    # (freeing a tensor gives the lock up as well)
+    try:
+        sys.setswitchinterval(1e3)
+        go.release()
+        while not ran and len(kept) < 20000:
+            kept.append(ops.rms_norm(x, None))
+    finally:
+        sys.setswitchinterval(interval)
+        other.join()
+    assert len(kept) < 20000
+
+
 def test_step_with_an_unaligned_v(ops):
     """v is read four elements at a time: a view at an odd offset is copied, in the plain and in the gated step."""
     torch.manual_seed(0)

@@ -32,6 +32,11 @@ int dtype_code(const Tensor &t) {
     if (t.scalar_type() == at::kFloat) return XLSTM_F32;
     throw py::type_error(std::string("xlstm_cuda kernels take float32 or bfloat16 activations, got ") + at::toString(t.scalar_type()));
 }
+// Launches run without the interpreter's lock, as calls through ctypes do: a full launch queue stalls this thread alone.
+template <typename Call> int unlocked(Call &&call) {
+    py::gil_scoped_release release;
+    return call();
+}
 void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 const void *ptr(const OptTensor &t) { return t ? t->data_ptr() : nullptr; }
 const float *fptr(const OptTensor &t) { return t ? static_cast<const float *>(t->data_ptr()) : nullptr; }
@@ -94,9 +99,11 @@ py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const Opt
     const Tensor h = token_dim ? at::empty({B, NH, 1, dv}, q.options()) : at::empty({B, NH, dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
     const int flags = st.step_flags(state_settled);
-    const int rc = xlstm_mlstm_step_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C),
-                                       fptr(st.n), fptr(st.m), h.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B,
-                                       (int)NH, (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    const int rc = unlocked([&] {
+        return xlstm_mlstm_step_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C), fptr(st.n),
+                                   fptr(st.m), h.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH, (int)dqk,
+                                   (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    });
     return py::make_tuple(rc, h, out.C, out.n, out.m);
 }
 
@@ -133,10 +140,12 @@ py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Ten
     const Tensor y = at::empty({B, NH * dv}, q.options());
     const NewState out(q, st, B, NH, dqk, dv, inplace);
     const int flags = st.step_flags(state_settled);
-    const int rc = xlstm_mlstm_step_gated_rows(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, fptr(st.C), fptr(st.n), fptr(st.m),
-        og.data_ptr(), ld, ptr(w), (float)norm_eps, y.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH,
-        (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    const int rc = unlocked([&] {
+        return xlstm_mlstm_step_gated_rows(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), pitch, fptr(st.C), fptr(st.n), fptr(st.m),
+            og.data_ptr(), ld, ptr(w), (float)norm_eps, y.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH,
+            (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
+    });
     return py::make_tuple(rc, y, out.C, out.n, out.m);
 }
 
@@ -171,10 +180,12 @@ py::tuple mlstm_chunkwise(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, cons
     if (need && (!workspace || workspace->nbytes() < need)) workspace = at::empty({(int64_t)need}, q.options().dtype(at::kByte));
     const size_t bytes = workspace ? workspace->nbytes() : 0;
     void *ws = workspace ? workspace->data_ptr() : nullptr;
-    const int rc = xlstm_mlstm_chunkwise_fwd_gatecap(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C), fptr(st.n), fptr(st.m), h.data_ptr(),
-        fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH, (int)S, (int)dqk, (int)dv, (int)chunk_size, (float)eps,
-        (float)gate_cap, dt, strides, ws, bytes, stream());
+    const int rc = unlocked([&] {
+        return xlstm_mlstm_chunkwise_fwd_gatecap(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), i.data_ptr(), f.data_ptr(), fptr(st.C), fptr(st.n), fptr(st.m),
+            h.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH, (int)S, (int)dqk, (int)dv, (int)chunk_size,
+            (float)eps, (float)gate_cap, dt, strides, ws, bytes, stream());
+    });
     return py::make_tuple(rc, h, out.C, out.n, out.m);
 }
 
@@ -207,11 +218,13 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
     const int epi = swiglu_pair ? 2 : (r ? 1 : 0);
     // a dense copy made here is written by the launch right before the call
     const int flags = weights_settled && w.is_same(weight) ? XLSTM_LINEAR_WEIGHTS_SETTLED : 0;
-    const int rc = max_rows <= 4
-        ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M, (int)N,
-                             (int)K, epi, XLSTM_BF16, stream())
-        : xlstm_linear_rows_ex(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, flags,
-                               XLSTM_BF16, stream());
+    const int rc = unlocked([&] {
+        return max_rows <= 4
+            ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M,
+                                 (int)N, (int)K, epi, XLSTM_BF16, stream())
+            : xlstm_linear_rows_ex(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, flags,
+                                   XLSTM_BF16, stream());
+    });
     return py::make_tuple(rc, y);
 }
 
@@ -222,8 +235,11 @@ py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
     const Tensor xc = x.contiguous();
     const OptTensor w = cast_contiguous(weight, xc.scalar_type());
     const Tensor y = at::empty_like(xc);
-    const int rc = xlstm_rms_norm(xc.data_ptr(), ptr(w), y.data_ptr(), cols ? xc.numel() / cols : 0, (int)cols, (float)eps,
-                                  dtype_code(xc), stream());
+    const int dt = dtype_code(xc);
+    const int rc = unlocked([&] {
+        return xlstm_rms_norm(xc.data_ptr(), ptr(w), y.data_ptr(), cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dt,
+                              stream());
+    });
     return py::make_tuple(rc, y);
 }
 
@@ -235,8 +251,11 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
     const Tensor xc = x.contiguous(), rc_ = residual.to(x.scalar_type()).contiguous();
     const OptTensor w = cast_contiguous(weight, xc.scalar_type());
     const Tensor s = at::empty_like(xc), y = at::empty_like(xc);
-    const int rc = xlstm_add_rms_norm(xc.data_ptr(), rc_.data_ptr(), ptr(w), s.data_ptr(), y.data_ptr(),
-                                      cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dtype_code(xc), stream());
+    const int dt = dtype_code(xc);
+    const int rc = unlocked([&] {
+        return xlstm_add_rms_norm(xc.data_ptr(), rc_.data_ptr(), ptr(w), s.data_ptr(), y.data_ptr(),
+                                  cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dt, stream());
+    });
     return py::make_tuple(rc, s, y);
 }
 
