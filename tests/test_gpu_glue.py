@@ -324,7 +324,67 @@ def test_block_token_step_matches_separate_launches(ops, B):
         assert relerr(host(a), host(b)) <= BF16_TOL
 
 
+def _blocks():
+    from xlstm_cuda.blocks import mLSTMBlock, sLSTMBlock, sLSTMBlockDiag
+    t = torch.bfloat16
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        m = mLSTMBlock(0, embedding_dim=512, num_heads=2, compute_dtype=t).to(t)
+        m.fuse_projections()
+        s = sLSTMBlock(0, embedding_dim=512, num_heads=2).to(t)
+
+        class Config:
+            inp_dim, head_dim, head_num, p_factor, norm_eps, gate_soft_cap = 128, 64, 2, (2.0, 1.5), 1e-6, 15.0
+        d = sLSTMBlockDiag(Config()).to(t)
+    return m, s, d
+
+
+@pytest.mark.parametrize("B", [8, 20])
+def test_fused_launches_leave_hooks_and_replaced_modules_alone(ops, B):
+    """Modules whose call a fused launch would leave out are called where somebody listens, or has put another module there."""
+    m, s, _ = _blocks()
+    x = torch.randn(B, 1, 512, device="cuda", dtype=torch.bfloat16)
+    seen = []
+    with torch.inference_mode():
+        y, ys = m(x)[0], s(x)[0]
+        for blk, mods in ((m, (m.norm_mlstm, m.mlstm_cell, m.mlstm_cell.recurrent_kernel, m.mlstm_cell.output_cell.out_proj,
+                               m.ffn_proj_down)), (s, (s.norm_ffn,))):
+            for mod in mods:
+                handle = mod.register_forward_hook(lambda mod, args, out: seen.append(mod))
+                out = blk(x)[0]
+                handle.remove()
+                assert seen == [mod] and relerr(host(out), host(y if blk is m else ys)) <= BF16_TOL
+                seen.clear()
+
+        class Doubled(torch.nn.Linear):
+            def forward(self, x):
+                return 2 * super().forward(x)
+        with torch.device("cuda"):
+            other = Doubled(512, 512, bias=False).to(torch.bfloat16)
+        other.weight.copy_(m.mlstm_cell.output_cell.out_proj.weight * 0.5)
+        m.mlstm_cell.output_cell.out_proj = other
+        assert relerr(host(m(x)[0]), host(y)) <= BF16_TOL
+
+
+def test_fused_launches_leave_gradients_alone(ops):
+    """Where gradients are recorded the blocks reach the same parameters and inputs as their separate ops do."""
+    m, s, d = _blocks()
+    x = torch.randn(8, 1, 512, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    s(x)[0].float().pow(2).sum().backward()
+    assert x.grad is not None and s.slstm_cell.output_cell.out_proj.weight.grad is not None
+    m(x)[0].float().pow(2).sum().backward()
+    assert m.ffn_proj_down.weight.grad is not None
+    xd = torch.randn(3, 5, 128, device="cuda", dtype=torch.bfloat16)
+    y = d(xd)[0]
+    y.float().pow(2).sum().backward()
+    assert d.up_proj.weight.grad is not None and d.hid_norm.weight.grad is not None
+    with torch.no_grad():
+        assert relerr(host(d(xd)[0]), host(y)) <= BF16_TOL
+
+
 def test_linear_token_rejects_what_it_does_not_do(ops):
+    with pytest.raises(ValueError):
+        ops.geglu(torch.zeros(4, 33, device="cuda"))
     t = torch.bfloat16
     with pytest.raises(ValueError):
         ops.linear_token(torch.zeros(8, 16, device="cuda", dtype=t), torch.zeros(5, 16, device="cuda", dtype=t))

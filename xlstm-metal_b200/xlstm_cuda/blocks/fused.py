@@ -1,0 +1,25 @@
+"""When a fused launch may stand in for calls of modules.
+
+The fused kernels have no backward and read the weights of the modules they replace.  They are taken where nobody can tell the
+difference: no gradient is recorded, and each of those modules is the class the kernel restates, with nothing attached to its call.
+"""
+from __future__ import annotations
+
+from typing import Tuple
+
+import torch
+import torch.nn as nn
+from torch.nn.modules import module as _module
+
+
+def may_fuse(owner: nn.Module, x: torch.Tensor, *replaced: Tuple[nn.Module, type]) -> bool:
+    """``replaced``: the modules whose calls the fused launch leaves out, with the class each is expected to be."""
+    if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in owner.parameters())):
+        return False
+    if _module._global_forward_hooks or _module._global_forward_pre_hooks:
+        return False
+    return all(type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+               for m, cls in replaced)
+
+
+__all__ = ["may_fuse"]

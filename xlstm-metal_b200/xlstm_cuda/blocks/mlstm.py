@@ -25,6 +25,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from ..utils import resolve_dtype
+from .fused import may_fuse
 from .rms_norm import MultiHeadRMSNorm, RMSNormCell
 from .soft_cap import SoftCap
 
@@ -417,9 +418,14 @@ class mLSTMBlock(nn.Module):
     def _token_step_ok(self, x: torch.Tensor) -> bool:
         if getattr(self.mlstm_cell, "_shard", None) is not None:
             return False   # the single-token launch sequence has no gather step
+        cell = self.mlstm_cell
         return (x.shape[1] == 1 and x.dtype == torch.bfloat16 and
-                self.mlstm_cell._fused_weights() is not None and self._fused_ffn() is not None and
-                self.mlstm_cell.compute_dtype == torch.bfloat16)
+                cell._fused_weights() is not None and self._fused_ffn() is not None and
+                cell.compute_dtype == torch.bfloat16 and
+                (x.shape[0] <= ops.LINEAR_TOKEN_MAX_ROWS or
+                 may_fuse(self, x, (self.norm_mlstm, RMSNormCell), (cell, mLSTMNeuron),
+                          (cell.parallel_kernel, mLSTMParallelKernelCell), (cell.recurrent_kernel, mLSTMRecurrentKernelCell),
+                          (cell.output_cell.out_proj, nn.Linear), (self.ffn_proj_down, nn.Linear))))
 
     def forward(self, x: torch.Tensor, state: Optional[State] = None):
         if self._token_step_ok(x):

@@ -23,6 +23,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
+from .fused import may_fuse
 from .rms_norm import RMSNormCell
 from .soft_cap import soft_cap
 
@@ -171,7 +172,11 @@ class sLSTMBlock(nn.Module):
 
     def forward(self, x: torch.Tensor, state=None):
         out, new_state = self.slstm_cell(self.norm_slstm(x), state)
-        x, xn = ops.add_rms_norm(x, out, self.norm_ffn.weight, self.norm_ffn.eps)   # residual + pre-norm
+        if may_fuse(self, x, (self.norm_ffn, RMSNormCell)):
+            x, xn = ops.add_rms_norm(x, out, self.norm_ffn.weight, self.norm_ffn.eps)   # residual + pre-norm
+        else:
+            x = x + out
+            xn = self.norm_ffn(x)
         x = x + self.ffn_proj_down(ops.swiglu(self.ffn_proj_up_gate(xn), self.ffn_proj_up(xn)))
         return x, new_state
 
@@ -300,7 +305,8 @@ class sLSTMBlockDiag(nn.Module):
         out = self.hid_norm(hs)
         Wu, bu, Wd, Pp = self._ffn_weights()
         y = F.linear(out, Wu, bu)
-        out = F.linear(ops.geglu(y), Wd, self.down_proj.bias) + xs
+        act = ops.geglu(y) if may_fuse(self, y) else y[..., :Pp] * F.gelu(y[..., Pp:])
+        out = F.linear(act, Wd, self.down_proj.bias) + xs
         return (out[:, 0] if single else out), state
 
     def _ffn_weights(self):

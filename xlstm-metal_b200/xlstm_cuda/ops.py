@@ -336,6 +336,8 @@ def geglu(x: torch.Tensor) -> torch.Tensor:
     """``x[..., :P] * gelu(x[..., P:])`` over the last dimension of size ``2 P`` (``P`` a multiple of 16 bytes)."""
     _need_cuda(x)
     P = x.shape[-1] // 2
+    if P == 0 or x.shape[-1] % 2:
+        raise ValueError(f"geglu takes rows [value | gate] of one width, got {x.shape[-1]} columns")
     xc = x.contiguous()
     y = torch.empty(*x.shape[:-1], P, dtype=x.dtype, device=x.device)
     _lib.check(_lib.load().xlstm_geglu(xc.data_ptr(), y.data_ptr(), y.numel() // P, P, _dtype_code(xc), _stream()), "xlstm_geglu")
