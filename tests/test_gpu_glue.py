@@ -324,6 +324,23 @@ def test_block_token_step_matches_separate_launches(ops, B):
         assert relerr(host(a), host(b)) <= BF16_TOL
 
 
+@pytest.mark.parametrize("B", [4, 8])
+def test_block_token_step_with_weights_at_odd_offsets(ops, B):
+    """Weights that are views at an odd offset, or transposed: the streaming kernels do not take them, the block does."""
+    m, _, _ = _blocks()
+    x = torch.randn(B, 1, 512, device="cuda", dtype=torch.bfloat16)
+    with torch.inference_mode():
+        y = m(x)[0]
+    out, down = m.mlstm_cell.output_cell.out_proj, m.ffn_proj_down
+    down.weight.data = down.weight.data.T.contiguous().T
+    if B > 4:
+        flat = torch.empty(out.weight.numel() + 1, device="cuda", dtype=torch.bfloat16)
+        flat[1:] = out.weight.data.reshape(-1)
+        out.weight.data = flat[1:].view_as(out.weight)
+    with torch.inference_mode():
+        assert relerr(host(m(x)[0]), host(y)) <= BF16_TOL
+
+
 def _blocks():
     from xlstm_cuda.blocks import mLSTMBlock, sLSTMBlock, sLSTMBlockDiag
     t = torch.bfloat16

@@ -405,7 +405,10 @@ class mLSTMBlock(nn.Module):
         return x3.view_as(x), rk._cast_state(new_state)
 
     def _rows_ok(self) -> bool:
-        return all(K % 32 == 0 for K in (self.embedding_dim, self.hidden_size, self.ffn_hidden_dim))
+        """The streaming kernel takes dense weights on 16-byte boundaries (the fused matrices are) and K in whole blocks."""
+        return (all(w.data_ptr() % 16 == 0 and w.is_contiguous()
+                    for w in (self.mlstm_cell.output_cell.out_proj.weight, self.ffn_proj_down.weight)) and
+                all(K % 32 == 0 for K in (self.embedding_dim, self.hidden_size, self.ffn_hidden_dim)))
 
     def shard_heads(self, rank: int, world: int, group=None) -> None:
         """Head-sharded mLSTM layer (see ``mLSTMNeuron.shard_heads``); norms and the FFN stay replicated."""
