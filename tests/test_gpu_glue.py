@@ -283,6 +283,18 @@ def test_linear_rows(ops, M, N, K):
     assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
 
 
+@pytest.mark.parametrize("K", [32, 64, 288, 1024])
+def test_linear_rows_keeps_infinities(ops, K):
+    """An infinite weight gives an infinite result in its row and none elsewhere, also in the last block of k."""
+    t = torch.bfloat16
+    torch.manual_seed(K)
+    x = torch.rand(5, K, device="cuda").to(t) + 0.5
+    W = torch.randn(40, K, device="cuda").to(t)
+    W[7, K - 1], W[33, 0] = float("inf"), float("-inf")
+    y = ops.linear_rows(W, x)
+    assert torch.equal(torch.isinf(y), torch.isinf(x.float() @ W.float().T)) and not torch.isnan(y).any()
+
+
 def test_linear_rows_reads_weights_written_just_before(ops):
     """A weight that the launch right before the call writes (an update in place; the dense copy that the call itself makes of a
     transposed one, also where the caller vouches for the weight it passes) is not read early."""

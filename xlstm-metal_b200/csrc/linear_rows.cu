@@ -57,10 +57,10 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
 
     // a ring of LR_U k blocks: slot u is refilled as soon as its block has been multiplied
     uint4 wr[LR_U][4], xr[LR_U][2];
+    // blocks beyond the end are zeros in both operands (0 times an infinite weight would be a NaN)
     auto load_w = [&](int u, int b) {
-        b = min(b, blocks - 1);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) wr[u][r] = ldg_weights(wp[r] + (size_t)b * 32);
+        for (int r = 0; r < 4; ++r) wr[u][r] = b < blocks ? ldg_weights(wp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
     };
     auto load_x = [&](int u, int b) {
 #pragma unroll
