@@ -6,6 +6,7 @@
 // kernels - one CTA of 16 warps per SM, inputs arriving through per-lane rings of 16-byte cp.async slots in
 // shared memory a fixed distance ahead, so the bytes in flight do not depend on the register allocation.
 #include "common.cuh"
+#include "cp_async.cuh"
 #include "vec16.cuh"
 
 namespace xl {
@@ -21,15 +22,6 @@ template <typename T> __device__ __forceinline__ float silu_t(float x) {
     if (sizeof(T) == 2) return __fdividef(x, 1.0f + __expf(-x));
     return x / (1.0f + expf(-x));
 }
-
-// 16-byte asynchronous copies global -> shared memory; a thread that only ever reads back the slots it filled
-// itself needs no barrier, only the wait on its own copy groups
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                 :: "r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
 // ---------------------------------------------------------------------------
 // RMSNorm: one CTA per row, the row cached in registers (NV 16-byte vectors per thread)

@@ -17,39 +17,19 @@
 //
 // Exponents are differences u_s - x_t <= 0 with u = i - b, x = max(m, running max of u) and b the summed log forget
 // gates of the chunk, kept in double until the difference is taken (b reaches 1e3 in a chunk of closed gates).
+#include "cp_async.cuh"
 #include "mlstm_chunkwise.cuh"
+#include "packed_f32.cuh"
 
 namespace xl {
 namespace {
 
-typedef unsigned long long u64;
 constexpr int CH = 64;          // tokens per chunk: distance of the stored states
 constexpr int TT = 32;          // tokens per tile of the state kernel: one lane of the gate warp each
 constexpr int JT = 64;          // rows of C per CTA of the state kernel
 constexpr int KP = 16;          // rows of dqk per piece of the output kernel
 constexpr int MAIN = 128;       // threads of the products: 8 row groups x 16 column groups
 constexpr size_t SLOT_BYTES = (size_t)192 << 20;
-
-__device__ __forceinline__ u64 ffma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ u64 fmul2(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 pack2(float x, float y) {
-    u64 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float2 unpack2(u64 v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
-}
 
 struct F32Params {
     ChunkwiseParams p;
@@ -98,13 +78,6 @@ __device__ __forceinline__ GateTile gate_tile(const GateRaw &r, float cap, int l
     }
     return g;
 }
-
-// 16 bytes global -> shared memory, zeros if not ok; arrives by cp_async_wait_all() in the issuing thread
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-                 "r"(ok ? 16u : 0u) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename T> __device__ __forceinline__ float4 ld4_or_zero(const T *ptr, bool ok) {
     return ok ? ld4(ptr) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -346,7 +319,7 @@ __global__ void __launch_bounds__(MAIN, 2) mlstm_f32_output_kernel(const F32Para
             for (int i = 0; i < CV; ++i) {
                 const int e = tid + i * MAIN, j = j0 + e / (DVT / 4), cc = (e % (DVT / 4)) * 4;
                 const bool ok = j < p.dqk && col0 + cc < p.dv;
-                cp_async16(reinterpret_cast<float4 *>(sC + buf * KP * DVT) + e, Cs + (ok ? (size_t)j * p.dv + col0 + cc : 0), ok);
+                cp_async16((uint32_t)__cvta_generic_to_shared(reinterpret_cast<float4 *>(sC + buf * KP * DVT) + e), Cs + (ok ? (size_t)j * p.dv + col0 + cc : 0), ok);
             }
         }
     };

@@ -1,9 +1,10 @@
 // Pieces shared by the kernels of the block-diagonal recurrent sLSTM whose CTAs exchange h_t through the shared memory of
-// their cluster: remote stores that complete bytes on the receiver's mbarrier, the bounded wait for them, cp.async.
+// their cluster: remote stores that complete bytes on the receiver's mbarrier, the bounded wait for them.
 #pragma once
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "cp_async.cuh"
 #include "tcgen05.cuh"
 
 namespace cg = cooperative_groups;
@@ -23,11 +24,6 @@ __device__ __forceinline__ void st_async16(uint32_t dst, uint32_t bar, const uin
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];"
                  ::"r"(dst), "r"(bar), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // bounded wait for bytes that other CTAs of the cluster write (hence the cluster-scope acquire); see tc::mbar_wait
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity, uint32_t ns) {

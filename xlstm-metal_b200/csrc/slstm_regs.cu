@@ -10,27 +10,21 @@
 //
 // R in shared memory (slstm.cu, kept for other head sizes) costs a shared-memory load per multiply-add group and has two
 // barriers per step, one of them across the cluster; half of its threads have no column at DH = 256.
+#include "packed_f32.cuh"
 #include "slstm_cluster.cuh"
 
 namespace xl {
 namespace {
 using namespace rec;
 
-typedef unsigned long long u64;
 constexpr int GU = 32;                 // units per CTA
 constexpr int GCOL = 4 * GU;           // gate columns per CTA
 constexpr int GK = 64;                 // k's per thread
 constexpr int BG = 4;                  // batch rows per cluster (8 doubled the step and saved no wave of clusters)
 
-__device__ __forceinline__ u64 ffma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 __device__ __forceinline__ float sum2(u64 v) {
-    float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-    return x + y;
+    const float2 f = unpack2(v);
+    return f.x + f.y;
 }
 
 template <int DH>
