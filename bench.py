@@ -3,7 +3,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-Headline workload (BASELINE configs[1]): the mLSTM decode step at the xLSTM-7B head shape,
+Headline workload: the mLSTM decode step at the xLSTM-7B head shape,
 B=16, NH=8, dqk=256, dv=512, bf16 activations, fp32 state.  A "step" is one decode step of the
 cell for the whole batch (16 tokens).  Consecutive steps walk a ring of independent layer
 states (8 layers x 2 buffers = 1 GiB), so every step streams a state that is cold in the
@@ -12,14 +12,14 @@ states (8 layers x 2 buffers = 1 GiB), so every step streams a state that is col
 ``value``  tokens/s with inputs resident in HBM (kernel launched straight through the C ABI).
 ``e2e``    tokens/s through the public tensor API with HOST inputs: pinned host -> device copies
            of q,k,v,i,f and a device -> host read of h inside the timed region, every step.
-``prefill``  chunkwise prefill of BASELINE configs[3] (B=4, S=32768, heads sharded over the
+``prefill``  chunkwise prefill (B=4, S=32768, heads sharded over the
            ranks, NCCL all-gather of h, 4096x4096 out-projection), reported beside the headline.
 At N > 1 the decode batch is sharded (global batch 16*N, no collective): weak scaling.
 ``--impl reference`` times the reference's own torch_native recurrent cell (the unmodified class, placed
 under oracle/_ref by oracle/make_ref.py) on all host cores for the same workload at the same global
 batch; where that file is absent it times the C restatement (oracle/, OpenMP over batch x heads).
 The JSON line stays short: the prefill / sLSTM / soft-cap figures ride inside ``roofline``; the long
-per-kernel tables (glue kernels, 7B-shaped model) go to ``bench_details_n{N}.json`` in the run's output folder.
+per-kernel tables (glue kernels, 7B-shaped model) go to ``bench_details_n{N}.json`` in the folder that ``--details`` names.
 """
 from __future__ import annotations
 
@@ -39,7 +39,7 @@ for _p in (ROOT, ROOT / "xlstm-metal_b200"):
 B, NH, DQK, DV = 16, 8, 256, 512
 N_LAYERS = 8          # ring of independent layer states (cold-L2 rule)
 N_INPUT_SETS = 64     # distinct per-step inputs cycled through
-WORKLOAD = "mlstm_decode_step B=16 NH=8 dqk=256 dv=512 bf16 act fp32 state (BASELINE configs[1])"
+WORKLOAD = "mlstm_decode_step B=16 NH=8 dqk=256 dv=512 bf16 act fp32 state"
 
 
 def workload_config(world):
@@ -407,8 +407,8 @@ def run_ours(args):
             "nccl_variant_ms": prefill["nccl_allgather_variant_ms"], "world": world,
             "gather_check": prefill["gather_check"], "gather_gbs_per_rank": prefill["gather_gbs_per_rank"],
             "token_sharded_outproj_ms": prefill["token_sharded_outproj_ms"], "token_sharded_check": prefill["token_sharded_check"],
-            "workload": f"B=4 S={args.prefill_seq} NH=8 256/512 bf16 (BASELINE configs[3]), heads x{world}",
-            "kernel": "mlstm_chunkwise_tc_kernel", "bound": "tensor"}
+            "workload": f"B=4 S={args.prefill_seq} NH=8 256/512 bf16, heads x{world}",
+            "kernel": "mlstm_chunkwise_tc_fast_kernel", "bound": "tensor"}
         details["prefill"] = prefill
     launches = K
     if not args.no_extras:
@@ -445,12 +445,10 @@ def run_ours(args):
         line["cpu_baseline"] = cpu_baseline() if world == 1 and not args.no_cpu else None
         line["roofline"] = roofline
         print(json.dumps(line), flush=True)
-        try:    # the long per-kernel tables: a file beside the run, not part of the line
-            out = ROOT / "gpurun_out"
-            out.mkdir(exist_ok=True)
+        if args.details:    # the long per-kernel tables: a file beside the run, not part of the line
+            out = Path(args.details)
+            out.mkdir(parents=True, exist_ok=True)
             (out / f"bench_details_n{world}.json").write_text(json.dumps({"line": line, "details": details}, indent=1))
-        except OSError:
-            pass
     if world > 1:
         dist.destroy_process_group()
 
@@ -461,7 +459,7 @@ TRAFFIC_PER_LAUNCH = 84_321_792   # 67.52 MB read + 16.80 MB written before the 
 
 
 def run_prefill(torch, dist, ops, device, world, rank, args):
-    """B=4, S=32768, NH=8, 256/512, L=64, bf16; heads sharded over the ranks,
+    """Chunkwise prefill: B=4, S=32768, NH=8, 256/512, L=64, bf16; heads sharded over the ranks,
     all-gather of h, then the replicated 4096x4096 out-projection.  Strong scaling."""
     Bp, Sp, L = 4, args.prefill_seq, 64
     nh_local = NH // world if NH % world == 0 else NH
@@ -572,7 +570,7 @@ def run_prefill(torch, dist, ops, device, world, rank, args):
     hbm, tf, which = peaks()
     # bytes of h every rank pushes to its peers during the cell (fused gather), over the cell time
     gather_gbs = (world - 1) * Bp * Sp * nh_local * DV * 2 / (cell_ms_gather * 1e-3) / 1e9 if fused is not None else None
-    return {"workload": f"mlstm_chunkwise_prefill B={Bp} S={Sp} NH={NH} dqk={DQK} dv={DV} L={L} bf16 (BASELINE configs[3])",
+    return {"workload": f"mlstm_chunkwise_prefill B={Bp} S={Sp} NH={NH} dqk={DQK} dv={DV} L={L} bf16",
             "parallelism": f"heads sharded x{world}, fused all-gather of h, replicated out-proj", "scaling": "strong",
             "cell_tokens_per_s": tokens / (cell_ms * 1e-3), "cell_ms": cell_ms, "cell_ms_burst": burst_ms, "clocks": prefill_clocks,
             "with_allgather_outproj_tokens_per_s": tokens / (full_ms * 1e-3), "with_allgather_outproj_ms": full_ms,
@@ -600,7 +598,7 @@ def _time_cuda(torch, fn, reps):
 
 
 def run_softcap(torch, ops, device):
-    """Logit soft-cap at the prefill shape of BASELINE configs[2]: [2048, 50304] fp32 (412 MB > L2)."""
+    """Logit soft-cap at a 2048-token prefill: [2048, 50304] fp32 (412 MB > L2)."""
     x = torch.randn(2048, 50304, device=device) * 20
     y = torch.empty_like(x)
     ops.softcap(x, 30.0, out=y)
@@ -686,7 +684,7 @@ def run_glue(torch, ops, device):
 
 
 def run_slstm(torch, dist, device, world, rank):
-    """BASELINE configs[4]: 4 sLSTM blocks with block-diagonal recurrent weights, d=1024, 4 heads x 256,
+    """4 sLSTM blocks with block-diagonal recurrent weights, d=1024, 4 heads x 256,
     B=32 (sharded over the ranks), S=1024, bf16 activations, fp32 state."""
     from xlstm_cuda.blocks import sLSTMBlockDiag
 
@@ -718,14 +716,14 @@ def run_slstm(torch, dist, device, world, rank):
     if world > 1:
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
     ms = float(t.item())
-    return {"workload": "4 sLSTM blocks (block-diagonal R), d=1024, 4x256, B=32, S=1024, bf16 (BASELINE configs[4])",
+    return {"workload": "4 sLSTM blocks (block-diagonal R), d=1024, 4x256, B=32, S=1024, bf16",
             "parallelism": f"batch-sharded x{world}", "scaling": "strong", "ms": ms,
             "tokens_per_s": Bs * world * S / (ms * 1e-3), "us_per_step_per_block": ms * 1e3 / (4 * S),
             "bound": "latency (sequential through h_{t-1}); includes the input-side GEMMs, norms and FFN of each block"}
 
 
 def run_model(torch, device, prompt_len, new_tokens):
-    """BASELINE configs[2]: xLSTM-7B-shaped random-init model, prefill then greedy decode, B=1."""
+    """xLSTM-7B-shaped random-init model, prefill then greedy decode, B=1."""
     import tempfile
     from xlstm_cuda.generate import xLSTMRunner
     from xlstm_cuda.utils import XLSTM_7B_CONFIG, write_model_dir
@@ -773,7 +771,7 @@ def run_model(torch, device, prompt_len, new_tokens):
     n_params = sum(p.numel() for p in runner.model.parameters())
     del runner
     torch.cuda.empty_cache()
-    return {"workload": f"xLSTM-7B-shaped random init, B=1, prompt {prompt_len} + {new_tokens} greedy tokens, bf16 (BASELINE configs[2])",
+    return {"workload": f"xLSTM-7B-shaped random init, B=1, prompt {prompt_len} + {new_tokens} greedy tokens, bf16",
             "params": n_params, "prefill_ms": pre_ms, "prefill_tokens_per_s": prompt_len / (pre_ms * 1e-3),
             "decode_ms_per_token": dec_ms / new_tokens, "decode_tokens_per_s": new_tokens / (dec_ms * 1e-3),
             "decode": "CUDA-graph replay of the single-token step", "decode_eager_ms_per_token": eager_ms,
@@ -794,7 +792,8 @@ def main():
     ap.add_argument("--no-model", action="store_true", help="skip the 7B-shaped full-model run")
     ap.add_argument("--glue-only", action="store_true",
                     help="time only the HBM-bound kernels either side of the cells (a small command to profile)")
-    ap.add_argument("--slstm-only", action="store_true", help="run only the sLSTM stack leg (BASELINE configs[4])")
+    ap.add_argument("--details", metavar="DIR", help="write the per-kernel tables into this folder")
+    ap.add_argument("--slstm-only", action="store_true", help="run only the sLSTM stack leg")
     ap.add_argument("--model-only", action="store_true",
                     help="run only the 7B-shaped full-model leg (prefill 2048 + 256 decode tokens)")
     args = ap.parse_args()

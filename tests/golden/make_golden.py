@@ -68,7 +68,7 @@ def main():
     enh = load(ref / "kernel_development/xlstm/implementations/pytorch/xlstm_pytorch_enhanced.py", "ref_enhanced")
     torch.set_grad_enabled(False)
 
-    # ---- mlstm_c1_fp32: BASELINE config 1 ---------------------------------
+    # ---- mlstm_c1_fp32: the smallest cell ---------------------------------
     g = torch.Generator().manual_seed(0)
     B, NH, S, dqk, dv = 1, 4, 256, 64, 64
     q = torch.randn(B, NH, S, dqk, generator=g)

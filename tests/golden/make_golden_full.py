@@ -48,7 +48,7 @@ def block_7b_input(seed: int = 52, tokens: int = 200, dim: int = 4096) -> torch.
 
 def fill_block_7b(blk, seed: int = 51) -> None:
     """Parameters of the 7B-shaped block: ``fill_parameters``, then the matrices brought to the N(0, 0.02) scale
-    that BASELINE configs[2] names (``fill_parameters`` draws them at 0.06 for the small fixtures)."""
+    of the 7B-shaped model (``fill_parameters`` draws them at 0.06 for the small fixtures)."""
     named = dict(blk.named_parameters())
     fill_parameters(named, seed=seed)
     with torch.no_grad():
@@ -142,7 +142,7 @@ def main():
     sblk = enh.sLSTMBlock(cfg).eval()
     named = {k: v for k, v in sblk.named_parameters() if not k.startswith("causal_conv")}
     fill_parameters(named, seed=61)
-    with torch.no_grad():   # recurrent weights at the scale BASELINE configs[4] names
+    with torch.no_grad():   # recurrent weights at the scale of the sLSTM stack
         for nme, prm in named.items():
             if ".R_" in nme or nme.startswith("R_"):
                 prm.mul_(0.02 / 0.3)

@@ -30,7 +30,7 @@ def from_bits(a):
 
 @pytest.mark.parametrize("fused", [True, False])
 def test_mlstm_block_7b_shape_bf16_teacher_forced(golden, fused):
-    """BASELINE configs[2], one layer: the reference mLSTMBlock at D=4096, NH=8 (256/512, FFN 10944) with bf16
+    """The 7B-shaped model, one layer: the reference mLSTMBlock at D=4096, NH=8 (256/512, FFN 10944) with bf16
     parameters (N(0, 0.02) matrices) and compute and fp32 state.  192 tokens (one 128-token tile on the tensor
     cores + a 64-token tail) in one call, then 8 single-token calls through the decode path, all on the
     reference's own input.  The fixture holds the reference's bf16 run AND its fp32 evaluation of the same
@@ -83,7 +83,7 @@ def test_mlstm_block_7b_shape_bf16_teacher_forced(golden, fused):
 
 
 def test_slstm_block_diagonal_config4_shape_bf16(golden):
-    """BASELINE configs[4], one block: d=1024, 4 heads x 256, bf16, B=4, S=64 - the tensor-core recurrence,
+    """The sLSTM stack, one block: d=1024, 4 heads x 256, bf16, B=4, S=64 - the tensor-core recurrence,
     the padded FFN and the fused LayerNorm together.  The reference class
     (kernel_development/xlstm/implementations/pytorch/xlstm_pytorch_enhanced.py:367-488) does not run with bf16
     parameters, so the fixture is its fp32 run on the bf16-rounded parameters and input."""
@@ -110,7 +110,7 @@ def test_slstm_block_diagonal_config4_shape_bf16(golden):
 
 
 def test_chunkwise_config3_full_length_final_state_and_last_tokens():
-    """BASELINE configs[3] length: S = 32768 at 256/512, bf16.  The last 256 tokens of h and the final (C, n, m)
+    """Full length: S = 32768 at 256/512, bf16.  The last 256 tokens of h and the final (C, n, m)
     against the CPU oracle's step-by-step recurrence over all 32768 tokens (follows
     xlstm_metal/torch_native/blocks/mlstm/mlstm_chunkwise/mlstm_recurrent_kernel_cell.py:106-153), through both
     tensor-core kernels."""

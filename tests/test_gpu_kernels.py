@@ -109,7 +109,7 @@ def test_mlstm_step_against_oracle(ops, B, NH, dqk, dv):
 
 
 def test_mlstm_step_config2_256_steps_bf16(ops):
-    """B=16, NH=8, 256/512, bf16 activations, fp32 state, 256 carried steps."""
+    """Decode of a serving batch: B=16, NH=8, 256/512, bf16 activations, fp32 state, 256 carried steps."""
     B, NH, dqk, dv, T = 16, 8, 256, 512, 256
     g = torch.Generator().manual_seed(1)
     C = torch.randn(B, NH, dqk, dv, generator=g) * 0.1
@@ -415,7 +415,7 @@ def test_chunkwise_bf16_extreme_gates_tensor_core_path(ops):
 
 
 def test_chunkwise_full_length_properties(ops):
-    """BASELINE configs[3] length (S = 32768, 256/512, bf16): the oracle cannot run this in seconds, so check
+    """Full length (S = 32768, 256/512, bf16): the oracle cannot run this in seconds, so check
     (a) the first 384 tokens against the oracle, (b) one pass == two half passes with the carried state,
     (c) run-to-run bitwise determinism."""
     B, NH, S, dqk, dv = 1, 4, 32768, 256, 512
@@ -448,6 +448,7 @@ def test_chunkwise_full_length_properties(ops):
     (1, 2, 200, 256, 192, torch.float32, False),   # 64-column CTAs, ragged last chunk
     (2, 8, 1606, 256, 512, torch.float32, True),   # 128-column CTAs, a second group of chunks continuing in place
     (1, 2, 130, 64, 128, torch.bfloat16, True),    # bf16 head shape outside the tensor-core kernels
+    (1, 2, 130, 640, 128, torch.float32, True),    # heads beyond the 512 rows of the one-kernel form
 ])
 def test_chunkwise_fp32_two_kernels(ops, B, NH, S, dqk, dv, dtype, with_state):
     """The fp32 forward at the edges of its tiles, chunks and groups, against the step-by-step oracle."""
@@ -502,6 +503,7 @@ def test_slstm_scan_oracle(ops, B, S, NH, H, dtype):
     (1, 1000, 2, 1024, torch.float32, True),  # many segments, several unit slices, ragged end
     (2, 333, 1, 37, torch.float32, False),    # width without 16-byte vectors
     (1, 1024, 4, 40, torch.bfloat16, True),   # a slice with idle lanes
+    (1, 200, 2, 1028, torch.float32, True),   # more than 1024 units
 ])
 def test_slstm_scan_segments(ops, B, S, NH, H, dtype, with_state):
     """Segments of the sequence in parallel against the oracle, raw gates capped inside, and an in-place state (which

@@ -14,9 +14,8 @@
 // with Q~ = Q * e^{m-x_t} * dqk^-1/2 and K~ = K * e^{u_t-x_last} scaled in place in
 // shared memory after S has consumed the raw tiles.  All exponents are
 // differences that are <= 0 (u_s = i_s - b_s, x_t = max(m, max_{s<=t} u_s)), so
-// nothing can overflow whatever the gates are.  The gate scalars come from a
-// small pre-pass kernel (one warp per head, sequential over tiles) that writes
-// them to caller-provided scratch.
+// nothing can overflow whatever the gates are.  The gate scalars come from the
+// gate pre-pass below, which writes them to caller-provided scratch.
 //
 // Roles (640 threads): warp 0 TMA producer, warp 1 MMA issuer (+TMEM alloc), warp 2 TMA stores of h,
 // warps 4-7 gate matrix P, then q~.n, then the C pass for rows [128,256) of C;
@@ -745,10 +744,11 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
 }
 
 // Two launches over the same (head, segment)s, for the gates of either kind; the choice is the pre-pass's path flag, so it
-// needs no host round trip, and a CTA of the other kind returns at once.  They run side by side: the general launch lets
-// the second one start as soon as its own CTAs have, and that one reads nothing the first has written, so the CTAs of both
-// kinds share the GPU (one after the other, heads with widely spread gates took twice as long).  One kernel with both bodies
-// made the bounded path spill (prefill of 4 x 32768: 1.61 -> 1.71 ms).
+// needs no host round trip, and a CTA of the other kind returns at once.  Up to FUSED_TILES tiles they run side by side: the
+// general launch lets the second one start as soon as its own CTAs have, and that one reads nothing the first has written, so
+// the CTAs of both kinds share the GPU (one after the other, heads with widely spread gates took twice as long); longer
+// sequences run them one after the other, see launch_tc().  One kernel with both bodies made the bounded path spill (prefill of
+// 4 x 32768: 1.61 -> 1.71 ms).
 template <int DQK>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
     grid_dependency_wait();
@@ -775,7 +775,8 @@ int launch_tc(const TcParams &tp, dim3 grid, cudaStream_t st) {
         cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return XLSTM_ERR_CUDA;
     // Long sequences: CTAs that start one by one as the kernel before drains land unevenly on the GPU's clusters of SMs and
-    // stay there for the whole pass (4 x 32768, 128 CTAs: 1.61 -> 1.71 ms), so each launch starts on an idle GPU.
+    // stay there for the whole pass (4 x 32768, 128 CTAs: 1.61 -> 1.71 ms), so each launch starts on an idle GPU.  Measured with
+    // gates of one kind; heads of both kinds pay for it with the sum of the two passes.
     if (tp.NCH > FUSED_TILES) {
         general<<<grid, THREADS, Smem<DQK>::TOTAL, st>>>(tp);
         if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
@@ -825,10 +826,13 @@ constexpr int MIN_SEG_TILES = 2, LONG_SEG_TILES = 16;
 // three more launches.  Microseconds fitted to forced segment counts at 256/512, 8 to 128 CTAs, 2 to 32 tiles a segment:
 //   one pass    13 + tiles x (4.55 up to 32 CTAs, 5.3 at 64, 6.75 at 128)
 //   two passes  35 + tiles of a segment x (7.1 at 64 CTAs, 9 at 128)
-// and with segments of less than LONG_SEG_TILES a quarter has to be gained (less is not worth states of 0.5 MB per head and
-// segment): 8 heads, S = 4096: 167 us in one
-// pass, 109 in 4 segments; 4 heads, S = 2048: 84 and 54 (8); 2 heads, S = 8192: 283, 127 in 4 segments and 72 in 16; but 8
-// heads, S = 2048: 85 and 74 (4), S = 1024: 51 and 54.  128/256 follows the same order (S = 8192, 4 heads: 250 and 51).
+// With segments of less than LONG_SEG_TILES a quarter has to be gained.  That is a choice for steady results and not for speed:
+// cutting moves the bf16 copy of C to other frames, and after the 16 blocks of a model the last states differ by 3e-2 from those
+// of one pass (the distance of any two correct bf16 evaluations there), which smaller gains were not given.  8 heads,
+// S = 4096: 167 us in one pass, 109 in 4 segments; 4 heads, S = 2048: 84 and 54 (8); 2 heads, S = 8192: 283, 127 in 4 segments
+// and 72 in 16; 8 heads, S = 2048, which the quarter keeps in one pass: 85 and 74 (4), S = 1024: 51 and 54.  The fit knows
+// bounded gates at 256/512 only: 128/256 follows the same order (S = 8192, 4 heads: 250 and 51), the general path costs 7.5 us
+// a tile where the bounded one costs 4.55.
 int plan_segments(int BH, int dv, int nch) {
     const int ctas = BH * (dv / DVS);
     int pmax = SM_COUNT / ctas;

@@ -355,9 +355,11 @@ class mLSTMBlock(nn.Module):
         its norm / bias / residual / SwiGLU folded in, so a block is five launches: projections, cell step with the
         output epilogue, out-projection, FFN up, FFN down.  Up to 16 the streaming kernel multiplies on the tensor cores
         (the CUDA-core one is bound by its multiply-adds from 3 rows on: 143 us for the four Linears of a 4096-wide block at 4
-        rows, 99 us on the tensor cores) and the two norms are launches of their own; beyond that the Linears are GEMMs (with
-        the separate gate and add 97 us at 8 rows and 92 at 16, against 96 and 98 streamed, but two more launches: 16
-        sequences through 8 blocks without a graph 1.54 ms against 1.31).  The cell step reads q, k, v and the gates where
+        rows, 99 us on the tensor cores) and the two norms are launches of their own; beyond that the Linears are GEMMs.
+        The line at 16 is drawn for calls without a graph, where two launches less count more than the Linears: 16 sequences
+        through 8 blocks take 1.31 ms streamed and 1.54 with GEMMs.  In a captured loop a block of 8 takes 125 us (133 as
+        separate launches), of 16 138 streamed, and GEMMs would be ahead from about 9 on (17 sequences: 129).
+        More than 4 sequences come here only where may_fuse() allows it.  The cell step reads q, k, v and the gates where
         the merged projection has written them."""
         cell = self.mlstm_cell
         W, b = cell._fused_weights()

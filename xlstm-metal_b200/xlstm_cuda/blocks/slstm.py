@@ -258,7 +258,7 @@ class sLSTMBlockDiag(nn.Module):
     reference's ``xLSTMConfig`` works as is).  ``forward(x [B,S,D] or [B,D], hidden_state=None)``
     returns ``(out, (c, n, h, m))`` with state tensors ``[B, head_num*head_dim]``.  The input-side
     projections are batched GEMMs over the whole sequence; the recurrence over ``t`` is one
-    kernel launch with the recurrent matrices resident in shared memory.
+    kernel launch with the recurrent matrices resident on chip.
     """
 
     def __init__(self, config):

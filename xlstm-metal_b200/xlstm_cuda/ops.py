@@ -109,7 +109,7 @@ def chunkwise_status(workspace: Optional[torch.Tensor] = None) -> None:
 
 
 def slstm_recurrent_status() -> None:
-    """The same for the tensor-core path of ``slstm_recurrent`` (all launches since the last query)."""
+    """The same for ``slstm_recurrent`` with head sizes 64, 128 and 256 (all launches since the last query)."""
     _lib.check(_lib.load().xlstm_slstm_recurrent_status(_stream()), "xlstm_slstm_recurrent_status")
 
 
