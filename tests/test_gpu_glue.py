@@ -262,6 +262,57 @@ def test_geglu_matches_separate_ops(ops, rows, cols, dtype):
     assert relerr(host(ops.geglu(x)), host(ref)) <= (2.0 ** -7 if dtype == torch.bfloat16 else 1e-6)
 
 
+@pytest.mark.parametrize("rows,groups,cols", [(1, 1, 8), (3, 4, 1024), (37, 1, 1368), (2, 1, 8192), (1500, 1, 4096), (700, 2, 2056), (5, 1, 512)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_layer_norm(ops, rows, groups, cols, dtype):
+    """A vector a row, the widths at which a lane holds another number of vectors, a warp and a CTA a row; rows far from zero
+    mean.  fp32: sums of up to 8192 terms, bf16: one rounding (2^-8 of the value) of a result within 1e-5 of the exact one."""
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, groups * cols, device="cuda") * 2 + 5).to(dtype)
+    w, b = (torch.randn(groups * cols, device="cuda").to(dtype) for _ in range(2))
+    assert ops.layer_norm_takes(x, w, b, groups)
+    y = ops.layer_norm(x, w, b, 1e-6, groups).double().cpu()
+    x64, w64, b64 = (t.double().cpu() for t in (x, w, b))
+    ref = torch.nn.functional.group_norm(x64, groups, w64, b64, 1e-6)
+    off = (y - ref).abs()
+    assert bool((off <= (2.0 ** -8 * ref.abs() if dtype == torch.bfloat16 else 0) + 1e-5 * (1 + w64.abs())).all()), float(off.max())
+
+
+def test_layer_norm_takes_what_the_kernel_does(ops):
+    x, w = torch.zeros(4, 64, device="cuda"), torch.zeros(64, device="cuda")
+    assert not ops.layer_norm_takes(x, w.bfloat16(), w, 1) and not ops.layer_norm_takes(x, None, w, 1)
+    assert not ops.layer_norm_takes(x.t(), w, w, 1) and not ops.layer_norm_takes(x, w, w, 32)          # 8-byte blocks
+    assert not ops.layer_norm_takes(torch.zeros(257, device="cuda")[1:].view(4, 64), w, w, 1)          # odd offset
+    with pytest.raises(Exception):
+        ops.layer_norm(torch.zeros(4, 6, device="cuda"), torch.zeros(6, device="cuda"), torch.zeros(6, device="cuda"))
+
+
+def test_norms_of_the_slstm_blocks_are_their_modules(ops):
+    """The fused norm stands in for the module only where nobody can tell: hooks, gradients, autocast and function transforms
+    see the module."""
+    from xlstm_cuda.blocks.slstm import sLSTMOutputCell
+    torch.manual_seed(0)
+    cell = sLSTMOutputCell(256, 4, 64).cuda()
+    with torch.no_grad():
+        cell.group_norm.weight.normal_()
+        cell.group_norm.bias.normal_()
+    h = torch.randn(2, 9, 4, 64, device="cuda")
+    with torch.inference_mode():
+        fused = cell(h)
+        seen = []
+        handle = cell.group_norm.register_forward_hook(lambda *a: seen.append(1))
+        plain = cell(h)
+        handle.remove()
+        assert seen and relerr(host(fused), host(plain)) <= 1e-5
+    h2 = h.clone().requires_grad_()
+    cell(h2).sum().backward()
+    assert h2.grad is not None and cell.group_norm.weight.grad is not None
+    with torch.no_grad():
+        _, tangent = torch.func.jvp(cell, (h,), (torch.ones_like(h),))
+        assert torch.isfinite(tangent).all()
+        assert relerr(host(torch.func.vmap(cell)(torch.stack([h, h]))[1]), host(plain)) <= 1e-5
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 4096, 4096), (5, 33, 64), (9, 264, 10944), (16, 31, 32), (1, 1, 288), (12, 50, 2080)])
 def test_linear_rows(ops, M, N, K):
     """Rows around the 8-row halves of the x operand, weight rows and k blocks around a CTA's and a warp's share."""

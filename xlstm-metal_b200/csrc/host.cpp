@@ -259,6 +259,23 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
     return py::make_tuple(rc, s, y);
 }
 
+// LayerNorm of each of `groups` column blocks of the rows of x; the status says if the kernel does not take the layout
+py::tuple layer_norm(const Tensor &x, const Tensor &weight, const Tensor &bias, double eps, int64_t groups) {
+    need_cuda(x); need_cuda(weight); need_cuda(bias);
+    const int64_t width = x.size(-1);
+    need(groups > 0 && width % groups == 0, "a row must split into equal groups");
+    need(weight.numel() == width && bias.numel() == width, "norm weight and bias must have one element per column");
+    const Tensor xc = x.contiguous();
+    const Tensor w = weight.to(xc.scalar_type()).contiguous(), b = bias.to(xc.scalar_type()).contiguous();
+    const Tensor y = at::empty_like(xc);
+    const int dt = dtype_code(xc);
+    const int rc = unlocked([&] {
+        return xlstm_layer_norm(xc.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), width ? xc.numel() / width : 0,
+                                (int)groups, (int)(width / groups), (float)eps, dt, stream());
+    });
+    return py::make_tuple(rc, y);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -268,4 +285,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("linear_token", &linear_token);
     m.def("rms_norm", &rms_norm);
     m.def("add_rms_norm", &add_rms_norm);
+    m.def("layer_norm", &layer_norm);
 }

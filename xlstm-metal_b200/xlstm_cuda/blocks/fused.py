@@ -9,7 +9,17 @@ from typing import Tuple
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad as _forward_ad
 from torch.nn.modules import module as _module
+
+
+def plain_tensor(x: torch.Tensor) -> bool:
+    """Whether ``x`` is an ordinary tensor whose memory a kernel may be handed: not a subclass, not wrapped by a function
+    transform (vmap, grad, jvp) or a forward-mode level, not being traced or compiled, and not under autocast (which would
+    pick another type for the module)."""
+    return (type(x) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(x) and
+            _forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and
+            not torch.is_autocast_enabled(x.device.type))
 
 
 def may_fuse(owner: nn.Module, x: torch.Tensor, *replaced: Tuple[nn.Module, type]) -> bool:
@@ -22,4 +32,4 @@ def may_fuse(owner: nn.Module, x: torch.Tensor, *replaced: Tuple[nn.Module, type
                for m, cls in replaced)
 
 
-__all__ = ["may_fuse"]
+__all__ = ["may_fuse", "plain_tensor"]

@@ -23,9 +23,17 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
-from .fused import may_fuse
+from .fused import may_fuse, plain_tensor
 from .rms_norm import RMSNormCell
 from .soft_cap import soft_cap
+
+
+def _norm(owner: nn.Module, norm: nn.Module, kind: type, x: torch.Tensor, groups: int = 1) -> torch.Tensor:
+    """``norm(x)`` on the last dimension: as one launch where nothing tells it from the module, else the module itself."""
+    if (may_fuse(owner, x, (norm, kind)) and plain_tensor(x) and
+            ops.layer_norm_takes(x, norm.weight, norm.bias, groups)):
+        return ops.layer_norm(x, norm.weight, norm.bias, norm.eps, groups)
+    return norm(x)
 
 
 class sLSTMStepwiseKernelCell(nn.Module):
@@ -114,7 +122,10 @@ class sLSTMOutputCell(nn.Module):
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
         B, S, NH, H = h.shape
-        return self.out_proj(self.group_norm(h.reshape(B * S, NH * H)).view(B, S, NH * H))
+        # groups of contiguous channels: a LayerNorm per head (the library's group norm and its affine pass took 341 us for
+        # 8192 tokens of 4 x 1024, this one reads and writes h once)
+        hn = _norm(self, self.group_norm, nn.GroupNorm, h.reshape(B * S, NH * H), self.group_norm.num_groups)
+        return self.out_proj(hn.view(B, S, NH * H))
 
 
 class sLSTMNeuron(nn.Module):
@@ -293,7 +304,7 @@ class sLSTMBlockDiag(nn.Module):
         single = x.dim() == 2
         xs = x.unsqueeze(1) if single else x
         B, S, _ = xs.shape
-        xn = self.inp_norm(xs)
+        xn = _norm(self, self.inp_norm, nn.LayerNorm, xs)
         # gate order of the kernel: i, f, z, o.  One GEMM over the four stacked input projections writes
         # gx [B,S,4,D] directly (no stack copy of four [B,S,D] results)
         Wg = torch.cat([self.W_i.weight, self.W_f.weight, self.W_z.weight, self.W_o.weight], dim=0)
@@ -302,7 +313,7 @@ class sLSTMBlockDiag(nn.Module):
         Rs, rbs = zip(*(lin.stacked() for lin in (self.R_i, self.R_f, self.R_z, self.R_o)))
         R, rb = torch.stack(Rs), torch.stack(rbs)
         hs, state = ops.slstm_recurrent(gx, R, rb, hidden_state, self.head_num, self.config.gate_soft_cap)
-        out = self.hid_norm(hs)
+        out = _norm(self, self.hid_norm, _HiddenLayerNorm, hs)
         Wu, bu, Wd, Pp = self._ffn_weights()
         y = F.linear(out, Wu, bu)
         act = ops.geglu(y) if may_fuse(self, y) else y[..., :Pp] * F.gelu(y[..., Pp:])

@@ -280,6 +280,26 @@ def add_rms_norm(x: torch.Tensor, residual: torch.Tensor, weight: Optional[torch
     return s, y
 
 
+def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5, groups: int = 1) -> torch.Tensor:
+    """Affine LayerNorm of each of ``groups`` equal column blocks of the last dimension (``groups`` = 1: ``nn.LayerNorm``;
+    heads: ``nn.GroupNorm`` over ``[tokens, heads * H]``); a block is a multiple of 16 bytes, at most 32 KB wide."""
+    rc, y = _lib.host().layer_norm(x, weight, bias, eps, groups)
+    if rc:
+        _lib.check(rc, "xlstm_layer_norm")
+    return y
+
+
+def layer_norm_takes(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Optional[torch.Tensor], groups: int = 1) -> bool:
+    """Whether ``layer_norm`` has a kernel for these operands (dense, of one type, 16-byte aligned blocks up to 32 KB)."""
+    if weight is None or bias is None or x.dtype not in _DT or weight.dtype != x.dtype or bias.dtype != x.dtype:
+        return False
+    if not (x.is_cuda and weight.is_cuda and bias.is_cuda and x.is_contiguous() and weight.is_contiguous() and bias.is_contiguous()):
+        return False
+    nbytes = x.shape[-1] // groups * x.element_size()
+    return (x.numel() > 0 and weight.numel() == bias.numel() == x.shape[-1] and x.shape[-1] % groups == 0 and nbytes % 16 == 0 and nbytes <= 32768 and
+            (x.data_ptr() | weight.data_ptr() | bias.data_ptr()) % 16 == 0)
+
+
 def mlstm_output_gate(h: torch.Tensor, ogate: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6) -> torch.Tensor:
     """Per-head RMS norm of ``h [B,NH,S,dv]`` (any strides with a contiguous last dimension) times the
     flat ``weight [NH*dv]`` times ``sigmoid(ogate [B,S,NH*dv])`` -> ``[B,S,NH*dv]``.  ``ogate`` may be a
