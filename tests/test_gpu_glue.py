@@ -313,6 +313,46 @@ def test_norms_of_the_slstm_blocks_are_their_modules(ops):
         assert relerr(host(torch.func.vmap(cell)(torch.stack([h, h]))[1]), host(plain)) <= 1e-5
 
 
+@pytest.mark.parametrize("B,S,C,NH", [(1, 1, 32, 4), (2, 3, 64, 1), (1, 16, 1024, 4), (3, 17, 416, 2), (1, 77, 4096, 4),
+                                      (4, 1801, 128, 3), (2, 3555, 64, 4)])
+@pytest.mark.parametrize("cap,bias", [(15.0, True), (None, False)])
+def test_slstm_gates(ops, B, S, C, NH, cap, bias):
+    """Both tile sizes, tokens around a tile's edge and before the first one, fewer channel blocks than warps.  Against float64
+    on the convolution kernel's own (rounded) result: the sums differ by fp32 summation order, 2^-8 is the one rounding, doubled
+    where the value rounded before the cap sits at a boundary."""
+    torch.manual_seed(S + C)
+    t = torch.bfloat16
+    x = torch.randn(B, S, C, device="cuda").to(t)
+    cw, cb = torch.randn(C, 1, 4, device="cuda").to(t) * 0.5, torch.randn(C, device="cuda").to(t) if bias else None
+    w = [(torch.randn(NH, C, device="cuda") * 2 / C ** 0.5).to(t) for _ in range(3)]
+    b = [torch.randn(NH, device="cuda").to(t) for _ in range(3)]
+    assert ops.slstm_gates_takes(x, cw, cb, w, b)
+    got = ops.slstm_gates(x, cw, cb, w, b, cap)
+    xc = ops.causal_conv1d(x, cw, cb, silu=True)
+    for k, src in enumerate((xc, xc, x)):
+        ref = src.double().cpu() @ w[k].double().cpu().t() + b[k].double().cpu()
+        if cap:
+            ref = cap * torch.tanh(ref / cap)
+        off = (got[k].double().cpu() - ref).abs()
+        assert got[k].shape == (B, S, NH) and bool((off <= 2.0 ** -7 * ref.abs() + 2e-4).all()), (k, float(off.max()))
+
+
+def test_slstm_projection_without_the_convolved_input(ops):
+    """The neuron's path equals the projection cell's, and goes through the modules where they carry hooks."""
+    from xlstm_cuda.blocks.slstm import sLSTMProjectionCell
+    torch.manual_seed(1)
+    pc = sLSTMProjectionCell(256, 4, 64).cuda().bfloat16()
+    x = torch.randn(2, 70, 256, device="cuda").bfloat16()
+    with torch.inference_mode():
+        z, i, f, o, _ = pc(x)
+        for a, b in zip(pc.gates_and_z(x), (z, i, f, o)):
+            assert relerr(host(a), host(b)) <= BF16_TOL
+        seen = []
+        pc.fgate_proj.register_forward_hook(lambda *a: seen.append(1))
+        pc.gates_and_z(x)
+        assert seen
+
+
 @pytest.mark.parametrize("M,N,K", [(16, 4096, 4096), (5, 33, 64), (9, 264, 10944), (16, 31, 32), (1, 1, 288), (12, 50, 2080)])
 def test_linear_rows(ops, M, N, K):
     """Rows around the 8-row halves of the x operand, weight rows and k blocks around a CTA's and a warp's share."""

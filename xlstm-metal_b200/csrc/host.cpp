@@ -276,6 +276,37 @@ py::tuple layer_norm(const Tensor &x, const Tensor &weight, const Tensor &bias, 
     return py::make_tuple(rc, y);
 }
 
+// Gates i, f, o of the packaged sLSTM for all tokens of x [B, S, C]
+py::tuple slstm_gates(const Tensor &x, const Tensor &conv_w, const OptTensor &conv_b, const std::vector<Tensor> &w,
+                      const std::vector<Tensor> &b, double gate_cap) {
+    need_cuda(x); need_cuda(conv_w); need_cuda(conv_b);
+    need(x.dim() == 3 && w.size() == 3 && b.size() == 3, "slstm_gates takes x as [B, S, C] and three weights and biases (i, f, o)");
+    const int64_t B = x.size(0), S = x.size(1), C = x.size(2), NH = w[0].size(0), K = conv_w.size(-1);
+    const int dt = dtype_code(x);
+    const auto type = x.scalar_type();
+    need(conv_w.numel() == C * K && (!conv_b || conv_b->numel() == C), "convolution weight or bias of another size than [C,K], [C]");
+    const Tensor xc = x.contiguous(), cw = conv_w.to(type).contiguous();
+    const OptTensor cb = cast_contiguous(conv_b, type);
+    std::vector<Tensor> keep, gates;
+    const void *wp[3], *bp[3];
+    void *gp[3];
+    for (int k = 0; k < 3; ++k) {
+        need_cuda(w[k]); need_cuda(b[k]);
+        need(w[k].numel() == NH * C && b[k].numel() == NH, "gate weight or bias of another size than [NH,C], [NH]");
+        keep.push_back(w[k].to(type).contiguous());
+        wp[k] = keep.back().data_ptr();
+        keep.push_back(b[k].to(type).contiguous());
+        bp[k] = keep.back().data_ptr();
+        gates.push_back(at::empty({B, S, NH}, x.options()));
+        gp[k] = gates.back().data_ptr();
+    }
+    const int rc = unlocked([&] {
+        return xlstm_slstm_gates(xc.data_ptr(), cw.data_ptr(), ptr(cb), wp, bp, gp, (int)B, (int)S, (int)C, (int)K, (int)NH,
+                                 (float)gate_cap, dt, stream());
+    });
+    return py::make_tuple(rc, gates[0], gates[1], gates[2]);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -286,4 +317,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("rms_norm", &rms_norm);
     m.def("add_rms_norm", &add_rms_norm);
     m.def("layer_norm", &layer_norm);
+    m.def("slstm_gates", &slstm_gates);
 }

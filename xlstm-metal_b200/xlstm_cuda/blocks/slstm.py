@@ -99,6 +99,20 @@ class sLSTMProjectionCell(nn.Module):
     def soft_cap(self, x: torch.Tensor) -> torch.Tensor:
         return x if self.gate_soft_cap is None else soft_cap(x, self.gate_soft_cap)
 
+    def gates_and_z(self, x: torch.Tensor):
+        """``z, i, f, o`` of ``forward`` for callers that do not need the convolved input: where nothing tells it from the
+        separate modules, the convolution and the three gate projections are one launch and its result is never stored."""
+        B, S, _ = x.shape
+        conv, lins = self.conv1d, (self.igate_proj, self.fgate_proj, self.ogate_proj)
+        if (type(conv) is CausalConv1d and type(conv.conv) is nn.Conv1d and conv.depthwise and
+                may_fuse(self, x, (self, sLSTMProjectionCell), (conv, CausalConv1d), *((lin, nn.Linear) for lin in lins)) and
+                plain_tensor(x) and
+                ops.slstm_gates_takes(x, conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins], [lin.bias for lin in lins])):
+            i, f, o = ops.slstm_gates(x, conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins],
+                                      [lin.bias for lin in lins], self.gate_soft_cap)
+            return self.z_proj(x).view(B, S, self.num_heads, self.head_dim), i, f, o
+        return self(x)[:4]
+
     def forward(self, x: torch.Tensor):
         B, S, _ = x.shape
         if self.conv1d is not None:
@@ -148,7 +162,8 @@ class sLSTMNeuron(nn.Module):
         return self.input_size
 
     def forward(self, x: torch.Tensor, state=None):
-        z, i_preact, f_preact, o_preact, _ = self.projection_cell(x)
+        pc = self.projection_cell
+        z, i_preact, f_preact, o_preact = pc.gates_and_z(x) if type(pc) is sLSTMProjectionCell else pc(x)[:4]
         h, state = self.kernel_cell.scan(z, i_preact, f_preact, o_preact, state)  # all S steps, one launch
         return self.output_cell(h), state
 

@@ -385,6 +385,29 @@ def causal_conv1d(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
     return (y, st_out) if return_state else y
 
 
+def slstm_gates(x: torch.Tensor, conv_weight: torch.Tensor, conv_bias: Optional[torch.Tensor], weights, biases,
+                gate_cap: Optional[float] = None):
+    """Gates ``(i, f, o)`` of the packaged sLSTM, each ``[B,S,NH]``, for all tokens of ``x [B,S,C]`` in one pass (bf16):
+    ``i`` and ``f`` project ``silu(causal_conv1d(x))``, ``o`` projects ``x``; all three soft-capped.  ``weights``,
+    ``biases``: the Linears' ``[NH,C]`` and ``[NH]`` in that order; ``NH <= 4``, four taps, ``C`` a multiple of 32."""
+    rc, i, f, o = _lib.host().slstm_gates(x, conv_weight, conv_bias, list(weights), list(biases), gate_cap or 0.0)
+    if rc:
+        _lib.check(rc, "xlstm_slstm_gates")
+    return i, f, o
+
+
+def slstm_gates_takes(x: torch.Tensor, conv_weight: torch.Tensor, conv_bias: Optional[torch.Tensor], weights, biases) -> bool:
+    """Whether ``slstm_gates`` has a kernel for these operands."""
+    ts = [x, conv_weight, *weights, *biases] + ([] if conv_bias is None else [conv_bias])
+    if any(t is None or t.dtype != torch.bfloat16 or not t.is_cuda or not t.is_contiguous() for t in ts):
+        return False
+    C, NH = x.shape[-1], weights[0].shape[0]
+    return (x.dim() == 3 and x.numel() > 0 and conv_weight.shape[-1] == 4 and conv_weight.numel() == 4 * C and NH <= 4 and
+            C % 32 == 0 and all(w.shape == (NH, C) and b.shape == (NH,) for w, b in zip(weights, biases)) and
+            all(t.data_ptr() % 16 == 0 for t in (x, conv_weight, *weights)) and
+            (conv_bias is None or (conv_bias.shape == (C,) and conv_bias.data_ptr() % 16 == 0)))
+
+
 LINEAR_TOKEN_MAX_ROWS = 4
 
 
