@@ -657,11 +657,13 @@ BF, FP = torch.bfloat16, torch.float32
 
 @pytest.mark.parametrize("B,S,NH,dh,dtype", [(1, 1, 1, 64, BF), (16, 2, 2, 64, BF), (17, 3, 4, 128, BF), (5, 64, 2, 128, BF),
                                              (16, 1, 1, 256, BF), (15, 2, 2, 256, BF), (34, 7, 3, 256, BF),
+                                             (8, 3, 2, 64, BF), (9, 3, 1, 128, BF), (7, 4, 1, 256, BF),
+                                             (209, 4, 4, 256, BF), (139, 3, 8, 128, BF), (265, 2, 8, 64, BF),
                                              (1, 1, 1, 256, FP), (4, 2, 2, 128, FP), (5, 3, 2, 64, FP), (33, 40, 4, 256, FP),
                                              (70, 5, 4, 128, FP), (140, 4, 4, 64, FP)])
 def test_slstm_recurrent_edges(ops, B, S, NH, dh, dtype):
-    """One, two and three steps (each h buffer unused, used once, reused), rows around the groups of a cluster (16 in bf16,
-    4 in fp32), a carried state.  bf16 heads of 64 and 128 feed h back unrounded and use the exact exponentials: their states stay within
+    """One, two and three steps (each h buffer unused, used once, reused), rows around the groups of a cluster (8 in bf16, 16
+    where those would not be resident at once, 4 in fp32), a carried state.  bf16 heads of 64 and 128 feed h back unrounded and use the exact exponentials: their states stay within
     the fp32 tolerance and their outputs within half a bf16 ulp (8 significant bits: 2^-8 of the value) of it."""
     rng = np.random.default_rng(dh + B)
     rd = xo.bf16_round if dtype == BF else (lambda a: a)
