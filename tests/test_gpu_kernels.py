@@ -895,6 +895,59 @@ def test_chunkwise_tail_forms(ops, S):
         assert relerr(host(C), host(st[0])) < FP32_TOL
 
 
+@pytest.mark.parametrize("T", [2, 15, 16, 17, 33, 63, 64, 65, 96, 97, 127])
+@pytest.mark.parametrize("dqk,dv,state,f_mean", [(256, 512, True, 3.0), (256, 128, False, -2.0), (128, 96, True, 6.0), (128, 256, False, 3.0)])
+def test_chunkwise_short_bf16(ops, T, dqk, dv, state, f_mean):
+    """Fewer tokens than a tensor-core tile, to fp32 accuracy in one launch: sizes around the 16-token blocks, the 32-token
+    passes and the two tile sizes, without and with a state, from strided q, k, v.  States within 1e-5 of the float64 recurrence
+    (sums of up to 127 products in fp32), h within that and one bf16 rounding (2^-8 of the value) on rows whose normaliser does
+    not cancel, and as near to float64 as the CUDA-core kernel is."""
+    rng = np.random.default_rng(T * 7 + dqk + dv)
+    B, NH = 2, 3
+    rd = xo.bf16_round
+    q, k = (rd(rng.standard_normal((B, NH, T, dqk)).astype(np.float32)) for _ in range(2))
+    v = rd(rng.standard_normal((B, NH, T, dv)).astype(np.float32))
+    i = rd(rng.standard_normal((B, NH, T)).astype(np.float32))
+    f = rd((rng.standard_normal((B, NH, T)) + f_mean).astype(np.float32))
+    st0 = None
+    if state:
+        st0 = (rng.standard_normal((B, NH, dqk, dv)).astype(np.float32), rng.standard_normal((B, NH, dqk)).astype(np.float32),
+               rng.standard_normal((B, NH)).astype(np.float32))
+    C, n, m = (np.zeros((B, NH, dqk, dv)), np.zeros((B, NH, dqk)), np.zeros((B, NH))) if st0 is None else (a.astype(np.float64) for a in st0)
+    h64, cond = [], []
+    for t in range(T):
+        fl = -np.logaddexp(0, -f[:, :, t].astype(np.float64))
+        mn = np.maximum(fl + m, i[:, :, t])
+        fg, ig = np.exp(fl + m - mn), np.exp(i[:, :, t] - mn)
+        C = fg[..., None, None] * C + ig[..., None, None] * k[:, :, t, :, None].astype(np.float64) * v[:, :, t, None, :]
+        n = fg[..., None] * n + ig[..., None] * k[:, :, t]
+        m = mn
+        qs = q[:, :, t].astype(np.float64) / np.sqrt(dqk)
+        qn = np.einsum("bhd,bhd->bh", qs, n)
+        den = np.maximum(np.abs(qn), np.exp(-m)) + 1e-6
+        h64.append(np.einsum("bhd,bhdv->bhv", qs, C) / den[..., None])
+        cond.append(np.linalg.norm(qs, axis=-1) * np.linalg.norm(n, axis=-1) / den)
+    h64, cond = np.stack(h64, 2), np.stack(cond, 2)
+    # q and k as column blocks of one wider projection, token-major
+    qk = dev(np.concatenate([q, k], -1), BF).permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3)
+    args = (qk[..., :dqk], qk[..., dqk:], dev(v, BF).permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3), dev(i, BF), dev(f, BF))
+    h, st = ops.mlstm_chunkwise(*args, None if st0 is None else tuple(dev(s) for s in st0))
+    hf, stf = ops.mlstm_chunkwise(*(dev(a) for a in (q, k, v, i, f)), None if st0 is None else tuple(dev(s) for s in st0))
+    for got, f32, want in zip(st, stf, (C, n, m)):
+        e = relerr(host(got), want)
+        assert e < 1e-5 and e <= 2 * relerr(host(f32), want) + 3e-7
+    ok = (cond < 20)[..., None]
+    off = np.abs(host(h) - h64) * ok
+    assert (off <= 2.0 ** -8 * np.abs(h64) + 1e-4 * np.abs(h64 * ok).max()).all()
+    if not state:   # a carried state equals the sequence that made it
+        from xlstm_cuda import _lib
+        h2, st2 = ops.mlstm_chunkwise(*(a[:, :, :1 + T // 2] for a in args), None)
+        if T - (1 + T // 2) > 0:
+            h3, st3 = ops.mlstm_chunkwise(*(a[:, :, 1 + T // 2:] for a in args), st2)
+            for got, want in zip(st3, st):
+                assert relerr(host(got), host(want)) < 1e-5
+
+
 @pytest.mark.parametrize("S", [128, 4096, 4224])
 def test_chunkwise_gate_prepass_forms_and_mixed_heads(ops, S):
     """1, 32 and 33 tiles: the one-launch gate pre-pass, its last size, and the three-launch form; one head of bounded gate

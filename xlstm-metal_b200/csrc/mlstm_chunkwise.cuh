@@ -34,6 +34,12 @@ int mlstm_chunkwise_f32(const ChunkwiseParams &p, int dtype, void *workspace, cu
 // the same in one launch without scratch: dqk <= 512, L <= 64
 int mlstm_chunkwise_simt(const ChunkwiseParams &p, int dtype, cudaStream_t st);
 
+// up to 128 bf16 tokens to the same accuracy in one launch without scratch: dqk == 256 or 128, dv % 32 == 0, 16-byte aligned
+// rows.  inputs_settled: q, k, v and the gates were not written by the launch before (only the state is waited for).  C1 may
+// be C0.
+bool mlstm_chunkwise_tail_supported(const ChunkwiseParams &p, int dtype);
+int mlstm_chunkwise_tail(const ChunkwiseParams &p, bool inputs_settled, cudaStream_t st);
+
 // tcgen05 / TMEM / TMA path: bf16, L == 64, dqk == 256 (or 128/64), dv % 128 == 0, whole chunks
 // shape_ok: the shape, strides and alignment fit the tensor-core kernel; driver_ok: the driver entry point
 // that encodes TMA descriptors could be resolved; supported = both

@@ -90,6 +90,7 @@ static int chunkwise_dispatch(const void *q, const void *k, const void *v, const
         if (n_peers) return XLSTM_ERR_UNSUPPORTED;   // peer stores exist in the tensor-core kernel only
         if (workspace && workspace_bytes >= sizeof(int) && !(reinterpret_cast<uintptr_t>(workspace) & 3u))
             p.status = static_cast<int *>(workspace);
+        if (xl::mlstm_chunkwise_tail_supported(p, dtype)) return xl::mlstm_chunkwise_tail(p, false, st);
         const size_t f32_need = xl::mlstm_chunkwise_f32_workspace(B, NH, S, dqk, dv);
         if (xl::mlstm_chunkwise_f32_supported(p, dtype) &&
             (f32_need == 0 || (workspace && workspace_bytes >= f32_need && !(reinterpret_cast<uintptr_t>(workspace) & 255u))))

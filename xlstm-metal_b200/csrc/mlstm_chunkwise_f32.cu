@@ -19,6 +19,7 @@
 // gates of the chunk, kept in double until the difference is taken (b reaches 1e3 in a chunk of closed gates).
 #include "cp_async.cuh"
 #include "mlstm_chunkwise.cuh"
+#include "mlstm_gate_tile.cuh"
 #include "packed_f32.cuh"
 
 namespace xl {
@@ -39,45 +40,6 @@ struct F32Params {
     int NC, c_begin, c_end, slots;   // chunks of the sequence, of the group, slots per head
     int slot0;                       // the first chunk's state is in slot 0 too (C1 may overwrite C0)
 };
-
-// Gate scalars of 32 tokens, lane = token: inclusive sums b (double), u = i - b, running maximum of u
-struct GateTile {
-    double b, u, mx;
-};
-// the raw gates of one token: loaded ahead of their use, the scan below is latency enough
-struct GateRaw {
-    float i, f;
-    bool valid;
-};
-template <typename T> __device__ __forceinline__ GateRaw gate_load(const ChunkwiseParams &p, int bb, int hd, int t) {
-    GateRaw r{0.f, 0.f, t < p.S};
-    if (r.valid) {
-        const int64_t off = bb * p.sg[0] + hd * p.sg[1] + (int64_t)t * p.sg[2];
-        r.i = Elem<T>::ld(static_cast<const T *>(p.ig) + off);
-        r.f = Elem<T>::ld(static_cast<const T *>(p.fg) + off);
-    }
-    return r;
-}
-__device__ __forceinline__ GateTile gate_tile(const GateRaw &r, float cap, int lane, double b_in) {
-    const float lf = r.valid ? logsigmoid(gate_softcap(r.f, cap)) : 0.f;
-    const float it = r.valid ? gate_softcap(r.i, cap) : -INFINITY;
-    GateTile g;
-    g.b = (double)lf;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, g.b, o);
-        if (lane >= o) g.b += up;
-    }
-    g.b += b_in;
-    g.u = (double)it - g.b;
-    g.mx = g.u;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, g.mx, o);
-        if (lane >= o) g.mx = fmax(g.mx, up);
-    }
-    return g;
-}
 
 template <typename T> __device__ __forceinline__ float4 ld4_or_zero(const T *ptr, bool ok) {
     return ok ? ld4(ptr) : make_float4(0.f, 0.f, 0.f, 0.f);

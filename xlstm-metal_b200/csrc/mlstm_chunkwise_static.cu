@@ -84,8 +84,9 @@ extern "C" int xlstm_mlstm_chunkwise_fwd_static(const void *q, const void *k, co
         p.sh[0] = p.sv[0]; p.sh[1] = p.sv[1]; p.sh[2] = p.sv[2];
         p.sg[0] = nh * s; p.sg[1] = s; p.sg[2] = 1;
     }
-    // the exact CUDA-core path needs no scratch at all
-    if (!xl::mlstm_chunkwise_tc_shape_ok(p, dtype)) return xl::mlstm_chunkwise_simt(p, dtype, st);
+    // the exact paths that need no scratch at all
+    if (!xl::mlstm_chunkwise_tc_shape_ok(p, dtype))
+        return xl::mlstm_chunkwise_tail_supported(p, dtype) ? xl::mlstm_chunkwise_tail(p, false, st) : xl::mlstm_chunkwise_simt(p, dtype, st);
 
     // size check before anything else can launch: a problem beyond the block is an error, never a fallback
     const size_t need = xl::mlstm_chunkwise_tc_workspace_min(B, NH, S, dqk, dv);   // the block is used by the single-pass mode

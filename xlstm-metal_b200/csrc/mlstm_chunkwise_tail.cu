@@ -1,0 +1,408 @@
+// Up to 128 bf16 tokens with a carried fp32 state in one launch, to fp32 accuracy: the tokens after the last whole 128-token
+// tile of the tensor-core kernels, and sequences that are shorter than one tile.
+//
+// The operands that are bf16 (Q, K, V) are exact; the fp32 ones (C, the gate matrix P, the weighted V) are cut into three
+// bf16 parts whose sum is the float, so mma.sync forms exact products and adds them in fp32:
+//   S = Q K^T                                         1 product
+//   H^T = (C^T Q^T) diag(w_in) + V^T P^T              3 products each (parts of C, of P)
+//   C^T = decay C^T + (w V)^T K                       3 products (parts of w V)
+// One CTA per (head, 32 columns of dv).  Its 8 warps share the dqk dimension: a warp keeps its rows of C in registers, as
+// accumulators of the update and, in the same places, as A fragments of the read-out; it takes its share of the keys s for
+// S, P and P V.  The read-outs of the 8 warps meet in shared memory, 32 tokens at a time.  Everything that does not need the
+// state (loads, S, gate sums) is done before the wait on the tensor-core kernel.
+//
+// Latency-bound: a few microseconds of products behind a chain of loads, two barriers a 32 tokens and the state's way through
+// registers.  As fp32 multiply-adds on CUDA cores a tail of 64 tokens took 52 us (8 heads of 256/512) in one launch, of 127
+// tokens 66 us in two; here 14 us behind the last tile (16 heads: 19).  Relative error of C against float64 6.9e-8 to 8.0e-8, as
+// fp32 multiply-adds 8.1e-8 to 1.0e-7; 5.6e-8 against 4.1e-8 where one token makes the state.
+#include "cp_async.cuh"
+#include "mlstm_gate_tile.cuh"
+
+namespace xl {
+namespace {
+
+constexpr int TW = 8;               // warps
+constexpr int TC_COLS = 32;         // columns of dv per CTA
+constexpr int TG = 32;              // tokens per read-out pass
+constexpr int V_LD = 40;            // bf16 elements between rows of V: 80 bytes, eight rows on different banks
+constexpr int PART_LD = 36;         // floats between tokens of a partial read-out
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&a)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t (&a)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma_k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+// Two floats as three packed pairs of bf16 whose sums are the floats: 8 significant bits each, cut off (a rounded leading
+// part could overflow).  An infinity is its leading part alone.
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
+        p[i] = __byte_perm(ux, uy, 0x7632);
+        x = fabsf(x) < INFINITY ? x - __uint_as_float(ux & 0xffff0000u) : 0.f;
+        y = fabsf(y) < INFINITY ? y - __uint_as_float(uy & 0xffff0000u) : 0.f;
+    }
+}
+
+template <int DQK, int TMAX> struct TailSmem {
+    static constexpr uint32_t QK_LD = DQK + 8;                                // elements between rows of Q and K
+    static constexpr uint32_t Q = 0;
+    static constexpr uint32_t K = Q + TMAX * QK_LD * 2;
+    static constexpr uint32_t V = K + TMAX * QK_LD * 2;
+    static constexpr uint32_t PART = V + TMAX * V_LD * 2;                     // float [TW][TG][PART_LD]
+    static constexpr uint32_t WV = PART;                                      // bf16 [3][TMAX][V_LD], after the last read-out
+    static constexpr uint32_t PART_BYTES = TW * TG * PART_LD * 4;
+    static constexpr uint32_t U = PART + PART_BYTES;                          // double [3][TMAX]: u, b, running maximum of u / x
+    static constexpr uint32_t F = U + 3 * TMAX * 8;                           // float [4][TMAX]: w_in, e^{-m_t}, w, q.n
+    static constexpr uint32_t RS = F + 4 * TMAX * 4;                          // float [TW][TMAX] row sums of P
+    static constexpr uint32_t N = RS + TW * TMAX * 4;                         // float [DQK]
+    static constexpr uint32_t TOTAL = N + DQK * 4;
+    static_assert(3 * TMAX * V_LD * 2 <= PART_BYTES, "weighted V fits the buffer it replaces");
+};
+
+template <int DQK, int TMAX>
+__global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel(const ChunkwiseParams p, int inputs_settled) {
+    using SM = TailSmem<DQK, TMAX>;
+    constexpr int JW = DQK / TW, KSJ = JW / 16, NTJ = JW / 8;                 // rows of C per warp; k-steps; n-tiles
+    constexpr int SW = TMAX / TW, NS = SW / 8;                                // keys per warp; n-tiles
+    constexpr int TB = TMAX / 16;
+    extern __shared__ __align__(16) unsigned char smem[];
+    double *sU = reinterpret_cast<double *>(smem + SM::U), *sB = sU + TMAX, *sX = sB + TMAX;
+    float *sWin = reinterpret_cast<float *>(smem + SM::F), *sEmt = sWin + TMAX, *sW = sEmt + TMAX, *sQn = sW + TMAX;
+    float *sRs = reinterpret_cast<float *>(smem + SM::RS), *sN = reinterpret_cast<float *>(smem + SM::N);
+    float *sPart = reinterpret_cast<float *>(smem + SM::PART);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+    const int col0 = blockIdx.x * TC_COLS, bh = blockIdx.y, b = bh / p.NH, hd = bh % p.NH;
+    const int T = p.S, nb = (T + 15) >> 4;                                    // tokens; blocks of 16 (the rest is zeros)
+    const int s0 = warp * SW, j0 = warp * JW;
+    const bool has_C = p.C0 != nullptr;
+    using bf16 = __nv_bfloat16;
+
+    if (!inputs_settled) grid_dependency_wait();
+    // ---- loads
+    const bf16 *qb = static_cast<const bf16 *>(p.q) + b * p.sq[0] + hd * p.sq[1];
+    const bf16 *kb = static_cast<const bf16 *>(p.k) + b * p.sk[0] + hd * p.sk[1];
+    const bf16 *vb = static_cast<const bf16 *>(p.v) + b * p.sv[0] + hd * p.sv[1] + col0;
+    for (int e = tid; e < nb * 16 * (DQK / 8); e += TW * 32) {
+        const int t = e / (DQK / 8), x = (e % (DQK / 8)) * 8;
+        const bool ok = t < T;
+        cp_async16(base + SM::Q + (t * SM::QK_LD + x) * 2, qb + (ok ? (int64_t)t * p.sq[2] + x : 0), ok);
+        cp_async16(base + SM::K + (t * SM::QK_LD + x) * 2, kb + (ok ? (int64_t)t * p.sk[2] + x : 0), ok);
+    }
+    for (int e = tid; e < nb * 16 * 4; e += TW * 32) {
+        const int t = e >> 2, x = (e & 3) * 8;
+        const bool ok = t < T;
+        cp_async16(base + SM::V + (t * V_LD + x) * 2, vb + (ok ? (int64_t)t * p.sv[2] + x : 0), ok);
+    }
+    if (warp == TW - 1) {                                                     // the warp with the fewest rows of P
+        double bsum = 0.0, mx = -INFINITY;
+#pragma unroll 1
+        for (int h = 0; h < TMAX; h += 32) {
+            const GateTile gt = gate_tile(gate_load<bf16>(p, b, hd, h + lane), p.gate_cap, lane, bsum);
+            const double x = fmax(mx, gt.mx);
+            sU[h + lane] = gt.u;
+            sB[h + lane] = gt.b;
+            sX[h + lane] = x;
+            bsum = __shfl_sync(0xffffffffu, gt.b, 31);
+            mx = __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    // ---- S = Q K^T: rows t of block tb (16), this warp's keys
+    float P[TB][NS][4];
+#pragma unroll
+    for (int tb = 0; tb < TB; ++tb)
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) P[tb][n][e] = 0.f;
+    const uint32_t a_row = base + SM::Q + ((lane & 15) * SM::QK_LD + (lane >> 4) * 8) * 2;
+    if (s0 < nb * 16) {
+#pragma unroll 1
+        for (int kk = 0; kk < DQK / 32; ++kk) {                               // two k-steps
+            uint32_t kf[NS][4];                                               // keys of n-tile n: registers 0, 1 and 2, 3
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+                ldsm4(base + SM::K + ((s0 + n * 8 + (lane & 7)) * SM::QK_LD + kk * 32 + (lane >> 3) * 8) * 2, kf[n]);
+#pragma unroll
+            for (int tb = 0; tb < TB; ++tb)
+                if (tb < nb && tb * 16 + 15 >= s0) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t a[4];
+                        ldsm4(a_row + (tb * 16 * SM::QK_LD + kk * 32 + h * 16) * 2, a);
+#pragma unroll
+                        for (int n = 0; n < NS; ++n) mma_k16(P[tb][n], a, kf[n][2 * h], kf[n][2 * h + 1]);
+                    }
+                }
+        }
+    }
+
+    if (inputs_settled) grid_dependency_wait();
+    allow_dependents();
+    if (p.status && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *p.status = 0;
+    // ---- the state: this warp's rows j of C^T, element e of tile (mt, nj): column 16 mt + g + 8 (e / 2), row 8 nj + 2c + (e & 1)
+    float Ct[2][NTJ][4];
+    const size_t c_off = ((size_t)bh * DQK + j0 + 2 * c) * p.dv + col0 + g;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nj = 0; nj < NTJ; ++nj)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                Ct[mt][nj][e] = has_C ? p.C0[c_off + (size_t)(nj * 8 + (e & 1)) * p.dv + mt * 16 + (e >> 1) * 8] : 0.f;
+    for (int j = tid; j < DQK; j += TW * 32) sN[j] = has_C ? p.n0[(size_t)bh * DQK + j] : 0.f;
+    const float m = has_C ? p.m0[bh] : 0.f;
+    const double x_last = fmax((double)m, sX[TMAX - 1]);
+    const float decay = expf((float)((double)m - x_last));
+    __syncthreads();                                                          // n; everyone has read the last maximum
+    if (tid < TMAX) {
+        const double x = fmax((double)m, sX[tid]);
+        sX[tid] = x;
+        sWin[tid] = expf((float)((double)m - x)) * p.qscale;
+        sEmt[tid] = expf(-(float)(sB[tid] + x));
+        sW[tid] = expf((float)(sU[tid] - x_last));                            // 0 beyond the last token
+    }
+    {   // q . n: TW * 32 / TMAX threads a token
+        constexpr int PT = TW * 32 / TMAX;
+        const int t = tid / PT;
+        float a = 0.f;
+        if (t < T) {
+            const bf16 *qrow = reinterpret_cast<const bf16 *>(smem + SM::Q) + t * SM::QK_LD;
+#pragma unroll 2
+            for (int x = (tid % PT) * 8; x < DQK; x += PT * 8) {
+                const uint4 w = *reinterpret_cast<const uint4 *>(qrow + x);
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    a = fmaf(__uint_as_float(ww[e] << 16), sN[x + 2 * e], a);
+                    a = fmaf(__uint_as_float(ww[e] & 0xffff0000u), sN[x + 2 * e + 1], a);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < PT; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (tid % PT == 0) sQn[t] = a;
+    }
+    __syncthreads();
+    // ---- P = tril(S) e^{u_s - x_t}, row sums
+#pragma unroll
+    for (int tb = 0; tb < TB; ++tb)
+        if (tb < nb)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = tb * 16 + r * 8 + g;
+                const double xt = sX[t];
+                float rs = 0.f;
+#pragma unroll
+                for (int n = 0; n < NS; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int s = s0 + n * 8 + 2 * c + e;
+                        float &v = P[tb][n][2 * r + e];
+                        v = s <= t ? v * p.qscale * expf((float)(sU[s] - xt)) : 0.f;
+                        rs += v;
+                    }
+                rs += __shfl_xor_sync(0xffffffffu, rs, 1);
+                rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+                if (c == 0) sRs[warp * TMAX + t] = rs;
+            }
+
+    // ---- read-out, TG tokens at a time
+    uint32_t Cp[3][2][KSJ][4];                                                // parts of C^T as A fragments (rows: columns of dv)
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int ks = 0; ks < KSJ; ++ks)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {                                     // register r: rows + 8 (r & 1), k + 8 (r / 2)
+                const float *src = Ct[mt][2 * ks + (r >> 1)] + 2 * (r & 1);
+                uint32_t w[3];
+                split3(src[0], src[1], w);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) Cp[x][mt][ks][r] = w[x];
+            }
+    bf16 *hb = static_cast<bf16 *>(p.h) + b * p.sh[0] + hd * p.sh[1] + col0;
+#pragma unroll
+    for (int th = 0; th < TMAX / TG; ++th) {
+        if (th * TG >= T) break;
+        float acc[2][TG / 8][4];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < TG / 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[mt][nt][e] = 0.f;
+        if (has_C) {
+#pragma unroll
+            for (int ks = 0; ks < KSJ; ++ks)
+#pragma unroll
+                for (int np = 0; np < TG / 16; ++np) {
+                    if (th * 2 + np >= nb) continue;
+                    uint32_t q[4];                                            // tokens of n-tiles 2 np (registers 0, 1), 2 np + 1
+                    ldsm4(base + SM::Q + ((th * TG + np * 16 + (lane & 7) + ((lane >> 4) << 3)) * SM::QK_LD + j0 + ks * 16 +
+                                          ((lane >> 3) & 1) * 8) * 2, q);
+#pragma unroll
+                    for (int x = 2; x >= 0; --x)
+#pragma unroll
+                        for (int mt = 0; mt < 2; ++mt) {
+                            mma_k16(acc[mt][2 * np], Cp[x][mt][ks], q[0], q[1]);
+                            mma_k16(acc[mt][2 * np + 1], Cp[x][mt][ks], q[2], q[3]);
+                        }
+                }
+#pragma unroll
+            for (int nt = 0; nt < TG / 8; ++nt) {
+                const float2 w = *reinterpret_cast<const float2 *>(sWin + th * TG + nt * 8 + 2 * c);
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    acc[mt][nt][0] *= w.x; acc[mt][nt][1] *= w.y;
+                    acc[mt][nt][2] *= w.x; acc[mt][nt][3] *= w.y;
+                }
+            }
+        }
+        if (s0 < nb * 16 && th * TG + TG > s0) {
+            uint32_t vf[2][4];                                                // V^T of this warp's keys
+            if (NS == 1) {
+                ldsm4_trans(base + SM::V + ((s0 + (lane & 7)) * V_LD + (lane >> 3) * 8) * 2, vf[0]);
+            } else {
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt)
+                    ldsm4_trans(base + SM::V + ((s0 + (lane & 7) + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, vf[mt]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < TG / 8; ++nt) {
+                const int tb = th * 2 + (nt >> 1), r = nt & 1;
+                uint32_t w[NS][3];
+#pragma unroll
+                for (int n = 0; n < NS; ++n) split3(P[tb][n][2 * r], P[tb][n][2 * r + 1], w[n]);
+#pragma unroll
+                for (int x = 2; x >= 0; --x)
+#pragma unroll
+                    for (int mt = 0; mt < 2; ++mt) {
+                        if (NS == 1) mma_k8(acc[mt][nt], vf[0][2 * mt], vf[0][2 * mt + 1], w[0][x]);
+                        else mma_k16(acc[mt][nt], vf[mt], w[0][x], w[NS - 1][x]);
+                    }
+            }
+        }
+        if (th > 0) __syncthreads();                                          // the previous pass has been read
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < TG / 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    sPart[(warp * TG + nt * 8 + 2 * c + (e & 1)) * PART_LD + mt * 16 + g + (e >> 1) * 8] = acc[mt][nt][e];
+        __syncthreads();
+        const int tl = tid >> 3, x4 = (tid & 7) * 4, t = th * TG + tl;        // a token's 32 columns in 8 threads
+        if (t < T) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            float rs = 0.f;
+#pragma unroll
+            for (int w = 0; w < TW; ++w) {
+                const float4 v = *reinterpret_cast<const float4 *>(sPart + (w * TG + tl) * PART_LD + x4);
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+                rs += sRs[w * TMAX + t];
+            }
+            const float den = sWin[t] * sQn[t] + rs;
+            const float inv = 1.0f / (fmaxf(fabsf(den), sEmt[t]) + p.eps);
+            st4(hb + (int64_t)t * p.sh[2] + x4, make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv));
+        }
+    }
+    __syncthreads();
+
+    // ---- C^T = decay C^T + (w V)^T K
+    bf16 *sWV = reinterpret_cast<bf16 *>(smem + SM::WV);
+    for (int e = tid; e < nb * 16 * (TC_COLS / 2); e += TW * 32) {
+        const int t = e / (TC_COLS / 2), x = (e % (TC_COLS / 2)) * 2;
+        const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + SM::V + (t * V_LD + x) * 2);
+        const float w = sW[t];
+        uint32_t pr[3];
+        split3(w * __uint_as_float(v << 16), w * __uint_as_float(v & 0xffff0000u), pr);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(sWV + (k * TMAX + t) * V_LD + x) = pr[k];
+    }
+    __syncthreads();
+    // The sum over the tokens has accumulators of its own, the leading parts and the remainders apart, and meets the state in
+    // one fp32 multiply-add: the tensor cores cut off below the last bit of a sum, so its terms should not be small beside it.
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+        float sum[2][NTJ][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int nj = 0; nj < NTJ; ++nj)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[h][nj][e] = 0.f;
+#pragma unroll 1
+        for (int ks = 0; ks < nb; ++ks) {
+            uint32_t wv[3][4], kf[NTJ / 2][4];
+            const int trow = ks * 16 + (lane & 7);
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+                ldsm4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wv[x]);
+#pragma unroll
+            for (int np = 0; np < NTJ / 2; ++np)
+                ldsm4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
+#pragma unroll
+            for (int x = 2; x >= 0; --x)
+#pragma unroll
+                for (int np = 0; np < NTJ / 2; ++np) {
+                    mma_k16(sum[x > 0][2 * np], wv[x], kf[np][0], kf[np][1]);
+                    mma_k16(sum[x > 0][2 * np + 1], wv[x], kf[np][2], kf[np][3]);
+                }
+        }
+#pragma unroll
+        for (int nj = 0; nj < NTJ; ++nj)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                p.C1[c_off + (size_t)(nj * 8 + (e & 1)) * p.dv + mt * 16 + (e >> 1) * 8] =
+                    fmaf(Ct[mt][nj][e], decay, sum[0][nj][e] + sum[1][nj][e]);
+    }
+    if (blockIdx.x == 0) {
+        const bf16 *sK = reinterpret_cast<const bf16 *>(smem + SM::K);
+        for (int j = tid; j < DQK; j += TW * 32) {
+            float a = decay * sN[j];
+            for (int t = 0; t < T; ++t) a = fmaf(sW[t], __bfloat162float(sK[t * SM::QK_LD + j]), a);
+            p.n1[(size_t)bh * DQK + j] = a;
+        }
+        if (tid == 0) p.m1[bh] = (float)(sB[TMAX - 1] + x_last);
+    }
+}
+
+template <int DQK, int TMAX> int tail_launch(const ChunkwiseParams &p, bool inputs_settled, cudaStream_t st) {
+    auto kern = mlstm_tail_kernel<DQK, TMAX>;
+    constexpr int bytes = (int)TailSmem<DQK, TMAX>::TOTAL;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return XLSTM_ERR_CUDA;
+    return launch_overlapped(kern, dim3(p.dv / TC_COLS, p.B * p.NH), dim3(TW * 32), bytes, st, p, inputs_settled ? 1 : 0);
+}
+
+}  // namespace
+
+bool mlstm_chunkwise_tail_supported(const ChunkwiseParams &p, int dtype) {
+    if (dtype != XLSTM_BF16 || p.S > 128 || (p.dqk != 256 && p.dqk != 128) || p.dv % TC_COLS || p.n_peer) return false;
+    for (int d = 0; d < 3; ++d)
+        if (p.sq[d] % 8 || p.sk[d] % 8 || p.sv[d] % 8 || p.sh[d] % 4) return false;
+    if ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15u) return false;
+    return !(reinterpret_cast<uintptr_t>(p.h) & 7u) && (int64_t)p.B * p.NH <= 65535;
+}
+
+int mlstm_chunkwise_tail(const ChunkwiseParams &p, bool inputs_settled, cudaStream_t st) {
+    if (p.dqk == 256) return p.S <= 64 ? tail_launch<256, 64>(p, inputs_settled, st) : tail_launch<256, 128>(p, inputs_settled, st);
+    return p.S <= 64 ? tail_launch<128, 64>(p, inputs_settled, st) : tail_launch<128, 128>(p, inputs_settled, st);
+}
+
+}  // namespace xl

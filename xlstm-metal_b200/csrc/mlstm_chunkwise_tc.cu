@@ -759,6 +759,8 @@ __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __
 // The wait for the general launch comes last, in one CTA: this launch is complete only when that one is.
 template <int DQK, bool STATE_ONLY>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(const __grid_constant__ TcParams p) {
+    // a tail launch follows, which reads only the inputs before its wait: let it start beside this one
+    if (!STATE_ONLY && p.early) allow_dependents();
     if (p.path[blockIdx.x] != 0) {
         if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
         else chunkwise_bounded<DQK>(p);
@@ -814,7 +816,7 @@ namespace {
 
 // Layout of the caller-provided scratch.  P > 1 adds the per-segment states of the segment-parallel mode.
 struct WsLayout {
-    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], decay, tail_C, tail_ws, total;
+    size_t gates, tail_n, tail_m, path, chain, seg_C[2], seg_n[2], decay, total;
     int P, seg_tiles;
 };
 
@@ -849,14 +851,7 @@ int plan_segments(int BH, int dv, int nch) {
     return best;
 }
 
-// Tokens after the last whole tile that run on the two-launch fp32 kernels (their state and scratch is in the workspace); 0:
-// none, or the one-kernel form in place.  That one walks 64-token chunks, 51 us each at 8 heads of 256/512; the two launches
-// take both chunks of a longer tail at once (101 -> 66 us; 64 heads: 486 -> 309 for 612 tokens in all), but for a single
-// chunk they gain nothing (52 and 51 us).
-int tail_for_f32(int S) { return S % LT > 64 ? S % LT : 0; }
-
-// tail: see tail_for_f32()
-WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P, int tail) {
+WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P) {
     WsLayout w{};
     const size_t BH = (size_t)B * NH, nch = (size_t)(S / LT);
     w.P = P;
@@ -877,10 +872,6 @@ WsLayout ws_layout(int B, int NH, int S, int dqk, int dv, int P, int tail) {
         }
         w.decay = o; o = up(o + VH * sizeof(float));
     }
-    if (tail) {
-        w.tail_C = o;  o = up(o + BH * dqk * dv * sizeof(float));
-        w.tail_ws = o; o = up(o + mlstm_chunkwise_f32_workspace(B, NH, tail, dqk, dv));
-    }
     w.total = o + 256;
     return w;
 }
@@ -896,11 +887,11 @@ size_t mlstm_chunkwise_tc_workspace(int B, int NH, int S, int dqk, int dv, int L
     if (nch < 1 || (dqk != 256 && dqk != 128) || dv % DVS) return 0;     // not a shape of this path
     const int forced = g_segments.load();
     const int P = forced >= 1 ? (forced > nch ? (nch > 0 ? nch : 1) : forced) : plan_segments(B * NH, dv, nch);
-    return ws_layout(B, NH, S, dqk, dv, P, tail_for_f32(S)).total;
+    return ws_layout(B, NH, S, dqk, dv, P).total;
 }
 
 size_t mlstm_chunkwise_tc_workspace_min(int B, int NH, int S, int dqk, int dv) {
-    return S < LT ? 0 : ws_layout(B, NH, S, dqk, dv, 1, 0).total;
+    return S < LT ? 0 : ws_layout(B, NH, S, dqk, dv, 1).total;
 }
 
 void mlstm_chunkwise_tc_set_general_only(int on) { g_general_only.store(on ? 1 : 0); }
@@ -911,14 +902,11 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     const int nch = s_full / LT;
     const int BH = p.B * p.NH;
     if (!workspace) return XLSTM_ERR_WORKSPACE;
-    // the segment-parallel mode, and the fp32 kernels for a tail, if the scratch holds their states; else the plain
-    // single pass, and the tail in place
+    // the segment-parallel mode if the scratch holds its states, else the plain single pass
     const int forced = g_segments.load();
     int P = forced >= 1 ? (forced > nch ? nch : forced) : plan_segments(BH, p.dv, nch);
-    int tail_f32 = tail_for_f32(p.S);
-    WsLayout w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, P, tail_f32);
-    if (workspace_bytes < w.total) w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1, tail_f32);
-    if (workspace_bytes < w.total) w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1, tail_f32 = 0);
+    WsLayout w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, P);
+    if (workspace_bytes < w.total) w = ws_layout(p.B, p.NH, s_full, p.dqk, p.dv, 1);
     if (workspace_bytes < w.total) return XLSTM_ERR_WORKSPACE;
     P = w.P;
     const int seg_tiles = w.seg_tiles;
@@ -961,8 +949,7 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         return state_only ? launch_tc<128, true>(tp, grid, st) : launch_tc<128, false>(tp, grid, st);
     };
     float *n_final = tail ? tail_n : p.n1, *m_final = tail ? tail_m : p.m1;
-    // the fp32 kernels write C1 before the last read of C0, so they start from a copy; the one-kernel form runs in place
-    ChunkwiseParams t = p;
+    ChunkwiseParams t = p;   // the tail: continues in place from (C1, tail_n, tail_m)
     if (tail) {
         const size_t esz = 2;
         t.q = static_cast<const unsigned char *>(p.q) + (size_t)s_full * p.sq[2] * esz;
@@ -973,11 +960,9 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         t.fg = static_cast<const unsigned char *>(p.fg) + (size_t)s_full * p.sg[2] * esz;
         t.S = p.S - s_full;
         t.L = 64;
-        t.C0 = tail_f32 ? reinterpret_cast<float *>(ws + w.tail_C) : p.C1;
-        t.n0 = tail_n; t.m0 = tail_m;
-        if (tail_f32 && !mlstm_chunkwise_f32_supported(t, XLSTM_BF16)) { tail_f32 = 0; t.C0 = p.C1; }
+        t.C0 = p.C1; t.n0 = tail_n; t.m0 = tail_m;
     }
-    float *C_final = tail ? const_cast<float *>(t.C0) : p.C1;
+    const bool fused_tail = tail && mlstm_chunkwise_tail_supported(t, XLSTM_BF16);
 
     // the gate pre-pass (chain, path flags and per-token scalars for both passes of the segment-parallel mode), then the
     // tensor-core kernel, whose CTAs read their path flag: the choice needs no host round trip
@@ -991,7 +976,8 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     int rc = gate_prepass<__nv_bfloat16>(gp, BH, st);
     if (rc != XLSTM_OK) return rc;
     if (P == 1) {
-        tp.C0 = p.C0; tp.n0 = p.n0; tp.C1 = C_final; tp.n1 = n_final; tp.n_h = n_dest;
+        tp.early = fused_tail;
+        tp.C0 = p.C0; tp.n0 = p.n0; tp.C1 = p.C1; tp.n1 = n_final; tp.n_h = n_dest;
         rc = forward(false);
         if (rc != XLSTM_OK) return rc;
     } else {
@@ -1004,17 +990,18 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         const int slabs = (int)(((CE + p.dqk) / COMB_VEC + COMB_THREADS - 1) / COMB_THREADS);   // one vector per thread
         rc = launch_overlapped(mlstm_segment_combine_kernel, dim3(BH, slabs), dim3(COMB_THREADS), 0, st, p.C0, p.n0,
                                static_cast<const float *>(segA_C), static_cast<const float *>(segA_n),
-                               static_cast<const float *>(decay), segB_C, segB_n, C_final, n_final, P, p.dqk, p.dv);
+                               static_cast<const float *>(decay), segB_C, segB_n, p.C1, n_final, P, p.dqk, p.dv);
         if (rc != XLSTM_OK) return rc;
         // pass 2: every segment from its true start state
+        tp.early = fused_tail;
         tp.C0 = segB_C; tp.n0 = segB_n; tp.C1 = segA_C; tp.n1 = segA_n; tp.n_h = n_dest;
         rc = forward(false);
         if (rc != XLSTM_OK) return rc;
     }
     if (!tail) return XLSTM_OK;
 
-    // S mod 128 tail on the exact path, continuing from (t.C0, tail_n, tail_m)
-    return tail_f32 ? mlstm_chunkwise_f32(t, XLSTM_BF16, ws + w.tail_ws, st) : mlstm_chunkwise_simt(t, XLSTM_BF16, st);
+    // S mod 128 tokens to fp32 accuracy; the launch does its loads and Q K^T while the last tiles run (tp.early)
+    return fused_tail ? mlstm_chunkwise_tail(t, true, st) : mlstm_chunkwise_simt(t, XLSTM_BF16, st);
 }
 
 }  // namespace xl
