@@ -38,6 +38,9 @@ __global__ void __launch_bounds__(RN_THREADS) rms_norm_kernel(const T *__restric
     __shared__ float s_part[2][RN_THREADS / 32];
     const int nvec = cols / VN;
     int par = 0;
+    // few rows: the launch is latency, and the single-token Linear behind it may bring its first weights meanwhile
+    grid_dependency_wait();
+    allow_dependents();
     for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
     const T *xr = x + (size_t)row * cols;
     T *yr = y + (size_t)row * cols;
@@ -289,11 +292,11 @@ static int rms_norm_launch(const void *x, const void *r, const void *w, void *su
         else rms_norm_warp_kernel<T, 16><<<wg, RW_WARPS * 32, 0, st>>>(xp, rp, wp, sp, yp, rows, cols, eps);
         return launch_status();
     }
-    if (aligned && nvec <= RN_THREADS * 1) rms_norm_kernel<T, 1><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, rows, cols, eps);
-    else if (aligned && nvec <= RN_THREADS * 2) rms_norm_kernel<T, 2><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, rows, cols, eps);
-    else if (aligned && nvec <= RN_THREADS * 4) rms_norm_kernel<T, 4><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, rows, cols, eps);
-    else if (aligned && nvec <= RN_THREADS * 8) rms_norm_kernel<T, 8><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, rows, cols, eps);
-    else rms_norm_generic_kernel<T><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, cols, eps);
+    if (aligned && nvec <= RN_THREADS * 1) return launch_overlapped(rms_norm_kernel<T, 1>, grid, dim3(RN_THREADS), 0, st, xp, rp, wp, sp, yp, rows, cols, eps);
+    if (aligned && nvec <= RN_THREADS * 2) return launch_overlapped(rms_norm_kernel<T, 2>, grid, dim3(RN_THREADS), 0, st, xp, rp, wp, sp, yp, rows, cols, eps);
+    if (aligned && nvec <= RN_THREADS * 4) return launch_overlapped(rms_norm_kernel<T, 4>, grid, dim3(RN_THREADS), 0, st, xp, rp, wp, sp, yp, rows, cols, eps);
+    if (aligned && nvec <= RN_THREADS * 8) return launch_overlapped(rms_norm_kernel<T, 8>, grid, dim3(RN_THREADS), 0, st, xp, rp, wp, sp, yp, rows, cols, eps);
+    rms_norm_generic_kernel<T><<<grid, RN_THREADS, 0, st>>>(xp, rp, wp, sp, yp, cols, eps);
     return launch_status();
 }
 

@@ -109,9 +109,15 @@ py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const Opt
 
 bool dense_heads(const Tensor &t) { return t.stride(2) == 1 && (t.size(1) == 1 || t.stride(1) == t.size(2)); }
 
-py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Tensor ogate, const OptTensor &norm_weight,
-                           const OptTensor &C0, const OptTensor &n0, const OptTensor &m0, double eps, double norm_eps,
-                           bool inplace, double gate_cap, bool state_settled) {
+struct Stepped {
+    int rc;
+    Tensor y;
+    NewState state;
+    py::tuple tuple() const { return py::make_tuple(rc, y, state.C, state.n, state.m); }
+};
+Stepped step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Tensor ogate, const OptTensor &norm_weight,
+                   const OptTensor &C0, const OptTensor &n0, const OptTensor &m0, double eps, double norm_eps,
+                   bool inplace, double gate_cap, bool state_settled) {
     for (const Tensor *t : {&q, &k, &v, &i, &f, &ogate}) need_cuda(*t);
     need_cuda(norm_weight);
     if (q.dim() != 3) throw py::value_error("mlstm_step_gated takes q as [B, NH, dqk]");
@@ -146,7 +152,12 @@ py::tuple mlstm_step_gated(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, Ten
             og.data_ptr(), ld, ptr(w), (float)norm_eps, y.data_ptr(), fptr(out.C), fptr(out.n), fptr(out.m), (int)B, (int)NH,
             (int)dqk, (int)dv, (float)eps, (float)gate_cap, flags, dt, stream());
     });
-    return py::make_tuple(rc, y, out.C, out.n, out.m);
+    return {rc, y, out};
+}
+py::tuple mlstm_step_gated(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &i, const Tensor &f, const Tensor &ogate,
+                           const OptTensor &norm_weight, const OptTensor &C0, const OptTensor &n0, const OptTensor &m0, double eps,
+                           double norm_eps, bool inplace, double gate_cap, bool state_settled) {
+    return step_gated(q, k, v, i, f, ogate, norm_weight, C0, n0, m0, eps, norm_eps, inplace, gate_cap, state_settled).tuple();
 }
 
 py::tuple mlstm_chunkwise(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const OptTensor &C0, const OptTensor &n0,
@@ -196,8 +207,13 @@ std::vector<int64_t> with_last(const Tensor &x, int64_t n) {
     return s;
 }
 
-py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight,
-                       double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows, bool weights_settled) {
+struct Result {
+    int rc;
+    Tensor y;
+    py::tuple tuple() const { return py::make_tuple(rc, y); }
+};
+Result linear(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight, double norm_eps,
+              const OptTensor &residual, bool swiglu_pair, int64_t max_rows, bool weights_settled) {
     need_cuda(weight); need_cuda(x); need_cuda(bias); need_cuda(norm_weight); need_cuda(residual);
     if (weight.scalar_type() != at::kBFloat16) throw py::type_error("linear_token and linear_rows are bf16 kernels");
     const int64_t K = x.size(-1);
@@ -225,10 +241,14 @@ py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &b
             : xlstm_linear_rows_ex(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, flags,
                                    XLSTM_BF16, stream());
     });
-    return py::make_tuple(rc, y);
+    return {rc, y};
+}
+py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight,
+                       double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows, bool weights_settled) {
+    return linear(weight, x, bias, norm_weight, norm_eps, residual, swiglu_pair, max_rows, weights_settled).tuple();
 }
 
-py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
+Result norm(const Tensor &x, const OptTensor &weight, double eps) {
     need_cuda(x); need_cuda(weight);
     const int64_t cols = x.size(-1);
     need(!weight || weight->numel() == cols, "norm weight must have one element per column");
@@ -240,8 +260,9 @@ py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) {
         return xlstm_rms_norm(xc.data_ptr(), ptr(w), y.data_ptr(), cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dt,
                               stream());
     });
-    return py::make_tuple(rc, y);
+    return {rc, y};
 }
+py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) { return norm(x, weight, eps).tuple(); }
 
 py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor &weight, double eps) {
     need_cuda(x); need_cuda(residual); need_cuda(weight);
@@ -257,6 +278,51 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
                                   cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dt, stream());
     });
     return py::make_tuple(rc, s, y);
+}
+
+// One token of B sequences through an mLSTM block, launch after launch as mLSTMBlock._token_step describes them: W, b are the
+// merged input projections, ffn the gate and up projections.  rows: the Linears for up to 16 rows with the norms as launches of
+// their own, else those for up to 4 with the norms in them.  Through Python the seven launches of a block took 140 us of host
+// time, as much as the GPU has work for 16 sequences of 4096.
+py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, const OptTensor &norm_w, double norm_eps, int64_t NH,
+                      int64_t dqk, int64_t dv, const OptTensor &C0, const OptTensor &n0, const OptTensor &m0,
+                      const OptTensor &head_norm_w, double eps, double head_norm_eps, bool inplace, double gate_cap,
+                      const Tensor &out_w, const OptTensor &out_b, const OptTensor &ffn_norm_w, double ffn_norm_eps,
+                      const Tensor &ffn, const Tensor &down_w, const OptTensor &down_b, bool rows) {
+    need(x.dim() == 2 && W.dim() == 2 && W.size(0) == 2 * NH * dqk + 2 * NH * dv + 2 * NH,
+         "token_block takes x as [B, D] and W as the merged q, k, v, i, f and o projections");
+    const OptTensor none;
+    const char *what = rows ? "xlstm_linear_rows_ex" : "xlstm_linear_token";
+    auto failed = [&](int rc, const char *call) { return py::make_tuple(rc, call, x, none, none, none); };
+    // weights_settled: the launches before the four Linears are a norm, the cell step, a norm and a Linear
+    auto project = [&](const Tensor &w, const Tensor &in, const OptTensor &bias, const OptTensor &nw, double ne, const OptTensor &res,
+                       bool pair) -> Result {
+        if (!rows) return linear(w, in, bias, nw, ne, res, pair, 4, false);
+        if (!nw) return linear(w, in, bias, none, 0.0, res, pair, 16, true);
+        const Result n = norm(in, nw, ne);
+        if (n.rc) return n;
+        return linear(w, n.y, bias, none, 0.0, res, pair, 16, true);
+    };
+    const Result y = project(W, x, b, norm_w, norm_eps, none, false);
+    if (y.rc) return failed(y.rc, what);
+    int64_t at = 0;
+    auto columns = [&](int64_t n) {
+        const Tensor t = y.y.narrow(1, at, n);
+        at += n;
+        return t;
+    };
+    const int64_t B = x.size(0);
+    const Tensor q = columns(NH * dqk).view({B, NH, dqk}), k = columns(NH * dqk).view({B, NH, dqk}), v = columns(NH * dv).view({B, NH, dv});
+    const Tensor i = columns(NH), f = columns(NH), o = columns(NH * dv);
+    // the launch before the step is the projection above: the state is settled
+    const Stepped st = step_gated(q, k, v, i, f, o, head_norm_w, C0, n0, m0, eps, head_norm_eps, inplace, gate_cap, true);
+    if (st.rc) return failed(st.rc, "xlstm_mlstm_step_gated_rows");
+    const Result x1 = project(out_w, st.y, out_b, none, 0.0, x, false);
+    if (x1.rc) return failed(x1.rc, what);
+    const Result act = project(ffn, x1.y, none, ffn_norm_w, ffn_norm_eps, none, true);
+    if (act.rc) return failed(act.rc, what);
+    const Result x3 = project(down_w, act.y, down_b, none, 0.0, x1.y, false);
+    return py::make_tuple(x3.rc, what, x3.y, st.state.C, st.state.n, st.state.m);
 }
 
 // LayerNorm of each of `groups` column blocks of the rows of x; the status says if the kernel does not take the layout
@@ -316,6 +382,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("linear_token", &linear_token);
     m.def("rms_norm", &rms_norm);
     m.def("add_rms_norm", &add_rms_norm);
+    m.def("token_block", &token_block);
     m.def("layer_norm", &layer_norm);
     m.def("slstm_gates", &slstm_gates);
 }

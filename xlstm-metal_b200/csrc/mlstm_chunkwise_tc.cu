@@ -141,17 +141,23 @@ __device__ __forceinline__ void gate_chain(double *ch, double m, int tile0, int 
     const int end = tile0 + n;
     for (int c0 = tile0; c0 < end; c0 += 32) {
         const int c = c0 + lane;
-        const double Gl = c < end ? ch[(size_t)c * GC + 0] : 0.0, Ul = c < end ? ch[(size_t)c * GC + 1] : 0.0;
-        double m_mine = 0.0;
-        const int nb = min(32, end - c0);
-        for (int j = 0; j < nb; ++j) {
-            const double Gj = __shfl_sync(0xffffffffu, Gl, j), Uj = __shfl_sync(0xffffffffu, Ul, j);
-            const double x_last = fmax(m, Uj);
-            if (x_last - m > SPREAD_LIMIT) bounded = false;
-            if (j == lane) m_mine = m;
-            m = Gj + x_last;
+        double G, M;
+        tile_map(c, end, G, M);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {         // inclusive: the map of the tiles c0 .. c
+            const double G1 = __shfl_up_sync(0xffffffffu, G, o), M1 = __shfl_up_sync(0xffffffffu, M, o);
+            if (lane >= o) {
+                M = fmax(G + M1, M);
+                G += G1;
+            }
         }
+        const double after = fmax(G + m, M);
+        const double up = __shfl_up_sync(0xffffffffu, after, 1);
+        const double m_mine = lane == 0 ? m : up;
+        const bool wide = c < end && fmax(m_mine, ch[(size_t)c * GC + 1]) - m_mine > SPREAD_LIMIT;
+        if (__any_sync(0xffffffffu, wide)) bounded = false;
         if (c < end) ch[(size_t)c * GC + 2] = m_mine;
+        m = __shfl_sync(0xffffffffu, after, 31);   // tiles beyond the end are the identity
     }
     if (lane == 0) { if (m_out) *m_out = (float)m; *path = bounded ? 1 : 0; }
     // C is kept in TMEM as C~ = C e^{-rho}: rho absorbs the per-tile decay so that the accumulator is
@@ -159,31 +165,42 @@ __device__ __forceinline__ void gate_chain(double *ch, double m, int tile0, int 
     // General path: the multiplication happens BEFORE tile c's update (mul also carries the decay of that
     // tile); bounded-spread path: AFTER tile c's update, so that update and read-out of a tile share one
     // frame.  rho_in = frame the read-out of tile c sees, rho_out = frame after tile c's update.
+    // Between two rescales rho is a prefix sum; a round finds the next rescale among the 32 tiles (every three or four
+    // tiles with usual gates).  Tile by tile, each step a chain of shuffles, 256 tiles took 39 us in all.
+    const double limit = bounded ? -RESCALE_AT_B : -RESCALE_AT;
     double rho = 0.0, total = 0.0;
     for (int c0 = tile0; c0 < end; c0 += 32) {
-        const int c = c0 + lane;
-        double ld = 0.0;
-        if (c < end) ld = ch[(size_t)c * GC + 2] - fmax(ch[(size_t)c * GC + 2], ch[(size_t)c * GC + 1]);   // m - x_last <= 0
-        double rin = 0.0, rout = 0.0, mul = 1.0;
-        const int nb = min(32, end - c0);
-        for (int j = 0; j < nb; ++j) {
-            const double logdec = __shfl_sync(0xffffffffu, ld, j);
-            const double r_in = rho;
-            double r_out, mu = 1.0;
-            total += logdec;
-            if (bounded) {
-                rho += logdec;
-                r_out = rho;
-                if (rho < -RESCALE_AT_B) { mu = exp(rho); rho = 0.0; }
-            } else {
-                if (rho + logdec < -RESCALE_AT) { mu = exp(rho + logdec); rho = 0.0; }
-                else rho += logdec;
-                r_out = rho;
+        const int c = c0 + lane, nb = min(32, end - c0);
+        double L = 0.0;                            // summed log decay (m - x_last <= 0) of the tiles c0 .. c
+        // (no state below e^-1e6 of it is left; unbounded, one such tile would take the digits of all sums after it)
+        if (c < end) L = fmax(ch[(size_t)c * GC + 2] - fmax(ch[(size_t)c * GC + 2], ch[(size_t)c * GC + 1]), -1e6);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double v = __shfl_up_sync(0xffffffffu, L, o);
+            if (lane >= o) L += v;
+        }
+        const double up = __shfl_up_sync(0xffffffffu, L, 1), Lx = lane == 0 ? 0.0 : up;
+        total += __shfl_sync(0xffffffffu, L, 31);
+        double rin = 0.0, rout = 0.0, at = -rho;   // rho of a tile's start: Lx - at
+        bool rescale = false;
+        for (int start = 0; start < nb;) {
+            const double r_out = L - at;
+            const unsigned hit = __ballot_sync(0xffffffffu, lane >= start && lane < nb && r_out < limit);
+            const int stop = hit ? __ffs(hit) - 1 : nb - 1;   // the tile that rescales, or the last one
+            if (lane >= start && lane <= stop) {
+                rin = Lx - at;
+                rout = r_out;
+                rescale = hit && lane == stop;
             }
-            if (j == lane) { rin = r_in; rout = r_out; mul = mu; }
+            const double L_stop = __shfl_sync(0xffffffffu, L, stop);
+            rho = hit ? 0.0 : L_stop - at;
+            at = L_stop - rho;
+            start = stop + 1;
         }
         if (c < end) {
-            ch[(size_t)c * GC + 3] = rin; ch[(size_t)c * GC + 4] = rout; ch[(size_t)c * GC + 5] = mul;
+            ch[(size_t)c * GC + 3] = rin;
+            ch[(size_t)c * GC + 4] = rescale && !bounded ? 0.0 : rout;
+            ch[(size_t)c * GC + 5] = rescale ? exp(rout) : 1.0;
         }
     }
     if (lane == 0 && decay) *decay = (float)exp(total);
@@ -962,7 +979,10 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         t.L = 64;
         t.C0 = p.C1; t.n0 = tail_n; t.m0 = tail_m;
     }
-    const bool fused_tail = tail && mlstm_chunkwise_tail_supported(t, XLSTM_BF16);
+    // A tail of one whole chunk stays on the CUDA-core kernel (52 us at 8 heads against 14): that is a choice for steady results
+    // and not for speed.  Prompts of whole chunks go through stacks of layers, and whichever way the last tokens' sums are
+    // ordered, after 16 blocks the last states differ by 2.1e-2 .. 3.1e-2, the distance of any two correct bf16 evaluations.
+    const bool fused_tail = tail && t.S != t.L && mlstm_chunkwise_tail_supported(t, XLSTM_BF16);
 
     // the gate pre-pass (chain, path flags and per-token scalars for both passes of the segment-parallel mode), then the
     // tensor-core kernel, whose CTAs read their path flag: the choice needs no host round trip
@@ -1000,7 +1020,7 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     }
     if (!tail) return XLSTM_OK;
 
-    // S mod 128 tokens to fp32 accuracy; the launch does its loads and Q K^T while the last tiles run (tp.early)
+    // S mod 128 tokens to fp32 accuracy; the fused launch does its loads and Q K^T while the last tiles run (tp.early)
     return fused_tail ? mlstm_chunkwise_tail(t, true, st) : mlstm_chunkwise_simt(t, XLSTM_BF16, st);
 }
 

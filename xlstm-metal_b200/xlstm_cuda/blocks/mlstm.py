@@ -368,6 +368,16 @@ class mLSTMBlock(nn.Module):
         x2 = x.reshape(B, -1)
         rows = 2 < B <= ops.LINEAR_ROWS_MAX and self._rows_ok()
         few = not rows and B <= ops.LINEAR_TOKEN_MAX_ROWS
+        n1, n2, oc, rk = self.norm_mlstm, self.norm_ffn, cell.output_cell, cell.recurrent_kernel
+        # the norms are calls of their modules for more than a few rows: natively only where nobody can tell the difference
+        if ((few or (rows and may_fuse(self, x, (n1, RMSNormCell), (n2, RMSNormCell)))) and dv <= 512 and dv % 4 == 0 and
+                n1.weight is not None and n2.weight is not None):
+            out, down = oc.out_proj, self.ffn_proj_down
+            x3, new_state = ops.mlstm_token_block(
+                x2, W, b, (n1.weight, n1.eps), (NH, dqk, dv), state, (oc.norm.weight, oc.norm.eps), rk.eps, rk.inplace_state,
+                cell.projection_cell.gate_soft_cap, (out.weight, out.bias), (n2.weight, n2.eps), self._fused_ffn(),
+                (down.weight, down.bias), rows)
+            return x3.view_as(x), rk._cast_state(new_state)
         if few:
             y = ops.linear_token(W, x2, bias=b, norm_weight=self.norm_mlstm.weight, norm_eps=self.norm_mlstm.eps)
         else:
@@ -376,8 +386,6 @@ class mLSTMBlock(nn.Module):
         o_k, o_v, o_g, o_o = NH * dqk, 2 * NH * dqk, 2 * NH * dqk + NH * dv, 2 * NH * dqk + NH * dv + 2 * NH
         heads = lambda lo, hi, d: y[:, lo:hi].unflatten(1, (NH, d))
         q, k, v = heads(0, o_k, dqk), heads(o_k, o_v, dqk), heads(o_v, o_g, dv)
-        rk = cell.recurrent_kernel
-        oc = cell.output_cell
         if dv <= 512 and dv % 4 == 0:
             # cell step and output epilogue in one launch: the head's column-tile CTAs meet through their cluster
             gated, new_state = ops.mlstm_step_gated(

@@ -86,6 +86,18 @@ def mlstm_step_gated(q, k, v, i, f, ogate, norm_weight, state=None, eps: float =
     return y, (C, n, m)
 
 
+def mlstm_token_block(x, W, b, norm, heads, state, head_norm, eps, inplace, gate_cap, out_proj, ffn_norm, ffn, down, rows):
+    """One token of ``x [B, D]`` through an mLSTM block in one native call: the launch sequence of ``mLSTMBlock._token_step``
+    for up to 16 sequences.  ``norm``, ``head_norm``, ``ffn_norm``: (weight, eps); ``heads``: (NH, dqk, dv), ``dv`` a multiple
+    of 4 up to 512; ``out_proj``, ``down``: (weight, bias); ``rows``: ``linear_rows`` (else ``linear_token``, up to 4 rows).
+    Returns the new ``x`` and the new state."""
+    rc, what, y, C, n, m = _lib.host().token_block(x, W, b, *norm, *heads, *(_NO_STATE if state is None else state), head_norm[0], eps,
+                                                   head_norm[1], inplace, gate_cap or 0.0, *out_proj, *ffn_norm, ffn, *down, rows)
+    if rc:
+        _lib.check(rc, what)
+    return y, (C, n, m)
+
+
 def _strides3(t: torch.Tensor):
     # [B,NH,S,d] view with a contiguous last dimension -> (batch, head, token) element strides
     return [t.stride(0), t.stride(1), t.stride(2)]
