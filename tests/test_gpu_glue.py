@@ -374,6 +374,24 @@ def test_linear_rows(ops, M, N, K):
     assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (2, 31, 32), (4, 5000, 4096), (3, 17, 1056), (16, 4800, 96), (5, 9600, 2080)])
+def test_linear_rows_with_norm(ops, M, N, K):
+    """One row and sixteen, fewer and more tiles than CTAs, k blocks around a warp's share: the norm in front equals its own
+    launch bit for bit, so the Linear does too."""
+    torch.manual_seed(M * 7 + N + K)
+    t = torch.bfloat16
+    x, nw = torch.randn(M, K, device="cuda").to(t) * 3, torch.rand(K, device="cuda").to(t) + 0.5
+    W, b = (torch.randn(N, K, device="cuda") * 0.05).to(t), torch.randn(N, device="cuda").to(t)
+    xn = ops.rms_norm(x, nw, 1e-6)
+    assert torch.equal(ops.linear_rows(W, x, bias=b, norm_weight=nw, norm_eps=1e-6), ops.linear_rows(W, xn, bias=b))
+    W2 = (torch.randn(2 * N, K, device="cuda") * 0.05).to(t)
+    assert torch.equal(ops.linear_rows(W2, x, swiglu_pair=True, norm_weight=nw), ops.linear_rows(W2, xn, swiglu_pair=True))
+    with pytest.raises(Exception):     # more rows than shared memory is given to
+        ops.linear_rows(W[:, :1].expand(N, 4096).contiguous(), torch.zeros(8, 4096, device="cuda", dtype=t), norm_weight=nw[:1].expand(4096))
+    with pytest.raises(Exception):
+        ops.linear_rows(W, x, residual=torch.zeros(M, N, device="cuda", dtype=t), norm_weight=nw)
+
+
 @pytest.mark.parametrize("K", [32, 64, 288, 1024])
 def test_linear_rows_keeps_infinities(ops, K):
     """An infinite weight gives an infinite result in its row and none elsewhere, also in the last block of k."""

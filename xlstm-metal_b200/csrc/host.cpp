@@ -238,8 +238,8 @@ Result linear(const Tensor &weight, const Tensor &x, const OptTensor &bias, cons
         return max_rows <= 4
             ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M,
                                  (int)N, (int)K, epi, XLSTM_BF16, stream())
-            : xlstm_linear_rows_ex(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(r), y.data_ptr(), (int)M, (int)N, (int)K, epi, flags,
-                                   XLSTM_BF16, stream());
+            : xlstm_linear_rows_norm(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M,
+                                     (int)N, (int)K, epi, flags, XLSTM_BF16, stream());
     });
     return {rc, y};
 }
@@ -281,8 +281,8 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
 }
 
 // One token of B sequences through an mLSTM block, launch after launch as mLSTMBlock._token_step describes them: W, b are the
-// merged input projections, ffn the gate and up projections.  rows: the Linears for up to 16 rows with the norms as launches of
-// their own, else those for up to 4 with the norms in them.  Through Python the seven launches of a block took 140 us of host
+// merged input projections, ffn the gate and up projections.  rows: the Linears for up to 16 rows, else those for up to 4; the
+// norms are in them (more than 48 KB of rows: launches of their own).  Through Python the seven launches of a block took 140 us of host
 // time, as much as the GPU has work for 16 sequences of 4096.
 py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, const OptTensor &norm_w, double norm_eps, int64_t NH,
                       int64_t dqk, int64_t dv, const OptTensor &C0, const OptTensor &n0, const OptTensor &m0,
@@ -294,16 +294,16 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
     const OptTensor none;
     const char *what = rows ? "xlstm_linear_rows_ex" : "xlstm_linear_token";
     auto failed = [&](int rc, const char *call) { return py::make_tuple(rc, call, x, none, none, none); };
-    // weights_settled: the launches before the four Linears are a norm, the cell step, a norm and a Linear
+    // settled: the launch before the Linear is one of this block's, none of which writes weights
     auto project = [&](const Tensor &w, const Tensor &in, const OptTensor &bias, const OptTensor &nw, double ne, const OptTensor &res,
-                       bool pair) -> Result {
+                       bool pair, bool settled) -> Result {
         if (!rows) return linear(w, in, bias, nw, ne, res, pair, 4, false);
-        if (!nw) return linear(w, in, bias, none, 0.0, res, pair, 16, true);
+        if (!nw || in.size(0) * (2 * in.size(1) + 64) + 2 * in.size(1) <= XLSTM_LINEAR_NORM_BYTES) return linear(w, in, bias, nw, ne, res, pair, 16, settled);
         const Result n = norm(in, nw, ne);
         if (n.rc) return n;
         return linear(w, n.y, bias, none, 0.0, res, pair, 16, true);
     };
-    const Result y = project(W, x, b, norm_w, norm_eps, none, false);
+    const Result y = project(W, x, b, norm_w, norm_eps, none, false, false);
     if (y.rc) return failed(y.rc, what);
     int64_t at = 0;
     auto columns = [&](int64_t n) {
@@ -317,11 +317,11 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
     // the launch before the step is the projection above: the state is settled
     const Stepped st = step_gated(q, k, v, i, f, o, head_norm_w, C0, n0, m0, eps, head_norm_eps, inplace, gate_cap, true);
     if (st.rc) return failed(st.rc, "xlstm_mlstm_step_gated_rows");
-    const Result x1 = project(out_w, st.y, out_b, none, 0.0, x, false);
+    const Result x1 = project(out_w, st.y, out_b, none, 0.0, x, false, true);
     if (x1.rc) return failed(x1.rc, what);
-    const Result act = project(ffn, x1.y, none, ffn_norm_w, ffn_norm_eps, none, true);
+    const Result act = project(ffn, x1.y, none, ffn_norm_w, ffn_norm_eps, none, true, true);
     if (act.rc) return failed(act.rc, what);
-    const Result x3 = project(down_w, act.y, down_b, none, 0.0, x1.y, false);
+    const Result x3 = project(down_w, act.y, down_b, none, 0.0, x1.y, false, true);
     return py::make_tuple(x3.rc, what, x3.y, st.state.C, st.state.n, st.state.m);
 }
 

@@ -7,21 +7,33 @@
 // one row) is used as the fragments of TWO k-steps, so weights go from global memory straight into the MMA's registers, 64
 // bytes of a row per quad of lanes, without passing through shared memory.
 //
-// A CTA owns 2 x 16 weight rows (16 gate and 16 up rows for the SwiGLU pair) and its 8 warps take the 32-wide k blocks in
-// turn; the partial sums meet in shared memory, where the epilogue (bias, residual, SwiGLU with the separate layers'
-// roundings) runs.  x comes through L2, half a byte per byte of W.  With XLSTM_LINEAR_WEIGHTS_SETTLED the first U blocks
-// of weights are loaded BEFORE the wait on the preceding kernel, which the caller promises not to have written them.
-// Measured (weights cold, 5 rows): 12304 x 4096 24 us (floor 15.2 at 6.65 TB/s; 385 CTAs in 1.3 waves), 4096 x 10944 23.6
-// (13.5), 21888 x 4096 36 (27).
-#include "common.cuh"
+// One persistent CTA of 16 warps per SM walks tiles of 2 x 16 weight rows (16 gate and 16 up rows for the SwiGLU pair); the
+// warps take the 32-wide k blocks of a tile in turn.  A warp's LR_U blocks in flight run on into the next tile, so the stream of
+// weights does not stop while the partial sums of the 16 warps meet in shared memory for the epilogue (bias, residual, SwiGLU
+// with the separate layers' roundings; two buffers, one barrier a tile).  x comes through L1 and L2, half a byte per byte of W.
+// With XLSTM_LINEAR_WEIGHTS_SETTLED the first weights are loaded BEFORE the wait on the preceding kernel, which the caller
+// promises not to have written them; without it they are only asked of L2.  With a norm in front every CTA normalises the rows
+// for itself, into shared memory, while its first weights are under way (a launch of its own takes 5.8 us between two of these).
+// That is for few rows only: shared memory is taken from the L1, where the weights in flight land.  16 rows of 4096 (132 KB)
+// cost 7 us, and a little more of it 25.
+// Measured (weights cold, 16 rows; a CTA of 8 warps per tile before): 12304 x 4096 21.6 us (26.1; floor 15.4), 4096 x 4096 8.5
+// (11.3; 5.1), 21888 x 4096 as a pair 33.8 (41.0; 27.3), 4096 x 10944 18.0 (24.8; 13.7), 1024 x 1024 2.4 (2.1).  LR_U = 2: 4 %
+// more, 12 warps with LR_U = 4 or 8 with 8: the same within 2 %.
+#include "cp_async.cuh"
+#include "vec16.cuh"
 
 namespace xl {
 namespace {
 
-constexpr int LR_THREADS = 256, LR_WARPS = LR_THREADS / 32;
-constexpr int LR_ROWS = 32;      // weight rows per CTA
+constexpr int LR_THREADS = 512, LR_WARPS = LR_THREADS / 32;
+constexpr int LR_ROWS = 32;      // weight rows per tile
 constexpr int LR_M = 16;         // rows of x
-constexpr int LR_U = 4;          // k blocks in flight per warp: 8 KB of weights
+constexpr int LR_U = 3;          // k blocks in flight per warp: 6 KB of weights
+constexpr int LR_LD = LR_ROWS + 1;
+constexpr uint32_t LR_SMEM = 2 * LR_WARPS * LR_M * LR_LD * sizeof(float);
+
+// bytes between normalised rows of x in shared memory: the eight rows and four 16-byte lanes of a load on different banks
+__host__ __device__ __forceinline__ int norm_ld(int K) { return 2 * K + 64; }
 
 __device__ __forceinline__ uint4 ldg_weights(const __nv_bfloat16 *p) {
     uint4 v;
@@ -36,22 +48,30 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 // EPI: 0 = bias only, 1 = + residual, 2 = SwiGLU pair (W has 2 N rows: gate rows, then up rows)
-template <int EPI>
-__global__ void __launch_bounds__(LR_THREADS, 2)
+template <int EPI, bool NORM>
+__global__ void __launch_bounds__(LR_THREADS, 1)
 linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, const __nv_bfloat16 *__restrict__ bias,
-                   const __nv_bfloat16 *residual, __nv_bfloat16 *__restrict__ y, int M, int N, int K, int weights_settled) {
-    constexpr int STRIDE = EPI == 2 ? 16 : 32;                 // outputs per CTA
-    __shared__ float s_part[LR_WARPS][LR_M][LR_ROWS + 1];
+                   const __nv_bfloat16 *residual, const __nv_bfloat16 *__restrict__ norm_w, float norm_eps,
+                   __nv_bfloat16 *__restrict__ y, int M, int N, int K, int weights_settled) {
+    constexpr int STRIDE = EPI == 2 ? 16 : 32;                 // outputs per tile
+    extern __shared__ __align__(16) float lr_part[];           // [2][LR_WARPS][LR_M][LR_LD]; NORM: the rows of x after it
+    unsigned char *sx = reinterpret_cast<unsigned char *>(lr_part) + LR_SMEM;
+    const int ldx = norm_ld(K);                                // bytes between them
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
-    const int n0 = blockIdx.x * STRIDE;
-    const int blocks = K >> 5;
-    // rows beyond the end read the last one again; their sums are not stored
+    const int blocks = K >> 5, tiles = (N + STRIDE - 1) / STRIDE;
+    const int groups = (blocks + LR_WARPS * LR_U - 1) / (LR_WARPS * LR_U);   // of LR_U blocks of this warp, per tile
+
+    // the load stream: weight rows of the tile it is in (rows beyond the end read the last one again; their sums are not
+    // stored), and the first block of the group
     const __nv_bfloat16 *wp[4], *xp[2];
+    auto rows_of = [&](int tile) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int base = EPI == 2 ? min(n0 + (r & 1) * 8 + g, N - 1) + (r >> 1) * N : min(n0 + r * 8 + g, N - 1);
-        wp[r] = W + (size_t)base * K + c * 8;
-    }
+        for (int r = 0; r < 4; ++r) {
+            const int n0 = tile * STRIDE;
+            const int row = EPI == 2 ? min(n0 + (r & 1) * 8 + g, N - 1) + (r >> 1) * N : min(n0 + r * 8 + g, N - 1);
+            wp[r] = W + (size_t)row * K + c * 8;
+        }
+    };
 #pragma unroll
     for (int r = 0; r < 2; ++r) xp[r] = x + (size_t)min(r * 8 + g, M - 1) * K + c * 8;
 
@@ -63,102 +83,176 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
         for (int r = 0; r < 4; ++r) wr[u][r] = b < blocks ? ldg_weights(wp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
     };
     auto load_x = [&](int u, int b) {
+        if (NORM) return;
 #pragma unroll
         for (int r = 0; r < 2; ++r)
             xr[u][r] = b < blocks ? *reinterpret_cast<const uint4 *>(xp[r] + (size_t)b * 32) : make_uint4(0, 0, 0, 0);
     };
     auto load_first = [&]() {
+        rows_of(blockIdx.x);
 #pragma unroll
         for (int u = 0; u < LR_U; ++u) load_w(u, warp + u * LR_WARPS);
     };
-    if (weights_settled) load_first();
+    if (weights_settled) {
+        load_first();
+    } else if (c == 0) {   // asked of L2 only: what the preceding kernel writes, it writes there
+        rows_of(blockIdx.x);
+#pragma unroll
+        for (int u = 0; u < LR_U; ++u)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (warp + u * LR_WARPS < blocks)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(wp[r] + (size_t)(warp + u * LR_WARPS) * 32));
+    }
     grid_dependency_wait();
     allow_dependents();
     if (!weights_settled) load_first();
-
-    float acc[2][2][4];
+    if (NORM) {   // RMSNorm of the rows, a warp each, summed and rounded as the norm's own launch does; in place
+        const int nvec = K >> 3;
+        unsigned char *snw = sx + (size_t)M * ldx;
+        for (int v = tid; v < nvec; v += LR_THREADS) {
+            for (int m = 0; m < M; ++m) cp_async16(sx + (size_t)m * ldx + v * 16, x + (size_t)m * K + v * 8);
+            cp_async16(snw + v * 16, norm_w + (size_t)v * 8);
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        for (int m = warp; m < M; m += LR_WARPS) {
+            uint4 *row = reinterpret_cast<uint4 *>(sx + (size_t)m * ldx);
+            float ss[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int v = lane; v < nvec; v += 128)
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+                for (int q = 0; q < 4; ++q)
+                    if (v + 32 * q < nvec) {
+                        float a[8];
+                        unpack16<__nv_bfloat16>(row[v + 32 * q], a);
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+                        for (int e = 0; e < 8; ++e) ss[q] += a[e] * a[e];
+                    }
+            float tot = 0.f;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[t][n][e] = 0.f;
+            for (int q = 0; q < 4; ++q) tot += warp_sum(ss[q]);
+            const float inv = rsqrtf(tot / (float)K + norm_eps);
+            for (int v = lane; v < nvec; v += 32) {
+                float a[8], w[8];
+                unpack16<__nv_bfloat16>(row[v], a);
+                ld16<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16 *>(snw + v * 16), w);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) a[e] = a[e] * inv * w[e];
+                st16<__nv_bfloat16>(reinterpret_cast<__nv_bfloat16 *>(row + v), a);
+            }
+        }
+        __syncthreads();
+    }
+    const unsigned char *sxp[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) sxp[r] = sx + min(r * 8 + g, M - 1) * ldx + c * 16;
 #pragma unroll
     for (int u = 0; u < LR_U; ++u) load_x(u, warp + u * LR_WARPS);
-    for (int b0 = warp; b0 < blocks; b0 += LR_U * LR_WARPS) {
+
+    int par = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, par ^= 1) {
+        float acc[2][2][4];
 #pragma unroll
-        for (int u = 0; u < LR_U; ++u) {
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int t = 0; t < 2; ++t)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    mma_bf16(acc[t][n], wr[u][2 * t].x, wr[u][2 * t + 1].x, wr[u][2 * t].y, wr[u][2 * t + 1].y, xr[u][n].x, xr[u][n].y);
-                    mma_bf16(acc[t][n], wr[u][2 * t].z, wr[u][2 * t + 1].z, wr[u][2 * t].w, wr[u][2 * t + 1].w, xr[u][n].z, xr[u][n].w);
+                for (int e = 0; e < 4; ++e) acc[t][n][e] = 0.f;
+        for (int gr = 0; gr < groups; ++gr) {
+            const bool tile_ends = gr + 1 == groups;
+            const int b0 = tile_ends ? warp : warp + (gr + 1) * LR_U * LR_WARPS;   // what the slots are refilled with
+            const bool more = !tile_ends || tile + (int)gridDim.x < tiles;
+            if (tile_ends && more) rows_of(tile + gridDim.x);
+#pragma unroll
+            for (int u = 0; u < LR_U; ++u) {
+                if (NORM) {
+                    const int b = warp + (gr * LR_U + u) * LR_WARPS;
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+                        xr[u][r] = b < blocks ? *reinterpret_cast<const uint4 *>(sxp[r] + b * 64) : make_uint4(0, 0, 0, 0);
                 }
-            const int b = b0 + (u + LR_U) * LR_WARPS;
-            if (b0 + LR_U * LR_WARPS < blocks) { load_w(u, b); load_x(u, b); }
-        }
-    }
-    // element e of a tile: weight row g + 8 (e / 2), x row 2c + (e & 1)
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+                for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s_part[warp][n * 8 + 2 * c + (e & 1)][t * 16 + g + 8 * (e >> 1)] = acc[t][n][e];
-    __syncthreads();
-    auto total = [&](int m, int r) {
-        float s = 0.f;
-#pragma unroll
-        for (int w = 0; w < LR_WARPS; ++w) s += s_part[w][m][r];
-        return s;
-    };
-    if (EPI == 2) {
-        const int m = tid >> 4, r = tid & 15, n = n0 + r;
-        if (m < M && n < N) {
-            // the two projections are rounded to bf16 before the gate, as separate GEMM outputs would be
-            const float gt = __bfloat162float(__float2bfloat16_rn(total(m, r) + (bias ? __bfloat162float(bias[n]) : 0.f)));
-            const float up = __bfloat162float(__float2bfloat16_rn(total(m, 16 + r) + (bias ? __bfloat162float(bias[n + N]) : 0.f)));
-            y[(size_t)m * N + n] = __float2bfloat16_rn(gt / (1.0f + expf(-gt)) * up);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int m = warp + i * LR_WARPS, n = n0 + lane;
-            if (m < M && n < N) {
-                float v = total(m, lane) + (bias ? __bfloat162float(bias[n]) : 0.f);
-                if (EPI == 1) v = __bfloat162float(__float2bfloat16_rn(v)) + __bfloat162float(residual[(size_t)m * N + n]);
-                y[(size_t)m * N + n] = __float2bfloat16_rn(v);
+                    for (int n = 0; n < 2; ++n) {
+                        mma_bf16(acc[t][n], wr[u][2 * t].x, wr[u][2 * t + 1].x, wr[u][2 * t].y, wr[u][2 * t + 1].y, xr[u][n].x, xr[u][n].y);
+                        mma_bf16(acc[t][n], wr[u][2 * t].z, wr[u][2 * t + 1].z, wr[u][2 * t].w, wr[u][2 * t + 1].w, xr[u][n].z, xr[u][n].w);
+                    }
+                if (more) { load_w(u, b0 + u * LR_WARPS); load_x(u, b0 + u * LR_WARPS); }
             }
+        }
+        // element e of an MMA tile: weight row g + 8 (e / 2), x row 2c + (e & 1)
+        float *part = lr_part + par * (LR_WARPS * LR_M * LR_LD);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[(warp * LR_M + n * 8 + 2 * c + (e & 1)) * LR_LD + t * 16 + g + 8 * (e >> 1)] = acc[t][n][e];
+        __syncthreads();
+        auto total = [&](int m, int r) {
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < LR_WARPS; ++w) s += part[(w * LR_M + m) * LR_LD + r];
+            return s;
+        };
+        const int n0 = tile * STRIDE;
+        if (EPI == 2) {
+            const int m = tid >> 4, r = tid & 15, n = n0 + r;
+            if (m < M && n < N) {   // (16 x 16 threads)
+                // the two projections are rounded to bf16 before the gate, as separate GEMM outputs would be
+                const float gt = __bfloat162float(__float2bfloat16_rn(total(m, r) + (bias ? __bfloat162float(bias[n]) : 0.f)));
+                const float up = __bfloat162float(__float2bfloat16_rn(total(m, 16 + r) + (bias ? __bfloat162float(bias[n + N]) : 0.f)));
+                y[(size_t)m * N + n] = __float2bfloat16_rn(gt / (1.0f + expf(-gt)) * up);
+            }
+        } else {
+            const int n = n0 + lane;
+            for (int m = warp; m < M; m += LR_WARPS)
+                if (n < N) {
+                    float v = total(m, lane) + (bias ? __bfloat162float(bias[n]) : 0.f);
+                    if (EPI == 1) v = __bfloat162float(__float2bfloat16_rn(v)) + __bfloat162float(residual[(size_t)m * N + n]);
+                    y[(size_t)m * N + n] = __float2bfloat16_rn(v);
+                }
         }
     }
 }
 
-template <int EPI>
-int linear_rows_launch(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N, int K,
-                       int settled, cudaStream_t st) {
-    const int per = EPI == 2 ? 16 : 32;
-    return launch_overlapped(linear_rows_kernel<EPI>, dim3((N + per - 1) / per), dim3(LR_THREADS), 0, st,
+template <int EPI, bool NORM>
+int linear_rows_launch(const void *W, const void *x, const void *bias, const void *residual, const void *norm_w, float norm_eps,
+                       void *y, int M, int N, int K, int settled, cudaStream_t st) {
+    const int per = EPI == 2 ? 16 : 32, tiles = (N + per - 1) / per;
+    const int64_t smem = (int64_t)LR_SMEM + (NORM ? (int64_t)M * norm_ld(K) + 2 * K : 0);   // rows of x, norm weight
+    if (smem > (int64_t)LR_SMEM + XLSTM_LINEAR_NORM_BYTES) return XLSTM_ERR_UNSUPPORTED;
+    auto kern = linear_rows_kernel<EPI, NORM>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return XLSTM_ERR_CUDA;
+    return launch_overlapped(kern, dim3(tiles < 148 ? tiles : 148), dim3(LR_THREADS), (size_t)smem, st,
                              static_cast<const __nv_bfloat16 *>(W), static_cast<const __nv_bfloat16 *>(x),
                              static_cast<const __nv_bfloat16 *>(bias), static_cast<const __nv_bfloat16 *>(residual),
-                             static_cast<__nv_bfloat16 *>(y), M, N, K, settled);
+                             static_cast<const __nv_bfloat16 *>(norm_w), norm_eps, static_cast<__nv_bfloat16 *>(y), M, N, K, settled);
 }
 
 }  // namespace
 }  // namespace xl
 
-extern "C" int xlstm_linear_rows_ex(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
-                                    int K, int epilogue, int flags, int dtype, void *stream) {
+extern "C" int xlstm_linear_rows_norm(const void *W, const void *x, const void *bias, const void *norm_w, float norm_eps,
+                                      const void *residual, void *y, int M, int N, int K, int epilogue, int flags, int dtype,
+                                      void *stream) {
     if (M <= 0 || N <= 0 || K <= 0 || !W || !x || !y) return XLSTM_ERR_INVALID;
     if (epilogue < 0 || epilogue > 2 || (epilogue == 1 && !residual)) return XLSTM_ERR_INVALID;
     if (flags & ~XLSTM_LINEAR_WEIGHTS_SETTLED) return XLSTM_ERR_INVALID;
-    if (dtype != XLSTM_BF16 || M > xl::LR_M || K % 32) return XLSTM_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x)) & 15u) return XLSTM_ERR_UNSUPPORTED;
+    if (dtype != XLSTM_BF16 || M > xl::LR_M || K % 32 || (norm_w && epilogue == 1)) return XLSTM_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w)) & 15u) return XLSTM_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int settled = flags & XLSTM_LINEAR_WEIGHTS_SETTLED ? 1 : 0;
-    if (epilogue == 2) return xl::linear_rows_launch<2>(W, x, bias, residual, y, M, N, K, settled, st);
-    if (epilogue == 1) return xl::linear_rows_launch<1>(W, x, bias, residual, y, M, N, K, settled, st);
-    return xl::linear_rows_launch<0>(W, x, bias, residual, y, M, N, K, settled, st);
+    auto run = [&](auto kern) { return kern(W, x, bias, residual, norm_w, norm_eps, y, M, N, K, settled, st); };
+    if (norm_w) return epilogue == 2 ? run(xl::linear_rows_launch<2, true>) : run(xl::linear_rows_launch<0, true>);
+    if (epilogue == 2) return run(xl::linear_rows_launch<2, false>);
+    return epilogue == 1 ? run(xl::linear_rows_launch<1, false>) : run(xl::linear_rows_launch<0, false>);
+}
+
+extern "C" int xlstm_linear_rows_ex(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
+                                    int K, int epilogue, int flags, int dtype, void *stream) {
+    return xlstm_linear_rows_norm(W, x, bias, nullptr, 0.f, residual, y, M, N, K, epilogue, flags, dtype, stream);
 }
 
 extern "C" int xlstm_linear_rows(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,

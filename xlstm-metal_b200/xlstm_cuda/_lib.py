@@ -57,6 +57,7 @@ _SIGNATURES = {
     "xlstm_linear_token": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "xlstm_linear_rows": (c_int, [c_void_p] * 5 + [c_int] * 5 + [c_void_p]),
     "xlstm_linear_rows_ex": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_void_p]),
+    "xlstm_linear_rows_norm": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p]),
     "xlstm_geglu": (c_int, [c_void_p] * 2 + [c_int64, c_int, c_int, c_void_p]),
     "xlstm_layer_norm": (c_int, [c_void_p] * 4 + [c_int64, c_int, c_int, c_float, c_int, c_void_p]),
     "xlstm_slstm_gates": (c_int, [c_void_p] * 3 + [ctypes.POINTER(c_void_p)] * 3 + [c_int] * 5 + [c_float, c_int, c_void_p]),

@@ -351,14 +351,14 @@ class mLSTMBlock(nn.Module):
         self.state_dtype = state_dtype
 
     def _token_step(self, x: torch.Tensor, state: Optional[State]):
-        """Single-token path (bf16, fused weights).  Up to 2 sequences every Linear is one weight-streaming kernel with
-        its norm / bias / residual / SwiGLU folded in, so a block is five launches: projections, cell step with the
-        output epilogue, out-projection, FFN up, FFN down.  Up to 16 the streaming kernel multiplies on the tensor cores
-        (the CUDA-core one is bound by its multiply-adds from 3 rows on: 143 us for the four Linears of a 4096-wide block at 4
-        rows, 99 us on the tensor cores) and the two norms are launches of their own; beyond that the Linears are GEMMs.
-        The line at 16 is drawn for calls without a graph, where two launches less count more than the Linears: 16 sequences
-        through 8 blocks take 1.31 ms streamed and 1.54 with GEMMs.  In a captured loop a block of 8 takes 125 us (133 as
-        separate launches), of 16 138 streamed, and GEMMs would be ahead from about 9 on (17 sequences: 129).
+        """Single-token path (bf16, fused weights).  Up to 16 sequences every Linear is one weight-streaming kernel with its
+        norm (for more than a few sequences a launch of its own) / bias / residual / SwiGLU folded in, so a block is five or seven
+        launches in one native call: projections, cell step with the output epilogue, out-projection, FFN up, FFN down.  Up to 2 they multiply on the CUDA cores (small CTAs that flow into the
+        gaps of the launch before: a token of one sequence through 16 blocks of 4096 takes 1.48 ms, 1.60 with the others), from 3 on,
+        where that kernel is bound by its multiply-adds, on the tensor cores.  Where the norms are more than their kernel to
+        somebody (hooks, gradients) the launches are separate calls.  Beyond 16, and from 5 on with weights that the tensor-core
+        kernel does not take, the Linears are GEMMs; the line at 16 is drawn for calls without a graph (16 sequences
+        through 8 blocks of 4096: 1.54 ms with GEMMs, 1.31 streamed when it was drawn).
         More than 4 sequences come here only where may_fuse() allows it.  The cell step reads q, k, v and the gates where
         the merged projection has written them."""
         cell = self.mlstm_cell
@@ -366,12 +366,12 @@ class mLSTMBlock(nn.Module):
         B = x.shape[0]
         NH, dqk, dv = cell.num_heads, cell.qk_dim_per_head, cell.v_dim_per_head
         x2 = x.reshape(B, -1)
+        n1, n2, oc, rk = self.norm_mlstm, self.norm_ffn, cell.output_cell, cell.recurrent_kernel
+        native = (dv <= 512 and dv % 4 == 0 and n1.weight is not None and n2.weight is not None and
+                  may_fuse(self, x, (n1, RMSNormCell), (n2, RMSNormCell)))
         rows = 2 < B <= ops.LINEAR_ROWS_MAX and self._rows_ok()
         few = not rows and B <= ops.LINEAR_TOKEN_MAX_ROWS
-        n1, n2, oc, rk = self.norm_mlstm, self.norm_ffn, cell.output_cell, cell.recurrent_kernel
-        # the norms are calls of their modules for more than a few rows: natively only where nobody can tell the difference
-        if ((few or (rows and may_fuse(self, x, (n1, RMSNormCell), (n2, RMSNormCell)))) and dv <= 512 and dv % 4 == 0 and
-                n1.weight is not None and n2.weight is not None):
+        if native and (rows or few):
             out, down = oc.out_proj, self.ffn_proj_down
             x3, new_state = ops.mlstm_token_block(
                 x2, W, b, (n1.weight, n1.eps), (NH, dqk, dv), state, (oc.norm.weight, oc.norm.eps), rk.eps, rk.inplace_state,
