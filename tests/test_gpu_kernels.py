@@ -948,6 +948,33 @@ def test_chunkwise_short_bf16(ops, T, dqk, dv, state, f_mean):
                 assert relerr(host(got), host(want)) < 1e-5
 
 
+@pytest.mark.parametrize("dqk,dv", [(256, 512), (128, 128)])
+@pytest.mark.parametrize("f_shift", [0.0, -8.0])
+def test_chunkwise_half_columns_equal_whole_ones(ops, dqk, dv, f_shift):
+    """Few heads run on CTAs of 64 columns, many on CTAs of 128: a head's results do not depend on how many others there are,
+    bit for bit, in both tensor-core paths, with a carried state and an uneven last tile."""
+    rng = np.random.default_rng(dqk)
+    few, many, S = 1, 40 * 512 // dv, 300
+    q, k = (dev(rng.standard_normal((1, many, S, dqk)), BF) for _ in range(2))
+    v = dev(rng.standard_normal((1, many, S, dv)), BF)
+    i, f = (dev(a, BF) for a in gates(rng, (1, many, S)))
+    f = f + f_shift
+    st = tuple(dev(rng.standard_normal(s) * 0.1) for s in ((1, many, dqk, dv), (1, many, dqk), (1, many)))
+    try:
+        ops.chunkwise_segments(1)
+        h, s1 = ops.mlstm_chunkwise(q, k, v, i, f, st)
+        hf, sf = ops.mlstm_chunkwise(*(a[:, :few] for a in (q, k, v, i, f)), tuple(s[:, :few].contiguous() for s in st))
+        assert torch.equal(h[:, :few], hf)
+        for a, b in zip(s1, sf):
+            assert torch.equal(a[:, :few], b)
+        for P in (2,):   # segments, whose second pass may be narrow
+            ops.chunkwise_segments(P)
+            hp, sp = ops.mlstm_chunkwise(*(a[:, :few] for a in (q, k, v, i, f)), tuple(s[:, :few].contiguous() for s in st))
+            assert relerr(host(hp), host(hf)) < BF16_TOL and relerr(host(sp[0]), host(sf[0])) < 1e-3
+    finally:
+        ops.chunkwise_segments(None)
+
+
 @pytest.mark.parametrize("S", [128, 4096, 4224])
 def test_chunkwise_gate_prepass_forms_and_mixed_heads(ops, S):
     """1, 32 and 33 tiles: the one-launch gate pre-pass, its last size, and the three-launch form; one head of bounded gate

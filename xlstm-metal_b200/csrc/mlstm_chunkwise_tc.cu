@@ -364,12 +364,12 @@ enum { B_QFULL = 0, B_KFULL, B_VFULL, B_SDONE, B_H1DONE, B_UPDDONE, B_H2DONE, B_
 
 // C pass for one 128-row half after the state update: TMEM -> Cb (bf16) and back to TMEM scaled by
 // the next tile's decay; after the last tile the fp32 rows go to `dst` instead.
-template <int DQK>
+template <int DQK, int W>
 __device__ __forceinline__ void c_pass_half(unsigned char *smem, uint32_t t_half, int j, bool last, float decay_next,
                                             float *dst) {
     using SM = Smem<DQK>;
 #pragma unroll 1
-    for (int c0 = 0; c0 < DVS; c0 += 64) {
+    for (int c0 = 0; c0 < W; c0 += 64) {
         uint32_t va[32], vb[32];
         tmem_ld32(t_half + c0, va);
         tmem_ld32(t_half + c0 + 32, vb);
@@ -414,7 +414,7 @@ __device__ __forceinline__ void c_pass_half(unsigned char *smem, uint32_t t_half
     }
 }
 
-template <int DQK>
+template <int DQK, int W>
 __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     using SM = Smem<DQK>;
     constexpr int NBOX = SM::NBOX;
@@ -431,7 +431,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     const int bh = blockIdx.x;     // (batch, head, segment): index of the states and of the path flag
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;   // (batch, head) and first tile of this segment
     const int b = bhr / p.NH, hd = bhr % p.NH;
-    const int col0 = blockIdx.y * DVS;
+    const int col0 = blockIdx.y * W;
     const int NCH = min(p.seg_tiles, p.NCH - tile0);
     const float *gbase = p.gates + ((size_t)bhr * p.NCH + tile0) * GW;
 
@@ -471,16 +471,16 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
                 mbar_expect_tx(&bars[B_QFULL], NBOX * SM::BOX);
                 for (int q = 0; q < NBOX; ++q) tma_load_4d(smem + SM::Q + q * SM::BOX, &p.tq, &bars[B_QFULL], q * 64, t0, hd, b);
                 if (k > 0 && !mbar_wait(&bars[B_VFREE], (k - 1) & 1, abort_flag)) break;   // h tile staged in V has been stored
-                mbar_expect_tx(&bars[B_VFULL], 2 * SM::BOX);
-                for (int q = 0; q < 2; ++q) tma_load_4d(smem + SM::V + q * SM::BOX, &p.tv, &bars[B_VFULL], col0 + q * 64, t0, hd, b);
+                mbar_expect_tx(&bars[B_VFULL], W / 64 * SM::BOX);
+                for (int q = 0; q < W / 64; ++q) tma_load_4d(smem + SM::V + q * SM::BOX, &p.tv, &bars[B_VFULL], col0 + q * 64, t0, hd, b);
             }
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
         if (lane == 0) {
             constexpr uint32_t ID_KK = idesc_bf16(128, 128, false, false);  // S
-            constexpr uint32_t ID_KM = idesc_bf16(128, 128, false, true);   // inter read-out, P V
-            constexpr uint32_t ID_MM = idesc_bf16(128, 128, true, true);    // state update
+            constexpr uint32_t ID_KM = idesc_bf16(128, W, false, true);   // inter read-out, P V
+            constexpr uint32_t ID_MM = idesc_bf16(128, W, true, true);    // state update
             // descriptors differ only in the start address (low word, units of 16 bytes)
             const uint64_t dQ = smem_desc_sw128(smem_u32(smem + SM::Q), 0, 1024);
             const uint64_t dK = smem_desc_sw128(smem_u32(smem + SM::K), 0, 1024);
@@ -536,11 +536,11 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
                 const int tk = (tile0 + k) * LT;
                 if (p.tok_per_rank > 0 && p.n_h > 0) {   // token-sharded: only the rank that owns these tokens gets the tile
                     const int d = tk / p.tok_per_rank;
-                    for (int bx = 0; bx < 2; ++bx)
+                    for (int bx = 0; bx < W / 64; ++bx)
                         tma_store_4d(&p.th[d], smem + SM::V + bx * SM::BOX, col0 + bx * 64, tk - d * p.tok_per_rank, hd, b);
                 } else {
                     for (int d = 0; d < p.n_h; ++d)
-                        for (int bx = 0; bx < 2; ++bx)
+                        for (int bx = 0; bx < W / 64; ++bx)
                             tma_store_4d(&p.th[d], smem + SM::V + bx * SM::BOX, col0 + bx * 64, tk, hd, b);
                 }
                 tma_store_commit();
@@ -556,7 +556,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
         const int t0w = t & ~31;                       // first row of this warp
         const uint32_t lane_off = (uint32_t)t0w << 16;
         if (NHALF == 2) {  // rows [128,256) of the initial state
-            c_init_half<DQK>(smem, T_C + 128 + lane_off, p.C0 ? p.C0 + ((size_t)bh * DQK + 128 + t) * p.dv + col0 : nullptr,
+            c_init_half<DQK, W>(smem, T_C + 128 + lane_off, p.C0 ? p.C0 + ((size_t)bh * DQK + 128 + t) * p.dv + col0 : nullptr,
                              128 + t, gbase[G_SCAL + 0]);
             tmem_wait_st();
             fence_proxy_async_smem();
@@ -609,7 +609,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
                 const bool last = (k == NCH - 1);
                 if (!(mbar_wait(&bars[B_UPDDONE], ph, abort_flag) && mbar_wait(&bars[B_H1DONE], ph, abort_flag))) break;
                 tc_fence_after_sync();
-                c_pass_half<DQK>(smem, T_C + 128 + lane_off, 128 + t, last, last ? g[G_SCAL + 2] : g[GW + G_SCAL + 0],
+                c_pass_half<DQK, W>(smem, T_C + 128 + lane_off, 128 + t, last, last ? g[G_SCAL + 2] : g[GW + G_SCAL + 0],
                                  p.C1 + ((size_t)bh * DQK + 128 + t) * p.dv + col0);
                 if (!last) {
                     tmem_wait_st();
@@ -643,7 +643,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
         const bool has_state = p.C0 != nullptr;
         // ---- prologue: rows [0,128) of the initial state (rows [128,256) by the P warps), and n
         {
-            c_init_half<DQK>(smem, T_C + lane_off, has_state ? p.C0 + ((size_t)bh * DQK + r) * p.dv + col0 : nullptr, r,
+            c_init_half<DQK, W>(smem, T_C + lane_off, has_state ? p.C0 + ((size_t)bh * DQK + r) * p.dv + col0 : nullptr, r,
                              gbase[G_SCAL + 0]);
             for (int j = r; j < DQK; j += 128) s_n[j] = has_state ? p.n0[(size_t)bh * DQK + j] : 0.f;
             tmem_wait_st();
@@ -665,7 +665,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
             // old Cb), pre-scale C for the next tile; after the last tile write C out instead.
             if (!(mbar_wait(&bars[B_UPDDONE], ph, abort_flag) && mbar_wait(&bars[B_H1DONE], ph, abort_flag))) break;
             tc_fence_after_sync();
-            c_pass_half<DQK>(smem, T_C + lane_off, r, last, decay_next, p.C1 + ((size_t)bh * DQK + r) * p.dv + col0);
+            c_pass_half<DQK, W>(smem, T_C + lane_off, r, last, decay_next, p.C1 + ((size_t)bh * DQK + r) * p.dv + col0);
             if (!last) {
                 tmem_wait_st();
                 fence_proxy_async_smem();
@@ -725,7 +725,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
             // tensor maps; one thread then issues TMA stores to this GPU's h and to every peer's buffer
             unsigned char *stage = smem + SM::V + r * 128;
 #pragma unroll 1
-            for (int c0 = 0; c0 < DVS; c0 += 64) {
+            for (int c0 = 0; c0 < W; c0 += 64) {
                 uint32_t va[32], vb[32];
                 tmem_ld32(T_H + lane_off + c0, va);
                 tmem_ld32(T_H + lane_off + c0 + 32, vb);
@@ -766,30 +766,30 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
 // the CTAs of both kinds share the GPU (one after the other, heads with widely spread gates took twice as long); longer
 // sequences run them one after the other, see launch_tc().  One kernel with both bodies made the bounded path spill (prefill of
 // 4 x 32768: 1.61 -> 1.71 ms).
-template <int DQK>
+template <int DQK, int W>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
     grid_dependency_wait();
     allow_dependents();
-    if (p.path[blockIdx.x] == 0) chunkwise_general<DQK>(p);
+    if (p.path[blockIdx.x] == 0) chunkwise_general<DQK, W>(p);
 }
 // STATE_ONLY: the first pass of the segment-parallel mode, where the bounded path needs no h.
 // The wait for the general launch comes last, in one CTA: this launch is complete only when that one is.
-template <int DQK, bool STATE_ONLY>
+template <int DQK, bool STATE_ONLY, int W>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(const __grid_constant__ TcParams p) {
     // a tail launch follows, which reads only the inputs before its wait: let it start beside this one
     if (!STATE_ONLY && p.early) allow_dependents();
     if (p.path[blockIdx.x] != 0) {
         if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
-        else chunkwise_bounded<DQK>(p);
+        else chunkwise_bounded<DQK, W>(p);
     }
     if (blockIdx.x == 0 && blockIdx.y == 0) grid_dependency_wait();
 }
 
-template <int DQK, bool STATE_ONLY>
+template <int DQK, bool STATE_ONLY, int W>
 int launch_tc(const TcParams &tp, dim3 grid, cudaStream_t st) {
     constexpr uint32_t bytes = STATE_ONLY ? ScanSmem<DQK>::TOTAL : Smem<DQK>::TOTAL;
-    auto general = mlstm_chunkwise_tc_kernel<DQK>;
-    auto fast = mlstm_chunkwise_tc_fast_kernel<DQK, STATE_ONLY>;
+    auto general = mlstm_chunkwise_tc_kernel<DQK, W>;
+    auto fast = mlstm_chunkwise_tc_fast_kernel<DQK, STATE_ONLY, W>;
     if (cudaFuncSetAttribute(general, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<DQK>::TOTAL) != cudaSuccess ||
         cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return XLSTM_ERR_CUDA;
@@ -961,9 +961,19 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     for (int d = 0; d < 3; ++d) tp.sh[d] = p.sh[d];
     const dim3 grid(BH * P, p.dv / DVS);
 
+    // Half the columns per CTA while every CTA still has a pair of SMs to itself: a tile is a chain of products and passes over
+    // the columns, and S, done once more, is the smaller part of it (256/512, 16 tiles: 4 to 16 CTAs 82 -> 66 us, 32 CTAs 85 -> 75).
+    // Beyond that tiles slow down as SMs are added (64 CTAs 89 us, as 128 of half the columns 99; with heads of both gate kinds
+    // 330 and 436).  The columns do not depend on one another: the results are the same bit for bit.
+    const bool narrow = 2 * grid.x * grid.y <= SM_COUNT / 2;
+    const dim3 half(grid.x, 2 * grid.y);
     auto forward = [&](bool state_only) -> int {
-        if (p.dqk == 256) return state_only ? launch_tc<256, true>(tp, grid, st) : launch_tc<256, false>(tp, grid, st);
-        return state_only ? launch_tc<128, true>(tp, grid, st) : launch_tc<128, false>(tp, grid, st);
+        if (p.dqk == 256) {
+            if (state_only) return launch_tc<256, true, DVS>(tp, grid, st);
+            return narrow ? launch_tc<256, false, DVS / 2>(tp, half, st) : launch_tc<256, false, DVS>(tp, grid, st);
+        }
+        if (state_only) return launch_tc<128, true, DVS>(tp, grid, st);
+        return narrow ? launch_tc<128, false, DVS / 2>(tp, half, st) : launch_tc<128, false, DVS>(tp, grid, st);
     };
     float *n_final = tail ? tail_n : p.n1, *m_final = tail ? tail_m : p.m1;
     ChunkwiseParams t = p;   // the tail: continues in place from (C1, tail_n, tail_m)

@@ -11,7 +11,7 @@ namespace tcw {
 using namespace tc;
 
 constexpr int LT = 128;        // tokens per tile
-constexpr int DVS = 128;       // dv columns per CTA
+constexpr int DVS = 128;       // dv columns per CTA; half of them (W = 64) where that still leaves SMs idle
 constexpr int THREADS = 640;
 constexpr int GW = 6 * LT;     // floats of gate scratch per (head, tile)
 constexpr int G_U2 = 0, G_X2 = LT, G_WINQ = 2 * LT, G_W = 3 * LT, G_EMT = 4 * LT, G_SCAL = 5 * LT;
@@ -161,11 +161,11 @@ __device__ __forceinline__ void scale_rows(unsigned char *tile, int row, float w
 
 // One 128-row half of the initial state: global fp32 -> Cb (bf16, swizzled MN-major) and TMEM
 // (pre-scaled by the first tile's decay).  `src` is this thread's row (NULL = zero state).
-template <int DQK>
+template <int DQK, int W>
 __device__ __forceinline__ void c_init_half(unsigned char *smem, uint32_t t_half, const float *src, int j, float decay0) {
     using SM = Smem<DQK>;
 #pragma unroll 1
-    for (int c0 = 0; c0 < DVS; c0 += 32) {
+    for (int c0 = 0; c0 < W; c0 += 32) {
         uint32_t v[32];
 #pragma unroll
         for (int x = 0; x < 32; x += 4) {

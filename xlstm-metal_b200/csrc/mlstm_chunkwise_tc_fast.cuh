@@ -48,12 +48,12 @@ static_assert(F_NBARS <= 24, "barrier slots");
 
 // C pass for one 128-row half after the state update: optional rescale of C~ in TMEM, then the bf16 copy
 // Cb (in the frame the next tile reads it in); after the last tile the fp32 rows go to `dst` instead.
-template <int DQK>
+template <int DQK, int W>
 __device__ __forceinline__ void c_pass_fast(unsigned char *smem, uint32_t t_half, int j, bool last, float mul,
                                             float frame, float *dst) {
     using SM = Smem<DQK>;
 #pragma unroll 1
-    for (int c0 = 0; c0 < DVS; c0 += 64) {
+    for (int c0 = 0; c0 < W; c0 += 64) {
         uint32_t va[32], vb[32];
         tmem_ld32(t_half + c0, va);
         tmem_ld32(t_half + c0 + 32, vb);
@@ -146,7 +146,7 @@ __device__ __forceinline__ float p_pass_part(uint32_t t_rows, int q, int lane, c
     return rowsum;
 }
 
-template <int DQK>
+template <int DQK, int W>
 __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
     using SM = Smem<DQK>;
     constexpr int NBOX = SM::NBOX;
@@ -166,7 +166,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;   // (batch, head) and first tile of this segment
     const int b = bhr / p.NH, hd = bhr % p.NH;
-    const int col0 = blockIdx.y * DVS;
+    const int col0 = blockIdx.y * W;
     const int NCH = min(p.seg_tiles, p.NCH - tile0);
     const float *gbase = p.gates + ((size_t)bhr * p.NCH + tile0) * GW;
 
@@ -210,16 +210,16 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
                 mbar_expect_tx(&bars[F_KFULL], NBOX * SM::BOX);
                 for (int q = 0; q < NBOX; ++q) tma_load_4d(smem + SM::K + q * SM::BOX, &p.tk, &bars[F_KFULL], q * 64, t0, hd, b);
                 if (k > 0 && !mbar_wait(&bars[F_VFREE], pp, abort_flag)) break;   // P V~ done and the h tile staged in V stored
-                mbar_expect_tx(&bars[F_VFULL], 2 * SM::BOX);
-                for (int q = 0; q < 2; ++q) tma_load_4d(smem + SM::V + q * SM::BOX, &p.tv, &bars[F_VFULL], col0 + q * 64, t0, hd, b);
+                mbar_expect_tx(&bars[F_VFULL], W / 64 * SM::BOX);
+                for (int q = 0; q < W / 64; ++q) tma_load_4d(smem + SM::V + q * SM::BOX, &p.tv, &bars[F_VFULL], col0 + q * 64, t0, hd, b);
             }
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
         if (lane == 0) {
             constexpr uint32_t ID_KK = idesc_bf16(128, 128, false, false);  // S
-            constexpr uint32_t ID_KM = idesc_bf16(128, 128, false, true);   // read-out, P V~
-            constexpr uint32_t ID_MM = idesc_bf16(128, 128, true, true);    // state update
+            constexpr uint32_t ID_KM = idesc_bf16(128, W, false, true);   // read-out, P V~
+            constexpr uint32_t ID_MM = idesc_bf16(128, W, true, true);    // state update
             const uint64_t dQ = smem_desc_sw128(smem_u32(smem + SM::Q), 0, 1024);
             const uint64_t dK = smem_desc_sw128(smem_u32(smem + SM::K), 0, 1024);
             const uint64_t dCb = smem_desc_sw128(smem_u32(smem + SM::CB), SM::CB_BLOCK, 1024);
@@ -283,11 +283,11 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
                 const int tk = (tile0 + k) * LT;
                 if (p.tok_per_rank > 0 && p.n_h > 0) {   // token-sharded: only the rank that owns these tokens gets the tile
                     const int d = tk / p.tok_per_rank;
-                    for (int bx = 0; bx < 2; ++bx)
+                    for (int bx = 0; bx < W / 64; ++bx)
                         tma_store_4d(&p.th[d], smem + SM::V + bx * SM::BOX, col0 + bx * 64, tk - d * p.tok_per_rank, hd, b);
                 } else {
                     for (int d = 0; d < p.n_h; ++d)
-                        for (int bx = 0; bx < 2; ++bx)
+                        for (int bx = 0; bx < W / 64; ++bx)
                             tma_store_4d(&p.th[d], smem + SM::V + bx * SM::BOX, col0 + bx * 64, tk, hd, b);
                 }
                 tma_store_commit();
@@ -302,7 +302,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
         const int t0w = t & ~31;                       // first row of this warp
         const uint32_t lane_off = (uint32_t)t0w << 16;
         if (NHALF == 2) {
-            c_init_half<DQK>(smem, T_C + 128 + lane_off, p.C0 ? p.C0 + ((size_t)bh * DQK + 128 + t) * p.dv + col0 : nullptr,
+            c_init_half<DQK, W>(smem, T_C + 128 + lane_off, p.C0 ? p.C0 + ((size_t)bh * DQK + 128 + t) * p.dv + col0 : nullptr,
                              128 + t, 1.0f);
             tmem_wait_st();
             fence_proxy_async_smem();
@@ -315,7 +315,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
             const float *g = gbase + (size_t)k * GW;
             // V~ = diag(a) V in place (these warps are idle until S completes; V arrives early in the tile)
             if (!mbar_wait(&bars[F_VFULL], ph, abort_flag)) break;
-            scale_tile_rows<2>(smem + SM::V, SM::BOX, t, g[G_W + t]);
+            scale_tile_rows<W / 64>(smem + SM::V, SM::BOX, t, g[G_W + t]);
             fence_proxy_async_smem();   // generic-proxy writes -> visible to the tensor-core (async) proxy
             mbar_arrive(&bars[F_VSCALED]);
             if (!(mbar_wait(&bars[F_SAREADY], ph, abort_flag) && mbar_wait(&bars[F_SDONE], ph, abort_flag))) break;
@@ -329,7 +329,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
                 const bool last = (k == NCH - 1);
                 if (!mbar_wait(&bars[F_UPDB], ph, abort_flag)) break;
                 tc_fence_after_sync();
-                c_pass_fast<DQK>(smem, T_C + 128 + lane_off, 128 + t, last, g[G_SCAL + 0], g[G_SCAL + 2],
+                c_pass_fast<DQK, W>(smem, T_C + 128 + lane_off, 128 + t, last, g[G_SCAL + 0], g[G_SCAL + 2],
                                  p.C1 + ((size_t)bh * DQK + 128 + t) * p.dv + col0);
                 if (!last) {
                     tmem_wait_st();
@@ -360,7 +360,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
         const uint32_t lane_off = (uint32_t)(r & ~31) << 16;
         const bool has_state = p.C0 != nullptr;
         {
-            c_init_half<DQK>(smem, T_C + lane_off, has_state ? p.C0 + ((size_t)bh * DQK + r) * p.dv + col0 : nullptr, r, 1.0f);
+            c_init_half<DQK, W>(smem, T_C + lane_off, has_state ? p.C0 + ((size_t)bh * DQK + r) * p.dv + col0 : nullptr, r, 1.0f);
             for (int j = r; j < DQK; j += 128) s_n[j] = has_state ? p.n0[(size_t)bh * DQK + j] : 0.f;
             tmem_wait_st();
             fence_proxy_async_smem();
@@ -401,7 +401,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
             mbar_arrive(&bars[F_NDONE]);   // K no longer read by the CUDA cores; n~ after this tile is final
             if (!mbar_wait(&bars[F_UPDA], ph, abort_flag)) break;
             tc_fence_after_sync();
-            c_pass_fast<DQK>(smem, T_C + lane_off, r, last, mul, frame, p.C1 + ((size_t)bh * DQK + r) * p.dv + col0);
+            c_pass_fast<DQK, W>(smem, T_C + lane_off, r, last, mul, frame, p.C1 + ((size_t)bh * DQK + r) * p.dv + col0);
             if (!last) {
                 tmem_wait_st();
                 fence_proxy_async_smem();
@@ -435,12 +435,12 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
             // tile and stall every other warp's shared-memory accesses.)
             unsigned char *stage = smem + SM::V + r * 128;
 #pragma unroll 1
-            for (int c0 = 0; c0 < DVS; c0 += 64) {
+            for (int c0 = 0; c0 < W; c0 += 64) {
                 uint32_t va[32], vb[32];
                 tmem_ld32(t_h(k) + lane_off + c0, va);
                 tmem_ld32(t_h(k) + lane_off + c0 + 32, vb);
                 tmem_wait_ld();
-                if (c0 == DVS - 64) {                 // H (and s_qn, s_rs) have been read: the next tile may proceed
+                if (c0 == W - 64) {                 // H (and s_qn, s_rs) have been read: the next tile may proceed
                     tc_fence_before_sync();
                     mbar_arrive(&bars[F_HFREE]);
                 }
