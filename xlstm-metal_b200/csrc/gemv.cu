@@ -100,11 +100,12 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_kernel(const __nv_bfloat16 *_
     const int total_warps = gridDim.x * (GV_THREADS / 32);
     const int n_first = blockIdx.x * (GV_THREADS / 32) + warp;
 
-    // ---- L2 prefetch of the head of this warp's first weight row (4 KB: what the first loads will ask for; more
-    //      would only push the running kernel's lines out of L2), then the wait for the preceding kernel
+    // ---- L2 prefetch of the head of this warp's first weight row (1 KB, two of its loads: a token through 16 blocks of 4096
+    //      takes 1.440 ms with 0.5 or 1 KB, 1.446 with 2, 1.471 with 4, 1.545 with 8, 1.457 without; loads into registers
+    //      instead cost resident CTAs, 1.56), then the wait for the preceding kernel
     if (n_first < N) {
         const char *row = reinterpret_cast<const char *>(W + (size_t)n_first * K);
-        const int head = K * 2 < 4096 ? K * 2 : 4096;
+        const int head = K * 2 < 1024 ? K * 2 : 1024;
         if (lane * 128 < head) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + lane * 128));
     }
     grid_dependency_wait();

@@ -20,6 +20,9 @@ namespace xl {
 
 // tile shape (the measured best on B200): dv columns per CTA, threads, rows in flight per thread, CTAs per SM
 constexpr int STEP_DVT = 64, STEP_THREADS = 256, STEP_UNROLL = 4, STEP_MIN_CTAS = 4;
+// with at most one CTA per SM (a sequence or two) the step is latency, not bandwidth: all rows of a thread in flight at once
+// (dqk up to 256), where the state is settled before the wait; a token of one sequence through 16 blocks: @MEASURED@
+constexpr int STEP_UNROLL_FEW = 16;
 
 // GATED: the output epilogue of the layer (per-head RMS norm x weight x sigmoid(output gate)) is applied before
 // the result leaves the chip.  The CTAs of one head (its dv / DVT column tiles) are then launched as ONE CLUSTER
@@ -41,7 +44,7 @@ struct StepRows {
 };
 
 template <typename T, int DVT, int THREADS, int UNROLL, bool GATED>
-__global__ void __launch_bounds__(THREADS, STEP_MIN_CTAS)
+__global__ void __launch_bounds__(THREADS, UNROLL > STEP_UNROLL ? 1 : STEP_MIN_CTAS)
 mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v,
                   const T *__restrict__ ig, const T *__restrict__ fg,
                   const float *C0, const float *__restrict__ n0, const float *__restrict__ m0,
@@ -69,42 +72,52 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     float *Cout = C1 + (size_t)bh * dqk * dv + col;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    // first batch of state rows: in flight while the prologue below runs (and, for a settled state, while the
-    // preceding kernel drains)
+    // first batch of state rows, and what the prologue needs of n and m: in flight while the prologue below runs (and, for a
+    // settled state, while the preceding kernel drains)
     float4 c[UNROLL];
-    if (state_settled) {
+    float mold = 0.0f, nold = 0.0f;
+    auto load_state = [&]() {
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
             const int j = rg + u * RG;
             c[u] = (active && has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
         }
-    }
+        if (has_state) {
+            mold = m0[bh];
+            if (tid < dqk) nold = n0[(size_t)bh * dqk + tid];
+        }
+    };
+    if (state_settled) load_state();
     grid_dependency_wait();
     allow_dependents();
-    if (!state_settled) {
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-            const int j = rg + u * RG;
-            c[u] = (active && has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
-        }
-    }
+    if (!state_settled) load_state();
 
     // stabilised gates (every thread: two exps and a log1p are cheaper than a broadcast)
-    const float it = gate_softcap(Elem<T>::ld(ig + gate_at), gate_cap);
-    const float flog = logsigmoid(gate_softcap(Elem<T>::ld(fg + gate_at), gate_cap));
-    const float mold = has_state ? m0[bh] : 0.0f;
+    const float graw = Elem<T>::ld(ig + gate_at), fraw = Elem<T>::ld(fg + gate_at);
+    // everything else that is read: its latency runs beside the gates'
+    const T *qrow = q + (GATED ? seq * rows.q + (size_t)head * dqk : (size_t)bh * dqk);
+    const T *krow = k + (GATED ? seq * rows.k + (size_t)head * dqk : (size_t)bh * dqk);
+    const float q0 = tid < dqk ? Elem<T>::ld(qrow + tid) : 0.f, k0 = tid < dqk ? Elem<T>::ld(krow + tid) : 0.f;
+    const float4 v4 = active ? ld4(v + (GATED ? seq * rows.v + (size_t)head * dv : (size_t)bh * dv) + col) : zero4;
+    float og = 0.f, ow = 1.f;
+    if (GATED && tid < DVT && tile * DVT + tid < dv) {
+        const int at = tile * DVT + tid;
+        if (gate.norm_w) ow = Elem<T>::ld(static_cast<const T *>(gate.norm_w) + (size_t)head * dv + at);
+        og = Elem<T>::ld(static_cast<const T *>(gate.ogate) + (size_t)seq * gate.ogate_ld + (size_t)head * dv + at);
+    }
+    const float it = gate_softcap(graw, gate_cap);
+    const float flog = logsigmoid(gate_softcap(fraw, gate_cap));
     const float mnew = fmaxf(flog + mold, it);
     const float fgate = expf(flog + mold - mnew);
     const float igate = expf(it - mnew);
 
     // q~, gated k, normaliser update and q~ . n'
-    const T *qrow = q + (GATED ? seq * rows.q + (size_t)head * dqk : (size_t)bh * dqk);
-    const T *krow = k + (GATED ? seq * rows.k + (size_t)head * dqk : (size_t)bh * dqk);
     float qn = 0.0f;
     for (int j = tid; j < dqk; j += THREADS) {
-        const float qj = Elem<T>::ld(qrow + j) * qscale;
-        const float kj = Elem<T>::ld(krow + j);
-        const float nj = fgate * (has_state ? n0[(size_t)bh * dqk + j] : 0.0f) + igate * kj;
+        const bool first = j == tid;
+        const float qj = (first ? q0 : Elem<T>::ld(qrow + j)) * qscale;
+        const float kj = first ? k0 : Elem<T>::ld(krow + j);
+        const float nj = fgate * (first ? nold : has_state ? n0[(size_t)bh * dqk + j] : 0.0f) + igate * kj;
         s_q[j] = qj;
         s_kw[j] = igate * kj;
         qn += nj * qj;
@@ -123,15 +136,17 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
 
     float4 acc = zero4;
     if (active) {
-        const float4 v4 = ld4(v + (GATED ? seq * rows.v + (size_t)head * dv : (size_t)bh * dv) + col);
         for (int j0 = rg; j0 < dqk; j0 += RG * UNROLL) {
-            // next batch goes out before this one is consumed
+            // next batch goes out before this one is consumed (few CTAs: there is none up to dqk = 256)
             float4 nx[UNROLL];
+            auto load_next = [&](float4 (&to)[UNROLL]) {
 #pragma unroll
-            for (int u = 0; u < UNROLL; ++u) {
-                const int j = j0 + (UNROLL + u) * RG;
-                nx[u] = (has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
-            }
+                for (int u = 0; u < UNROLL; ++u) {
+                    const int j = j0 + (UNROLL + u) * RG;
+                    to[u] = (has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
+                }
+            };
+            if (UNROLL == STEP_UNROLL) load_next(nx);
 #pragma unroll
             for (int u = 0; u < UNROLL; ++u) {
                 const int j = j0 + u * RG;
@@ -149,8 +164,12 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
                     acc.w = fmaf(o.w, qj, acc.w);
                 }
             }
+            if (UNROLL == STEP_UNROLL) {
 #pragma unroll
-            for (int u = 0; u < UNROLL; ++u) c[u] = nx[u];
+                for (int u = 0; u < UNROLL; ++u) c[u] = nx[u];
+            } else {
+                load_next(c);
+            }
         }
     }
     st4(s_red + rg * DVT + cv * 4, acc);
@@ -189,20 +208,18 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
             for (unsigned p = 0; p < nc; ++p) tot += cluster.map_shared_rank(s_ss, p)[0];
             const float inv = 1.0f / sqrtf(tot / (float)dv + gate.norm_eps);
             const int c = tile * DVT + tid;
-            const float w = gate.norm_w ? Elem<T>::ld(static_cast<const T *>(gate.norm_w) + (size_t)head * dv + c) : 1.0f;
-            const float og = Elem<T>::ld(static_cast<const T *>(gate.ogate) + (size_t)seq * gate.ogate_ld + (size_t)head * dv + c);
-            Elem<T>::st(h + (size_t)bh * dv + c, hv * inv * w * gate_sigmoid<T>(og));
+            Elem<T>::st(h + (size_t)bh * dv + c, hv * inv * ow * gate_sigmoid<T>(og));
         }
         cluster.sync();                    // nobody leaves while a peer still reads its shared memory
     }
 }
 
-template <typename T>
+template <typename T, int UNROLL>
 static int mlstm_step_launch(const void *q, const void *k, const void *v, const void *ig, const void *fg,
                              const float *C0, const float *n0, const float *m0, void *h, float *C1, float *n1,
                              float *m1, int BH, int dqk, int dv, float eps, float gate_cap, int state_settled,
                              const StepRows &rows, const StepGate *gate, cudaStream_t st) {
-    constexpr int DVT = STEP_DVT, THREADS = STEP_THREADS, UNROLL = STEP_UNROLL;
+    constexpr int DVT = STEP_DVT, THREADS = STEP_THREADS;
     dim3 grid(BH, (dv + DVT - 1) / DVT);
     size_t smem = sizeof(float) * (2 * (size_t)dqk + (THREADS / (DVT / 4)) * DVT);
     if (smem > 200 * 1024) return XLSTM_ERR_UNSUPPORTED;
@@ -269,11 +286,13 @@ static int mlstm_step_checked(const void *q, const void *k, const void *v, const
         ((reinterpret_cast<uintptr_t>(C0) | reinterpret_cast<uintptr_t>(C1)) & 15u))
         return XLSTM_ERR_UNSUPPORTED;
     const int settled = (flags & XLSTM_STEP_STATE_SETTLED) ? 1 : 0;
+    auto run = [&](auto launch) {
+        return launch(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap, settled, rows, gate, st);
+    };
+    const bool few = (int64_t)B * NH * ((dv + xl::STEP_DVT - 1) / xl::STEP_DVT) <= 148 && dqk <= 256;
     if (dtype == XLSTM_F32)
-        return xl::mlstm_step_launch<float>(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap,
-                                            settled, rows, gate, st);
-    return xl::mlstm_step_launch<__nv_bfloat16>(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap,
-                                                settled, rows, gate, st);
+        return few ? run(xl::mlstm_step_launch<float, xl::STEP_UNROLL_FEW>) : run(xl::mlstm_step_launch<float, xl::STEP_UNROLL>);
+    return few ? run(xl::mlstm_step_launch<__nv_bfloat16, xl::STEP_UNROLL_FEW>) : run(xl::mlstm_step_launch<__nv_bfloat16, xl::STEP_UNROLL>);
 }
 
 extern "C" int xlstm_mlstm_step(const void *q, const void *k, const void *v, const void *ig, const void *fg,
