@@ -28,9 +28,14 @@ from .rms_norm import RMSNormCell
 from .soft_cap import soft_cap
 
 
+# elements from which the library's norms are bound by the GPU (a million in bf16: 3 us, as a launch here); below it, the few
+# microseconds that the checks of a fused launch take would be all there is to see
+NORM_MIN_NUMEL = 1 << 20
+
+
 def _norm(owner: nn.Module, norm: nn.Module, kind: type, x: torch.Tensor, groups: int = 1) -> torch.Tensor:
     """``norm(x)`` on the last dimension: as one launch where nothing tells it from the module, else the module itself."""
-    if (may_fuse(owner, x, (norm, kind)) and plain_tensor(x) and
+    if (x.numel() >= NORM_MIN_NUMEL and may_fuse(owner, x, (norm, kind)) and plain_tensor(x) and
             ops.layer_norm_takes(x, norm.weight, norm.bias, groups)):
         return ops.layer_norm(x, norm.weight, norm.bias, norm.eps, groups)
     return norm(x)
@@ -104,7 +109,7 @@ class sLSTMProjectionCell(nn.Module):
         separate modules, the convolution and the three gate projections are one launch and its result is never stored."""
         B, S, _ = x.shape
         conv, lins = self.conv1d, (self.igate_proj, self.fgate_proj, self.ogate_proj)
-        if (type(conv) is CausalConv1d and type(conv.conv) is nn.Conv1d and conv.depthwise and
+        if (x.dtype == torch.bfloat16 and type(conv) is CausalConv1d and type(conv.conv) is nn.Conv1d and conv.depthwise and
                 may_fuse(self, x, (self, sLSTMProjectionCell), (conv, CausalConv1d), *((lin, nn.Linear) for lin in lins)) and
                 plain_tensor(x) and
                 ops.slstm_gates_takes(x, conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins], [lin.bias for lin in lins])):
