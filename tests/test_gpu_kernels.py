@@ -948,6 +948,26 @@ def test_chunkwise_short_bf16(ops, T, dqk, dv, state, f_mean):
                 assert relerr(host(got), host(want)) < 1e-5
 
 
+@pytest.mark.parametrize("shape,f_mean", [((2, 8, 3968, 256, 512), -2.0), ((2, 8, 3968, 256, 512), 3.0), ((1, 4, 2048, 128, 256), -2.0)])
+def test_chunkwise_is_deterministic(ops, shape, f_mean):
+    """The same call gives the same bits, in the general path (gates that forget within a few tokens) and the bounded one, call
+    after call without a wait between them.  A row of Q scaled in place before the last warp had taken its part of q . n showed
+    as single elements of h, in one call of twelve at the first shape."""
+    B, NH, S, dqk, dv = shape
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    args = [rnd(B, NH, S, dqk).to(BF), rnd(B, NH, S, dqk).to(BF), rnd(B, NH, S, dv).to(BF), rnd(B, NH, S).to(BF),
+            (rnd(B, NH, S) + f_mean).to(BF)]
+    try:
+        ops.chunkwise_segments(1)
+        first = ops.mlstm_chunkwise(*args)
+        for _ in range(20):
+            for h, st in [ops.mlstm_chunkwise(*args) for _ in range(6)]:
+                assert torch.equal(h, first[0]) and all(torch.equal(a, b) for a, b in zip(st, first[1]))
+    finally:
+        ops.chunkwise_segments(None)
+
+
 @pytest.mark.parametrize("dqk,dv", [(256, 512), (128, 128)])
 @pytest.mark.parametrize("f_shift", [0.0, -8.0])
 def test_chunkwise_half_columns_equal_whole_ones(ops, dqk, dv, f_shift):

@@ -632,6 +632,8 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
             if (k > 0 && !mbar_wait(&bars[B_HFREE], (k - 1) & 1, abort_flag)) break;
             qn_pass<DQK>(smem, s_n, s_qn, gbase + (size_t)k * GW + G_WINQ, warp - 8, lane);
             mbar_arrive(&bars[B_QNDONE]);
+            // a warp's rows of q . n are spread over the tile, its rows of the scaling are not: all four must have read
+            if (!mbar_wait(&bars[B_QNDONE], ph, abort_flag)) break;
             scale_rows<DQK>(smem + SM::Q, t, winq);
             fence_proxy_async_smem();   // generic-proxy writes -> visible to the tensor-core (async) proxy
             mbar_arrive(&bars[B_QSCALED]);
