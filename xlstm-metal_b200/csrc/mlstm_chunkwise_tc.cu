@@ -691,7 +691,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
             if (q < NBOX) {
                 const unsigned char *box = smem + SM::K + q * SM::BOX + ((cp & 3) << 2);
                 float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
+#pragma unroll 2
                 for (int tt = 0; tt < LT; tt += 4) {
 #pragma unroll
                     for (int x = 0; x < 4; ++x) {

@@ -91,14 +91,14 @@ __device__ __forceinline__ void qn_pass(const unsigned char *smem, const float *
     using SM = Smem<DQK>;
     constexpr int NBOX = SM::NBOX;
     const int c = lane & 7, g = lane >> 3;
-    float part[2][4];
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
+#pragma unroll 1
+    for (int rr = 0; rr < 2; ++rr) {                  // rolled loops: small code (unrolled it was the largest piece of a tile's)
+        float part[4];
         const int rho = 2 * wl + rr;
         const int row0 = rho + 8 * g;                 // rows row0 + 32 i
 #pragma unroll
-        for (int i = 0; i < 4; ++i) part[rr][i] = 0.f;
-#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i] = 0.f;
+#pragma unroll 1
         for (int q = 0; q < NBOX; ++q) {
             // the lane's 8 values of n: two 16-byte loads, issued in an order that puts the 8 lanes of a
             // quarter-warp on 8 different 16-byte bank groups (lanes with logical chunk >= 4 take the upper half first)
@@ -112,24 +112,22 @@ __device__ __forceinline__ void qn_pass(const unsigned char *smem, const float *
             for (int i = 0; i < 4; ++i) {
                 const uint4 v = *reinterpret_cast<const uint4 *>(base + i * 32 * 128);
                 const float2 f0 = unpack_bf16(v.x), f1 = unpack_bf16(v.y), f2 = unpack_bf16(v.z), f3 = unpack_bf16(v.w);
-                part[rr][i] += (f0.x * na.x + f0.y * na.y + f1.x * na.z + f1.y * na.w) +
+                part[i] += (f0.x * na.x + f0.y * na.y + f1.x * na.z + f1.y * na.w) +
                                (f2.x * nb.x + f2.y * nb.y + f3.x * nb.z + f3.y * nb.w);
             }
         }
-    }
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            float v = part[rr][i];
+            float v = part[i];
             v += __shfl_xor_sync(0xffffffffu, v, 1);
             v += __shfl_xor_sync(0xffffffffu, v, 2);
             v += __shfl_xor_sync(0xffffffffu, v, 4);
             if (c == 0) {
-                const int row = (2 * wl + rr) + 8 * g + 32 * i;
+                const int row = row0 + 32 * i;
                 s_qn[row] = row_scale ? v * row_scale[row] : v;
             }
         }
+    }
 }
 
 // In-place row scaling of a [128 x NB*64] bf16 tile (NB boxes of 64 columns, `box_bytes` apart, 128-byte
@@ -139,7 +137,7 @@ template <int NB>
 __device__ __forceinline__ void scale_tile_rows(unsigned char *tile, uint32_t box_bytes, int row, float w) {
     uint32_t whi, wlo;
     split_scale(w, whi, wlo);
-#pragma unroll 2
+#pragma unroll 1
     for (int q = 0; q < NB; ++q) {
         unsigned char *rowp = tile + q * box_bytes + row * 128;
         uint4 v[8];

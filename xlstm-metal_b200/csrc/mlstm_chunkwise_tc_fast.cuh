@@ -32,6 +32,13 @@
 // once P V~ has read it).
 // Every mbarrier wait is bounded; a time-out sets the status word in the scratch buffer, releases all roles
 // and frees TMEM before the CTA returns.
+//
+// The roles' code together is what a tile executes, and it did not fit the instruction caches: 28 % of the fetches missed, and
+// "no instruction" was the largest stall that was not a wait for another role.  So the passes on CUDA cores are loops (q . n over
+// the boxes, the normaliser over the tokens, the scaling over the boxes), the pass over the gate matrix and the slow half of a
+// wait are functions; the MMA issue stays unrolled (rolled: 72 -> 81 us at 64 CTAs).  Before and after, same bits: 4 x 8 heads of
+// 256/512 and 4096 tokens (128 CTAs) 215 -> 179 us; 2 x 8 heads, 3968 tokens, every second head on the general path, whose CTAs
+// share the fetch of a pair of SMs with those of this kernel, 343 -> 235 us; 32 CTAs of half the columns 75 -> 72.
 #pragma once
 #include "mlstm_chunkwise_tc.cuh"
 
@@ -130,7 +137,7 @@ __device__ __forceinline__ float p_piece(const uint32_t (&r)[32], uint32_t t_row
 // warp takes the pieces [0, nl), the "upper" warp [nl, q] and zero-fills the pieces above the diagonal, with
 // nl = (q + 2) / 2: at most two pieces per warp.  This function does the pieces [first, last) and zero-fills
 // [zfirst, 4); it returns the warp's part of the row sums of tril(S) diag(a).
-__device__ __forceinline__ float p_pass_part(uint32_t t_rows, int q, int lane, const float4 *a4, int first, int last,
+static __device__ __noinline__ float p_pass_part(uint32_t t_rows, int q, int lane, const float4 *a4, int first, int last,
                                              int zfirst) {
     float rowsum = 0.f;
     uint32_t r[32];
@@ -378,7 +385,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
             if (q < NBOX) {
                 const unsigned char *box = smem + SM::K + q * SM::BOX + ((cp & 3) << 2);
                 float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
+#pragma unroll 2
                 for (int tt = 0; tt < LT; tt += 4) {
                     const float4 av = *reinterpret_cast<const float4 *>(s_a + tt);
                     const float aw[4] = {av.x, av.y, av.z, av.w};

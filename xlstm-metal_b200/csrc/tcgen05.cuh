@@ -49,8 +49,9 @@ __device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, uint32_t parity
 #ifndef XL_TC_WAIT_CLOCKS
 #define XL_TC_WAIT_CLOCKS (4ll << 30)
 #endif
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
+// Out of line: the kernels wait at dozens of places, and their code does not fit the instruction caches (see the bounded-gate
+// kernel).
+static __device__ __noinline__ bool mbar_wait_on(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
     const long long t0 = clock64();
     for (;;) {
         if (mbar_try_wait_for(bar, parity, 20000u)) return true;
@@ -59,6 +60,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     }
     *abort_flag = 1;
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+    return mbar_try_wait(bar, parity) || mbar_wait_on(bar, parity, abort_flag);
 }
 
 // ---- fences -------------------------------------------------------------------
