@@ -995,6 +995,32 @@ def test_chunkwise_half_columns_equal_whole_ones(ops, dqk, dv, f_shift):
         ops.chunkwise_segments(None)
 
 
+@pytest.mark.parametrize("B,NH,S,dqk,dv,P", [(2, 9, 300, 256, 512, 1), (2, 20, 256, 256, 512, 1), (1, 40, 133, 128, 256, 1),
+                                             (1, 3, 33 * 128 + 5, 128, 256, 1), (1, 5, 9 * 128 + 70, 128, 256, 4)])
+def test_chunkwise_heads_of_both_kinds_equal_each_on_its_own(ops, B, NH, S, dqk, dv, P):
+    """The two launches run side by side, in the order that the number of CTAs and tiles asks for: up to one CTA per SM (of half
+    the columns), more than that, a long pass, segments.  Heads do not depend on one another, so every head gives bit for bit what
+    it gives in a call of its own, where only its kind runs (few CTAs, general launch first)."""
+    rng = np.random.default_rng(NH * S)
+    q, k = (dev(rng.standard_normal((B, NH, S, dqk)), BF) for _ in range(2))
+    v = dev(rng.standard_normal((B, NH, S, dv)), BF)
+    i, f = (dev(a, BF) for a in gates(rng, (B, NH, S)))
+    f[:, 1::2] -= 5
+    st = tuple(dev(rng.standard_normal(s) * 0.1) for s in ((B, NH, dqk, dv), (B, NH, dqk), (B, NH)))
+    try:
+        ops.chunkwise_segments(P)
+        for _ in range(3):
+            h, s1 = ops.mlstm_chunkwise(q, k, v, i, f, st)
+            for hd in (0, 1, NH - 1):
+                one = slice(hd, hd + 1)
+                ho, so = ops.mlstm_chunkwise(*(a[-1:, one] for a in (q, k, v, i, f)), tuple(s[-1:, one].contiguous() for s in st))
+                assert torch.equal(h[-1:, one], ho)
+                for a, b in zip(s1, so):
+                    assert torch.equal(a[-1:, one], b)
+    finally:
+        ops.chunkwise_segments(None)
+
+
 @pytest.mark.parametrize("S", [128, 4096, 4224])
 def test_chunkwise_gate_prepass_forms_and_mixed_heads(ops, S):
     """1, 32 and 33 tiles: the one-launch gate pre-pass, its last size, and the three-launch form; one head of bounded gate

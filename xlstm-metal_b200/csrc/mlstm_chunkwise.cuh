@@ -26,7 +26,7 @@ struct ChunkwiseParams {
 // the first bytes of every scratch buffer: the status word that xlstm_mlstm_chunkwise_status() reads
 constexpr size_t WS_HEADER = 256;
 
-// fp32 arithmetic, any dqk, dv, S: two launches per group of chunks, chunk states in scratch
+// fp32 arithmetic, any dqk, dv, S: launches over groups of chunks, chunk states in scratch
 size_t mlstm_chunkwise_f32_workspace(int B, int NH, int S, int dqk, int dv);
 bool mlstm_chunkwise_f32_supported(const ChunkwiseParams &p, int dtype);
 int mlstm_chunkwise_f32(const ChunkwiseParams &p, int dtype, void *workspace, cudaStream_t st);

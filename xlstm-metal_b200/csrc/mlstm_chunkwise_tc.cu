@@ -428,10 +428,10 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     float *s_rs = reinterpret_cast<float *>(smem + SM::INV);   // row sums of P, by tile parity
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int bh = blockIdx.x;     // (batch, head, segment): index of the states and of the path flag
+    const int bh = head_of_cta<W>(p);     // (batch, head, segment): index of the states and of the path flag
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;   // (batch, head) and first tile of this segment
     const int b = bhr / p.NH, hd = bhr % p.NH;
-    const int col0 = blockIdx.y * W;
+    const int col0 = (int)blockIdx.x % (p.dv / W) * W;
     const int NCH = min(p.seg_tiles, p.NCH - tile0);
     const float *gbase = p.gates + ((size_t)bhr * p.NCH + tile0) * GW;
 
@@ -711,7 +711,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
                 const float n0v = decay * s_n[j] + s0, n1v = decay * s_n[j + 1] + s1;
                 s_n[j] = n0v;
                 s_n[j + 1] = n1v;
-                if (last && blockIdx.y == 0) {
+                if (last && col0 == 0) {
                     const float fr = g[G_SCAL + 2];   // n = n~ e^{rho}
                     p.n1[(size_t)bh * DQK + j] = n0v * fr; p.n1[(size_t)bh * DQK + j + 1] = n1v * fr;
                 }
@@ -762,51 +762,66 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
     if (tid == 0 && *abort_flag) atomicExch(p.status, 1);
 }
 
+constexpr int SM_COUNT = 148;          // B200
+
 // Two launches over the same (head, segment)s, for the gates of either kind; the choice is the pre-pass's path flag, so it
-// needs no host round trip, and a CTA of the other kind returns at once.  Up to FUSED_TILES tiles they run side by side: the
-// general launch lets the second one start as soon as its own CTAs have, and that one reads nothing the first has written, so
-// the CTAs of both kinds share the GPU (one after the other, heads with widely spread gates took twice as long); longer
-// sequences run them one after the other, see launch_tc().  One kernel with both bodies made the bounded path spill (prefill of
-// 4 x 32768: 1.61 -> 1.71 ms).
-template <int DQK, int W>
+// needs no host round trip, and a CTA of the other kind returns at once.  They run side by side: the first lets the second one
+// start as soon as its CTAs run or have returned, and the second reads nothing the first has written, so the CTAs of both kinds
+// share the GPU.  The second one's wait for the first comes last, in one CTA: it is complete only when the first is.
+// One kernel with both bodies made the bounded path spill (prefill of 4 x 32768: 1.61 -> 1.71 ms).
+template <int DQK, int W, bool SECOND>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_kernel(const __grid_constant__ TcParams p) {
-    grid_dependency_wait();
-    allow_dependents();
-    if (p.path[blockIdx.x] == 0) chunkwise_general<DQK, W>(p);
+    if constexpr (!SECOND) {
+        grid_dependency_wait();
+        allow_dependents();
+    } else if (p.early) {
+        allow_dependents();     // a tail follows, which reads only the inputs before its wait: let it start beside this launch
+    }
+    if (p.path[head_of_cta<W>(p)] == 0) chunkwise_general<DQK, W>(p);
+    if (SECOND && blockIdx.x == 0) grid_dependency_wait();
 }
 // STATE_ONLY: the first pass of the segment-parallel mode, where the bounded path needs no h.
-// The wait for the general launch comes last, in one CTA: this launch is complete only when that one is.
-template <int DQK, bool STATE_ONLY, int W>
+template <int DQK, bool STATE_ONLY, int W, bool SECOND>
 __global__ void __launch_bounds__(THREADS, 1) mlstm_chunkwise_tc_fast_kernel(const __grid_constant__ TcParams p) {
-    // a tail launch follows, which reads only the inputs before its wait: let it start beside this one
-    if (!STATE_ONLY && p.early) allow_dependents();
-    if (p.path[blockIdx.x] != 0) {
+    if constexpr (!SECOND) grid_dependency_wait();
+    else if (!STATE_ONLY && p.early) allow_dependents();
+    if (p.path[head_of_cta<W>(p)] != 0) {
+        // as the first launch only now: where no head is of this kind, the other one's CTAs find the GPU empty
+        if constexpr (!SECOND) allow_dependents();
         if constexpr (STATE_ONLY) chunkwise_state_scan<DQK>(p);
         else chunkwise_bounded<DQK, W>(p);
     }
-    if (blockIdx.x == 0 && blockIdx.y == 0) grid_dependency_wait();
+    if (SECOND && blockIdx.x == 0) grid_dependency_wait();
 }
 
-template <int DQK, bool STATE_ONLY, int W>
-int launch_tc(const TcParams &tp, dim3 grid, cudaStream_t st) {
+template <int DQK, bool STATE_ONLY, int W, bool BOUNDED_FIRST>
+int launch_both(const TcParams &tp, int grid, cudaStream_t st) {
     constexpr uint32_t bytes = STATE_ONLY ? ScanSmem<DQK>::TOTAL : Smem<DQK>::TOTAL;
-    auto general = mlstm_chunkwise_tc_kernel<DQK, W>;
-    auto fast = mlstm_chunkwise_tc_fast_kernel<DQK, STATE_ONLY, W>;
+    auto general = mlstm_chunkwise_tc_kernel<DQK, W, BOUNDED_FIRST>;
+    auto fast = mlstm_chunkwise_tc_fast_kernel<DQK, STATE_ONLY, W, !BOUNDED_FIRST>;
     if (cudaFuncSetAttribute(general, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<DQK>::TOTAL) != cudaSuccess ||
         cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
         return XLSTM_ERR_CUDA;
-    // Long sequences: CTAs that start one by one as the kernel before drains land unevenly on the GPU's clusters of SMs and
-    // stay there for the whole pass (4 x 32768, 128 CTAs: 1.61 -> 1.71 ms), so each launch starts on an idle GPU.  Measured with
-    // gates of one kind; heads of both kinds pay for it with the sum of the two passes.
-    if (tp.NCH > FUSED_TILES) {
-        general<<<grid, THREADS, Smem<DQK>::TOTAL, st>>>(tp);
-        if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
+    if constexpr (BOUNDED_FIRST) {
         fast<<<grid, THREADS, bytes, st>>>(tp);
-        return cudaGetLastError() == cudaSuccess ? XLSTM_OK : XLSTM_ERR_CUDA;
+        if (cudaGetLastError() != cudaSuccess) return XLSTM_ERR_CUDA;
+        return launch_overlapped(general, dim3(grid), dim3(THREADS), Smem<DQK>::TOTAL, st, tp);
+    } else {
+        const int rc = launch_overlapped(general, dim3(grid), dim3(THREADS), Smem<DQK>::TOTAL, st, tp);
+        return rc == XLSTM_OK ? launch_overlapped(fast, dim3(grid), dim3(THREADS), bytes, st, tp) : rc;
     }
-    const int rc = launch_overlapped(general, grid, dim3(THREADS), Smem<DQK>::TOTAL, st, tp);
-    if (rc != XLSTM_OK) return rc;
-    return launch_overlapped(fast, grid, dim3(THREADS), bytes, st, tp);
+}
+
+// CTAs that start one by one as the kernel before drains land unevenly on the GPU's clusters of SMs and stay there for the whole
+// pass (4 x 32768, 128 CTAs: 1.61 -> 1.71 ms).  So the bounded kernel, which most sequences take, comes first and on an idle GPU
+// where the pass is long or most SMs get a CTA.  With the general launch in front and only short sequences side by side, heads of
+// both kinds took, us at 256/512: 32 heads, 4001 tokens 387 (now 270), 32 x 8192 730 (450), 16 x 16384 1396 (833).  Short passes of
+// few CTAs keep the general launch in front and both overlapped with what precedes them: an idle GPU costs 2 of 70 us there, and the
+// general path 3 of 104.
+template <int DQK, bool STATE_ONLY, int W>
+int launch_tc(const TcParams &tp, int grid, cudaStream_t st) {
+    const bool idle = tp.NCH > FUSED_TILES || grid > SM_COUNT / 2;
+    return idle ? launch_both<DQK, STATE_ONLY, W, true>(tp, grid, st) : launch_both<DQK, STATE_ONLY, W, false>(tp, grid, st);
 }
 
 }  // namespace
@@ -839,7 +854,6 @@ struct WsLayout {
     int P, seg_tiles;
 };
 
-constexpr int SM_COUNT = 148;          // B200
 constexpr int MIN_SEG_TILES = 2, LONG_SEG_TILES = 16;
 
 // Number of segments every sequence is cut into.  Cutting buys parallelism while the grid of persistent CTAs (one per head
@@ -961,21 +975,20 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
     tp.NH = p.NH; tp.dv = p.dv; tp.NCH = nch; tp.eps = p.eps; tp.log2_qscale = log2f(p.qscale); tp.status = status;
     tp.path = path; tp.h = p.h; tp.P = P; tp.seg_tiles = seg_tiles;
     for (int d = 0; d < 3; ++d) tp.sh[d] = p.sh[d];
-    const dim3 grid(BH * P, p.dv / DVS);
+    const int ctas = BH * P * (p.dv / DVS);
 
-    // Half the columns per CTA while every CTA still has a pair of SMs to itself: a tile is a chain of products and passes over
-    // the columns, and S, done once more, is the smaller part of it (256/512, 16 tiles: 4 to 16 CTAs 82 -> 66 us, 32 CTAs 85 -> 75).
-    // Beyond that tiles slow down as SMs are added (64 CTAs 89 us, as 128 of half the columns 99; with heads of both gate kinds
-    // 330 and 436).  The columns do not depend on one another: the results are the same bit for bit.
-    const bool narrow = 2 * grid.x * grid.y <= SM_COUNT / 2;
-    const dim3 half(grid.x, 2 * grid.y);
+    // Half the columns per CTA while every CTA still has an SM to itself: a tile is a chain of products and passes over
+    // the columns, and S, done once more, is the smaller part of it (256/512, 16 tiles: 4 to 16 CTAs 82 -> 66 us, 32 CTAs 85 -> 75;
+    // 64 CTAs 94 -> 81, with 128 tiles 617 -> 523; on the general path 126 -> 121 and 812 -> 825).  The columns do not depend on one
+    // another: the results are the same bit for bit.
+    const bool narrow = 2 * ctas <= SM_COUNT;
     auto forward = [&](bool state_only) -> int {
         if (p.dqk == 256) {
-            if (state_only) return launch_tc<256, true, DVS>(tp, grid, st);
-            return narrow ? launch_tc<256, false, DVS / 2>(tp, half, st) : launch_tc<256, false, DVS>(tp, grid, st);
+            if (state_only) return launch_tc<256, true, DVS>(tp, ctas, st);
+            return narrow ? launch_tc<256, false, DVS / 2>(tp, 2 * ctas, st) : launch_tc<256, false, DVS>(tp, ctas, st);
         }
-        if (state_only) return launch_tc<128, true, DVS>(tp, grid, st);
-        return narrow ? launch_tc<128, false, DVS / 2>(tp, half, st) : launch_tc<128, false, DVS>(tp, grid, st);
+        if (state_only) return launch_tc<128, true, DVS>(tp, ctas, st);
+        return narrow ? launch_tc<128, false, DVS / 2>(tp, 2 * ctas, st) : launch_tc<128, false, DVS>(tp, ctas, st);
     };
     float *n_final = tail ? tail_n : p.n1, *m_final = tail ? tail_m : p.m1;
     ChunkwiseParams t = p;   // the tail: continues in place from (C1, tail_n, tail_m)

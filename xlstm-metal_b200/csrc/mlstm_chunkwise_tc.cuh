@@ -30,11 +30,16 @@ struct TcParams {
     int *status;
     const int *path;               // [B*NH*P] 1: this (head, segment) fits the bounded-spread kernel, 0: general kernel
     int P, seg_tiles;              // the sequence of every head is cut into P segments of seg_tiles tiles (P = 1: no cut);
-                                   // blockIdx.x = (batch * NH + head) * P + segment; C0, n0, C1, n1 and path are per segment
-    int early;                     // the launch after the bounded kernel may start as soon as all its CTAs have
+                                   // C0, n0, C1, n1 and path are per (batch * NH + head) * P + segment
+    int early;                     // the launch after the second kernel may start as soon as all CTAs of that one have
     void *h;                       // h of this GPU as a plain pointer with its element strides (batch, head, token)
     int64_t sh[3];
 };
+
+// (batch, head, segment) of this CTA.  Its columns vary fastest: CTAs next to one another share a pair of SMs and its
+// instruction cache, so that a pair runs only one of the two kernels where heads take different ones (32 heads, 2048 tokens, every
+// second head on the general path: 195 us with the heads fastest, 147 so).
+template <int W> __device__ __forceinline__ int head_of_cta(const TcParams &p) { return (int)blockIdx.x / (p.dv / W); }
 
 template <int DQK> struct Smem {
     static constexpr int NBOX = DQK / 64;                  // 64-column TMA boxes of a Q / K tile

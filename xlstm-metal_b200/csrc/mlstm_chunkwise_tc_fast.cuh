@@ -160,7 +160,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
     constexpr int NHALF = DQK / 128;
     constexpr int F_UPDLAST = (NHALF == 2) ? F_UPDB : F_UPDA;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int bh = blockIdx.x;     // (batch, head, segment): index of the states and of the path flag
+    const int bh = head_of_cta<W>(p);     // (batch, head, segment): index of the states and of the path flag
 
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + SM::BARS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + SM::MISC);
@@ -173,7 +173,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;   // (batch, head) and first tile of this segment
     const int b = bhr / p.NH, hd = bhr % p.NH;
-    const int col0 = blockIdx.y * W;
+    const int col0 = (int)blockIdx.x % (p.dv / W) * W;
     const int NCH = min(p.seg_tiles, p.NCH - tile0);
     const float *gbase = p.gates + ((size_t)bhr * p.NCH + tile0) * GW;
 
@@ -401,7 +401,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
                 const float n1v = s_n[j + 1] + (a1[0] + a1[1]) + (a1[2] + a1[3]);
                 s_n[j] = n0v * mul;
                 s_n[j + 1] = n1v * mul;
-                if (last && blockIdx.y == 0) {   // n = n~ e^{rho'}
+                if (last && col0 == 0) {   // n = n~ e^{rho'}
                     p.n1[(size_t)bh * DQK + j] = n0v * frame; p.n1[(size_t)bh * DQK + j + 1] = n1v * frame;
                 }
             }

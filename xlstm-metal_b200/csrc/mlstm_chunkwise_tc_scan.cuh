@@ -44,7 +44,7 @@ __device__ __forceinline__ void chunkwise_state_scan(const TcParams &p) {
     constexpr int NBOX = SM::NBOX;
     constexpr int NHALF = DQK / 128;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int bh = blockIdx.x;     // (batch, head, segment)
+    const int bh = head_of_cta<DVS>(p);     // (batch, head, segment)
 
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + SM::BARS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + SM::MISC);
@@ -54,7 +54,7 @@ __device__ __forceinline__ void chunkwise_state_scan(const TcParams &p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bhr = bh / p.P, tile0 = (bh % p.P) * p.seg_tiles;
     const int b = bhr / p.NH, hd = bhr % p.NH;
-    const int col0 = blockIdx.y * DVS;
+    const int col0 = (int)blockIdx.x % (p.dv / DVS) * DVS;
     const int NCH = min(p.seg_tiles, p.NCH - tile0);
     const float *gbase = p.gates + ((size_t)bhr * p.NCH + tile0) * GW;
 
@@ -153,7 +153,7 @@ __device__ __forceinline__ void chunkwise_state_scan(const TcParams &p) {
                 const float n1v = s_n[j + 1] + (a1[0] + a1[1]) + (a1[2] + a1[3]);
                 s_n[j] = n0v * mul;
                 s_n[j + 1] = n1v * mul;
-                if (last && blockIdx.y == 0) {
+                if (last && col0 == 0) {
                     p.n1[(size_t)bh * DQK + j] = n0v * frame; p.n1[(size_t)bh * DQK + j + 1] = n1v * frame;
                 }
             }
