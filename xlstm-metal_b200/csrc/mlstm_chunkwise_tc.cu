@@ -858,27 +858,30 @@ constexpr int MIN_SEG_TILES = 2, LONG_SEG_TILES = 16;
 
 // Number of segments every sequence is cut into.  Cutting buys parallelism while the grid of persistent CTAs (one per head
 // and 128 dv columns) leaves SMs idle, at the price of the state-only first pass, of the states going through HBM and of
-// three more launches.  Microseconds fitted to forced segment counts at 256/512, 8 to 128 CTAs, 2 to 32 tiles a segment:
-//   one pass    13 + tiles x (4.55 up to 32 CTAs, 5.3 at 64, 6.75 at 128)
-//   two passes  35 + tiles of a segment x (7.1 at 64 CTAs, 9 at 128)
+// three more launches.  Microseconds at 256/512, bounded gates, forced segment counts, 2 to 64 tiles a segment:
+//   up to 32 CTAs in one pass   one 13 + tiles x 4.55, two 35 + tiles of a segment x (5.2 + 0.03 a CTA of all segments)
+//   more of them                one 20 + tiles x (3.05 + 0.014 a CTA), two 43 + tiles of a segment x (5.6 + 0.0117 a CTA)
+// The first line is above what bounded gates take now (one pass 10 + 3.9, 8 heads, S = 2048: 72 us) and asks for the cuts that suit
+// both kinds of gates: the lines that fit these best would cut 4 heads of 2048 tokens in 4 instead of 8 (54 and 56 us, but general
+// 85 and 71), while 6 heads in one pass instead of 6 segments take 71 and 62 us (general 104 and 86).
 // With segments of less than LONG_SEG_TILES a quarter has to be gained.  That is a choice for steady results and not for speed:
 // cutting moves the bf16 copy of C to other frames, and after the 16 blocks of a model the last states differ by 3e-2 from those
-// of one pass (the distance of any two correct bf16 evaluations there), which smaller gains were not given.  8 heads,
-// S = 4096: 167 us in one pass, 109 in 4 segments; 4 heads, S = 2048: 84 and 54 (8); 2 heads, S = 8192: 283, 127 in 4 segments
-// and 72 in 16; 8 heads, S = 2048, which the quarter keeps in one pass: 85 and 74 (4), S = 1024: 51 and 54.  The fit knows
-// bounded gates at 256/512 only: 128/256 follows the same order (S = 8192, 4 heads: 250 and 51), the general path costs 7.5 us
-// a tile where the bounded one costs 4.55.
+// of one pass (the distance of any two correct bf16 evaluations there), which smaller gains were not given.
+// us, bounded / general: 8 heads, S = 4096: 139 / 214 in one pass, 101 / 159 in 4 segments, S = 2048, which stays in one pass: 72 /
+// 105 and 70 / 99 (4); 16 heads, S = 4096: 145 / 223 in one pass, 159 / 264 in two, S = 8192: 268 and 261 (2); 18 heads, S = 6144:
+// 212 / 333 and 219 / 381; 4 heads, S = 8192: 257 and 101 (8).  128/256 follows the same order.
 int plan_segments(int BH, int dv, int nch) {
     const int ctas = BH * (dv / DVS);
     int pmax = SM_COUNT / ctas;
     if (pmax > nch / MIN_SEG_TILES) pmax = nch / MIN_SEG_TILES;
     if (pmax > 64) pmax = 64;
-    const float one = 13.0f + nch * (ctas <= 32 ? 4.55f : 3.9f + 0.022f * ctas);
+    const bool few = ctas <= 32;
+    const float one = few ? 13.0f + nch * 4.55f : 20.0f + nch * (3.05f + 0.014f * ctas);
     int best = 1;
     float best_us = one;
     for (int P = 2; P <= pmax; ++P) {
         const int tiles = (nch + P - 1) / P;
-        const float us = 35.0f + tiles * (5.2f + 0.03f * ctas * P);
+        const float us = few ? 35.0f + tiles * (5.2f + 0.03f * ctas * P) : 43.0f + tiles * (5.6f + 0.0117f * ctas * P);
         if (us < best_us && (tiles >= LONG_SEG_TILES || us < 0.75f * one)) { best_us = us; best = P; }
     }
     return best;
