@@ -473,6 +473,7 @@ __device__ __forceinline__ void chunkwise_general(const TcParams &p) {
                 if (k > 0 && !mbar_wait(&bars[B_VFREE], (k - 1) & 1, abort_flag)) break;   // h tile staged in V has been stored
                 mbar_expect_tx(&bars[B_VFULL], W / 64 * SM::BOX);
                 for (int q = 0; q < W / 64; ++q) tma_load_4d(smem + SM::V + q * SM::BOX, &p.tv, &bars[B_VFULL], col0 + q * 64, t0, hd, b);
+                if (k + 1 < NCH) prefetch_tile<DQK, W>(p, t0 + LT, hd, b, col0);
             }
         }
     } else if (warp == 1) {

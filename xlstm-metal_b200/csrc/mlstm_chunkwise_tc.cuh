@@ -41,6 +41,18 @@ struct TcParams {
 // second head on the general path: 195 us with the heads fastest, 147 so).
 template <int W> __device__ __forceinline__ int head_of_cta(const TcParams &p) { return (int)blockIdx.x / (p.dv / W); }
 
+// Q, K and V of the tile at token t0 into L2.  Shared memory holds one tile, so its loads wait for the tile before, and what they
+// would find in HBM only is latency of the tile's chain.  The CTAs of a head share the boxes of Q and K among them.  us, bounded /
+// general gates: 32 heads, 2048 tokens 100.5 -> 95.7 / 130 -> 128, 32 x 8192 330 -> 311 / 437 -> 428, 16 x 16384 at 128/256 475 -> 433 /
+// 629 -> 592; inputs that are in L2 do not change (8 x 2048: 71, from HBM 83 -> 81).  Two tiles ahead gave the same or less; the one
+// loss seen is the general path alone on 128 CTAs of 64 columns, 16 x 16384 at 256/512: 825 -> 850.
+template <int DQK, int W> __device__ __forceinline__ void prefetch_tile(const TcParams &p, int t0, int hd, int b, int col0) {
+    constexpr int NBOX = DQK / 64;
+    const int cols = p.dv / W;
+    for (int q = col0 / W; q < 2 * NBOX; q += cols) tma_prefetch_4d(q < NBOX ? &p.tq : &p.tk, q % NBOX * 64, t0, hd, b);
+    for (int q = 0; q < W / 64; ++q) tma_prefetch_4d(&p.tv, col0 + q * 64, t0, hd, b);
+}
+
 template <int DQK> struct Smem {
     static constexpr int NBOX = DQK / 64;                  // 64-column TMA boxes of a Q / K tile
     static constexpr uint32_t BOX = LT * 128;              // bytes of one box: 128 rows x 128 B

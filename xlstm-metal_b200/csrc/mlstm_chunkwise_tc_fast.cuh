@@ -212,6 +212,7 @@ __device__ __forceinline__ void chunkwise_bounded(const TcParams &p) {
                 if (k > 0 && !(mbar_wait(&bars[F_SDONE], pp, abort_flag) && mbar_wait(&bars[F_QNDONE], pp, abort_flag))) break;
                 mbar_expect_tx(&bars[F_QFULL], NBOX * SM::BOX);
                 for (int q = 0; q < NBOX; ++q) tma_load_4d(smem + SM::Q + q * SM::BOX, &p.tq, &bars[F_QFULL], q * 64, t0, hd, b);
+                if (k + 1 < NCH) prefetch_tile<DQK, W>(p, t0 + LT, hd, b, col0);
                 // the normaliser update of tile k-1 is completion k of its barrier (completion 0 = initial n)
                 if (k > 0 && !(mbar_wait(&bars[F_UPDLAST], pp, abort_flag) && mbar_wait(&bars[F_NDONE], k & 1, abort_flag))) break;
                 mbar_expect_tx(&bars[F_KFULL], NBOX * SM::BOX);
