@@ -88,6 +88,12 @@ __device__ __forceinline__ void chunkwise_state_scan(const TcParams &p) {
                 mbar_expect_tx(&bars[S_VFULL0 + s], 2 * SM::BOX);
                 for (int q = 0; q < 2; ++q)
                     tma_load_4d(smem + SM::V + s * SM::VSTAGE + q * SM::BOX, &p.tv, &bars[S_VFULL0 + s], col0 + q * 64, t0, hd, b);
+                // the next stage's tile into L2, as in prefetch_tile() (8 heads, 8192 tokens in 4 segments 150 -> 148.5 us for both
+                // passes, 16 x 8192 at 128/256 130 -> 127); the first two tiles are loaded at once
+                if (k >= 1 && k + 1 < NCH) {
+                    for (int q = col0 / DVS; q < NBOX; q += p.dv / DVS) tma_prefetch_4d(&p.tk, q * 64, t0 + LT, hd, b);
+                    for (int q = 0; q < 2; ++q) tma_prefetch_4d(&p.tv, col0 + q * 64, t0 + LT, hd, b);
+                }
             }
         }
     } else if (warp == 1) {
