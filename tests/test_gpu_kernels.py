@@ -807,6 +807,67 @@ def test_step_with_a_state_that_is_converted(ops, state_dtype, strided):
         assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("part", ["n", "m"])
+@pytest.mark.parametrize("form", ["bf16", "strided", "written"])
+@pytest.mark.parametrize("B,dqk,dv", [(1, 256, 512), (16, 256, 512)])
+def test_step_with_a_normaliser_or_stabiliser_written_just_before(ops, part, form, B, dqk, dv):
+    """A settled state vouches for C alone.  n or m in bf16 or with strides is copied by the launch right before the step, or the
+    caller writes it there: the step sees what was written, bit for bit, through the plain step, the gated one and a block's token."""
+    from xlstm_cuda.blocks import mLSTMBlock
+    torch.manual_seed(2)
+    NH, bf = 8, torch.bfloat16
+    rnd = lambda *s: torch.randn(*s, device="cuda")
+    q, k, v = rnd(B, NH, dqk).to(bf), rnd(B, NH, dqk).to(bf), rnd(B, NH, dv).to(bf)
+    i, f, og = rnd(B, NH).to(bf), rnd(B, NH).to(bf), rnd(B, NH * dv).to(bf)
+    w = torch.ones(NH * dv, device="cuda", dtype=bf)
+    with torch.inference_mode():
+        blk = mLSTMBlock(0, embedding_dim=512, num_heads=4, compute_dtype=bf).cuda().to(bf)
+        blk.fuse_projections()
+        cell = blk.mlstm_cell
+        bh, bk, bv = cell.num_heads, cell.qk_dim_per_head, cell.v_dim_per_head
+        x = rnd(B, 1, 512).to(bf)
+
+        def states(shape_heads, dk, dvv):
+            """(what the step is given, the same values settled long ago)"""
+            C, n, m = rnd(B, shape_heads, dk, dvv), rnd(B, shape_heads, dk), rnd(B, shape_heads)
+            src = n if part == "n" else m
+            if form == "bf16":
+                src.copy_(src.to(bf))
+            plain = (C, n.clone(), m.clone())
+            if form == "bf16":
+                given = src.to(bf)
+            elif form == "strided":
+                given = torch.stack([src, src], -1)[..., 0]
+            else:
+                given = torch.full_like(src, 7.0)
+            torch.cuda.synchronize()
+
+            def write():
+                if form == "written":
+                    given.copy_(src)
+            return ((C, given, m) if part == "n" else (C, n, given)), plain, write
+
+        for _ in range(10):
+            st, plain, write = states(NH, dqk, dv)
+            ref = ops.mlstm_step(q, k, v, i, f, plain)
+            write()
+            got = ops.mlstm_step(q, k, v, i, f, st, state_settled=True)
+            for a, b in zip((got[0], *got[1]), (ref[0], *ref[1])):
+                assert torch.equal(a, b)
+            st, plain, write = states(NH, dqk, dv)
+            ref = ops.mlstm_step_gated(q, k, v, i, f, og, w, plain)
+            write()
+            got = ops.mlstm_step_gated(q, k, v, i, f, og, w, st, state_settled=True)
+            for a, b in zip((got[0], *got[1]), (ref[0], *ref[1])):
+                assert torch.equal(a, b)
+            st, plain, write = states(bh, bk, bv)
+            ref = blk(x, plain)
+            write()
+            got = blk(x, st)
+            for a, b in zip((got[0], *got[1]), (ref[0], *ref[1])):
+                assert torch.equal(a, b)
+
+
 # ---- error behaviour of the C ABI --------------------------------------------------
 def test_errors_are_statuses_not_crashes(ops):
     from xlstm_cuda import _lib

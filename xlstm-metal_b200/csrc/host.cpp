@@ -47,7 +47,9 @@ OptTensor cast_contiguous(const OptTensor &t, at::ScalarType dt) {
 
 struct State {
     OptTensor C, n, m;
-    bool converted;   // C is a copy made here, by the launch right before the step's: not settled, whatever the caller says
+    // C, which a step of a settled state reads early, is a copy made here, by the launch right before the step's: not settled,
+    // whatever the caller says
+    bool converted;
     State(const OptTensor &c, const OptTensor &nn, const OptTensor &mm, int64_t B, int64_t NH, int64_t dqk, int64_t dv)
         : C(cast_contiguous(c, at::kFloat)), n(cast_contiguous(nn, at::kFloat)), m(cast_contiguous(mm, at::kFloat)) {
         need(C.has_value() == n.has_value() && C.has_value() == m.has_value(), "a state is (C, n, m), all three or None");

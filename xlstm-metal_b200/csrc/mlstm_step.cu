@@ -73,19 +73,14 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     float *Cout = C1 + (size_t)bh * dqk * dv + col;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    // first batch of state rows, and what the prologue needs of n and m: in flight while the prologue below runs (and, for a
-    // settled state, while the preceding kernel drains)
+    // first batch of state rows: in flight while the prologue below runs (and, for a settled state, while the preceding kernel
+    // drains)
     float4 c[UNROLL];
-    float mold = 0.0f, nold = 0.0f;
     auto load_state = [&]() {
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
             const int j = rg + u * RG;
             c[u] = (active && has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
-        }
-        if (has_state) {
-            mold = m0[bh];
-            if (tid < dqk) nold = n0[(size_t)bh * dqk + tid];
         }
     };
     if (state_settled) load_state();
@@ -95,7 +90,9 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
 
     // stabilised gates (every thread: two exps and a log1p are cheaper than a broadcast)
     const float graw = Elem<T>::ld(ig + gate_at), fraw = Elem<T>::ld(fg + gate_at);
-    // everything else that is read: its latency runs beside the gates'
+    // everything else that is read: its latency runs beside the gates'.  n and m too: a settled state promises C alone, and the
+    // preceding kernel may have written them (a copy that converts their type, a reset)
+    const float mold = has_state ? m0[bh] : 0.f, nold = has_state && tid < dqk ? n0[(size_t)bh * dqk + tid] : 0.f;
     const T *qrow = q + (GATED ? seq * rows.q + (size_t)head * dqk : (size_t)bh * dqk);
     const T *krow = k + (GATED ? seq * rows.k + (size_t)head * dqk : (size_t)bh * dqk);
     const float q0 = tid < dqk ? Elem<T>::ld(qrow + tid) : 0.f, k0 = tid < dqk ? Elem<T>::ld(krow + tid) : 0.f;

@@ -64,9 +64,9 @@ def mlstm_step(q, k, v, i, f, state=None, eps: float = 1e-6, inplace: bool = Fal
     Returns ``h [B,NH,dv]`` and the new state.  ``inplace=True`` overwrites the
     caller's ``C`` (the 2 x dqk x dv x 4 byte stream then hits one buffer).
     ``gate_cap`` > 0: ``i`` and ``f`` are the raw gate projections and are soft-capped inside the kernel.
-    ``state_settled=True`` promises that ``state`` was not written by the kernel launched just before this call
-    (a layer stack: the launch before a layer's step is its projection); the kernel then starts streaming the
-    state while that kernel drains.
+    ``state_settled=True`` promises that ``C`` was not written by the kernel launched just before this call
+    (a layer stack: the launch before a layer's step is its projection); the kernel then starts streaming ``C``
+    while that kernel drains, and reads ``n`` and ``m`` once it is done.
     """
     rc, h, C, n, m = _lib.host().mlstm_step(q, k, v, i, f, *(_NO_STATE if state is None else state), eps, inplace, gate_cap or 0.0, state_settled)
     if rc:
