@@ -315,6 +315,34 @@ def test_norms_of_the_slstm_blocks_are_their_modules(ops, monkeypatch):
         assert relerr(host(torch.func.vmap(cell)(torch.stack([h, h]))[1]), host(plain)) <= 1e-5
 
 
+def test_ensembles_of_slstm_cells_go_through_the_modules(ops, monkeypatch):
+    """Stacked weights of an ensemble under vmap, an input that is shared: the weights have no memory of their own to hand to a
+    kernel, so the cells call their modules, as for a member at a time."""
+    from xlstm_cuda.blocks import slstm as blocks_slstm
+    monkeypatch.setattr(blocks_slstm, "NORM_MIN_NUMEL", 1)
+
+    class Gates(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.cell = blocks_slstm.sLSTMProjectionCell(64, 4, 16, gate_soft_cap=None)
+
+        def forward(self, x):
+            return torch.cat([t.flatten(2) for t in self.cell.gates_and_z(x)], -1)
+    torch.manual_seed(3)
+    with torch.no_grad():
+        for make, x, part in ((lambda: blocks_slstm.sLSTMOutputCell(64, 4, 16), torch.randn(2, 9, 4, 16, device="cuda"), "group_norm"),
+                              (Gates, torch.randn(2, 9, 64, device="cuda"), "gate_proj")):
+            cells = [make().cuda().bfloat16() for _ in range(3)]
+            x = x.bfloat16()
+            base = dict(cells[0].named_parameters())
+            members = [{k: (torch.randn_like(v) if part in k else v) for k, v in base.items()} for _ in cells]
+            stacked = {k: torch.stack([m[k] for m in members]) for k in base if part in k}
+            call = lambda p: torch.func.functional_call(cells[0], {**base, **p}, (x,))
+            y = torch.func.vmap(call)(stacked)
+            for n, m in enumerate(members):
+                assert relerr(host(y[n]), host(call(m))) <= BF16_TOL
+
+
 @pytest.mark.parametrize("B,S,C,NH", [(1, 1, 32, 4), (2, 3, 64, 1), (1, 16, 1024, 4), (3, 17, 416, 2), (1, 77, 4096, 4),
                                       (4, 1801, 128, 3), (2, 3555, 64, 4)])
 @pytest.mark.parametrize("cap,bias", [(15.0, True), (None, False)])

@@ -5,7 +5,7 @@ difference: no gradient is recorded, and each of those modules is the class the 
 """
 from __future__ import annotations
 
-from typing import Tuple
+from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
@@ -13,11 +13,13 @@ from torch.autograd import forward_ad as _forward_ad
 from torch.nn.modules import module as _module
 
 
-def plain_tensor(x: torch.Tensor) -> bool:
-    """Whether ``x`` is an ordinary tensor whose memory a kernel may be handed: not a subclass, not wrapped by a function
-    transform (vmap, grad, jvp) or a forward-mode level, not being traced or compiled, and not under autocast (which would
-    pick another type for the module)."""
+def plain_tensor(x: torch.Tensor, *weights: Optional[torch.Tensor]) -> bool:
+    """Whether ``x`` and the weights are ordinary tensors whose memory a kernel may be handed: not subclasses, not wrapped by a
+    function transform (vmap, grad, jvp; an ensemble's stacked weights are wrapped where ``x`` is not) or a forward-mode level,
+    not being traced or compiled, and not under autocast (which would pick another type for the module)."""
     return (type(x) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(x) and
+            all(w is None or (type(w) in (nn.Parameter, torch.Tensor) and not torch._C._functorch.is_functorch_wrapped_tensor(w))
+                for w in weights) and
             _forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and
             not torch.is_autocast_enabled(x.device.type))
 

@@ -35,7 +35,7 @@ NORM_MIN_NUMEL = 1 << 20
 
 def _norm(owner: nn.Module, norm: nn.Module, kind: type, x: torch.Tensor, groups: int = 1) -> torch.Tensor:
     """``norm(x)`` on the last dimension: as one launch where nothing tells it from the module, else the module itself."""
-    if (x.numel() >= NORM_MIN_NUMEL and may_fuse(owner, x, (norm, kind)) and plain_tensor(x) and
+    if (x.numel() >= NORM_MIN_NUMEL and may_fuse(owner, x, (norm, kind)) and plain_tensor(x, norm.weight, norm.bias) and
             ops.layer_norm_takes(x, norm.weight, norm.bias, groups)):
         return ops.layer_norm(x, norm.weight, norm.bias, norm.eps, groups)
     return norm(x)
@@ -110,12 +110,11 @@ class sLSTMProjectionCell(nn.Module):
         B, S, _ = x.shape
         conv, lins = self.conv1d, (self.igate_proj, self.fgate_proj, self.ogate_proj)
         if (x.dtype == torch.bfloat16 and type(conv) is CausalConv1d and type(conv.conv) is nn.Conv1d and conv.depthwise and
-                may_fuse(self, x, (self, sLSTMProjectionCell), (conv, CausalConv1d), *((lin, nn.Linear) for lin in lins)) and
-                plain_tensor(x) and
-                ops.slstm_gates_takes(x, conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins], [lin.bias for lin in lins])):
-            i, f, o = ops.slstm_gates(x, conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins],
-                                      [lin.bias for lin in lins], self.gate_soft_cap)
-            return self.z_proj(x).view(B, S, self.num_heads, self.head_dim), i, f, o
+                may_fuse(self, x, (self, sLSTMProjectionCell), (conv, CausalConv1d), *((lin, nn.Linear) for lin in lins))):
+            cw, cb, w, b = conv.conv.weight, conv.conv.bias, [lin.weight for lin in lins], [lin.bias for lin in lins]
+            if plain_tensor(x, cw, cb, *w, *b) and ops.slstm_gates_takes(x, cw, cb, w, b):
+                i, f, o = ops.slstm_gates(x, cw, cb, w, b, self.gate_soft_cap)
+                return self.z_proj(x).view(B, S, self.num_heads, self.head_dim), i, f, o
         return self(x)[:4]
 
     def forward(self, x: torch.Tensor):
