@@ -1009,6 +1009,30 @@ def test_chunkwise_short_bf16(ops, T, dqk, dv, state, f_mean):
                 assert relerr(host(got), host(want)) < 1e-5
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 8, 16, 17, 33, 64, 65, 127])
+@pytest.mark.parametrize("dqk,dv,f_mean", [(256, 512, -2.0), (256, 512, 3.0), (128, 256, -2.0)])
+def test_chunkwise_short_bf16_state_is_no_further_off_than_fp32(ops, T, dqk, dv, f_mean):
+    """The state after up to 127 bf16 tokens against float64, beside the same values through the fp32 multiply-adds (2-norms over
+    2 dqk dv elements, so equal errors agree to a few percent: 1.1), from a carried state; gates that forget within a few tokens
+    leave single roundings to see (3e-8), where the tensor cores' cut-off sums were 6e-8 off."""
+    g = torch.Generator(device="cuda").manual_seed(T * 3 + dqk)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k, v = rnd(1, 2, T, dqk).to(BF), rnd(1, 2, T, dqk).to(BF), rnd(1, 2, T, dv).to(BF)
+    i, f = rnd(1, 2, T).to(BF), (rnd(1, 2, T) + f_mean).to(BF)
+    st = (rnd(1, 2, dqk, dv), rnd(1, 2, dqk), rnd(1, 2))
+    C, n, m = (s.double() for s in st)
+    for t in range(T):
+        fl, it = torch.nn.functional.logsigmoid(f[:, :, t].double()), i[:, :, t].double()
+        mn = torch.maximum(fl + m, it)
+        fg, ig = torch.exp(fl + m - mn), torch.exp(it - mn)
+        C = fg[..., None, None] * C + ig[..., None, None] * k[:, :, t, :, None].double() * v[:, :, t, None, :].double()
+        m = mn
+    _, (Cb, _, _) = ops.mlstm_chunkwise(q, k, v, i, f, st)
+    _, (Cf, _, _) = ops.mlstm_chunkwise(*(a.float() for a in (q, k, v, i, f)), st)
+    eb, ef = (float((a.double() - C).norm() / C.norm()) for a in (Cb, Cf))
+    assert eb <= 1.1 * ef, (eb, ef)
+
+
 @pytest.mark.parametrize("shape,f_mean", [((2, 8, 3968, 256, 512), -2.0), ((2, 8, 3968, 256, 512), 3.0), ((1, 4, 2048, 128, 256), -2.0)])
 def test_chunkwise_is_deterministic(ops, shape, f_mean):
     """The same call gives the same bits, in the general path (gates that forget within a few tokens) and the bounded one, call

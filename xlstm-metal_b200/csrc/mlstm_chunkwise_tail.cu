@@ -5,7 +5,7 @@
 // bf16 parts whose sum is the float, so mma.sync forms exact products and adds them in fp32:
 //   S = Q K^T                                         1 product
 //   H^T = (C^T Q^T) diag(w_in) + V^T P^T              3 products each (parts of C, of P)
-//   C^T = decay C^T + (w V)^T K                       3 products (parts of w V)
+//   C^T = decay C^T + (w V)^T K                       4 products (parts of w V; K in two for the leading one, see below)
 // One CTA per (head, 32 columns of dv).  Its 8 warps share the dqk dimension: a warp keeps its rows of C in registers, as
 // accumulators of the update and, in the same places, as A fragments of the read-out; it takes its share of the keys s for
 // S, P and P V.  The read-outs of the 8 warps meet in shared memory, 32 tokens at a time.  Everything that does not need the
@@ -13,10 +13,17 @@
 //
 // Latency-bound: a few microseconds of products behind a chain of loads, two barriers a 32 tokens and the state's way through
 // registers.  As fp32 multiply-adds on CUDA cores a tail of 64 tokens took 52 us (8 heads of 256/512) in one launch, of 127
-// tokens 66 us in two; here 14 us behind the last tile (16 heads: 19).  Relative error of C against float64 6.9e-8 to 8.0e-8, as
-// fp32 multiply-adds 8.1e-8 to 1.0e-7; 5.6e-8 against 4.1e-8 where one token makes the state.
+// tokens 66 us in two; here 14 us behind the last tile (16 heads: 19).
+//
+// The tensor cores cut off what does not fit 24 bits of a sum, they do not round: with plain parts C was 5.5e-8 from float64 where
+// gates forget within a few tokens (fp32 multiply-adds 3.0e-8).  So the leading parts of w V and of K are multiples of one power of
+// two each, for the whole sum: their products and all partial sums of up to 128 of them fit 22 bits, nothing is cut off, and the
+// other three products are 2^-6 of it.  The two sums and the state meet with one rounding.  C of 1 to 127 tokens is 1.5e-8 to 5.7e-8
+// from float64 where fp32 multiply-adds are 1.6e-8 to 9.4e-8 (2-norms; never more than 2 % further, which is the spread of the
+// samples).  It costs 1 us of 7 to 25; multiply-adds on the CUDA cores, as exact, cost nothing for one token and 5 us for 127.
 #include "cp_async.cuh"
 #include "mlstm_gate_tile.cuh"
+#include "packed_f32.cuh"
 
 namespace xl {
 namespace {
@@ -55,6 +62,42 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
     }
 }
 
+// The same with the leading part on a grid, the multiples of 2^-7 of the power of two of `largest`, the largest magnitude there
+// is: adding and subtracting 1.5 * 2^23 of that rounds to it.  No grid near the end of the range, or beside an infinity.
+__device__ __forceinline__ float grid_of(uint32_t largest) {
+    const uint32_t e = largest >> 23;
+    return e < 235u ? __uint_as_float(((e + 16u) << 23) | 0x400000u) : 0.f;
+}
+__device__ __forceinline__ void split3_on_grid(float x, float y, float gx, float gy, uint32_t (&p)[3]) {
+    const uint32_t hx = __float_as_uint(__fsub_rn(__fadd_rn(x, gx), gx)) & 0xffff0000u;
+    const uint32_t hy = __float_as_uint(__fsub_rn(__fadd_rn(y, gy), gy)) & 0xffff0000u;
+    p[0] = __byte_perm(hx, hy, 0x7632);
+    x = fabsf(x) < INFINITY ? x - __uint_as_float(hx) : 0.f;
+    y = fabsf(y) < INFINITY ? y - __uint_as_float(hy) : 0.f;
+#pragma unroll
+    for (int i = 1; i < 3; ++i) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        p[i] = *reinterpret_cast<const uint32_t *>(&v);
+        x -= __uint_as_float(p[i] << 16);
+        y -= __uint_as_float(p[i] & 0xffff0000u);
+    }
+}
+// K on the multiples of 2^-5 of its largest magnitude's power of two, and the rest: in bf16 itself, 1.5 * 2^7 of that added and
+// subtracted (g: bf16 bits, 0: no grid).
+__device__ __forceinline__ uint32_t k_grid_of(uint32_t largest) { return largest < (250u << 7) ? ((largest >> 7) + 2u) << 7 | 0x40u : 0u; }
+__device__ __forceinline__ void k_on_grid(uint32_t k, __nv_bfloat162 g, uint32_t &lead, uint32_t &rest) {
+    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(&k), h = __hsub2(__hadd2(v, g), g), r = __hsub2(v, h);
+    lead = *reinterpret_cast<const uint32_t *>(&h);
+    rest = *reinterpret_cast<const uint32_t *>(&r);
+}
+// c d + a + b for |b| far below |a|, with one rounding that counts: the sum of c d and a with what its rounding leaves.  nd: -d
+__device__ __forceinline__ float2 scaled_sum(u64 c, u64 d, u64 nd, u64 a, u64 b) {
+    const u64 np = fmul2(c, nd), ep = ffma2(c, d, np);
+    const u64 s = fsub2(a, np), t = fsub2(s, a), left = fsub2(fsub2(a, fsub2(s, t)), fadd2(np, t));
+    const float2 r = unpack2(fadd2(s, fadd2(left, fadd2(ep, b)))), plain = unpack2(s);
+    return make_float2(fabsf(plain.x) < INFINITY ? r.x : plain.x, fabsf(plain.y) < INFINITY ? r.y : plain.y);
+}
+
 template <int DQK, int TMAX> struct TailSmem {
     static constexpr uint32_t QK_LD = DQK + 8;                                // elements between rows of Q and K
     static constexpr uint32_t Q = 0;
@@ -67,7 +110,8 @@ template <int DQK, int TMAX> struct TailSmem {
     static constexpr uint32_t F = U + 3 * TMAX * 8;                           // float [4][TMAX]: w_in, e^{-m_t}, w, q.n
     static constexpr uint32_t RS = F + 4 * TMAX * 4;                          // float [TW][TMAX] row sums of P
     static constexpr uint32_t N = RS + TW * TMAX * 4;                         // float [DQK]
-    static constexpr uint32_t TOTAL = N + DQK * 4;
+    static constexpr uint32_t KMAX = N + DQK * 4;                             // uint32 [TW]: largest |K|, bf16 bits, by warps
+    static constexpr uint32_t TOTAL = KMAX + TW * 4;
     static_assert(3 * TMAX * V_LD * 2 <= PART_BYTES, "weighted V fits the buffer it replaces");
 };
 
@@ -121,6 +165,18 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
     }
     cp_async_wait_all();
     __syncthreads();
+    {
+        uint32_t k2 = 0u;
+#pragma unroll 2
+        for (int e = tid; e < nb * 16 * (DQK / 8); e += TW * 32) {
+            const uint4 k = *reinterpret_cast<const uint4 *>(smem + SM::K + ((e / (DQK / 8)) * SM::QK_LD + (e % (DQK / 8)) * 8) * 2);
+            const uint32_t kk[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) k2 = __vmaxu2(k2, kk[x] & 0x7fff7fffu);
+        }
+        k2 = __reduce_max_sync(0xffffffffu, max(k2 & 0xffffu, k2 >> 16));
+        if (lane == 0) *reinterpret_cast<uint32_t *>(smem + SM::KMAX + warp * 4) = k2;   // read after the barriers below
+    }
 
     // ---- S = Q K^T: rows t of block tb (16), this warp's keys
     float P[TB][NS][4];
@@ -326,18 +382,48 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
 
     // ---- C^T = decay C^T + (w V)^T K
     bf16 *sWV = reinterpret_cast<bf16 *>(smem + SM::WV);
-    for (int e = tid; e < nb * 16 * (TC_COLS / 2); e += TW * 32) {
-        const int t = e / (TC_COLS / 2), x = (e % (TC_COLS / 2)) * 2;
-        const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + SM::V + (t * V_LD + x) * 2);
+    static_assert(TW * 32 == 16 * (TC_COLS / 2), "a thread has two columns, of the tokens tid / 16 + 16 i");
+    const int vx = (tid % (TC_COLS / 2)) * 2, vt = tid / (TC_COLS / 2);
+    auto weighted = [&](int t) {
+        const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + SM::V + (t * V_LD + vx) * 2);
         const float w = sW[t];
-        uint32_t pr[3];
-        split3(w * __uint_as_float(v << 16), w * __uint_as_float(v & 0xffff0000u), pr);
+        return make_float2(w * __uint_as_float(v << 16), w * __uint_as_float(v & 0xffff0000u));
+    };
+    uint32_t ex = 0u, ey = 0u, kmax = 0u;
+#pragma unroll 2
+    for (int i = 0; i < nb; ++i) {
+        const float2 wv = weighted(vt + 16 * i);
+        ex = max(ex, __float_as_uint(fabsf(wv.x)));
+        ey = max(ey, __float_as_uint(fabsf(wv.y)));
+    }
+    ex = max(ex, __shfl_xor_sync(0xffffffffu, ex, 16));
+    ey = max(ey, __shfl_xor_sync(0xffffffffu, ey, 16));
+    uint2 *sMax = reinterpret_cast<uint2 *>(sRs);                             // [TW][TC_COLS / 2], after the last row sums
+    if (lane < 16) sMax[warp * (TC_COLS / 2) + lane] = make_uint2(ex, ey);
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(sWV + (k * TMAX + t) * V_LD + x) = pr[k];
+    for (int w = 0; w < TW; ++w) {
+        const uint2 o = sMax[w * (TC_COLS / 2) + (lane & 15)];
+        ex = max(ex, o.x);
+        ey = max(ey, o.y);
+        kmax = max(kmax, *reinterpret_cast<const uint32_t *>(smem + SM::KMAX + w * 4));
+    }
+    // an infinity keeps its products with all of the other factor: no grids then
+    const bool finite = __all_sync(0xffffffffu, max(ex, ey) < 0x7f800000u) && kmax < 0x7f80u;
+    const float gx = finite ? grid_of(ex) : 0.f, gy = finite ? grid_of(ey) : 0.f;
+    const uint32_t kg = finite ? k_grid_of(kmax) * 0x10001u : 0u;
+    const __nv_bfloat162 kgrid = *reinterpret_cast<const __nv_bfloat162 *>(&kg);
+#pragma unroll 2
+    for (int i = 0; i < nb; ++i) {
+        const float2 wv = weighted(vt + 16 * i);
+        uint32_t pr[3];
+        split3_on_grid(wv.x, wv.y, gx, gy, pr);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(sWV + (k * TMAX + vt + 16 * i) * V_LD + vx) = pr[k];
     }
     __syncthreads();
-    // The sum over the tokens has accumulators of its own, the leading parts and the remainders apart, and meets the state in
-    // one fp32 multiply-add: the tensor cores cut off below the last bit of a sum, so its terms should not be small beside it.
+    const u64 decay2 = pack2(decay, decay), minus_decay2 = pack2(-decay, -decay);
+    // The sum over the tokens has accumulators of its own, that of the leading parts (exact) and that of the rest
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
         float sum[2][NTJ][4];
@@ -349,28 +435,39 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                 for (int e = 0; e < 4; ++e) sum[h][nj][e] = 0.f;
 #pragma unroll 1
         for (int ks = 0; ks < nb; ++ks) {
-            uint32_t wv[3][4], kf[NTJ / 2][4];
+            uint32_t wp[3][4], kf[NTJ / 2][4];
             const int trow = ks * 16 + (lane & 7);
 #pragma unroll
             for (int x = 0; x < 3; ++x)
-                ldsm4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wv[x]);
+                ldsm4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wp[x]);
 #pragma unroll
             for (int np = 0; np < NTJ / 2; ++np)
                 ldsm4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
 #pragma unroll
-            for (int x = 2; x >= 0; --x)
+            for (int np = 0; np < NTJ / 2; ++np)
 #pragma unroll
-                for (int np = 0; np < NTJ / 2; ++np) {
-                    mma_k16(sum[x > 0][2 * np], wv[x], kf[np][0], kf[np][1]);
-                    mma_k16(sum[x > 0][2 * np + 1], wv[x], kf[np][2], kf[np][3]);
+                for (int half = 0; half < 2; ++half) {
+                    const int nj = 2 * np + half;
+                    const uint32_t k0 = kf[np][2 * half], k1 = kf[np][2 * half + 1];
+                    uint32_t l0, l1, r0, r1;
+                    k_on_grid(k0, kgrid, l0, r0);
+                    k_on_grid(k1, kgrid, l1, r1);
+                    mma_k16(sum[1][nj], wp[2], k0, k1);
+                    mma_k16(sum[0][nj], wp[0], l0, l1);
+                    mma_k16(sum[1][nj], wp[1], k0, k1);
+                    mma_k16(sum[1][nj], wp[0], r0, r1);
                 }
         }
 #pragma unroll
         for (int nj = 0; nj < NTJ; ++nj)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                p.C1[c_off + (size_t)(nj * 8 + (e & 1)) * p.dv + mt * 16 + (e >> 1) * 8] =
-                    fmaf(Ct[mt][nj][e], decay, sum[0][nj][e] + sum[1][nj][e]);
+            for (int h = 0; h < 2; ++h) {
+                const float *C = Ct[mt][nj] + 2 * h, *s0 = sum[0][nj] + 2 * h, *s1 = sum[1][nj] + 2 * h;
+                const float2 v = scaled_sum(pack2(C[0], C[1]), decay2, minus_decay2, pack2(s0[0], s0[1]), pack2(s1[0], s1[1]));
+                float *dst = p.C1 + c_off + (size_t)(nj * 8) * p.dv + mt * 16 + h * 8;
+                dst[0] = v.x;
+                dst[p.dv] = v.y;
+            }
     }
     if (blockIdx.x == 0) {
         const bf16 *sK = reinterpret_cast<const bf16 *>(smem + SM::K);
