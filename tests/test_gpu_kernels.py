@@ -1009,6 +1009,28 @@ def test_chunkwise_short_bf16(ops, T, dqk, dv, state, f_mean):
                 assert relerr(host(got), host(want)) < 1e-5
 
 
+@pytest.mark.parametrize("T", [30, 60, 100, 127])
+@pytest.mark.parametrize("dqk,dv", [(256, 512), (128, 96)])
+def test_chunkwise_short_bf16_keeps_an_infinity_to_later_tokens(ops, T, dqk, dv):
+    """An infinite v reaches its own column of its block of 16 tokens and of those after it, as in the fp32 kernels: the blocks
+    before it and the other columns of h are bit for bit what they are without it, those of C to fp32 rounding (their sums go
+    without the grids then)."""
+    torch.manual_seed(T + dqk)
+    q, k, v = (torch.randn(1, 2, T, d, device="cuda").to(BF) for d in (dqk, dqk, dv))
+    i, f = torch.randn(1, 2, T, device="cuda").to(BF), (torch.randn(1, 2, T, device="cuda") + 3).to(BF)
+    st = (torch.randn(1, 2, dqk, dv, device="cuda"), torch.randn(1, 2, dqk, device="cuda"), torch.zeros(1, 2, device="cuda"))
+    h, (C, n, m) = ops.mlstm_chunkwise(q, k, v, i, f, st)
+    for at in (17, T - 1):
+        vi = v.clone()
+        vi[:, :, at, 5] = float("inf")
+        hi, (Ci, ni, mi) = ops.mlstm_chunkwise(q, k, vi, i, f, st)
+        assert torch.equal(hi[:, :, :at // 16 * 16], h[:, :, :at // 16 * 16])
+        others = torch.arange(dv, device="cuda") != 5
+        assert torch.equal(hi[..., others], h[..., others]) and torch.equal(ni, n) and torch.equal(mi, m)
+        assert not torch.isfinite(hi[:, :, at:, 5].float()).any()
+        assert (Ci[..., 5][k[:, :, at] != 0].isinf()).all() and relerr(host(Ci[..., others]), host(C[..., others])) < 1e-6
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 8, 16, 17, 33, 64, 65, 127])
 @pytest.mark.parametrize("dqk,dv,f_mean", [(256, 512, -2.0), (256, 512, 3.0), (128, 256, -2.0)])
 def test_chunkwise_short_bf16_state_is_no_further_off_than_fp32(ops, T, dqk, dv, f_mean):

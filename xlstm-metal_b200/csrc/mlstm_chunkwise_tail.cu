@@ -342,6 +342,7 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
 #pragma unroll
             for (int nt = 0; nt < TG / 8; ++nt) {
                 const int tb = th * 2 + (nt >> 1), r = nt & 1;
+                if (th * TG + nt * 8 + 8 <= s0) continue;                     // all earlier than the keys: P is 0, V may be infinite
                 uint32_t w[NS][3];
 #pragma unroll
                 for (int n = 0; n < NS; ++n) split3(P[tb][n][2 * r], P[tb][n][2 * r + 1], w[n]);
