@@ -492,6 +492,26 @@ def test_block_token_step_with_weights_at_odd_offsets(ops, B):
         assert relerr(host(m(x)[0]), host(y)) <= BF16_TOL
 
 
+@pytest.mark.parametrize("B", [3, 16])
+@pytest.mark.parametrize("what", ["input", "norm_mlstm", "norm_ffn"])
+def test_block_token_step_with_inputs_or_norms_at_odd_offsets(ops, B, what):
+    """An input or a norm weight off a 16-byte boundary: the norm is a launch of its own, with the same bits."""
+    m, _, _ = _blocks()
+    x = torch.randn(B, 1, 512, device="cuda", dtype=torch.bfloat16)
+    with torch.inference_mode():
+        for mod in (m.norm_mlstm, m.norm_ffn):
+            mod.weight.uniform_(0.5, 1.5)
+        y, st = m(x)
+        off = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+        if what == "input":
+            x = off(x)
+        else:
+            mod = getattr(m, what)
+            mod.weight.data = off(mod.weight.data)
+        y2, st2 = m(x)
+        assert torch.equal(y, y2) and all(torch.equal(a, b) for a, b in zip(st, st2))
+
+
 def _blocks():
     from xlstm_cuda.blocks import mLSTMBlock, sLSTMBlock, sLSTMBlockDiag
     t = torch.bfloat16

@@ -85,6 +85,8 @@ Tensor aligned4(const Tensor &t) {
     return reinterpret_cast<uintptr_t>(t.data_ptr()) % (4 * t.element_size()) ? t.clone() : t;
 }
 
+bool aligned16(const Tensor &t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
 // q, k: [B, NH, dqk], v: [B, NH, dv], i, f: [B, NH], or the same with a token dimension of one ([B, NH, 1, d], [B, NH, 1])
 py::tuple mlstm_step(Tensor q, Tensor k, Tensor v, Tensor i, Tensor f, const OptTensor &C0, const OptTensor &n0,
                      const OptTensor &m0, double eps, bool inplace, double gate_cap, bool state_settled) {
@@ -284,7 +286,7 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
 
 // One token of B sequences through an mLSTM block, launch after launch as mLSTMBlock._token_step describes them: W, b are the
 // merged input projections, ffn the gate and up projections.  rows: the Linears for up to 16 rows, else those for up to 4; the
-// norms are in them (more than 48 KB of rows: launches of their own).  Through Python the seven launches of a block took 140 us of host
+// norms are in them (more than 48 KB of rows, or rows or a norm weight off 16 bytes: launches of their own, which take both).  Through Python the seven launches of a block took 140 us of host
 // time, as much as the GPU has work for 16 sequences of 4096.
 py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, const OptTensor &norm_w, double norm_eps, int64_t NH,
                       int64_t dqk, int64_t dv, const OptTensor &C0, const OptTensor &n0, const OptTensor &m0,
@@ -300,7 +302,8 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
     auto project = [&](const Tensor &w, const Tensor &in, const OptTensor &bias, const OptTensor &nw, double ne, const OptTensor &res,
                        bool pair, bool settled) -> Result {
         if (!rows) return linear(w, in, bias, nw, ne, res, pair, 4, false);
-        if (!nw || in.size(0) * (2 * in.size(1) + 64) + 2 * in.size(1) <= XLSTM_LINEAR_NORM_BYTES) return linear(w, in, bias, nw, ne, res, pair, 16, settled);
+        const bool fits = in.size(0) * (2 * in.size(1) + 64) + 2 * in.size(1) <= XLSTM_LINEAR_NORM_BYTES;
+        if (!nw || (fits && aligned16(in) && aligned16(*nw))) return linear(w, in, bias, nw, ne, res, pair, 16, settled);
         const Result n = norm(in, nw, ne);
         if (n.rc) return n;
         return linear(w, n.y, bias, none, 0.0, res, pair, 16, true);
