@@ -315,6 +315,35 @@ def test_norms_of_the_slstm_blocks_are_their_modules(ops, monkeypatch):
         assert relerr(host(torch.func.vmap(cell)(torch.stack([h, h]))[1]), host(plain)) <= 1e-5
 
 
+def test_slstm_cells_under_modes_go_through_the_modules(ops, monkeypatch):
+    """A graph of the output cell made by make_fx computes with its own input, and a mode that listens sees the norm and the gate
+    projections; a default device is no such mode."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from xlstm_cuda.blocks import slstm as blocks_slstm
+    monkeypatch.setattr(blocks_slstm, "NORM_MIN_NUMEL", 1)
+    torch.manual_seed(4)
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func._opname)
+            return func(*args, **(kwargs or {}))
+    seen = []
+    cell, pc = blocks_slstm.sLSTMOutputCell(64, 4, 16).cuda(), blocks_slstm.sLSTMProjectionCell(64, 4, 16).cuda().bfloat16()
+    h, h2 = torch.randn(2, 9, 4, 16, device="cuda"), torch.randn(2, 9, 4, 16, device="cuda")
+    with torch.no_grad():
+        assert relerr(host(make_fx(cell)(h)(h2)), host(cell(h2))) <= 1e-5
+        with Log():
+            cell(h)
+            pc.gates_and_z(h.flatten(2).bfloat16())
+        assert "native_group_norm" in seen and sum(name in ("mm", "addmm") for name in seen) == 1 + 4
+        seen.clear()
+        with torch.device("cuda"):
+            monkeypatch.setattr(torch.nn.GroupNorm, "forward", None)     # not called: the fused launch is taken
+            cell(h)
+
+
 def test_ensembles_of_slstm_cells_go_through_the_modules(ops, monkeypatch):
     """Stacked weights of an ensemble under vmap, an input that is shared: the weights have no memory of their own to hand to a
     kernel, so the cells call their modules, as for a member at a time."""

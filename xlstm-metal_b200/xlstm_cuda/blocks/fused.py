@@ -9,15 +9,25 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
+from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
 from torch.autograd import forward_ad as _forward_ad
 from torch.nn.modules import module as _module
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
+
+
+def _no_mode() -> bool:
+    """No dispatch mode, and no function mode but the default device's."""
+    return (_len_torch_dispatch_stack() == 0 and
+            (_len_torch_function_stack() == 0 or all(type(m) is DeviceContext for m in _get_current_function_mode_stack())))
 
 
 def plain_tensor(x: torch.Tensor, *weights: Optional[torch.Tensor]) -> bool:
     """Whether ``x`` and the weights are ordinary tensors whose memory a kernel may be handed: not subclasses, not wrapped by a
     function transform (vmap, grad, jvp; an ensemble's stacked weights are wrapped where ``x`` is not) or a forward-mode level,
-    not being traced or compiled, and not under autocast (which would pick another type for the module)."""
-    return (type(x) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(x) and
+    not being traced or compiled, no mode listens to the operators (make_fx, a counter), and not under autocast (which would pick
+    another type for the module)."""
+    return (_no_mode() and type(x) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(x) and
             all(w is None or (type(w) in (nn.Parameter, torch.Tensor) and not torch._C._functorch.is_functorch_wrapped_tensor(w))
                 for w in weights) and
             _forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and
