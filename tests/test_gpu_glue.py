@@ -451,6 +451,27 @@ def test_linear_rows_with_norm(ops, M, N, K):
         ops.linear_rows(W, x, residual=torch.zeros(M, N, device="cuda", dtype=t), norm_weight=nw)
 
 
+def test_linear_rows_with_norm_from_several_threads(ops):
+    """Calls that need different amounts of shared memory, from threads that run beside one another: none is refused."""
+    import threading
+    from xlstm_cuda import _lib
+    lib, t, failed = _lib.load(), torch.bfloat16, []
+
+    def calls(M, K, N=16):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            W, x, nw, y = (torch.randn(s, device="cuda").to(t) for s in ((N, K), (M, K), (K,), (M, N)))
+        args = (W.data_ptr(), x.data_ptr(), None, nw.data_ptr(), 1e-6, None, y.data_ptr(), M, N, K, 0, 0, _lib.BF16, stream.cuda_stream)
+        failed.extend(rc for rc in (lib.xlstm_linear_rows_norm(*args) for _ in range(20000)) if rc)
+        stream.synchronize()
+    threads = [threading.Thread(target=calls, args=a) for a in ((1, 32), (16, 1408), (2, 32), (15, 1408))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not failed, (len(failed), failed[:3])
+
+
 @pytest.mark.parametrize("K", [32, 64, 288, 1024])
 def test_linear_rows_keeps_infinities(ops, K):
     """An infinite weight gives an infinite result in its row and none elsewhere, also in the last block of k."""

@@ -79,6 +79,12 @@ __device__ __forceinline__ void stg_stream(float *p, float4 v) {
                  :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
+// The most dynamic shared memory that any launch of a kernel asks for.  The limit is the function's, not the launch's: set to what
+// one launch needs, it could be lowered by another thread between the setting and the launch, which is then refused.
+template <typename Kernel> inline bool allow_smem(Kernel kern, size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
+}
+
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? XLSTM_OK : XLSTM_ERR_CUDA; }
 
 // ---- programmatic dependent launch ---------------------------------------------------

@@ -193,10 +193,9 @@ int gemv_launch(const void *W, const void *x, const void *bias, const void *norm
                 int N, int K, cudaStream_t st) {
     auto kern = gemv_kernel<M, EPI>;
     const size_t smem = (size_t)M * K * sizeof(__nv_bfloat16);
-    if (smem > 200 * 1024) return XLSTM_ERR_UNSUPPORTED;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return XLSTM_ERR_CUDA;
+    constexpr size_t most = 200 * 1024;
+    if (smem > most) return XLSTM_ERR_UNSUPPORTED;
+    if (smem > 48 * 1024 && !allow_smem(kern, most)) return XLSTM_ERR_CUDA;
     // rows are spread over all SMs: enough CTAs of 8 warps for one row per warp, at most 8 CTAs per SM
     const int want = (N + GV_THREADS / 32 - 1) / (GV_THREADS / 32);
     const int grid = want < 148 * 8 ? want : 148 * 8;

@@ -224,7 +224,7 @@ int linear_rows_launch(const void *W, const void *x, const void *bias, const voi
     const int64_t smem = (int64_t)LR_SMEM + (NORM ? (int64_t)M * norm_ld(K) + 2 * K : 0);   // rows of x, norm weight
     if (smem > (int64_t)LR_SMEM + XLSTM_LINEAR_NORM_BYTES) return XLSTM_ERR_UNSUPPORTED;
     auto kern = linear_rows_kernel<EPI, NORM>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return XLSTM_ERR_CUDA;
+    if (!allow_smem(kern, LR_SMEM + (NORM ? XLSTM_LINEAR_NORM_BYTES : 0))) return XLSTM_ERR_CUDA;
     return launch_overlapped(kern, dim3(tiles < 148 ? tiles : 148), dim3(LR_THREADS), (size_t)smem, st,
                              static_cast<const __nv_bfloat16 *>(W), static_cast<const __nv_bfloat16 *>(x),
                              static_cast<const __nv_bfloat16 *>(bias), static_cast<const __nv_bfloat16 *>(residual),

@@ -313,18 +313,17 @@ int mlstm_chunkwise_simt(const ChunkwiseParams &p_in, int dtype, cudaStream_t st
          reinterpret_cast<uintptr_t>(p.h)) & mask)
         return XLSTM_ERR_UNSUPPORTED;
     const int dqkp = (p.dqk + KP - 1) / KP * KP;
-    const size_t smem = sizeof(float) * ((size_t)dqkp * DVT + dqkp + 3 * LT * LDP + 2 * LT * DVT + 7 * LT);
-    if (smem > 227 * 1024) return XLSTM_ERR_UNSUPPORTED;
+    auto smem_of = [](int rows) { return sizeof(float) * ((size_t)rows * DVT + rows + 3 * LT * LDP + 2 * LT * DVT + 7 * LT); };
+    const size_t smem = smem_of(dqkp), most = smem_of(512);
+    if (smem > most) return XLSTM_ERR_UNSUPPORTED;
     dim3 grid(p.B * p.NH, (p.dv + DVT - 1) / DVT);
     if (dtype == XLSTM_F32) {
         auto kern = mlstm_chunkwise_simt_kernel<float>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
+        if (!allow_smem(kern, most)) return XLSTM_ERR_CUDA;
         kern<<<grid, THREADS, smem, st>>>(p, dqkp);
     } else {
         auto kern = mlstm_chunkwise_simt_kernel<__nv_bfloat16>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
+        if (!allow_smem(kern, most)) return XLSTM_ERR_CUDA;
         kern<<<grid, THREADS, smem, st>>>(p, dqkp);
     }
     return launch_status();

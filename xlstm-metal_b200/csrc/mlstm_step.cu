@@ -220,13 +220,12 @@ static int mlstm_step_launch(const void *q, const void *k, const void *v, const 
     constexpr int DVT = STEP_DVT, THREADS = STEP_THREADS;
     dim3 grid(BH, (dv + DVT - 1) / DVT);
     size_t smem = sizeof(float) * (2 * (size_t)dqk + (THREADS / (DVT / 4)) * DVT);
-    if (smem > 200 * 1024) return XLSTM_ERR_UNSUPPORTED;
+    constexpr size_t most = 200 * 1024;
+    if (smem > most) return XLSTM_ERR_UNSUPPORTED;
     const float qscale = 1.0f / sqrtf((float)dqk);
     if (!gate) {
         auto kern = mlstm_step_kernel<T, DVT, THREADS, UNROLL, false>;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return XLSTM_ERR_CUDA;
+        if (smem > 48 * 1024 && !allow_smem(kern, most)) return XLSTM_ERR_CUDA;
         return launch_overlapped(kern, grid, dim3(THREADS), smem, st, static_cast<const T *>(q), static_cast<const T *>(k),
                                  static_cast<const T *>(v), static_cast<const T *>(ig), static_cast<const T *>(fg), C0, n0,
                                  m0, static_cast<T *>(h), C1, n1, m1, dqk, dv, eps, qscale, gate_cap, state_settled,
@@ -235,9 +234,7 @@ static int mlstm_step_launch(const void *q, const void *k, const void *v, const 
     // fused output epilogue: the column tiles of a head form one cluster (portable size: at most 8)
     if (grid.y > 8) return XLSTM_ERR_UNSUPPORTED;
     auto kern = mlstm_step_kernel<T, DVT, THREADS, UNROLL, true>;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return XLSTM_ERR_CUDA;
+    if (smem > 48 * 1024 && !allow_smem(kern, most)) return XLSTM_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(THREADS);

@@ -161,13 +161,15 @@ static int slstm_recurrent_launch(const void *gx, const void *R, const float *rb
     // units per CTA: at most 64, and the resident weight slice must fit in shared memory
     int CL = 1;
     auto slice_bytes = [&](int cl) { return (size_t)dh * 4 * (dh / cl) * sizeof(T); };
-    while (CL <= 8 && (dh / CL > 64 || slice_bytes(CL) > 160 * 1024 || dh % CL)) CL *= 2;
+    constexpr size_t slice_most = 160 * 1024;
+    while (CL <= 8 && (dh / CL > 64 || slice_bytes(CL) > slice_most || dh % CL)) CL *= 2;
     if (CL > 8 || dh % 4) return XLSTM_ERR_UNSUPPORTED;
     const int U = dh / CL;
-    const size_t smem = slice_bytes(CL) + sizeof(float) * (2 * REC_BG * dh + REC_BG * 4 * U);
+    // (at most 64 units in each of 8 CTAs)
+    auto smem_of = [](size_t slice, int dims, int units) { return slice + sizeof(float) * (2 * REC_BG * dims + REC_BG * 4 * units); };
+    const size_t smem = smem_of(slice_bytes(CL), dh, U);
     auto kern = slstm_recurrent_kernel<T>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return XLSTM_ERR_CUDA;
+    if (!allow_smem(kern, smem_of(slice_most, 512, 64))) return XLSTM_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CL, NH, (B + REC_BG - 1) / REC_BG);
     cfg.blockDim = dim3(REC_THREADS);
