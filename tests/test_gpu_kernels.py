@@ -470,6 +470,22 @@ def test_chunkwise_fp32_two_kernels(ops, B, NH, S, dqk, dv, dtype, with_state):
         assert relerr(host(a), r) < FP32_TOL
 
 
+@pytest.mark.parametrize("NH,S,dqk,dv", [(48, 50, 128, 256), (32, 65, 128, 256), (40, 130, 128, 256), (16, 600, 128, 256), (60, 130, 72, 200)])
+def test_chunkwise_fp32_heads_do_not_depend_on_how_many_there_are(ops, NH, S, dqk, dv):
+    """The number of heads decides on the columns of a CTA, of the states and of the outputs (128 and 128 in one chunk; 128 and 64;
+    128 and 128; 64 and 128; the last part of dv in half a CTA), and on when the output kernel starts: bit for bit a head of its own."""
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(1, NH, S, d, device="cuda") for d in (dqk, dqk, dv))
+    i, f = torch.randn(1, NH, S, device="cuda"), torch.randn(1, NH, S, device="cuda") + 3
+    st = (torch.randn(1, NH, dqk, dv, device="cuda"), torch.randn(1, NH, dqk, device="cuda"), torch.randn(1, NH, device="cuda"))
+    for _ in range(3):
+        h, s1 = ops.mlstm_chunkwise(q, k, v, i, f, st)
+        for n in (0, NH // 2, NH - 1):
+            one = slice(n, n + 1)
+            ho, so = ops.mlstm_chunkwise(*(a[:, one] for a in (q, k, v, i, f)), tuple(s[:, one].contiguous() for s in st))
+            assert torch.equal(h[:, one], ho) and all(torch.equal(a[:, one], b) for a, b in zip(s1, so))
+
+
 # ---- sLSTM ------------------------------------------------------------------------
 @pytest.mark.parametrize("tag", ["a", "b", "x", "z"])
 def test_slstm_scan_fixture(ops, golden, tag):

@@ -3,20 +3,19 @@
 //
 //   chain   one CTA per head: the stabiliser m at the start of every 64-token chunk (sums and maxima of the gates by warps,
 //           then a scan over the chunks; whole sequence, first group only);
-//   state   one CTA per (head, 64 rows x 64 NG columns of C): keeps its piece of C in registers, walks the sequence in
+//   state   one CTA per (head, 64 rows x 64 or 128 columns of C): keeps its piece of C in registers, walks the sequence in
 //           tiles of 32 tokens, C <- decay C + (w K)^T V, and leaves the state at the start of every chunk in scratch (the
 //           only sequential part).  The weights of the chunks ahead and the normaliser are the work of two further warps;
 //   matrix  one CTA per (head, chunk): S = Q K^T, P = tril(S) with its gates, beside the state kernel;
-//   output  one CTA per (head, chunk, 64 NG columns of h): H = w_in Q C_start + P V as one contraction over dqk and the 64
+//   output  one CTA per (head, chunk, 64 or 128 columns of h): H = w_in Q C_start + P V as one contraction over dqk and the 64
 //           keys, normaliser.  All chunks at once.
 // A single chunk needs no scratch: its state and its output, which forms P itself, are two launches side by side.
 //
-// Both products are bound by FMA issue: a thread's tile is 8 rows x 4 NG columns of packed fp32 pairs (fma.rn.f32x2: two IEEE
-// multiply-adds per instruction), the pairs lie along the columns as they are stored, the row operand is doubled in registers.
-// The loops alone reach 98 (NG = 2) and 107 (NG = 4) multiply-adds a clock and SM of 128 (with the doubled operand in shared
-// memory 91 and 95).  16 heads of 256/512, 1024 tokens: 280 us in all, 142 of it states, 147 outputs (378 with the output
-// kernel forming S for every 128 columns, 8 x 8 tiles and doubled operands in shared memory); 4 heads of 64/64, 256 tokens:
-// 27 us (32), a chain of launches of 3, 14 and 8 us.
+// Both products are bound by FMA issue: a thread's tile is 8 rows x 4 NG columns (NG = 1, 2) of packed fp32 pairs (fma.rn.f32x2:
+// two IEEE multiply-adds per instruction), the pairs lie along the columns as they are stored, the row operand is doubled in
+// registers.  The loops alone reach 98 multiply-adds a clock and SM of 128 (with the doubled operand in shared memory 91).  16 heads of
+// 256/512, 1024 tokens: 267 us (378 with the output kernel forming S for every 128 columns and doubled operands in shared memory);
+// pieces of 256 columns, one CTA an SM, 279; 4 heads of 64/64, 256 tokens: 26 us (32).
 //
 // Exponents are differences u_s - x_t <= 0 with u = i - b, x = max(m, running max of u) and b the summed log forget
 // gates of the chunk, kept in double until the difference is taken (b reaches 1e3 in a chunk of closed gates).
@@ -46,6 +45,7 @@ struct F32Params {
     double *m_all;                   // [BH][NC + 1], NULL: a single chunk, which starts at m0
     float *pm;                       // [BH][g][CHUNK_PM]: gate matrix and scalars of every chunk (NULL with m_all)
     int NC, c_begin, c_end, slots;   // chunks of the sequence, of the group, slots per head
+    int early;                       // the output kernel may become resident while this group's states are worked on
     int slot0;                       // the first chunk's state is in slot 0 too (C1 may overwrite C0)
 };
 
@@ -181,14 +181,13 @@ template <typename T, int ROWS, int COLS, int THREADS> struct BlockStage {
     }
 };
 
-// K and V tiles; at NG = 4 a copy of the CTA's piece of C, from where it leaves for its slot
-template <int NG> constexpr uint32_t state_smem() { return 2 * TT * JT * 4 + 2 * TT * 64 * NG * 4 + (NG == 4 ? JT * 64 * NG * 4 : 0); }
+// K and V tiles
+template <int NG> constexpr uint32_t state_smem() { return 2 * TT * JT * 4 + 2 * TT * 64 * NG * 4; }
 
-// The products are one warp per scheduler at NG = 4, so whatever else those warps did would stand beside the multiply-adds, not
-// behind them (144 us alone at the size above when they brought their tiles themselves, 55 of it without the products; 135 now): two warps
-// bring K and V of the next tile and scale K, a third turns gates into weights a chunk ahead.
+// The products are two warps per scheduler at most, so whatever else those warps did would stand beside the multiply-adds, not
+// behind them: two warps bring K and V of the next tile and scale K, a third turns gates into weights a chunk ahead.
 template <typename T, int NG>
-__global__ void __launch_bounds__(MAIN + LOAD + 32, NG == 4 ? 1 : 2) mlstm_f32_state_kernel(const F32Params P) {
+__global__ void __launch_bounds__(MAIN + LOAD + 32, 2) mlstm_f32_state_kernel(const F32Params P) {
     constexpr int CT = 64 * NG;
     extern __shared__ __align__(16) unsigned char smem[];
     float *sK = reinterpret_cast<float *>(smem);                       // [2][TT][JT] w k
@@ -350,39 +349,12 @@ __global__ void __launch_bounds__(MAIN + LOAD + 32, NG == 4 ? 1 : 2) mlstm_f32_s
             d += p.dv;
         }
     };
-    // The slots of all CTAs are written at the same moments; from registers the stores of 64 KB a CTA held up the products
-    // (27 of 135 us).  A warp owns 16 whole rows: it leaves them in shared memory and the copy engine takes them from there.
-    float *sC = sV + 2 * TT * CT + (ty & ~1) * 8 * CT;
-    auto put_async = [&](float *base) {
-        if (lane < 16) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the rows of the slot before have left
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int g = 0; g < NG; ++g) {
-                const float2 x = unpack2(acc[r][2 * g]), y = unpack2(acc[r][2 * g + 1]);
-                *reinterpret_cast<float4 *>(sC + ((ty & 1) * 8 + r) * CT + g * 64 + tx * 4) = make_float4(x.x, x.y, y.x, y.y);
-            }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        const int row = j0 + (ty & ~1) * 8 + lane;
-        if (lane < 16) {
-            if (row < p.dqk)
-                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                             ::"l"(base + (size_t)row * p.dv + col0), "r"(smem_addr(sC + lane * CT)), "r"(min(CT, p.dv - col0) * 4) : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-    };
     __syncthreads();
     __syncthreads();
     for (int k = 0; k < tiles; ++k) {
         if ((k & 1) == 0) {
             const int c = k >> 1;
-            if (P.slot_C && (c > 0 || P.slot0)) {
-                float *slot = P.slot_C + ((size_t)bh * P.slots + c) * CE;
-                if constexpr (NG == 4) put_async(slot);
-                else put(slot);
-            }
+            if (P.slot_C && (c > 0 || P.slot0)) put(P.slot_C + ((size_t)bh * P.slots + c) * CE);
             const u64 d2 = pack2(s_decay[c & 1], s_decay[c & 1]);
 #pragma unroll
             for (int r = 0; r < 8; ++r)
@@ -393,7 +365,6 @@ __global__ void __launch_bounds__(MAIN + LOAD + 32, NG == 4 ? 1 : 2) mlstm_f32_s
         __syncthreads();
     }
     put(P.C1 + bh * CE);
-    if (NG == 4 && lane < 16) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -502,7 +473,7 @@ template <typename T> __global__ void __launch_bounds__(MAIN, 3) mlstm_f32_gate_
     const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 4, tx = tid & 15;
     const int ci = blockIdx.x, c = P.c_begin + ci, bh = blockIdx.y, b = bh / p.NH, hd = bh % p.NH;
     // the state kernel has waited for the chain kernel before it let this one start
-    allow_dependents();
+    if (P.early) allow_dependents();
     GateRaw raw[2];
     chunk_load<T>(p, b, hd, c * CH, lane, raw);
     const ChunkQK<T> qk(p, b, hd, c * CH, tid);
@@ -695,21 +666,31 @@ template <typename T> int run_group(const F32Params &P, cudaStream_t st) {
         const int rc = launch_overlapped(mlstm_f32_chain_kernel<T>, dim3(p.B * p.NH), dim3(CHAIN_WARPS * 32), 0, st, P);
         if (rc != XLSTM_OK) return rc;
     }
-    // columns per CTA: as many as still give most SMs a CTA (fewer passes over K, and over Q and K and S in the output)
-    const int64_t state = (int64_t)p.B * p.NH * ((p.dqk + JT - 1) / JT), output = (int64_t)p.B * p.NH * (P.c_end - P.c_begin);
-    auto columns = [&](int64_t rows) {
-        for (int ng = 4; ng > 1; ng >>= 1)
-            if (p.dv > 32 * ng && rows * ((p.dv + 64 * ng - 1) / (64 * ng)) >= 111) return ng;
-        return 1;
-    };
-    const int ns = columns(state);
-    int rc = ns == 4 ? launch_state<T, 4>(P, st) : ns == 2 ? launch_state<T, 2>(P, st) : launch_state<T, 1>(P, st);
+    const int chunks = P.c_end - P.c_begin;
+    auto state_ctas = [&](int ng) { return (int64_t)p.B * p.NH * ((p.dqk + JT - 1) / JT) * ((p.dv + 64 * ng - 1) / (64 * ng)); };
+    auto output_ctas = [&](int ng) { return (int64_t)p.B * p.NH * chunks * ((p.dv + 64 * ng - 1) / (64 * ng)); };
+    // 128 columns a CTA or 64.  States: 64 make the shorter tile and twice the CTAs, each of which starts, leaves its slots and ends,
+    // so the more chunks, the more CTAs are worth it (us with 64 and 128 columns: 16 heads of 256/512, 65 tokens 63 and 58; 8 of 128/256
+    // 256 tokens 29 and 40; 24 of 128/256 256 tokens 49 and 47, 512 tokens 79 and 84).  Outputs: 128 where 64 would be more than fit at
+    // once, three an SM (24 of 256/512, 256 tokens 123 and 117; 12 heads 74 and 77).  A single chunk's two kernels share the SMs: 32
+    // of 256/512, 64 tokens 58 and 42 with 128 output CTAs of 128 columns, 12 heads 27.4 and 28.7 with 48.
+    const int ns = p.dv > 64 && state_ctas(2) >= (chunks == 1 ? 111 : chunks < 10 ? 24 * chunks : 222) ? 2 : 1;
+    const int no = p.dv > 64 && (chunks == 1 ? output_ctas(2) >= 80 : output_ctas(1) > 444) ? 2 : 1;
+    // Output CTAs that become resident beside the state kernel crowd the SMs it leaves free, up to three on one, and stay there: with
+    // one wave of them that lasts longer than their start costs (16 heads of 256/512, 128 tokens 85 us, 56 when they start after the
+    // states; 24 of 128/256, 192 tokens 60 and 39).  They come early where every CTA of the group has an SM, where several waves
+    // even it out (32 of 128/256, 512 tokens: 115 and 119), or where they are short and half the SMs are free (64 of 64/64, 320
+    // tokens: 38 and 41).
+    F32Params G = P;
+    G.early = state_ctas(ns) + (int64_t)p.B * p.NH * chunks + output_ctas(no) <= 148 || output_ctas(no) >= 370 ||
+              (p.dqk <= 64 && state_ctas(ns) <= 74);
+    int rc = ns == 2 ? launch_state<T, 2>(G, st) : launch_state<T, 1>(G, st);
     if (rc != XLSTM_OK) return rc;
     if (P.m_all) {
-        rc = launch_overlapped(mlstm_f32_gate_matrix_kernel<T>, dim3(P.c_end - P.c_begin, p.B * p.NH), dim3(MAIN), 0, st, P);
+        rc = launch_overlapped(mlstm_f32_gate_matrix_kernel<T>, dim3(chunks, p.B * p.NH), dim3(MAIN), 0, st, G);
         if (rc != XLSTM_OK) return rc;
     }
-    return columns(output) >= 2 ? launch_output<T, 2>(P, st) : launch_output<T, 1>(P, st);
+    return no == 2 ? launch_output<T, 2>(G, st) : launch_output<T, 1>(G, st);
 }
 
 // scratch of one chunk of a head: its state and its gate matrix (a multiple of 16 bytes, as each of the three arrays is)
