@@ -20,9 +20,12 @@ namespace xl {
 
 // tile shape (the measured best on B200): dv columns per CTA, threads, rows in flight per thread, CTAs per SM
 constexpr int STEP_DVT = 64, STEP_THREADS = 256, STEP_UNROLL = 4, STEP_MIN_CTAS = 4;
-// with at most one CTA per SM (a sequence or two) the step is latency, not bandwidth: all rows of a thread in flight at once
-// (dqk up to 256), where the state is settled before the wait; a token of one sequence through 16 blocks
-// 1.44 -> 1.40 ms (with the loads of the prologue all on their way at once, which takes a step of 16 sequences from 24.9 to 23.9 us)
+// With at most one CTA per SM (a sequence or two) the step is latency, not bandwidth: all rows of a thread in flight at once (dqk up
+// to 256), where the state is settled before the wait.  Cold states, us with and without: 256/512, 4 heads 3.8 / 5.2, 16 heads 5.2 /
+// 6.4 (gated 5.7 / 7.2); 128/256, gated, 32 heads 4.4 / 5.2.  With few bytes to wait for it only keeps registers and rows that are not
+// there busy (128/256, 4 heads 3.0 / 2.4; any number of heads of 64/64 2.7 / 2.0), hence the lower limits in mlstm_step_checked().
+// Two CTAs must fit an SM (128 registers), or the next step's cannot be there when the last ones of this leave (gated, 16 heads of
+// 256/512: 5.7 us, with 138 registers 8.9).
 constexpr int STEP_UNROLL_FEW = 16;
 
 // GATED: the output epilogue of the layer (per-head RMS norm x weight x sigmoid(output gate)) is applied before
@@ -45,7 +48,7 @@ struct StepRows {
 };
 
 template <typename T, int DVT, int THREADS, int UNROLL, bool GATED>
-__global__ void __launch_bounds__(THREADS, UNROLL > STEP_UNROLL ? 1 : STEP_MIN_CTAS)
+__global__ void __launch_bounds__(THREADS, UNROLL > STEP_UNROLL ? 2 : STEP_MIN_CTAS)
 mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v,
                   const T *__restrict__ ig, const T *__restrict__ fg,
                   const float *C0, const float *__restrict__ n0, const float *__restrict__ m0,
@@ -86,13 +89,25 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     if (state_settled) load_state();
     grid_dependency_wait();
     allow_dependents();
-    if (!state_settled) load_state();
+    // n and m after the wait always: a settled state promises C alone, and the preceding kernel may have written them (a copy that
+    // converts their type, a reset)
+    float mold = 0.f, nold = 0.f;
+    auto load_nm = [&]() {
+        if (has_state) {
+            mold = m0[bh];
+            if (tid < dqk) nold = n0[(size_t)bh * dqk + tid];
+        }
+    };
+    if (!state_settled) {
+        load_state();
+        load_nm();      // (in each branch: 16 sequences of 8 heads 24.5 us, behind both 25.0)
+    } else {
+        load_nm();
+    }
 
     // stabilised gates (every thread: two exps and a log1p are cheaper than a broadcast)
     const float graw = Elem<T>::ld(ig + gate_at), fraw = Elem<T>::ld(fg + gate_at);
-    // everything else that is read: its latency runs beside the gates'.  n and m too: a settled state promises C alone, and the
-    // preceding kernel may have written them (a copy that converts their type, a reset)
-    const float mold = has_state ? m0[bh] : 0.f, nold = has_state && tid < dqk ? n0[(size_t)bh * dqk + tid] : 0.f;
+    // everything else that is read: its latency runs beside the gates'
     const T *qrow = q + (GATED ? seq * rows.q + (size_t)head * dqk : (size_t)bh * dqk);
     const T *krow = k + (GATED ? seq * rows.k + (size_t)head * dqk : (size_t)bh * dqk);
     const float q0 = tid < dqk ? Elem<T>::ld(qrow + tid) : 0.f, k0 = tid < dqk ? Elem<T>::ld(krow + tid) : 0.f;
@@ -135,16 +150,16 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
     float4 acc = zero4;
     if (active) {
         for (int j0 = rg; j0 < dqk; j0 += RG * UNROLL) {
-            // next batch goes out before this one is consumed (few CTAs: there is none up to dqk = 256)
-            float4 nx[UNROLL];
-            auto load_next = [&](float4 (&to)[UNROLL]) {
+            // next batch goes out before this one is consumed (few CTAs: there is none, dqk <= 256)
+            static_assert(UNROLL == STEP_UNROLL || UNROLL * RG >= 256, "one batch");
+            float4 nx[UNROLL == STEP_UNROLL ? UNROLL : 1];
+            if constexpr (UNROLL == STEP_UNROLL) {
 #pragma unroll
                 for (int u = 0; u < UNROLL; ++u) {
                     const int j = j0 + (UNROLL + u) * RG;
-                    to[u] = (has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
+                    nx[u] = (has_state && j < dqk) ? ldg_stream(Cin + (size_t)j * dv) : zero4;
                 }
-            };
-            if (UNROLL == STEP_UNROLL) load_next(nx);
+            }
 #pragma unroll
             for (int u = 0; u < UNROLL; ++u) {
                 const int j = j0 + u * RG;
@@ -162,11 +177,9 @@ mlstm_step_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__r
                     acc.w = fmaf(o.w, qj, acc.w);
                 }
             }
-            if (UNROLL == STEP_UNROLL) {
+            if constexpr (UNROLL == STEP_UNROLL) {
 #pragma unroll
                 for (int u = 0; u < UNROLL; ++u) c[u] = nx[u];
-            } else {
-                load_next(c);
             }
         }
     }
@@ -284,7 +297,8 @@ static int mlstm_step_checked(const void *q, const void *k, const void *v, const
     auto run = [&](auto launch) {
         return launch(q, k, v, ig, fg, C0, n0, m0, h, C1, n1, m1, B * NH, dqk, dv, eps, gate_cap, settled, rows, gate, st);
     };
-    const bool few = (int64_t)B * NH * ((dv + xl::STEP_DVT - 1) / xl::STEP_DVT) <= 148 && dqk <= 256;
+    const int64_t ctas = (int64_t)B * NH * ((dv + xl::STEP_DVT - 1) / xl::STEP_DVT);
+    const bool few = ctas <= 148 && ctas * dqk >= 6144 && dqk > 64 && dqk <= 256;
     if (dtype == XLSTM_F32)
         return few ? run(xl::mlstm_step_launch<float, xl::STEP_UNROLL_FEW>) : run(xl::mlstm_step_launch<float, xl::STEP_UNROLL>);
     return few ? run(xl::mlstm_step_launch<__nv_bfloat16, xl::STEP_UNROLL_FEW>) : run(xl::mlstm_step_launch<__nv_bfloat16, xl::STEP_UNROLL>);
