@@ -433,6 +433,27 @@ def test_linear_rows(ops, M, N, K):
     assert relerr(host(act), xo.swiglu(bf(xo.linear(x, W2[:N])), bf(xo.linear(x, W2[N:])))) <= BF16_TOL
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 4736, 2048), (3, 4737, 2048), (16, 9472, 2048), (5, 9473, 2048), (7, 70, 1024), (16, 70, 1056)])
+def test_linear_rows_forms(ops, M, N, K):
+    """Both sides of the lines between a CTA a tile and CTAs that walk (148 and 296 tiles, rows of 1024), plain, as a pair and with a
+    norm, against float64: fp32 sums of K products (within K 2^-24 of their absolute sum) and the bf16 roundings on the way."""
+    torch.manual_seed(M + N + K)
+    t = torch.bfloat16
+    W, x = (torch.randn(N, K, device="cuda") * 0.05).to(t), torch.randn(M, K, device="cuda").to(t)
+    W64, x64 = W.double(), x.double()
+    ref = x64 @ W64.t()
+    room = 2.0 ** -8 * ref.abs() + K * 2.0 ** -24 * (x64.abs() @ W64.abs().t())
+    assert bool(((ops.linear_rows(W, x).double() - ref).abs() <= room).all())
+    half = N // 2 * 2
+    gate, up = (a.to(t).double() for a in ref[:, :half].split(half // 2, 1))
+    pair = gate * torch.sigmoid(gate) * up
+    got = ops.linear_rows(W[:half].contiguous(), x, swiglu_pair=True).double()
+    assert float((got - pair).abs().max()) <= BF16_TOL * float(pair.abs().max())
+    if M * (2 * K + 64) + 2 * K <= 49152:
+        nw = torch.rand(K, device="cuda").to(t) + 0.5
+        assert torch.equal(ops.linear_rows(W, x, norm_weight=nw), ops.linear_rows(W, ops.rms_norm(x, nw)))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (2, 31, 32), (4, 5000, 4096), (3, 17, 1056), (16, 4800, 96), (5, 9600, 2080)])
 def test_linear_rows_with_norm(ops, M, N, K):
     """One row and sixteen, fewer and more tiles than CTAs, k blocks around a warp's share: the norm in front equals its own

@@ -7,30 +7,36 @@
 // one row) is used as the fragments of TWO k-steps, so weights go from global memory straight into the MMA's registers, 64
 // bytes of a row per quad of lanes, without passing through shared memory.
 //
-// One persistent CTA of 16 warps per SM walks tiles of 2 x 16 weight rows (16 gate and 16 up rows for the SwiGLU pair); the
-// warps take the 32-wide k blocks of a tile in turn.  A warp's LR_U blocks in flight run on into the next tile, so the stream of
-// weights does not stop while the partial sums of the 16 warps meet in shared memory for the epilogue (bias, residual, SwiGLU
-// with the separate layers' roundings; two buffers, one barrier a tile).  x comes through L1 and L2, half a byte per byte of W.
+// A CTA's tile is 2 x 16 weight rows (16 gate and 16 up rows for the SwiGLU pair); its warps take the 32-wide k blocks in turn, and
+// their partial sums meet in shared memory for the epilogue (bias, residual, SwiGLU with the separate layers' roundings).  x comes
+// through L1 and L2, half a byte per byte of W.  Two forms: a persistent CTA of 16 warps per SM walks the tiles, and a warp's LR_U
+// blocks in flight run on into the next one, so the stream of weights does not stop for the epilogue (two buffers, one barrier a
+// tile); or a CTA of 8 warps has one tile (which is taken when: linear_rows_form()).
 // With XLSTM_LINEAR_WEIGHTS_SETTLED the first weights are loaded BEFORE the wait on the preceding kernel, which the caller
 // promises not to have written them; without it they are only asked of L2.  With a norm in front every CTA normalises the rows
 // for itself, into shared memory, while its first weights are under way (a launch of its own takes 5.8 us between two of these).
 // That is for few rows only: shared memory is taken from the L1, where the weights in flight land.  16 rows of 4096 (132 KB)
 // cost 7 us, and a little more of it 25.
-// Measured (weights cold, 16 rows; a CTA of 8 warps per tile before): 12304 x 4096 21.6 us (26.1; floor 15.4), 4096 x 4096 8.5
-// (11.3; 5.1), 21888 x 4096 as a pair 33.8 (41.0; 27.3), 4096 x 10944 18.0 (24.8; 13.7), 1024 x 1024 2.4 (2.1).  LR_U = 2: 4 %
-// more, 12 warps with LR_U = 4 or 8 with 8: the same within 2 %.
+// Measured (weights cold, 16 rows; 8 warps and one tile): 12304 x 4096 21.1 us (25.1; floor 15.4), 4096 x 4096 8.0 (10.2; 5.1),
+// 21888 x 4096 as a pair 33.3 (38.0; 27.3), 4096 x 10944 16.9 (22.9; 13.7).  LR_U = 2: 4 % more, 12 warps with LR_U = 4 or 8 with 8:
+// the same within 2 %.
 #include "cp_async.cuh"
 #include "vec16.cuh"
 
 namespace xl {
 namespace {
 
-constexpr int LR_THREADS = 512, LR_WARPS = LR_THREADS / 32;
 constexpr int LR_ROWS = 32;      // weight rows per tile
 constexpr int LR_M = 16;         // rows of x
-constexpr int LR_U = 3;          // k blocks in flight per warp: 6 KB of weights
 constexpr int LR_LD = LR_ROWS + 1;
-constexpr uint32_t LR_SMEM = 2 * LR_WARPS * LR_M * LR_LD * sizeof(float);
+// the two forms of a CTA: 16 warps that walk tiles, 8 warps with one tile
+template <int WARPS> struct Form {
+    static constexpr int THREADS = WARPS * 32;
+    static constexpr int U = WARPS == 16 ? 3 : 4;            // k blocks in flight per warp: 6 or 8 KB of weights
+    static constexpr int BUFFERS = WARPS == 16 ? 2 : 1;      // of partial sums
+    static constexpr int PART = WARPS * LR_M * LR_LD;
+    static constexpr uint32_t SMEM = BUFFERS * PART * sizeof(float);
+};
 
 // bytes between normalised rows of x in shared memory: the eight rows and four 16-byte lanes of a load on different banks
 __host__ __device__ __forceinline__ int norm_ld(int K) { return 2 * K + 64; }
@@ -48,14 +54,15 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 // EPI: 0 = bias only, 1 = + residual, 2 = SwiGLU pair (W has 2 N rows: gate rows, then up rows)
-template <int EPI, bool NORM>
-__global__ void __launch_bounds__(LR_THREADS, 1)
+template <int EPI, bool NORM, int LR_WARPS>
+__global__ void __launch_bounds__(LR_WARPS * 32, LR_WARPS == 16 ? 1 : 2)
 linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, const __nv_bfloat16 *__restrict__ bias,
                    const __nv_bfloat16 *residual, const __nv_bfloat16 *__restrict__ norm_w, float norm_eps,
                    __nv_bfloat16 *__restrict__ y, int M, int N, int K, int weights_settled) {
     constexpr int STRIDE = EPI == 2 ? 16 : 32;                 // outputs per tile
-    extern __shared__ __align__(16) float lr_part[];           // [2][LR_WARPS][LR_M][LR_LD]; NORM: the rows of x after it
-    unsigned char *sx = reinterpret_cast<unsigned char *>(lr_part) + LR_SMEM;
+    constexpr int LR_U = Form<LR_WARPS>::U, LR_THREADS = Form<LR_WARPS>::THREADS;
+    extern __shared__ __align__(16) float lr_part[];           // [BUFFERS][LR_WARPS][LR_M][LR_LD]; NORM: the rows of x after it
+    unsigned char *sx = reinterpret_cast<unsigned char *>(lr_part) + Form<LR_WARPS>::SMEM;
     const int ldx = norm_ld(K);                                // bytes between them
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const int blocks = K >> 5, tiles = (N + STRIDE - 1) / STRIDE;
@@ -150,7 +157,7 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
     for (int u = 0; u < LR_U; ++u) load_x(u, warp + u * LR_WARPS);
 
     int par = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, par ^= 1) {
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, par ^= Form<LR_WARPS>::BUFFERS - 1) {
         float acc[2][2][4];
 #pragma unroll
         for (int t = 0; t < 2; ++t)
@@ -161,8 +168,8 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
         for (int gr = 0; gr < groups; ++gr) {
             const bool tile_ends = gr + 1 == groups;
             const int b0 = tile_ends ? warp : warp + (gr + 1) * LR_U * LR_WARPS;   // what the slots are refilled with
-            const bool more = !tile_ends || tile + (int)gridDim.x < tiles;
-            if (tile_ends && more) rows_of(tile + gridDim.x);
+            const bool more = !tile_ends || (LR_WARPS == 16 && tile + (int)gridDim.x < tiles);
+            if (LR_WARPS == 16 && tile_ends && more) rows_of(tile + gridDim.x);
 #pragma unroll
             for (int u = 0; u < LR_U; ++u) {
                 if (NORM) {
@@ -182,7 +189,7 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
             }
         }
         // element e of an MMA tile: weight row g + 8 (e / 2), x row 2c + (e & 1)
-        float *part = lr_part + par * (LR_WARPS * LR_M * LR_LD);
+        float *part = lr_part + par * Form<LR_WARPS>::PART;
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -217,18 +224,31 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
     }
 }
 
-template <int EPI, bool NORM>
-int linear_rows_launch(const void *W, const void *x, const void *bias, const void *residual, const void *norm_w, float norm_eps,
-                       void *y, int M, int N, int K, int settled, cudaStream_t st) {
-    const int per = EPI == 2 ? 16 : 32, tiles = (N + per - 1) / per;
-    const int64_t smem = (int64_t)LR_SMEM + (NORM ? (int64_t)M * norm_ld(K) + 2 * K : 0);   // rows of x, norm weight
-    if (smem > (int64_t)LR_SMEM + XLSTM_LINEAR_NORM_BYTES) return XLSTM_ERR_UNSUPPORTED;
-    auto kern = linear_rows_kernel<EPI, NORM>;
-    if (!allow_smem(kern, LR_SMEM + (NORM ? XLSTM_LINEAR_NORM_BYTES : 0))) return XLSTM_ERR_CUDA;
-    return launch_overlapped(kern, dim3(tiles < 148 ? tiles : 148), dim3(LR_THREADS), (size_t)smem, st,
-                             static_cast<const __nv_bfloat16 *>(W), static_cast<const __nv_bfloat16 *>(x),
-                             static_cast<const __nv_bfloat16 *>(bias), static_cast<const __nv_bfloat16 *>(residual),
-                             static_cast<const __nv_bfloat16 *>(norm_w), norm_eps, static_cast<__nv_bfloat16 *>(y), M, N, K, settled);
+struct Args {
+    const void *W, *x, *bias, *residual, *norm_w;
+    float norm_eps;
+    void *y;
+    int M, N, K, settled;
+};
+template <int EPI, bool NORM, int WARPS> int linear_rows_launch(const Args &a, int tiles, cudaStream_t st) {
+    using F = Form<WARPS>;
+    using B = const __nv_bfloat16 *;
+    const int64_t norm = NORM ? (int64_t)a.M * norm_ld(a.K) + 2 * a.K : 0;   // rows of x, norm weight
+    if (norm > XLSTM_LINEAR_NORM_BYTES) return XLSTM_ERR_UNSUPPORTED;
+    auto kern = linear_rows_kernel<EPI, NORM, WARPS>;
+    if (!allow_smem(kern, F::SMEM + (NORM ? XLSTM_LINEAR_NORM_BYTES : 0))) return XLSTM_ERR_CUDA;
+    return launch_overlapped(kern, dim3(WARPS == 16 && tiles > 148 ? 148 : tiles), dim3(F::THREADS), (size_t)(F::SMEM + norm), st,
+                             static_cast<B>(a.W), static_cast<B>(a.x), static_cast<B>(a.bias), static_cast<B>(a.residual),
+                             static_cast<B>(a.norm_w), a.norm_eps, static_cast<__nv_bfloat16 *>(a.y), a.M, a.N, a.K, a.settled);
+}
+template <int EPI, bool NORM> int linear_rows_form(const Args &a, cudaStream_t st) {
+    const int per = EPI == 2 ? 16 : 32, tiles = (a.N + per - 1) / per;
+    // Tiles of short rows are over before a second one pays for the walk, and with one and a bit to two rounds of tiles half the CTAs
+    // would be idle in the last one; two small CTAs an SM hold all of them at once.  us, 16 rows of x, one tile a CTA and walking:
+    // 1024 x 1024 2.3 / 2.6, 3088 x 1024 as a pair 3.6 / 5.1, 16384 x 1024 8.4 / 10.3; 6160 x 1536 5.7 / 5.5; 8192 x 2048 7.5 / 8.4,
+    // 6144 x 4096 12.6 / 13.9; 12288 x 2048 13.8 / 11.6, 4096 x 2048 6.1 / 4.9.
+    if (a.K <= 1024 || (a.K >= 2048 && tiles > 148 && tiles <= 2 * 148)) return linear_rows_launch<EPI, NORM, 8>(a, tiles, st);
+    return linear_rows_launch<EPI, NORM, 16>(a, tiles, st);
 }
 
 }  // namespace
@@ -244,10 +264,10 @@ extern "C" int xlstm_linear_rows_norm(const void *W, const void *x, const void *
     if ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w)) & 15u) return XLSTM_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int settled = flags & XLSTM_LINEAR_WEIGHTS_SETTLED ? 1 : 0;
-    auto run = [&](auto kern) { return kern(W, x, bias, residual, norm_w, norm_eps, y, M, N, K, settled, st); };
-    if (norm_w) return epilogue == 2 ? run(xl::linear_rows_launch<2, true>) : run(xl::linear_rows_launch<0, true>);
-    if (epilogue == 2) return run(xl::linear_rows_launch<2, false>);
-    return epilogue == 1 ? run(xl::linear_rows_launch<1, false>) : run(xl::linear_rows_launch<0, false>);
+    const xl::Args a{W, x, bias, residual, norm_w, norm_eps, y, M, N, K, settled};
+    if (norm_w) return epilogue == 2 ? xl::linear_rows_form<2, true>(a, st) : xl::linear_rows_form<0, true>(a, st);
+    if (epilogue == 2) return xl::linear_rows_form<2, false>(a, st);
+    return epilogue == 1 ? xl::linear_rows_form<1, false>(a, st) : xl::linear_rows_form<0, false>(a, st);
 }
 
 extern "C" int xlstm_linear_rows_ex(const void *W, const void *x, const void *bias, const void *residual, void *y, int M, int N,
