@@ -100,12 +100,15 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_kernel(const __nv_bfloat16 *_
     const int total_warps = gridDim.x * (GV_THREADS / 32);
     const int n_first = blockIdx.x * (GV_THREADS / 32) + warp;
 
-    // ---- L2 prefetch of the head of this warp's first weight row (1 KB, two of its loads: a token through 16 blocks of 4096
-    //      takes 1.440 ms with 0.5 or 1 KB, 1.446 with 2, 1.471 with 4, 1.545 with 8, 1.457 without; loads into registers
-    //      instead cost resident CTAs, 1.56), then the wait for the preceding kernel
+    // ---- L2 prefetch of the head of this warp's first weight row, then the wait for the preceding kernel.  4 KB: a row of 2048, or what
+    //      the first loads will ask for.  With one row of x and large weights (every warp has a row of 8 KB and more, the launch before
+    //      is as long as this one) what is brought early pushes the running kernel's lines out of L2, and 1 KB is the better: a token
+    //      through 16 blocks of 4096 1.44 ms with 0.5 or 1 KB, 1.45 with 2, 1.47 with 4, 1.55 with 8.  Elsewhere 1 KB loses, us with 4
+    //      and 1 KB: 2048 x 2048 4.0 / 4.7, 8192 x 2048 9.1 / 10.2, 2048 x 5504 9.9 / 10.5, 3 rows of x with 10944 x 4096 29.5 / 32.4, a token
+    //      of one sequence through blocks of 1024 20.3 / 21.8.  Loads into registers instead cost resident CTAs (1.56 ms).
     if (n_first < N) {
         const char *row = reinterpret_cast<const char *>(W + (size_t)n_first * K);
-        const int head = K * 2 < 1024 ? K * 2 : 1024;
+        const int most = M == 1 && N >= 4096 && K >= 4096 ? 1024 : 4096, head = K * 2 < most ? K * 2 : most;
         if (lane * 128 < head) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + lane * 128));
     }
     grid_dependency_wait();
