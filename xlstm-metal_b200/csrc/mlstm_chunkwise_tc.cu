@@ -818,10 +818,14 @@ int launch_both(const TcParams &tp, int grid, cudaStream_t st) {
 // where the pass is long or most SMs get a CTA.  With the general launch in front and only short sequences side by side, heads of
 // both kinds took, us at 256/512: 32 heads, 4001 tokens 387 (now 270), 32 x 8192 730 (450), 16 x 16384 1396 (833).  Short passes of
 // few CTAs keep the general launch in front and both overlapped with what precedes them: an idle GPU costs 2 of 70 us there, and the
-// general path 3 of 104.
+// general path 3 of 104.  So do segments of up to two tiles of 256 rows or four of 128, whose two passes would wait for it twice: general
+// in front and bounded in front, 4 heads of 128/256, 3072 tokens, usual / general / mixed gates 38.7 / 46.6 / 45.9 and 39.2 / 50.4 / 50.7
+// us, 2 of 256/512, 3072 tokens 52.3 / 65.5 / 64.1 and 52.3 / 68.7 / 69.2; with longer segments the usual gates lose (4 of 256/512, 4001
+// tokens 85.7 and 82.3).
 template <int DQK, bool STATE_ONLY, int W>
 int launch_tc(const TcParams &tp, int grid, cudaStream_t st) {
-    const bool idle = tp.NCH > FUSED_TILES || grid > SM_COUNT / 2;
+    const bool short_segments = tp.P > 1 && tp.seg_tiles * DQK <= 512;
+    const bool idle = !short_segments && (tp.NCH > FUSED_TILES || grid > SM_COUNT / 2);
     return idle ? launch_both<DQK, STATE_ONLY, W, true>(tp, grid, st) : launch_both<DQK, STATE_ONLY, W, false>(tp, grid, st);
 }
 
