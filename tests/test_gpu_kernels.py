@@ -1047,6 +1047,38 @@ def test_chunkwise_short_bf16_keeps_an_infinity_to_later_tokens(ops, T, dqk, dv)
         assert (Ci[..., 5][k[:, :, at] != 0].isinf()).all() and relerr(host(Ci[..., others]), host(C[..., others])) < 1e-6
 
 
+@pytest.mark.parametrize("T", [65, 80, 127, 128])
+@pytest.mark.parametrize("dqk,dv,NH,f_mean", [(256, 480, 10, -2.0), (256, 480, 10, 3.0), (128, 96, 50, 3.0)])
+def test_chunkwise_short_bf16_in_turn(ops, T, dqk, dv, NH, f_mean):
+    """More heads than SMs: 64 tokens at a time in one launch.  As two calls, the second from the first one's state: h to one bf16
+    rounding (2^-7 of the value across a rounding boundary) on rows whose normaliser does not cancel, the state to fp32 rounding;
+    and no further from float64 than the fp32 kernels (as above)."""
+    torch.manual_seed(T + dqk)
+    rnd = lambda *s: torch.randn(*s, device="cuda")
+    q, k, v = rnd(1, NH, T, dqk).to(BF), rnd(1, NH, T, dqk).to(BF), rnd(1, NH, T, dv).to(BF)
+    i, f = rnd(1, NH, T).to(BF), (rnd(1, NH, T) + f_mean).to(BF)
+    st = (rnd(1, NH, dqk, dv), rnd(1, NH, dqk), rnd(1, NH))
+    part = lambda a, b: [x[:, :, a:b] for x in (q, k, v, i, f)]
+    for start in (st, None):
+        h, s1 = ops.mlstm_chunkwise(*part(0, T), start)
+        ha, sa = ops.mlstm_chunkwise(*part(0, 64), start)
+        hb, sb = ops.mlstm_chunkwise(*part(64, T), sa)
+        assert torch.equal(h[:, :, :64], ha)
+        off = (h[:, :, 64:].float() - hb.float()).abs()
+        assert float((off > 2.0 ** -7 * hb.float().abs() + 1e-5 * hb.float().abs().amax(-1, keepdim=True)).float().mean()) < 1e-3
+        for a, b in zip(s1, sb):
+            assert relerr(host(a), host(b)) < 1e-6
+    C, m = st[0].double(), st[2].double()
+    for t in range(T):
+        fl, it = torch.nn.functional.logsigmoid(f[:, :, t].double()), i[:, :, t].double()
+        mn = torch.maximum(fl + m, it)
+        fg, ig = torch.exp(fl + m - mn), torch.exp(it - mn)
+        C = fg[..., None, None] * C + ig[..., None, None] * k[:, :, t, :, None].double() * v[:, :, t, None, :].double()
+        m = mn
+    (Cb, Cf) = (ops.mlstm_chunkwise(*args, st)[1][0].double() for args in (part(0, T), [x.float() for x in part(0, T)]))
+    assert float((Cb - C).norm()) <= 1.1 * float((Cf - C).norm())
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 8, 16, 17, 33, 64, 65, 127])
 @pytest.mark.parametrize("dqk,dv,f_mean", [(256, 512, -2.0), (256, 512, 3.0), (128, 256, -2.0)])
 def test_chunkwise_short_bf16_state_is_no_further_off_than_fp32(ops, T, dqk, dv, f_mean):
