@@ -486,6 +486,20 @@ def test_chunkwise_fp32_heads_do_not_depend_on_how_many_there_are(ops, NH, S, dq
             assert torch.equal(h[:, one], ho) and all(torch.equal(a[:, one], b) for a, b in zip(s1, so))
 
 
+def test_chunkwise_fp32_normaliser_of_one_token_is_rounded_once(ops):
+    """With an input gate that weighs the token with exactly one, n' = decay n + k is one multiply-add: bit for bit the float64
+    value rounded to fp32, for the decay that the kernel itself uses (read off n = 1, k = 0)."""
+    torch.manual_seed(0)
+    NH, dqk, dv = 3, 256, 64
+    k, n, v = torch.randn(1, NH, 1, dqk, device="cuda"), torch.randn(1, NH, dqk, device="cuda"), torch.randn(1, NH, 1, dv, device="cuda")
+    i, f, m, C = (torch.zeros(1, NH, 1, device="cuda"), torch.randn(1, NH, 1, device="cuda"), torch.zeros(1, NH, device="cuda"),
+                  torch.zeros(1, NH, dqk, dv, device="cuda"))
+    after = lambda k, n: ops.mlstm_chunkwise(k, k, v, i, f, (C, n, m))[1][1]
+    decay = after(torch.zeros_like(k), torch.ones_like(n))
+    assert bool((decay < 1).all())
+    assert torch.equal(after(k, n), (decay.double() * n.double() + k[:, :, 0].double()).float())
+
+
 # ---- sLSTM ------------------------------------------------------------------------
 @pytest.mark.parametrize("tag", ["a", "b", "x", "z"])
 def test_slstm_scan_fixture(ops, golden, tag):

@@ -290,14 +290,14 @@ __global__ void __launch_bounds__(MAIN + LOAD + 32, 2) mlstm_f32_state_kernel(co
             if (k + 1 < tiles) stage(k + 1);   // into the other buffer: last read before the previous barrier
             if (my_n) {
                 const int c = k >> 1;
+                float decay = 1.f;
                 if ((k & 1) == 0) {
                     if (P.slot_n && (c > 0 || P.slot0)) {
                         float *dst = P.slot_n + ((size_t)bh * P.slots + c) * p.dqk;
                         if (j < p.dqk) dst[j] = n0;
                         if (j + 1 < p.dqk) dst[j + 1] = n1;
                     }
-                    n0 *= s_decay[c & 1];
-                    n1 *= s_decay[c & 1];
+                    decay = s_decay[c & 1];
                 }
                 const float2 *row = reinterpret_cast<const float2 *>(sK + (k & 1) * TT * JT) + lane;
                 float a0 = 0.f, a1 = 0.f;
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(MAIN + LOAD + 32, 2) mlstm_f32_state_kernel(co
                     a0 += v.x;
                     a1 += v.y;
                 }
-                n0 += a0;
-                n1 += a1;
+                n0 = fmaf(n0, decay, a0);
+                n1 = fmaf(n1, decay, a1);
             }
             cp_async_wait_all();
             __syncthreads();
