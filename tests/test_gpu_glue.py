@@ -583,6 +583,47 @@ def test_block_token_step_with_inputs_or_norms_at_odd_offsets(ops, B, what):
         assert torch.equal(y, y2) and all(torch.equal(a, b) for a, b in zip(st, st2))
 
 
+@pytest.mark.parametrize("d,NH,B", [(4096, 8, 5), (4096, 8, 16), (2048, 8, 16)])
+def test_block_token_step_with_norms_of_their_own(ops, d, NH, B):
+    """Rows beyond what the Linears take a norm for (48 KB): the norms are launches, in the same native call.  Against the block cell by
+    cell, the state carried over several tokens."""
+    from xlstm_cuda.blocks import mLSTMBlock
+    t = torch.bfloat16
+    assert B * (2 * d + 64) + 2 * d > 49152
+    torch.manual_seed(B)
+    with torch.device("cuda"):
+        blk = mLSTMBlock(0, embedding_dim=d, num_heads=NH, compute_dtype=t).to(t)
+    blk.fuse_projections()
+    with torch.inference_mode():
+        for mod in (blk.norm_mlstm, blk.norm_ffn):
+            mod.weight.uniform_(0.5, 1.5)
+        st = ref_st = None
+        for _ in range(4):
+            x = torch.randn(B, 1, d, device="cuda", dtype=t)
+            y, st = blk(x, st)
+            out, ref_st = blk.mlstm_cell(blk.norm_mlstm(x), ref_st)
+            x1, xn = ops.add_rms_norm(x, out, blk.norm_ffn.weight, blk.norm_ffn.eps)
+            ref = x1 + blk.ffn_proj_down(ops.swiglu(blk.ffn_proj_up_gate(xn), blk.ffn_proj_up(xn)))
+            assert relerr(host(y), host(ref)) <= BF16_TOL
+            for a, b in zip(st, ref_st):
+                assert relerr(host(a), host(b)) <= BF16_TOL
+
+
+def test_block_token_reports_the_call_that_failed(ops):
+    """A weight that the Linear does not take (odd offset): the status comes with that Linear's name, for both kinds of it."""
+    from xlstm_cuda._lib import XlstmCudaError
+    m, _, _ = _blocks()
+    cell = m.mlstm_cell
+    W, b = cell._fused_weights()
+    out, down, rk = cell.output_cell.out_proj, m.ffn_proj_down, cell.recurrent_kernel
+    odd = torch.cat([out.weight.new_zeros(1), out.weight.detach().flatten()])[1:].view_as(out.weight)
+    for B, rows, name in ((2, False, "xlstm_linear_token"), (8, True, "xlstm_linear_rows_norm")):
+        with torch.inference_mode(), pytest.raises(XlstmCudaError, match=name):
+            ops.mlstm_token_block(torch.zeros(B, 512, device="cuda", dtype=torch.bfloat16), W, b, (m.norm_mlstm.weight, 1e-6),
+                                  (cell.num_heads, cell.qk_dim_per_head, cell.v_dim_per_head), None, (None, 1e-6), rk.eps, False, 15.0,
+                                  (odd, None), (m.norm_ffn.weight, 1e-6), m._fused_ffn(), (down.weight, None), rows)
+
+
 def _blocks():
     from xlstm_cuda.blocks import mLSTMBlock, sLSTMBlock, sLSTMBlockDiag
     t = torch.bfloat16

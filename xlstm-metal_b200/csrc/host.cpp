@@ -214,6 +214,7 @@ std::vector<int64_t> with_last(const Tensor &x, int64_t n) {
 struct Result {
     int rc;
     Tensor y;
+    const char *what;   // the call that gave rc
     py::tuple tuple() const { return py::make_tuple(rc, y); }
 };
 Result linear(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight, double norm_eps,
@@ -238,14 +239,15 @@ Result linear(const Tensor &weight, const Tensor &x, const OptTensor &bias, cons
     const int epi = swiglu_pair ? 2 : (r ? 1 : 0);
     // a dense copy made here is written by the launch right before the call
     const int flags = weights_settled && w.is_same(weight) ? XLSTM_LINEAR_WEIGHTS_SETTLED : 0;
+    const bool token = max_rows <= 4;
     const int rc = unlocked([&] {
-        return max_rows <= 4
+        return token
             ? xlstm_linear_token(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M,
                                  (int)N, (int)K, epi, XLSTM_BF16, stream())
             : xlstm_linear_rows_norm(w.data_ptr(), x2.data_ptr(), ptr(b), ptr(nw), (float)norm_eps, ptr(r), y.data_ptr(), (int)M,
                                      (int)N, (int)K, epi, flags, XLSTM_BF16, stream());
     });
-    return {rc, y};
+    return {rc, y, token ? "xlstm_linear_token" : "xlstm_linear_rows_norm"};
 }
 py::tuple linear_token(const Tensor &weight, const Tensor &x, const OptTensor &bias, const OptTensor &norm_weight,
                        double norm_eps, const OptTensor &residual, bool swiglu_pair, int64_t max_rows, bool weights_settled) {
@@ -264,7 +266,7 @@ Result norm(const Tensor &x, const OptTensor &weight, double eps) {
         return xlstm_rms_norm(xc.data_ptr(), ptr(w), y.data_ptr(), cols ? xc.numel() / cols : 0, (int)cols, (float)eps, dt,
                               stream());
     });
-    return {rc, y};
+    return {rc, y, "xlstm_rms_norm"};
 }
 py::tuple rms_norm(const Tensor &x, const OptTensor &weight, double eps) { return norm(x, weight, eps).tuple(); }
 
@@ -296,7 +298,6 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
     need(x.dim() == 2 && W.dim() == 2 && W.size(0) == 2 * NH * dqk + 2 * NH * dv + 2 * NH,
          "token_block takes x as [B, D] and W as the merged q, k, v, i, f and o projections");
     const OptTensor none;
-    const char *what = rows ? "xlstm_linear_rows_ex" : "xlstm_linear_token";
     auto failed = [&](int rc, const char *call) { return py::make_tuple(rc, call, x, none, none, none); };
     // settled: the launch before the Linear is one of this block's, none of which writes weights
     auto project = [&](const Tensor &w, const Tensor &in, const OptTensor &bias, const OptTensor &nw, double ne, const OptTensor &res,
@@ -309,7 +310,7 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
         return linear(w, n.y, bias, none, 0.0, res, pair, 16, true);
     };
     const Result y = project(W, x, b, norm_w, norm_eps, none, false, false);
-    if (y.rc) return failed(y.rc, what);
+    if (y.rc) return failed(y.rc, y.what);
     int64_t at = 0;
     auto columns = [&](int64_t n) {
         const Tensor t = y.y.narrow(1, at, n);
@@ -323,11 +324,11 @@ py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, cons
     const Stepped st = step_gated(q, k, v, i, f, o, head_norm_w, C0, n0, m0, eps, head_norm_eps, inplace, gate_cap, true);
     if (st.rc) return failed(st.rc, "xlstm_mlstm_step_gated_rows");
     const Result x1 = project(out_w, st.y, out_b, none, 0.0, x, false, true);
-    if (x1.rc) return failed(x1.rc, what);
+    if (x1.rc) return failed(x1.rc, x1.what);
     const Result act = project(ffn, x1.y, none, ffn_norm_w, ffn_norm_eps, none, true, true);
-    if (act.rc) return failed(act.rc, what);
+    if (act.rc) return failed(act.rc, act.what);
     const Result x3 = project(down_w, act.y, down_b, none, 0.0, x1.y, false, true);
-    return py::make_tuple(x3.rc, what, x3.y, st.state.C, st.state.n, st.state.m);
+    return py::make_tuple(x3.rc, x3.what, x3.y, st.state.C, st.state.n, st.state.m);
 }
 
 // LayerNorm of each of `groups` column blocks of the rows of x; the status says if the kernel does not take the layout
