@@ -94,6 +94,10 @@ inline int launch_status() { return cudaGetLastError() == cudaSuccess ? XLSTM_OK
 // kernel has completed and its writes are visible.  allow_dependents() is issued right AFTER the wait, so the
 // pre-wait part of launch k+1 can only ever overlap launch k, never anything older.  Both instructions do
 // nothing in a kernel launched the ordinary way, or after a stream operation that is not such a kernel.
+// Two kernels are an exception: mlstm_f32_gate_matrix_kernel, and the second of the two tensor-core prefill launches where a
+// tail follows (TcParams::early), call allow_dependents() before they wait for the launch in front of them (one CTA waits at their
+// end, so they are complete only when that launch is).  What is launched behind them may overlap BOTH, and may read before its own
+// wait only what neither of them writes: mlstm_f32_output_kernel reads nothing before it, mlstm_tail_kernel q, k, v and gates.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
