@@ -288,8 +288,8 @@ py::tuple add_rms_norm(const Tensor &x, const Tensor &residual, const OptTensor 
 
 // One token of B sequences through an mLSTM block, launch after launch as mLSTMBlock._token_step describes them: W, b are the
 // merged input projections, ffn the gate and up projections.  rows: the Linears for up to 16 rows, else those for up to 4; the
-// norms are in them (more than 48 KB of rows, or rows or a norm weight off 16 bytes: launches of their own, which take both).  Through Python the seven launches of a block took 140 us of host
-// time, as much as the GPU has work for 16 sequences of 4096.
+// norms are in them (more than 48 KB of rows, or rows or a norm weight off 16 bytes: launches of their own, which take both).
+// Through Python the seven launches of a block took 140 us of host time, as much as the GPU has work for 16 sequences of 4096.
 py::tuple token_block(const Tensor &x, const Tensor &W, const OptTensor &b, const OptTensor &norm_w, double norm_eps, int64_t NH,
                       int64_t dqk, int64_t dv, const OptTensor &C0, const OptTensor &n0, const OptTensor &m0,
                       const OptTensor &head_norm_w, double eps, double head_norm_eps, bool inplace, double gate_cap,

@@ -21,6 +21,7 @@
 // 21888 x 4096 as a pair 33.3 (38.0; 27.3), 4096 x 10944 16.9 (22.9; 13.7).  LR_U = 2: 4 % more, 12 warps with LR_U = 4 or 8 with 8:
 // the same within 2 %.
 #include "cp_async.cuh"
+#include "mma_sync.cuh"
 #include "vec16.cuh"
 
 namespace xl {
@@ -47,12 +48,6 @@ __device__ __forceinline__ uint4 ldg_weights(const __nv_bfloat16 *p) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // EPI: 0 = bias only, 1 = + residual, 2 = SwiGLU pair (W has 2 N rows: gate rows, then up rows)
 template <int EPI, bool NORM, int LR_WARPS>
 __global__ void __launch_bounds__(LR_WARPS * 32, LR_WARPS == 16 ? 1 : 2)
@@ -182,8 +177,8 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ W, const __nv_bfloat16 *x, 
                 for (int t = 0; t < 2; ++t)
 #pragma unroll
                     for (int n = 0; n < 2; ++n) {
-                        mma_bf16(acc[t][n], wr[u][2 * t].x, wr[u][2 * t + 1].x, wr[u][2 * t].y, wr[u][2 * t + 1].y, xr[u][n].x, xr[u][n].y);
-                        mma_bf16(acc[t][n], wr[u][2 * t].z, wr[u][2 * t + 1].z, wr[u][2 * t].w, wr[u][2 * t + 1].w, xr[u][n].z, xr[u][n].w);
+                        mma_m16n8k16(acc[t][n], wr[u][2 * t].x, wr[u][2 * t + 1].x, wr[u][2 * t].y, wr[u][2 * t + 1].y, xr[u][n].x, xr[u][n].y);
+                        mma_m16n8k16(acc[t][n], wr[u][2 * t].z, wr[u][2 * t + 1].z, wr[u][2 * t].w, wr[u][2 * t + 1].w, xr[u][n].z, xr[u][n].w);
                     }
                 if (more) { load_w(u, b0 + u * LR_WARPS); load_x(u, b0 + u * LR_WARPS); }
             }

@@ -24,6 +24,7 @@
 // samples).  It costs 1 us of 7 to 25; multiply-adds on the CUDA cores, as exact, cost nothing for one token and 5 us for 127.
 #include "cp_async.cuh"
 #include "mlstm_gate_tile.cuh"
+#include "mma_sync.cuh"
 #include "packed_f32.cuh"
 
 namespace xl {
@@ -35,22 +36,6 @@ constexpr int TG = 32;              // tokens per read-out pass
 constexpr int V_LD = 40;            // bf16 elements between rows of V: 80 bytes, eight rows on different banks
 constexpr int PART_LD = 36;         // floats between tokens of a partial read-out
 
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void mma_k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
-}
 // Two floats as three packed pairs of bf16 whose sums are the floats: 8 significant bits each, cut off (a rounded leading
 // part could overflow).  An infinity is its leading part alone.
 __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
@@ -200,16 +185,16 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                 uint32_t kf[NS][4];                                           // keys of n-tile n: registers 0, 1 and 2, 3
 #pragma unroll
                 for (int n = 0; n < NS; ++n)
-                    ldsm4(base + SM::K + ((s0 + n * 8 + (lane & 7)) * SM::QK_LD + kk * 32 + (lane >> 3) * 8) * 2, kf[n]);
+                    ldmatrix4(base + SM::K + ((s0 + n * 8 + (lane & 7)) * SM::QK_LD + kk * 32 + (lane >> 3) * 8) * 2, kf[n]);
 #pragma unroll
                 for (int tb = 0; tb < TB; ++tb)
                     if (tb < nb && tb * 16 + 15 >= s0) {
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             uint32_t a[4];
-                            ldsm4(a_row + (tb * 16 * SM::QK_LD + kk * 32 + h * 16) * 2, a);
+                            ldmatrix4(a_row + (tb * 16 * SM::QK_LD + kk * 32 + h * 16) * 2, a);
 #pragma unroll
-                            for (int n = 0; n < NS; ++n) mma_k16(P[tb][n], a, kf[n][2 * h], kf[n][2 * h + 1]);
+                            for (int n = 0; n < NS; ++n) mma_m16n8k16(P[tb][n], a, kf[n][2 * h], kf[n][2 * h + 1]);
                         }
                     }
             }
@@ -316,14 +301,14 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                     for (int np = 0; np < TG / 16; ++np) {
                         if (th * 2 + np >= nb) continue;
                         uint32_t q[4];                                        // tokens of n-tiles 2 np (registers 0, 1), 2 np + 1
-                        ldsm4(base + SM::Q + ((th * TG + np * 16 + (lane & 7) + ((lane >> 4) << 3)) * SM::QK_LD + j0 + ks * 16 +
+                        ldmatrix4(base + SM::Q + ((th * TG + np * 16 + (lane & 7) + ((lane >> 4) << 3)) * SM::QK_LD + j0 + ks * 16 +
                                               ((lane >> 3) & 1) * 8) * 2, q);
 #pragma unroll
                         for (int x = 2; x >= 0; --x)
 #pragma unroll
                             for (int mt = 0; mt < 2; ++mt) {
-                                mma_k16(acc[mt][2 * np], Cp[x][mt][ks], q[0], q[1]);
-                                mma_k16(acc[mt][2 * np + 1], Cp[x][mt][ks], q[2], q[3]);
+                                mma_m16n8k16(acc[mt][2 * np], Cp[x][mt][ks], q[0], q[1]);
+                                mma_m16n8k16(acc[mt][2 * np + 1], Cp[x][mt][ks], q[2], q[3]);
                             }
                     }
 #pragma unroll
@@ -339,11 +324,11 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
             if (s0 < nb * 16 && th * TG + TG > s0) {
                 uint32_t vf[2][4];                                            // V^T of this warp's keys
                 if (NS == 1) {
-                    ldsm4_trans(base + SM::V + ((s0 + (lane & 7)) * V_LD + (lane >> 3) * 8) * 2, vf[0]);
+                    ldmatrix4_trans(base + SM::V + ((s0 + (lane & 7)) * V_LD + (lane >> 3) * 8) * 2, vf[0]);
                 } else {
 #pragma unroll
                     for (int mt = 0; mt < 2; ++mt)
-                        ldsm4_trans(base + SM::V + ((s0 + (lane & 7) + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, vf[mt]);
+                        ldmatrix4_trans(base + SM::V + ((s0 + (lane & 7) + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, vf[mt]);
                 }
 #pragma unroll
                 for (int nt = 0; nt < TG / 8; ++nt) {
@@ -356,8 +341,8 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                     for (int x = 2; x >= 0; --x)
 #pragma unroll
                         for (int mt = 0; mt < 2; ++mt) {
-                            if (NS == 1) mma_k8(acc[mt][nt], vf[0][2 * mt], vf[0][2 * mt + 1], w[0][x]);
-                            else mma_k16(acc[mt][nt], vf[mt], w[0][x], w[NS - 1][x]);
+                            if (NS == 1) mma_m16n8k8(acc[mt][nt], vf[0][2 * mt], vf[0][2 * mt + 1], w[0][x]);
+                            else mma_m16n8k16(acc[mt][nt], vf[mt], w[0][x], w[NS - 1][x]);
                         }
                 }
             }
@@ -446,10 +431,10 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                 const int trow = ks * 16 + (lane & 7);
 #pragma unroll
                 for (int x = 0; x < 3; ++x)
-                    ldsm4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wp[x]);
+                    ldmatrix4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wp[x]);
 #pragma unroll
                 for (int np = 0; np < NTJ / 2; ++np)
-                    ldsm4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
+                    ldmatrix4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
 #pragma unroll
                 for (int np = 0; np < NTJ / 2; ++np)
 #pragma unroll
@@ -459,10 +444,10 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
                         uint32_t l0, l1, r0, r1;
                         k_on_grid(k0, kgrid, l0, r0);
                         k_on_grid(k1, kgrid, l1, r1);
-                        mma_k16(sum[1][nj], wp[2], k0, k1);
-                        mma_k16(sum[0][nj], wp[0], l0, l1);
-                        mma_k16(sum[1][nj], wp[1], k0, k1);
-                        mma_k16(sum[1][nj], wp[0], r0, r1);
+                        mma_m16n8k16(sum[1][nj], wp[2], k0, k1);
+                        mma_m16n8k16(sum[0][nj], wp[0], l0, l1);
+                        mma_m16n8k16(sum[1][nj], wp[1], k0, k1);
+                        mma_m16n8k16(sum[1][nj], wp[0], r0, r1);
                     }
             }
 #pragma unroll

@@ -863,12 +863,13 @@ constexpr int MIN_SEG_TILES = 2, LONG_SEG_TILES = 16;
 
 // Number of segments every sequence is cut into.  Cutting buys parallelism while the grid of persistent CTAs (one per head
 // and 128 dv columns) leaves SMs idle, at the price of the state-only first pass, of the states going through HBM and of
-// three more launches.  Microseconds at 256/512, bounded gates, forced segment counts, 2 to 64 tiles a segment:
-//   up to 32 CTAs in one pass   one 13 + tiles x 4.55, two 35 + tiles of a segment x (5.2 + 0.03 a CTA of all segments)
-//   more of them                one 20 + tiles x (3.05 + 0.014 a CTA), two 43 + tiles of a segment x (5.6 + 0.0117 a CTA)
-// The first line is above what bounded gates take now (one pass 10 + 3.9, 8 heads, S = 2048: 72 us) and asks for the cuts that suit
-// both kinds of gates: the lines that fit these best would cut 4 heads of 2048 tokens in 4 instead of 8 (54 and 56 us, but general
-// 85 and 71), while 6 heads in one pass instead of 6 segments take 71 and 62 us (general 104 and 86).
+// three more launches.  The two lines below are compared, they are not predictions for one kind of gates:
+//   more than 32 CTAs in one pass: fitted to bounded gates at 256/512 with forced segment counts, 2 to 64 tiles a segment.
+//   up to 32 CTAs: between the two kinds.  One pass takes 10 + 3.9 us a tile with bounded gates and 15 + 5.6 on the general path;
+//   which it will be is decided on the device, so the line for one pass, 13 + 4.55, and that for two were kept at values whose
+//   cuts are near the best of both: 4 heads of 2048 tokens in 8 segments take 56 us bounded and 71 general (in 4, which the bounded
+//   line alone would choose, 54 and 85), 6 heads in 6 segments 62 and 86 (in one pass 71 and 104).  A refit takes, over forced
+//   segment counts of both kinds, the lines whose choices lose least against the sum of the two best times.
 // With segments of less than LONG_SEG_TILES a quarter has to be gained.  That is a choice for steady results and not for speed:
 // cutting moves the bf16 copy of C to other frames, and after the 16 blocks of a model the last states differ by 3e-2 from those
 // of one pass (the distance of any two correct bf16 evaluations there), which smaller gains were not given.

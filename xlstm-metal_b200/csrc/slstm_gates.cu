@@ -11,6 +11,7 @@
 // heads: one product with (i, f) of xc, one with o of x.
 // Bound by issue (about 35 instructions per 4 elements, the window and the SiLU) and by the latency of 2 J + 3 loads a block;
 // HBM would allow 10 us at the size above, it takes 36.  J = 1 gives the SMs more CTAs where there are few tokens.
+#include "mma_sync.cuh"
 #include "vec16.cuh"
 
 namespace xl {
@@ -25,11 +26,6 @@ struct GateArgs {
     float cap;
 };
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 // SiLU rounded to bf16: the sigmoid from one tanh.approx, as the convolution kernel takes it
 __device__ __forceinline__ float silu_bf16(float x) {
     float t;
@@ -106,10 +102,10 @@ template <int J> __global__ void __launch_bounds__(SG_WARPS * 32, 1) slstm_gates
             }
             // rows g and g + 8 of the tile: tokens tf + 2 j and tf + 2 j + 1
             const uint4 x0 = raw[2 * j + 3], x1 = raw[2 * j + 4];
-            mma_bf16(aif[j], xc[0].x, xc[1].x, xc[0].y, xc[1].y, bif.x, bif.y);
-            mma_bf16(aif[j], xc[0].z, xc[1].z, xc[0].w, xc[1].w, bif.z, bif.w);
-            mma_bf16(ao[j], x0.x, x1.x, x0.y, x1.y, bo.x, bo.y);
-            mma_bf16(ao[j], x0.z, x1.z, x0.w, x1.w, bo.z, bo.w);
+            mma_m16n8k16(aif[j], xc[0].x, xc[1].x, xc[0].y, xc[1].y, bif.x, bif.y);
+            mma_m16n8k16(aif[j], xc[0].z, xc[1].z, xc[0].w, xc[1].w, bif.z, bif.w);
+            mma_m16n8k16(ao[j], x0.x, x1.x, x0.y, x1.y, bo.x, bo.y);
+            mma_m16n8k16(ao[j], x0.z, x1.z, x0.w, x1.w, bo.z, bo.w);
         }
     }
     // the upper half of the warps hands its sums to the lower half, whose parts are added in order below

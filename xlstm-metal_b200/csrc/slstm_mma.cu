@@ -27,6 +27,7 @@
 //
 // Buffer reuse without further synchronisation: h_t goes to buffer (t + 1) & 1, which held h_{t-2}.  A block of h_t is
 // sent only after all blocks of h_{t-1} have arrived, and a warp sends its block of h_{t-1} after it has read h_{t-2}.
+#include "mma_sync.cuh"
 #include "slstm_cluster.cuh"
 
 namespace xl {
@@ -49,24 +50,11 @@ __device__ __forceinline__ float tanh_sfu(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldmatrix4_trans(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
-}
 // 8x8 matrix of bf16 in fragment layout (lane (g, c) holds row g, columns 2c and 2c + 1) -> its transpose
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t a) {
     uint32_t d;
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
     return d;
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
@@ -215,7 +203,7 @@ slstm_recurrent_mma_kernel(const __nv_bfloat16 *__restrict__ gx, const __nv_bflo
                     const int kk = NT == 1 ? 2 * ld + half : ld, n = NT == 1 ? 0 : half;
 #pragma unroll
                     for (int m = 0; m < 2; ++m)
-                        mma16816(acc[s][kk % KX][m][n], Rr[m][kk], b[s][NT == 1 ? 2 * half : half], b[s][NT == 1 ? 2 * half + 1 : half + 2]);
+                        mma_m16n8k16(acc[s][kk % KX][m][n], Rr[m][kk], b[s][NT == 1 ? 2 * half : half], b[s][NT == 1 ? 2 * half + 1 : half + 2]);
                 }
         }
 #pragma unroll

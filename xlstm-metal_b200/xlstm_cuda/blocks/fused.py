@@ -10,10 +10,14 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
+from torch._C._functorch import peek_interpreter_stack
 from torch.autograd import forward_ad as _forward_ad
 from torch.nn.modules import module as _module
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
+
+
+_PLAIN = frozenset((nn.Parameter, torch.Tensor, type(None)))
 
 
 def _no_mode() -> bool:
@@ -27,11 +31,12 @@ def plain_tensor(x: torch.Tensor, *weights: Optional[torch.Tensor]) -> bool:
     function transform (vmap, grad, jvp; an ensemble's stacked weights are wrapped where ``x`` is not) or a forward-mode level,
     not being traced or compiled, no mode listens to the operators (make_fx, a counter), and not under autocast (which would pick
     another type for the module)."""
-    return (_no_mode() and type(x) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(x) and
-            all(w is None or (type(w) in (nn.Parameter, torch.Tensor) and not torch._C._functorch.is_functorch_wrapped_tensor(w))
-                for w in weights) and
-            _forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and
-            not torch.is_autocast_enabled(x.device.type))
+    if type(x) is not torch.Tensor or peek_interpreter_stack() is not None or _forward_ad._current_level >= 0 or not _no_mode():
+        return False   # (the interpreter stack: every function transform that is running, whatever it has wrapped)
+    for w in weights:
+        if type(w) not in _PLAIN:
+            return False
+    return not (torch.jit.is_tracing() or torch.compiler.is_compiling() or torch.is_autocast_enabled(x.device.type))
 
 
 def may_fuse(owner: nn.Module, x: torch.Tensor, *replaced: Tuple[nn.Module, type]) -> bool:

@@ -351,14 +351,15 @@ class mLSTMBlock(nn.Module):
         self.state_dtype = state_dtype
 
     def _token_step(self, x: torch.Tensor, state: Optional[State]):
-        """Single-token path (bf16, fused weights).  Up to 16 sequences every Linear is one weight-streaming kernel with its
-        norm (for more than a few sequences a launch of its own) / bias / residual / SwiGLU folded in, so a block is five or seven
-        launches in one native call: projections, cell step with the output epilogue, out-projection, FFN up, FFN down.  Up to 2 they multiply on the CUDA cores (small CTAs that flow into the
-        gaps of the launch before: a token of one sequence through 16 blocks of 4096 takes 1.48 ms, 1.60 with the others), from 3 on,
-        where that kernel is bound by its multiply-adds, on the tensor cores.  Where the norms are more than their kernel to
-        somebody (hooks, gradients) the launches are separate calls.  Beyond 16, and from 5 on with weights that the tensor-core
-        kernel does not take, the Linears are GEMMs; the line at 16 is drawn for calls without a graph (16 sequences
-        through 8 blocks of 4096: 1.54 ms with GEMMs, 1.31 streamed when it was drawn).
+        """Single-token path (bf16, fused weights).  Up to 16 sequences every Linear is one weight-streaming kernel with its norm
+        (for more than 48 KB of rows, or rows and norm weights off a 16-byte boundary, a launch of its own), bias, residual and SwiGLU
+        folded in, so a block is five or seven launches in one native call: projections, cell step with the output epilogue,
+        out-projection, FFN up, FFN down.  Up to 2 they multiply on the CUDA cores (small CTAs that flow into the gaps of the launch
+        before: a token of one sequence through 16 blocks of 4096 takes 1.41 ms, 1.60 with the others), from 3 on, where that kernel is
+        bound by its multiply-adds, on the tensor cores.  Where the norms are more than their kernel to somebody (hooks, gradients)
+        the launches are separate calls.  Beyond 16, and from 5 on with weights that the tensor-core kernel does not take, the
+        Linears are GEMMs; the line at 16 is drawn for calls without a graph (16 sequences through 8 blocks of 4096: 1.54 ms with
+        GEMMs, 1.31 streamed when it was drawn, 1.05 now).
         More than 4 sequences come here only where may_fuse() allows it.  The cell step reads q, k, v and the gates where
         the merged projection has written them."""
         cell = self.mlstm_cell

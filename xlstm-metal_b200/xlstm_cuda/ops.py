@@ -443,8 +443,8 @@ LINEAR_ROWS_MAX = 16
 def linear_rows(weight: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 residual: Optional[torch.Tensor] = None, swiglu_pair: bool = False, weights_settled: bool = False,
                 norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 1e-6) -> torch.Tensor:
-    """The same for up to 16 token rows (bf16, ``K`` a multiple of 32); with a norm, rows of up to 46 KB in all and no
-    ``residual``.  ``weights_settled`` promises that the launch right before this one on the stream does not write ``weight``:
+    """The same for up to 16 token rows (bf16, ``K`` a multiple of 32); with a norm, rows of up to 48 KB in all (with the norm
+    weight and 64 bytes a row) and no ``residual``.  ``weights_settled`` promises that the launch right before this one on the stream does not write ``weight``:
     its first blocks are then loaded while that launch drains."""
     rc, y = _lib.host().linear_token(weight, x, bias, norm_weight, norm_eps, residual, swiglu_pair, LINEAR_ROWS_MAX, weights_settled)
     if rc:
