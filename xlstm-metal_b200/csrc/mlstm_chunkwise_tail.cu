@@ -5,7 +5,8 @@
 // bf16 parts whose sum is the float, so mma.sync forms exact products and adds them in fp32:
 //   S = Q K^T                                         1 product
 //   H^T = (C^T Q^T) diag(w_in) + V^T P^T              3 products each (parts of C, of P)
-//   C^T = decay C^T + (w V)^T K                       4 products (parts of w V; K in two for the leading one, see below)
+//   C^T = decay C^T + (w V)^T K                       4 products (parts of w V; K in two for the leading one, see below);
+//                                                     few tokens: fp32 multiply-adds
 // One CTA per (head, 32 columns of dv), for all tokens at once or for 64 in turn, C, n and m staying with it.  Its 8 warps share
 // the dqk dimension: a warp keeps its rows of C in registers, as accumulators of the update and, in the same places, as A
 // fragments of the read-out; it takes its share of the keys s for S, P and P V.  The read-outs of the 8 warps meet in shared
@@ -21,7 +22,11 @@
 // two each, for the whole sum: their products and all partial sums of up to 128 of them fit 22 bits, nothing is cut off, and the
 // other three products are 2^-6 of it.  The two sums and the state meet with one rounding.  C of 1 to 127 tokens is 1.5e-8 to 5.7e-8
 // from float64 where fp32 multiply-adds are 1.6e-8 to 9.4e-8 (2-norms; never more than 2 % further, which is the spread of the
-// samples).  It costs 1 us of 7 to 25; multiply-adds on the CUDA cores, as exact, cost nothing for one token and 5 us for 127.
+// samples).  That is 1 to 2.5 us of 7 to 25 more than plain parts.
+//
+// Up to FEW_TOKENS the update is fp32 multiply-adds on the CUDA cores instead, as exact and without the splits: us at 256/512, that /
+// tensor cores, 1 head, 1 / 17 / 24 / 32 tokens 6.8 8.1 / 8.7 9.4 / 9.1 9.4 / 9.7 9.6; 16 heads 8.3 10.4 / 11.3 12.1 / 12.3 12.2 /
+// 13.4 12.5; 64 heads 28.5 35.8 / 38.7 42.2 / 42.0 42.6 / 45.8 43.2.
 #include "cp_async.cuh"
 #include "mlstm_gate_tile.cuh"
 #include "mma_sync.cuh"
@@ -33,6 +38,7 @@ namespace {
 constexpr int TW = 8;               // warps
 constexpr int TC_COLS = 32;         // columns of dv per CTA
 constexpr int TG = 32;              // tokens per read-out pass
+constexpr int FEW_TOKENS = 24;      // up to so many the update of C is fp32 multiply-adds
 constexpr int V_LD = 40;            // bf16 elements between rows of V: 80 bytes, eight rows on different banks
 constexpr int PART_LD = 36;         // floats between tokens of a partial read-out
 
@@ -90,7 +96,7 @@ template <int DQK, int TMAX> struct TailSmem {
     static constexpr uint32_t K = Q + TMAX * QK_LD * 2;
     static constexpr uint32_t V = K + TMAX * QK_LD * 2;
     static constexpr uint32_t PART = V + TMAX * V_LD * 2;                     // float [TW][TG][PART_LD]
-    static constexpr uint32_t WV = PART;                                      // bf16 [3][TMAX][V_LD], after the last read-out
+    static constexpr uint32_t WV = PART;                                      // bf16 [3][TMAX][V_LD], few: float [T][TC_COLS]; after the read-outs
     static constexpr uint32_t PART_BYTES = TW * TG * PART_LD * 4;
     static constexpr uint32_t U = PART + PART_BYTES;                          // double [3][TMAX]: u, b, running maximum of u / x
     static constexpr uint32_t F = U + 3 * TMAX * 8;                           // float [4][TMAX]: w_in, e^{-m_t}, w, q.n
@@ -101,7 +107,7 @@ template <int DQK, int TMAX> struct TailSmem {
     static_assert(3 * TMAX * V_LD * 2 <= PART_BYTES, "weighted V fits the buffer it replaces");
 };
 
-template <int DQK, int TMAX>
+template <int DQK, int TMAX, bool FEW>
 __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel(const ChunkwiseParams p, int inputs_settled) {
     using SM = TailSmem<DQK, TMAX>;
     constexpr int JW = DQK / TW, KSJ = JW / 16, NTJ = JW / 8;                 // rows of C per warp; k-steps; n-tiles
@@ -126,7 +132,7 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
     if (!inputs_settled) grid_dependency_wait();
     for (int t0 = 0;; t0 += TMAX) {
         const int T = min(p.S - t0, TMAX), nb = (T + 15) >> 4;                // tokens; blocks of 16 (the rest is zeros)
-        const bool last = TMAX == 128 || t0 + TMAX >= p.S;
+        const bool last = FEW || TMAX == 128 || t0 + TMAX >= p.S;
         // ---- loads
         const bf16 *qb = static_cast<const bf16 *>(p.q) + b * p.sq[0] + hd * p.sq[1] + t0 * p.sq[2];
         const bf16 *kb = static_cast<const bf16 *>(p.k) + b * p.sk[0] + hd * p.sk[1] + t0 * p.sk[2];
@@ -157,7 +163,7 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
         }
         cp_async_wait_all();
         __syncthreads();
-        {
+        if constexpr (!FEW) {
             uint32_t k2 = 0u;
 #pragma unroll 2
             for (int e = tid; e < nb * 16 * (DQK / 8); e += TW * 32) {
@@ -373,98 +379,137 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
         __syncthreads();
 
         // ---- C^T = decay C^T + (w V)^T K
-        bf16 *sWV = reinterpret_cast<bf16 *>(smem + SM::WV);
-        static_assert(TW * 32 == 16 * (TC_COLS / 2), "a thread has two columns, of the tokens tid / 16 + 16 i");
-        const int vx = (tid % (TC_COLS / 2)) * 2, vt = tid / (TC_COLS / 2);
-        auto weighted = [&](int t) {
-            const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + SM::V + (t * V_LD + vx) * 2);
-            const float w = sW[t];
-            return make_float2(w * __uint_as_float(v << 16), w * __uint_as_float(v & 0xffff0000u));
-        };
-        uint32_t ex = 0u, ey = 0u, kmax = 0u;
+        const u64 decay2 = pack2(decay, decay);
+        if constexpr (FEW) {   // token after token on the CUDA cores: a pair is two rows of a column
+            float *sWV = reinterpret_cast<float *>(smem + SM::WV);            // [T][TC_COLS]
+            for (int e = tid; e < T * TC_COLS; e += TW * 32)
+                sWV[e] = sW[e / TC_COLS] * __bfloat162float(*reinterpret_cast<const bf16 *>(smem + SM::V + (e / TC_COLS * V_LD + e % TC_COLS) * 2));
+            __syncthreads();
+            u64 acc[4][NTJ];                                                  // column 8 x + g, rows 8 nj + 2c and + 1
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int nj = 0; nj < NTJ; ++nj)
+                    acc[x][nj] = fmul2(pack2(Ct[x >> 1][nj][2 * (x & 1)], Ct[x >> 1][nj][2 * (x & 1) + 1]), decay2);
+            const unsigned char *krow = smem + SM::K + (j0 + 2 * c) * 2;
+#pragma unroll 4
+            for (int t = 0; t < T; ++t) {
+                u64 kk[NTJ];
+#pragma unroll
+                for (int nj = 0; nj < NTJ; ++nj) {
+                    const uint32_t k2 = *reinterpret_cast<const uint32_t *>(krow + t * SM::QK_LD * 2 + nj * 16);
+                    kk[nj] = pack2(__uint_as_float(k2 << 16), __uint_as_float(k2 & 0xffff0000u));
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const float wv = sWV[t * TC_COLS + x * 8 + g];
+#pragma unroll
+                    for (int nj = 0; nj < NTJ; ++nj) acc[x][nj] = ffma2(kk[nj], pack2(wv, wv), acc[x][nj]);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int nj = 0; nj < NTJ; ++nj) {
+                    const float2 v = unpack2(acc[x][nj]);
+                    float *dst = p.C1 + c_off + (size_t)(nj * 8) * p.dv + x * 8;
+                    dst[0] = v.x;
+                    dst[p.dv] = v.y;
+                }
+        } else {
+            bf16 *sWV = reinterpret_cast<bf16 *>(smem + SM::WV);
+            static_assert(TW * 32 == 16 * (TC_COLS / 2), "a thread has two columns, of the tokens tid / 16 + 16 i");
+            const int vx = (tid % (TC_COLS / 2)) * 2, vt = tid / (TC_COLS / 2);
+            auto weighted = [&](int t) {
+                const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + SM::V + (t * V_LD + vx) * 2);
+                const float w = sW[t];
+                return make_float2(w * __uint_as_float(v << 16), w * __uint_as_float(v & 0xffff0000u));
+            };
+            uint32_t ex = 0u, ey = 0u, kmax = 0u;
 #pragma unroll 2
-        for (int i = 0; i < nb; ++i) {
-            const float2 wv = weighted(vt + 16 * i);
-            ex = max(ex, __float_as_uint(fabsf(wv.x)));
-            ey = max(ey, __float_as_uint(fabsf(wv.y)));
-        }
-        ex = max(ex, __shfl_xor_sync(0xffffffffu, ex, 16));
-        ey = max(ey, __shfl_xor_sync(0xffffffffu, ey, 16));
-        uint2 *sMax = reinterpret_cast<uint2 *>(sRs);                         // [TW][TC_COLS / 2], after the last row sums
-        if (lane < 16) sMax[warp * (TC_COLS / 2) + lane] = make_uint2(ex, ey);
-        __syncthreads();
+            for (int i = 0; i < nb; ++i) {
+                const float2 wv = weighted(vt + 16 * i);
+                ex = max(ex, __float_as_uint(fabsf(wv.x)));
+                ey = max(ey, __float_as_uint(fabsf(wv.y)));
+            }
+            ex = max(ex, __shfl_xor_sync(0xffffffffu, ex, 16));
+            ey = max(ey, __shfl_xor_sync(0xffffffffu, ey, 16));
+            uint2 *sMax = reinterpret_cast<uint2 *>(sRs);                         // [TW][TC_COLS / 2], after the last row sums
+            if (lane < 16) sMax[warp * (TC_COLS / 2) + lane] = make_uint2(ex, ey);
+            __syncthreads();
 #pragma unroll
-        for (int w = 0; w < TW; ++w) {
-            const uint2 o = sMax[w * (TC_COLS / 2) + (lane & 15)];
-            ex = max(ex, o.x);
-            ey = max(ey, o.y);
-            kmax = max(kmax, *reinterpret_cast<const uint32_t *>(smem + SM::KMAX + w * 4));
-        }
-        // an infinity keeps its products with all of the other factor: no grids then
-        const bool finite = __all_sync(0xffffffffu, max(ex, ey) < 0x7f800000u) && kmax < 0x7f80u;
-        const float gx = finite ? grid_of(ex) : 0.f, gy = finite ? grid_of(ey) : 0.f;
-        const uint32_t kg = finite ? k_grid_of(kmax) * 0x10001u : 0u;
-        const __nv_bfloat162 kgrid = *reinterpret_cast<const __nv_bfloat162 *>(&kg);
+            for (int w = 0; w < TW; ++w) {
+                const uint2 o = sMax[w * (TC_COLS / 2) + (lane & 15)];
+                ex = max(ex, o.x);
+                ey = max(ey, o.y);
+                kmax = max(kmax, *reinterpret_cast<const uint32_t *>(smem + SM::KMAX + w * 4));
+            }
+            // an infinity keeps its products with all of the other factor: no grids then
+            const bool finite = __all_sync(0xffffffffu, max(ex, ey) < 0x7f800000u) && kmax < 0x7f80u;
+            const float gx = finite ? grid_of(ex) : 0.f, gy = finite ? grid_of(ey) : 0.f;
+            const uint32_t kg = finite ? k_grid_of(kmax) * 0x10001u : 0u;
+            const __nv_bfloat162 kgrid = *reinterpret_cast<const __nv_bfloat162 *>(&kg);
 #pragma unroll 2
-        for (int i = 0; i < nb; ++i) {
-            const float2 wv = weighted(vt + 16 * i);
-            uint32_t pr[3];
-            split3_on_grid(wv.x, wv.y, gx, gy, pr);
+            for (int i = 0; i < nb; ++i) {
+                const float2 wv = weighted(vt + 16 * i);
+                uint32_t pr[3];
+                split3_on_grid(wv.x, wv.y, gx, gy, pr);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(sWV + (k * TMAX + vt + 16 * i) * V_LD + vx) = pr[k];
-        }
-        __syncthreads();
-        const u64 decay2 = pack2(decay, decay), minus_decay2 = pack2(-decay, -decay);
-        // The sum over the tokens has accumulators of its own, that of the leading parts (exact) and that of the rest
+                for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(sWV + (k * TMAX + vt + 16 * i) * V_LD + vx) = pr[k];
+            }
+            __syncthreads();
+            const u64 minus_decay2 = pack2(-decay, -decay);
+            // The sum over the tokens has accumulators of its own, that of the leading parts (exact) and that of the rest
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            float sum[2][NTJ][4];
+            for (int mt = 0; mt < 2; ++mt) {
+                float sum[2][NTJ][4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int nj = 0; nj < NTJ; ++nj)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sum[h][nj][e] = 0.f;
+#pragma unroll 1
+                for (int ks = 0; ks < nb; ++ks) {
+                    uint32_t wp[3][4], kf[NTJ / 2][4];
+                    const int trow = ks * 16 + (lane & 7);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                        ldmatrix4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wp[x]);
+#pragma unroll
+                    for (int np = 0; np < NTJ / 2; ++np)
+                        ldmatrix4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
+#pragma unroll
+                    for (int np = 0; np < NTJ / 2; ++np)
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            const int nj = 2 * np + half;
+                            const uint32_t k0 = kf[np][2 * half], k1 = kf[np][2 * half + 1];
+                            uint32_t l0, l1, r0, r1;
+                            k_on_grid(k0, kgrid, l0, r0);
+                            k_on_grid(k1, kgrid, l1, r1);
+                            mma_m16n8k16(sum[1][nj], wp[2], k0, k1);
+                            mma_m16n8k16(sum[0][nj], wp[0], l0, l1);
+                            mma_m16n8k16(sum[1][nj], wp[1], k0, k1);
+                            mma_m16n8k16(sum[1][nj], wp[0], r0, r1);
+                        }
+                }
 #pragma unroll
                 for (int nj = 0; nj < NTJ; ++nj)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) sum[h][nj][e] = 0.f;
-#pragma unroll 1
-            for (int ks = 0; ks < nb; ++ks) {
-                uint32_t wp[3][4], kf[NTJ / 2][4];
-                const int trow = ks * 16 + (lane & 7);
-#pragma unroll
-                for (int x = 0; x < 3; ++x)
-                    ldmatrix4_trans(base + SM::WV + ((x * TMAX + trow + ((lane >> 4) << 3)) * V_LD + mt * 16 + ((lane >> 3) & 1) * 8) * 2, wp[x]);
-#pragma unroll
-                for (int np = 0; np < NTJ / 2; ++np)
-                    ldmatrix4_trans(base + SM::K + ((trow + (((lane >> 3) & 1) << 3)) * SM::QK_LD + j0 + np * 16 + ((lane >> 4) << 3)) * 2, kf[np]);
-#pragma unroll
-                for (int np = 0; np < NTJ / 2; ++np)
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int nj = 2 * np + half;
-                        const uint32_t k0 = kf[np][2 * half], k1 = kf[np][2 * half + 1];
-                        uint32_t l0, l1, r0, r1;
-                        k_on_grid(k0, kgrid, l0, r0);
-                        k_on_grid(k1, kgrid, l1, r1);
-                        mma_m16n8k16(sum[1][nj], wp[2], k0, k1);
-                        mma_m16n8k16(sum[0][nj], wp[0], l0, l1);
-                        mma_m16n8k16(sum[1][nj], wp[1], k0, k1);
-                        mma_m16n8k16(sum[1][nj], wp[0], r0, r1);
+                    for (int h = 0; h < 2; ++h) {
+                        float *C = Ct[mt][nj] + 2 * h;
+                        const float *s0 = sum[0][nj] + 2 * h, *s1 = sum[1][nj] + 2 * h;
+                        const float2 v = scaled_sum(pack2(C[0], C[1]), decay2, minus_decay2, pack2(s0[0], s0[1]), pack2(s1[0], s1[1]));
+                        C[0] = v.x;
+                        C[1] = v.y;
+                        if (last) {
+                            float *dst = p.C1 + c_off + (size_t)(nj * 8) * p.dv + mt * 16 + h * 8;
+                            dst[0] = v.x;
+                            dst[p.dv] = v.y;
+                        }
                     }
             }
-#pragma unroll
-            for (int nj = 0; nj < NTJ; ++nj)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float *C = Ct[mt][nj] + 2 * h;
-                    const float *s0 = sum[0][nj] + 2 * h, *s1 = sum[1][nj] + 2 * h;
-                    const float2 v = scaled_sum(pack2(C[0], C[1]), decay2, minus_decay2, pack2(s0[0], s0[1]), pack2(s1[0], s1[1]));
-                    C[0] = v.x;
-                    C[1] = v.y;
-                    if (last) {
-                        float *dst = p.C1 + c_off + (size_t)(nj * 8) * p.dv + mt * 16 + h * 8;
-                        dst[0] = v.x;
-                        dst[p.dv] = v.y;
-                    }
-                }
         }
         static_assert(DQK <= TW * 32, "a thread per element of n");
         m = sB[TMAX - 1] + x_last;
@@ -484,8 +529,8 @@ __global__ void __launch_bounds__(TW * 32, TMAX == 64 ? 2 : 1) mlstm_tail_kernel
     }
 }
 
-template <int DQK, int TMAX> int tail_launch(const ChunkwiseParams &p, bool inputs_settled, cudaStream_t st) {
-    auto kern = mlstm_tail_kernel<DQK, TMAX>;
+template <int DQK, int TMAX, bool FEW = false> int tail_launch(const ChunkwiseParams &p, bool inputs_settled, cudaStream_t st) {
+    auto kern = mlstm_tail_kernel<DQK, TMAX, FEW>;
     constexpr int bytes = (int)TailSmem<DQK, TMAX>::TOTAL;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return XLSTM_ERR_CUDA;
     return launch_overlapped(kern, dim3(p.dv / TC_COLS, p.B * p.NH), dim3(TW * 32), bytes, st, p, inputs_settled ? 1 : 0);
@@ -505,6 +550,7 @@ int mlstm_chunkwise_tail(const ChunkwiseParams &p, bool inputs_settled, cudaStre
     // 64 tokens at a time fit an SM twice, 128 once: in turn while every CTA has an SM it takes longer, beyond that it is the faster (127
     // tokens, at once and 64 at a time: 8 heads of 256/512 24.8 / 28.5 us, 16 heads 48.0 / 40.0; 64 of 128/256 75.2 / 51.3)
     const bool in_turn = p.S <= 64 || (int64_t)(p.dv / TC_COLS) * p.B * p.NH > 148;
+    if (p.S <= FEW_TOKENS) return p.dqk == 256 ? tail_launch<256, 64, true>(p, inputs_settled, st) : tail_launch<128, 64, true>(p, inputs_settled, st);
     if (p.dqk == 256) return in_turn ? tail_launch<256, 64>(p, inputs_settled, st) : tail_launch<256, 128>(p, inputs_settled, st);
     return in_turn ? tail_launch<128, 64>(p, inputs_settled, st) : tail_launch<128, 128>(p, inputs_settled, st);
 }
