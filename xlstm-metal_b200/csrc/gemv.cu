@@ -1,7 +1,7 @@
 // Single-token projections: y[m] = epilogue(W . norm(x[m]) + bias) for M <= 4 rows of x, bf16 weights.
 // At one token per sequence a Linear layer is a weight-streaming pass (2 bytes of W per multiply-add), so
 // it is written as one: a warp per output row reads the row with 16-byte loads (512 contiguous bytes per
-// warp and trip, four trips in flight), x sits in shared memory, fp32 accumulation, one warp reduction
+// warp and trip, up to eight trips in flight), x sits in shared memory, fp32 accumulation, one warp reduction
 // per row.  What a separate kernel would do before or after is folded in:
 //   prologue  RMSNorm of x (every CTA recomputes the 1/rms of the few rows: 8 KB from L2),
 //   epilogue  + bias, + residual (the block's residual stream), or silu(gate) * up when W holds the two

@@ -15,7 +15,7 @@
 //
 // Latency-bound while a CTA has an SM to itself: a few microseconds of products behind a chain of loads, two barriers a 32 tokens
 // and the state's way through registers.  As fp32 multiply-adds on CUDA cores a tail of 64 tokens took 52 us (8 heads of 256/512)
-// in one launch, of 127 tokens 66 us in two; here 14 and 25 us.
+// in one launch, of 127 tokens 66 us in two; here 15 and 25 us.
 //
 // The tensor cores cut off what does not fit 24 bits of a sum, they do not round: with plain parts C was 5.5e-8 from float64 where
 // gates forget within a few tokens (fp32 multiply-adds 3.0e-8).  So the leading parts of w V and of K are multiples of one power of

@@ -1013,7 +1013,7 @@ int mlstm_chunkwise_tc(const ChunkwiseParams &p, void *workspace, size_t workspa
         t.L = 64;
         t.C0 = p.C1; t.n0 = tail_n; t.m0 = tail_m;
     }
-    // A tail of one whole chunk stays on the CUDA-core kernel (52 us at 8 heads against 14): that is a choice for steady results
+    // A tail of one whole chunk stays on the CUDA-core kernel (52 us at 8 heads against 15): that is a choice for steady results
     // and not for speed.  Prompts of whole chunks go through stacks of layers, and whichever way the last tokens' sums are
     // ordered, after 16 blocks the last states differ by 2.1e-2 .. 3.1e-2, the distance of any two correct bf16 evaluations.
     const bool fused_tail = tail && t.S != t.L && mlstm_chunkwise_tail_supported(t, XLSTM_BF16);
